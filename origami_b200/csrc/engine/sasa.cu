@@ -20,6 +20,8 @@
 //    test gives the same answer, and the transitions it adds to other
 //    circles lie strictly inside the larger cap, where they only split
 //    buried segments.  The exposed arcs and vertices are unchanged.
+//  * A circle that the other caps bury all around is dropped before its
+//    transitions are built (cover_pair): it has no exposed segment.
 //  * Transitions on a circle are ordered by a pseudo-angle (monotone in the
 //    reference's atan2 angle, one division instead of an atan2), and the
 //    exposure test point of the segment from a to b -- a rotated by half the
@@ -66,8 +68,8 @@ constexpr double kPi = 3.14159265358979323846;
 // 4 transitions, 5 rank sort, 6 walk over the sorted order (ties,
 // duplicates, burial bookkeeping, toggle scan; de-duplication), 7 exposure and arcs, 8 vertex
 // signs and links, 9 term records; sums of 10 caps, 11 live circles,
-// 12 transitions, 13 atoms.
-constexpr int kPhases = 14;
+// 12 transitions, 13 atoms, 14 circles left after the buried ones.
+constexpr int kPhases = 15;
 #ifdef OG_SASA_PHASE_CLOCKS
 __device__ unsigned long long g_sasa_phase[kPhases];
 __device__ __forceinline__ long long cycles() {
@@ -123,6 +125,7 @@ __device__ __forceinline__ bool contains_strict(Cap c, D3 p) { return dot(p, c.a
 // pass (each ordered pair) classify every pair bit for bit alike.
 struct PairClass {
   double sigma, denom;
+  double nn;  // c_sq denom
   int count;  // transitions: 0, 1 (tangent) or 2
 };
 
@@ -130,12 +133,14 @@ __device__ __forceinline__ PairClass classify(Cap c1, Cap c2) {
   PairClass r;
   r.sigma = __fma_rn(c1.axis.x, c2.axis.x, __fma_rn(c1.axis.y, c2.axis.y, __dmul_rn(c1.axis.z, c2.axis.z)));
   r.denom = __fma_rn(-r.sigma, r.sigma, 1.0);
+  r.nn = 0.0;
   r.count = 0;
   if (fabs(r.denom) < 1e-12) return r;
   // every step is symmetric in the two caps, so (1, 2) and (2, 1) agree too
   const double t = __fma_rn(2.0 * r.sigma, __dmul_rn(c1.c, c2.c), r.denom);
   const double nn = __dsub_rn(t, __dadd_rn(__dmul_rn(c1.c, c1.c), __dmul_rn(c2.c, c2.c)));
   const double eps = 1e-9 * r.denom;
+  r.nn = nn;
   r.count = nn > eps ? 2 : (nn >= -eps ? 1 : 0);
   return r;
 }
@@ -250,6 +255,8 @@ struct WarpSmemT {
   double cx[kCaps], cy[kCaps], cz[kCaps], cc[kCaps];
   int32_t owner[kCaps];
   uint8_t live[kCaps];
+  // live circles that may have an exposed segment (indices into live)
+  uint8_t circ[kCaps];
   // per live circle either its transitions (low 16 bits) and kContained,
   // or -- up to kMaskCircles live circles, no tangent pair -- the mask of
   // the live circles it crosses (bit lm) and kMaskContained
@@ -328,6 +335,71 @@ __device__ __forceinline__ int32_t circle_tally(const W& w, int li, bool masks) 
   return 2 * __popcll(mk & ~kMaskContained) | ((mk & kMaskContained) ? kContained : 0);
 }
 
+// ------------------------------------------------------- buried circles
+// On the circle of cap k, a cap m that it crosses buries one interval.  The
+// circle's angle range is divided into 64 bins of the pseudo-angle; each
+// crossing pair sets, on both circles, the bins that lie wholly inside its
+// interval, and a circle whose 64 bins are all set is buried all around: it
+// has no exposed segment, so none of its transitions is built, sorted or
+// tested.  Protein atoms have 20 to 50 live circles and a handful of exposed
+// arcs, so most circles go this way (about 15 in 20 on the relaxed 300-residue
+// chain, which took 546 transitions per atom before).
+//
+// With sigma = a_k.a_m, the interval is centred on the direction of a_m
+// projected on the circle's plane, (wx, wy) in the circle's frame (fu, fv) of
+// slot_frame, and its half width has cosine : sine = (c_m - c_k sigma) :
+// sqrt(nn) (nn as in classify; the squares sum to (1 - c_k^2) denom), so the
+// end points follow without a division or an arc function.  All of it is
+// FP32, from FP64 differences rounded once: each end's pseudo-angle is within
+// 4e-6 of the exact one, and bins are taken kCoverMargin / 16 = 2.4e-4 inside
+// the interval.  A point there is inside cap m by more than
+// (1 - c_k^2)^(1/2) denom^(1/2) 2e-8, above the 1e-12 of the exposure tests
+// for the pairs used here.
+constexpr float kCoverMargin = 1.0f / 256.0f;  // of a bin
+
+__device__ __forceinline__ float cover_bin(float x, float y) {
+  const float d = fabsf(x) + fabsf(y);
+  const float r = __fdividef(x, d);
+  return 16.0f * ((y >= 0.0f ? 1.0f - r : r - 1.0f) + 2.0f);
+}
+
+// Bins [0, b) of 64.
+__device__ __forceinline__ uint64_t bins_below(int b) { return b >= 64 ? ~0ull : (b <= 0 ? 0ull : (1ull << b) - 1ull); }
+
+// The bins of circle k that cap m buries; root = sqrt(nn).
+__device__ __forceinline__ uint64_t covered_bins(Cap ck, Cap cm, double sigma, float root) {
+  const D3 a = ck.axis, b = cm.axis;
+  const double ax = fabs(a.x), ay = fabs(a.y), az = fabs(a.z);
+  // b.fu and b.fv of slot_frame(a): e - a (a.e) and a x e for helper axis e
+  double u, v;
+  if (ax < ay && ax < az) {
+    u = b.x - a.x * sigma;
+    v = b.y * a.z - b.z * a.y;
+  } else if (ay < az) {
+    u = b.y - a.y * sigma;
+    v = b.z * a.x - b.x * a.z;
+  } else {
+    u = b.z - a.z * sigma;
+    v = b.x * a.y - b.y * a.x;
+  }
+  const float wx = __double2float_rn(u), wy = __double2float_rn(v);
+  const float h = __double2float_rn(cm.c - ck.c * sigma);
+  if (!(h * h + root * root > 1e-6f)) return 0ull;
+  const float ts = cover_bin(h * wx + root * wy, h * wy - root * wx);
+  const float te = cover_bin(h * wx - root * wy, h * wy + root * wx);
+  const int bs = __float2int_ru(ts + kCoverMargin), be = __float2int_rd(te - kCoverMargin);
+  if (te > ts + kCoverMargin) return be > bs ? bins_below(be) & ~bins_below(bs) : 0ull;
+  if (ts > te + kCoverMargin) return ~bins_below(bs) | bins_below(be);
+  return 0ull;  // the ends coincide to rounding
+}
+
+__device__ __forceinline__ void cover_or(uint64_t* cover, int li, uint64_t m) {
+  unsigned* p = reinterpret_cast<unsigned*>(cover + li);
+  const unsigned lo = static_cast<unsigned>(m), hi = static_cast<unsigned>(m >> 32);
+  if (lo) atomicOr(p, lo);
+  if (hi) atomicOr(p + 1, hi);
+}
+
 // Sets bit b of circle li's crossing mask by a 32-bit atomic on the word
 // holding it (little-endian halves), which shared memory does natively.
 template <class W>
@@ -385,7 +457,7 @@ __device__ __noinline__ void reorder_tied(W& w, unsigned tied, int b0, int lane)
     tied &= tied - 1;
     const int sb = w.sbeg[j], se = w.sbeg[j + 1];
     D3 fu, fv;
-    slot_frame(cap_at(w, w.live[b0 + j]).axis, &fu, &fv);
+    slot_frame(cap_at(w, w.live[w.circ[b0 + j]]).axis, &fu, &fv);
     for (int sl = sb + lane; sl < se; sl += 32) {
       const double as = slot_angle(tpoint(w, sl), fu, fv);
       int rank = 0;
@@ -563,6 +635,12 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // quotient at least 0.5 / n_live from an integer, far above the rounding
   const float inv_live = 1.0f / static_cast<float>(n_live);
   bool masks = n_live <= kMaskCircles;
+  // buried bins per live circle, over the transition arrays (not in use yet)
+  static_assert(offsetof(W, ty) == offsetof(W, tx) + sizeof(w.tx) &&
+                    sizeof(w.tx) + sizeof(w.ty) >= W::kCaps * sizeof(uint64_t),
+                "cover scratch");
+  uint64_t* cover = reinterpret_cast<uint64_t*>(w.tx);
+  for (int li = lane; li < n_live; li += 32) cover[li] = 0;
   for (int pass = 0; pass < 2; ++pass) {
     if (masks) {
       for (int li = lane; li < n_live; li += 32) w.xmask[li] = 0;
@@ -590,6 +668,11 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       const int lm = li + 1 + p - li * (2 * n_live - 1 - li) / 2;
       const Cap ck = cap_at(w, w.live[li]), cm = cap_at(w, w.live[lm]);
       const PairClass pc = classify(ck, cm);
+      if (pc.count == 2) {
+        const float root = sqrtf(__double2float_rn(pc.nn));
+        cover_or(cover, li, covered_bins(ck, cm, pc.sigma, root));
+        cover_or(cover, lm, covered_bins(cm, ck, pc.sigma, root));
+      }
       // a circle inside the other cap without crossing its rim
       const bool in_m = !pc.count && ck.c * pc.sigma - cm.c > -1e-9;
       const bool in_k = !pc.count && cm.c * pc.sigma - ck.c > -1e-9;
@@ -614,22 +697,34 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     if (!masks || !__any_sync(kFull, tangent)) break;
     masks = false;
   }
+  // the circles left to process, in live order
+  int n_circ = 0;
+  for (int l0 = 0; l0 < n_live; l0 += 32) {
+    const int li = l0 + lane;
+    const bool open = li < n_live && cover[li] != ~0ull;
+    const unsigned m = __ballot_sync(kFull, open);
+    if (open) w.circ[n_circ + __popc(m & ((1u << lane) - 1u))] = static_cast<uint8_t>(li);
+    n_circ += __popc(m);
+  }
+  __syncwarp();
   ph.mark(2);
+  ph.count(14, n_circ);
 
   int n_arcs = 0, n_verts = 0;
   bool bad = false;
-  for (int b0 = 0; b0 < n_live && !bad;) {
-    // the batch: consecutive live circles whose (padded) lists fit.  Lane j
-    // takes circle b0 + j (kSasaBatch == 32): an inclusive warp prefix of
+  for (int b0 = 0; b0 < n_circ && !bad;) {
+    // the batch: consecutive circles of circ whose (padded) lists fit.  Lane j
+    // takes circle circ[b0 + j] (kSasaBatch == 32): an inclusive warp prefix of
     // the list sizes gives every circle's first slot, and the lanes whose
     // prefix fits the buffer form the batch (a leading run, since the prefix
     // grows with j).  (Lane 0 alone walking the circles took twice as long.)
     static_assert(kSasaBatch == 32, "one batch circle per lane");
     const int cj = b0 + lane;
-    const int tally = cj < n_live ? circle_tally(w, cj, masks) : 0;
+    const int lj = cj < n_circ ? w.circ[cj] : 0;
+    const int tally = cj < n_circ ? circle_tally(w, lj, masks) : 0;
     const int cnt_j = tally & kCountMask;
-    const int sz = cj < n_live ? max(cnt_j, 1) : 0;
-    const int zero_j = (cj < n_live && cnt_j == 0) ? 1 : 0;
+    const int sz = cj < n_circ ? max(cnt_j, 1) : 0;
+    const int zero_j = (cj < n_circ && cnt_j == 0) ? 1 : 0;
     int incl = sz, zincl = zero_j;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -639,7 +734,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         zincl += z;
       }
     }
-    const int nb = __popc(__ballot_sync(kFull, cj < n_live && incl <= W::kTrans));
+    const int nb = __popc(__ballot_sync(kFull, cj < n_circ && incl <= W::kTrans));
     if (nb == 0) {
       bad = true;  // one circle alone has more transitions than the buffer
       break;
@@ -648,7 +743,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     if (lane < nb) {
       w.sbeg[lane] = static_cast<uint16_t>(incl - sz);
       w.zpre[lane] = static_cast<uint8_t>(zincl - zero_j);
-      const double c = w.cc[w.live[cj]];
+      const double c = w.cc[w.live[lj]];
       const double sk = sqrt(fmax(1.0 - c * c, 0.0));
       w.bsk[lane] = sk;
       w.binv[lane] = sk > 0.0 ? 1.0 / sk : 0.0;
@@ -713,7 +808,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       // intersection between the pairs (k, m) and (m, k) of two batch
       // circles was measured slower: the lane holding both does two
       // circles' slot work while the others wait.)
-      const uint64_t mj = lane < nb ? (w.xmask[b0 + lane] & ~kMaskContained) : 0ull;
+      const uint64_t mj = lane < nb ? (w.xmask[lj] & ~kMaskContained) : 0ull;
       int incl = __popcll(mj);
       for (int d = 1; d < 32; d <<= 1) {
         const int v = __shfl_up_sync(kFull, incl, d);
@@ -734,7 +829,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
           const int clo = __popc(lo);
           const int lm = r < clo ? nth_set_bit(lo, r) : 32 + nth_set_bit(static_cast<unsigned>(mk >> 32), r - clo);
           const int m = w.live[lm];
-          const Cap ck = cap_at(w, w.live[b0 + j]), cm = cap_at(w, m);
+          const Cap ck = cap_at(w, w.live[w.circ[b0 + j]]), cm = cap_at(w, m);
           const PairClass pc = classify(ck, cm);
           if (pc.count != 2) mismatch = true;  // never expected: classify is symmetric
           D3 pt{}, qt{};
@@ -753,7 +848,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
           const int pidx = static_cast<int>(qentry & 0xFFFFu), base = static_cast<int>(qentry >> 16);
           const int j = __float2int_rz((static_cast<float>(pidx) + 0.5f) * inv_live);
           const int m = w.live[pidx - j * n_live];
-          const Cap ck = cap_at(w, w.live[b0 + j]), cm = cap_at(w, m);
+          const Cap ck = cap_at(w, w.live[w.circ[b0 + j]]), cm = cap_at(w, m);
           const PairClass pc = classify(ck, cm);
           D3 pt{}, qt{};
           double rate_sk = 0.0;
@@ -767,7 +862,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         if (p < np) {
           j = __float2int_rz((static_cast<float>(p) + 0.5f) * inv_live);
           const int lm = p - j * n_live;
-          const int k = w.live[b0 + j], m = w.live[lm];
+          const int k = w.live[w.circ[b0 + j]], m = w.live[lm];
           if (k != m) cnt = classify(cap_at(w, k), cap_at(w, m)).count;
         }
         // prefix of the counts (0, 1 or 2) from two ballots
@@ -801,12 +896,12 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       bad = true;
       break;
     }
-    if (run + w.zpre[nb - 1] + ((circle_tally(w, b1 - 1, masks) & kCountMask) == 0 ? 1 : 0) != w.sbeg[nb]) {
+    if (run + w.zpre[nb - 1] + ((circle_tally(w, w.circ[b1 - 1], masks) & kCountMask) == 0 ? 1 : 0) != w.sbeg[nb]) {
       bad = true;  // the two passes disagree: never expected, but never written past
       break;
     }
     for (int j = lane; j < nb; j += 32) {
-      if ((circle_tally(w, b0 + j, masks) & kCountMask) != 0) continue;
+      if ((circle_tally(w, w.circ[b0 + j], masks) & kCountMask) != 0) continue;
       const int sl = w.sbeg[j];
       w.tseg[sl] = static_cast<uint8_t>(j);
       w.tother[sl] = kNoOther;
@@ -906,7 +1001,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       // start the bookkeeping of the batch again
       __syncwarp();
       if (lane < nb) {
-        w.bmode[lane] = (circle_tally(w, b0 + lane, masks) & kContained) ? 1 : 0;
+        w.bmode[lane] = (circle_tally(w, lj, masks) & kContained) ? 1 : 0;
         w.bbase[lane] = 0;
       }
       reorder_tied(w, tied, b0, lane);
@@ -944,7 +1039,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         if (pos < kept) {
           j = jr;
           sa = w.torder[r];
-          k = w.live[b0 + j];
+          k = w.live[w.circ[b0 + j]];
           const int nxt = pos + 1 == kept ? 0 : pos + 1;
           if (w.tother[sa] == kNoOther) {
             // no transitions: exposed unless a probe on the circle is buried

@@ -22,7 +22,7 @@ namespace ogk {
 // exposed arcs).
 constexpr int kSasaMaxCaps = 112;
 constexpr int kSasaMaxTrans = 96;
-constexpr int kSasaMaxArcs = 36;
+constexpr int kSasaMaxArcs = 34;
 constexpr int kSasaBigCaps = 254;
 constexpr int kSasaBigTrans = 254;
 constexpr int kSasaBigArcs = 128;
