@@ -202,9 +202,9 @@ struct og_engine {
 
   // per padded atom
   DVec<double> x, y, z, vx, vy, vz, rx, ry, rz, mass, inv_mass, q, rmin, eps, rmin14, eps14, rho, rho_tilde, srho;
-  DVec<double> born_r, born_r64, integral64, e_lj, e_coul, e_gb, e_self;
+  DVec<double> born_r, born_r64;
   DVec<unsigned long long> fx, fy, fz, born_sum;
-  DVec<int32_t> atom_sys, local_idx, atom_valid, n_pairs;
+  DVec<int32_t> atom_sys, local_idx, atom_valid;
   // real atom (systems in order) -> padded index; AoS staging of og_state
   DVec<int32_t> real_map;
   int64_t n_real = 0;
@@ -218,28 +218,22 @@ struct og_engine {
   DVec<int32_t> jlist, mask_begin;
   DVec<ogk::TileMaskRef> mask_refs;
   DVec<uint32_t> mask_ex, mask_14;
-  DVec<int32_t> excl_row, excl_col;
-  DVec<int8_t> excl_kind;
   DVec<int4> near;
   // Host side of the exclusion tables, kept so that an append
   // (og_engine_append_atoms) adds only the new exclusions' bits: mask block
   // of each ordered tile pair, the blocks' words, per-tile block references
-  // (sorted by j tile) and their CSR, per-atom exclusion rows and their CSR,
-  // the unordered near-field block list.
+  // (sorted by j tile) and their CSR, the unordered near-field block list.
   std::map<std::pair<int, int>, int> mask_of;
   std::vector<uint32_t> h_mex, h_m14;
   std::vector<std::vector<ogk::TileMaskRef>> tile_refs;
   std::vector<int32_t> h_mask_begin;
   std::vector<ogk::TileMaskRef> h_mask_refs;
-  std::vector<std::vector<std::pair<int, int8_t>>> excl_rows;
-  std::vector<int32_t> h_excl_row, h_excl_col;
-  std::vector<int8_t> h_excl_kind;
   std::vector<int4> h_near;
   int n_terms = 0;  // dihedral Fourier terms on the device
-  // FP64 energy path: j ranges per i atom and their partial sums
+  // FP64 energy path: warps per i-tile and their partial sums
   int e_chunks = 1;
-  DVec<double> epart;
-  DVec<int32_t> epart_pairs;
+  DVec<double> epart, epair;
+  DVec<int32_t> epair_count;
   DVec<ogk::PairWork> work_f;   // far-field force: upper-triangle tile pairs
   DVec<int32_t> jlist_f;
   // cutoff mode: i-blocks of the two lists, their culled j lists and ends
@@ -255,7 +249,7 @@ struct og_engine {
   // device-side replica exchange (og_remd_run): temperature slots, counters
   bool remd_ready = false;
   uint32_t remd_round = 0;
-  DVec<int32_t> remd_slot, remd_begin, remd_count;
+  DVec<int32_t> remd_slot;
   DVec<double> remd_temps, remd_total, remd_vscale;
   DVec<long long> remd_attempts, remd_accepts;
   // bonded
@@ -581,7 +575,7 @@ struct og_engine {
       }
       {
         Timer t(this, "born_finalize");
-        ogk::launch_born_finalize(at, nullptr, born_r.p, true, nullptr, stream);
+        ogk::launch_born_finalize(at, nullptr, 0, born_r.p, true, nullptr, stream);
       }
     }
     {
@@ -971,8 +965,8 @@ void sasa_lists(const og_engine* e, int si, int k0, int k1, std::vector<int32_t>
 
 // ---- exclusion tables.  One 32-word block per ordered tile pair holding an
 // exclusion (bit c of word a: atoms a, c excluded; 1-4 pairs in the second
-// array), each tile's blocks referenced in j-tile order; per-atom exclusion
-// rows for the FP64 paths; the unordered block list of the near field.
+// array), each tile's blocks referenced in j-tile order; the unordered block
+// list of the near field.
 
 // The block of (ti, tj), made (and referenced) when missing; *t_min takes
 // the lowest tile whose reference list changed.
@@ -1002,13 +996,10 @@ void mask_diagonal(og_engine* e, int t0, int t1, int* t_min, std::set<int>* touc
 }
 
 // Exclusion k of system si (kind 1: excluded, else a scaled 1-4 pair).
-void mask_exclusion(og_engine* e, int si, size_t k, int* t_min, int* a_min, std::set<int>* touched) {
+void mask_exclusion(og_engine* e, int si, size_t k, int* t_min, std::set<int>* touched) {
   const SysHost& s = e->sys[si];
   const int i = s.atom_begin + s.topo.excl[2 * k], j = s.atom_begin + s.topo.excl[2 * k + 1];
   const int8_t kind = s.topo.excl_kind[k];
-  e->excl_rows[i].push_back({j, kind});
-  e->excl_rows[j].push_back({i, kind});
-  *a_min = std::min(*a_min, std::min(i, j));
   for (int dir = 0; dir < 2; ++dir) {
     const int a = dir ? j : i, c = dir ? i : j;
     const int b = mask_block(e, a / kTile, c / kTile, t_min);
@@ -1021,11 +1012,10 @@ void mask_exclusion(og_engine* e, int si, size_t k, int* t_min, int* a_min, std:
 
 // Device copies of the exclusion tables after blocks up to n_blocks_before
 // existed on the device: the touched old blocks, the new blocks, the tile
-// CSR from tile t_min on, the atom CSR from atom a_min on and the near-field
-// blocks past n_near_before.
-og_status upload_exclusions(og_engine* e, int n_blocks_before, int t_min, int a_min, int n_near_before,
+// CSR from tile t_min on and the near-field blocks past n_near_before.
+og_status upload_exclusions(og_engine* e, int n_blocks_before, int t_min, int n_near_before,
                             const std::set<int>& touched, cudaStream_t st) {
-  const int nt = e->n_tiles, np = e->n_padded;
+  const int nt = e->n_tiles;
   // tile CSR
   t_min = std::min(t_min, std::max(static_cast<int>(e->h_mask_begin.size()) - 1, 0));
   if (e->h_mask_begin.empty()) t_min = 0;
@@ -1049,25 +1039,6 @@ og_status upload_exclusions(og_engine* e, int n_blocks_before, int t_min, int a_
     }
   e->n_near = static_cast<int>(e->h_near.size());
   OG_CUDA(e->near.upload_tail(e->h_near, n_near_before, st));
-  // atom CSR (rows sorted by partner)
-  a_min = std::min(a_min, std::max(static_cast<int>(e->h_excl_row.size()) - 1, 0));
-  if (e->h_excl_row.empty()) a_min = 0;
-  e->h_excl_col.resize(e->h_excl_row.empty() ? 0 : e->h_excl_row[a_min]);
-  e->h_excl_kind.resize(e->h_excl_col.size());
-  e->h_excl_row.resize(a_min);
-  for (int i = a_min; i < np; ++i) {
-    auto& r = e->excl_rows[i];
-    std::sort(r.begin(), r.end());
-    e->h_excl_row.push_back(static_cast<int32_t>(e->h_excl_col.size()));
-    for (auto& pr : r) {
-      e->h_excl_col.push_back(pr.first);
-      e->h_excl_kind.push_back(pr.second);
-    }
-  }
-  e->h_excl_row.push_back(static_cast<int32_t>(e->h_excl_col.size()));
-  OG_CUDA(e->excl_row.upload_tail(e->h_excl_row, a_min, st));
-  OG_CUDA(e->excl_col.upload_tail(e->h_excl_col, e->h_excl_row[a_min], st));
-  OG_CUDA(e->excl_kind.upload_tail(e->h_excl_kind, e->h_excl_row[a_min], st));
   return OG_OK;
 }
 
@@ -1241,14 +1212,13 @@ og_status size_lgb_scratch(og_engine* e, cudaStream_t st) {
 
 // Partial-sum buffers of the FP64 energy path for the current layout.
 og_status size_energy_scratch(og_engine* e, cudaStream_t st) {
-  int max_n = 1;
-  for (const auto& s : e->sys) max_n = std::max(max_n, s.topo.n);
-  e->e_chunks = ogk::energy_chunks(e->n_padded, max_n, e->n_sm);
-  if (e->e_chunks > 1) {
-    const size_t m = static_cast<size_t>(e->e_chunks) * e->n_padded;
-    OG_CUDA(e->epart.grow(3 * m, st));
-    OG_CUDA(e->epart_pairs.grow(m, st));
-  }
+  int max_t = 1;
+  for (const auto& s : e->sys) max_t = std::max(max_t, s.n_tiles);
+  e->e_chunks = ogk::energy_chunks(e->n_tiles, max_t, e->n_sm);
+  const size_t m = static_cast<size_t>(e->e_chunks) * e->n_tiles;
+  OG_CUDA(e->epart.grow(m * kTile, st));
+  OG_CUDA(e->epair.grow(3 * m, st));
+  OG_CUDA(e->epair_count.grow(m, st));
   return OG_OK;
 }
 
@@ -1302,10 +1272,8 @@ og_status finalize_impl(og_engine* e) {
     e->n_real = static_cast<int64_t>(hmap.size());
     OG_CUDA(e->real_map.upload(hmap, st));
   }
-  for (auto* v : {&e->born_r, &e->born_r64, &e->integral64, &e->e_lj, &e->e_coul, &e->e_gb, &e->e_self})
-    OG_CUDA(v->alloc(np));
+  for (auto* v : {&e->born_r, &e->born_r64}) OG_CUDA(v->alloc(np));
   for (auto* v : {&e->fx, &e->fy, &e->fz, &e->born_sum}) OG_CUDA(v->alloc(np));
-  OG_CUDA(e->n_pairs.alloc(np));
   OG_CUDA(e->pq.alloc(4 * static_cast<size_t>(np)));
   OG_CUDA(e->origin.alloc(e->n_tiles));
 
@@ -1393,16 +1361,15 @@ og_status finalize_impl(og_engine* e) {
     if (ls != OG_OK) return ls;
   }
 
-  // ---- exclusion masks (per ordered tile pair) and the FP64 CSR
+  // ---- exclusion masks (per ordered tile pair)
   {
     e->tile_refs.assign(e->n_tiles, {});
-    e->excl_rows.assign(np, {});
-    int t_min = 0, a_min = 0;
+    int t_min = 0;
     std::set<int> touched;
     for (const auto& s : e->sys) mask_diagonal(e, s.tile_begin, s.tile_begin + s.n_tiles, &t_min, &touched);
     for (int si = 0; si < n_sys; ++si)
-      for (size_t k = 0; k < e->sys[si].topo.excl_kind.size(); ++k) mask_exclusion(e, si, k, &t_min, &a_min, &touched);
-    og_status xs = upload_exclusions(e, 0, 0, 0, 0, touched, st);
+      for (size_t k = 0; k < e->sys[si].topo.excl_kind.size(); ++k) mask_exclusion(e, si, k, &t_min, &touched);
+    og_status xs = upload_exclusions(e, 0, 0, 0, touched, st);
     if (xs != OG_OK) return xs;
   }
 
@@ -1415,7 +1382,7 @@ og_status finalize_impl(og_engine* e) {
     og_status ss = upload_segments(e, st);
     if (ss != OG_OK) return ss;
   }
-  OG_CUDA(e->seg_out.alloc(9 * static_cast<size_t>(n_sys)));  // energy terms: 5 per-atom + 4 bonded
+  OG_CUDA(e->seg_out.alloc(ogk::kEnergyTerms * static_cast<size_t>(n_sys)));
   OG_CUDA(append(e->cl_start, std::vector<int32_t>(1, 0), st));
   if (e->p.constrain_h_bonds)
     for (int si = 0; si < n_sys; ++si) {
@@ -1610,7 +1577,7 @@ og_status append_impl(og_engine* e, int si, const TopoCopy& grown, const double*
   if (!why.empty()) return og_fail(OG_E_BADARG, "og_engine_append_atoms: " + why);
   cudaStream_t st = e->stream;
   const int n_old = sh.topo.n, n_new = grown.n, n_add = n_new - n_old;
-  const int old_tiles = e->n_tiles, old_np = e->n_padded;
+  const int old_tiles = e->n_tiles;
   std::set<int> old_heavy;  // system-local heavy atoms with a SHAKE cluster on the device
   for (size_t k = 0; k < sh.topo.cons_d.size(); ++k) {
     const int a = sh.topo.cons[2 * k], b = sh.topo.cons[2 * k + 1];
@@ -1628,12 +1595,10 @@ og_status append_impl(og_engine* e, int si, const TopoCopy& grown, const double*
   // of the tiles from the first new atom's on and the new atoms' state
   for (auto* v : {&e->x, &e->y, &e->z, &e->vx, &e->vy, &e->vz, &e->rx, &e->ry, &e->rz, &e->mass, &e->inv_mass,
                   &e->q, &e->rmin, &e->eps, &e->rmin14, &e->eps14, &e->rho, &e->rho_tilde, &e->srho, &e->born_r,
-                  &e->born_r64, &e->integral64, &e->e_lj, &e->e_coul, &e->e_gb, &e->e_self, &e->sasa_r,
-                  &e->sasa_gamma, &e->sasa_area, &e->sasa_energy})
+                  &e->born_r64, &e->sasa_r, &e->sasa_gamma, &e->sasa_area, &e->sasa_energy})
     OG_CUDA(v->grow(np, st));
   for (auto* v : {&e->fx, &e->fy, &e->fz, &e->born_sum}) OG_CUDA(v->grow(np, st));
-  for (auto* v : {&e->atom_sys, &e->local_idx, &e->atom_valid, &e->n_pairs, &e->lgb_class})
-    OG_CUDA(v->grow(np, st));
+  for (auto* v : {&e->atom_sys, &e->local_idx, &e->atom_valid, &e->lgb_class}) OG_CUDA(v->grow(np, st));
   for (auto* v : {&e->pq, &e->lj, &e->gb}) OG_CUDA(v->grow(4 * static_cast<size_t>(np), st));
   OG_CUDA(e->origin.grow(e->n_tiles, st));
   const int a_first = sh.atom_begin + n_old;
@@ -1675,14 +1640,11 @@ og_status append_impl(og_engine* e, int si, const TopoCopy& grown, const double*
   {
     const int n_blocks = static_cast<int>(e->mask_of.size()), n_near = static_cast<int>(e->h_near.size());
     e->tile_refs.resize(e->n_tiles);
-    e->excl_rows.resize(np);
-    int t_min = e->n_tiles, a_min = np;
+    int t_min = e->n_tiles;
     std::set<int> touched;
     mask_diagonal(e, old_tiles, e->n_tiles, &t_min, &touched);
-    for (int k : d.excl) mask_exclusion(e, si, static_cast<size_t>(k), &t_min, &a_min, &touched);
-    if ((s = upload_exclusions(e, n_blocks, std::min(t_min, old_tiles), std::min(a_min, old_np), n_near, touched,
-                               st)) != OG_OK)
-      return s;
+    for (int k : d.excl) mask_exclusion(e, si, static_cast<size_t>(k), &t_min, &touched);
+    if ((s = upload_exclusions(e, n_blocks, std::min(t_min, old_tiles), n_near, touched, st)) != OG_OK) return s;
   }
 
   // bonded terms and SHAKE clusters of the new atoms, appended
@@ -1981,6 +1943,57 @@ og_status og_get_born_integrals(og_engine* e, int32_t s, double* out) {
   return OG_OK;
 }
 
+namespace {
+
+// Every system's energy terms at the current positions into seg_out
+// ([term][system]); the surface term when `areas`.
+og_status enqueue_energies(og_engine* e, bool areas, cudaStream_t stream) {
+  const int n_sys = static_cast<int>(e->sys.size());
+  ogk::EnergyArgs a{};
+  a.x = e->x.p; a.y = e->y.p; a.z = e->z.p; a.q = e->q.p;
+  a.rmin = e->rmin.p; a.eps = e->eps.p; a.rmin14 = e->rmin14.p; a.eps14 = e->eps14.p;
+  a.rho_tilde = e->rho_tilde.p; a.srho = e->srho.p; a.born_r = e->born_r64.p;
+  a.origin = e->origin.p;
+  a.atom_sys = e->atom_sys.p;
+  a.sys_tiles = e->sys_tiles.p;
+  a.sys_state = e->sys_state.p;
+  a.mask_begin = e->mask_begin.p; a.mask_refs = e->mask_refs.p; a.mask_ex = e->mask_ex.p; a.mask_14 = e->mask_14.p;
+  a.n_tiles = e->n_tiles;
+  const bool all_nb = no_cutoff(e->p.nb_cutoff), all_born = no_cutoff(e->p.born_cutoff);
+  a.nb_cutoff = all_nb ? INFINITY : e->p.nb_cutoff;
+  a.nb_c2 = all_nb ? INFINITY : e->p.nb_cutoff * e->p.nb_cutoff;
+  a.born_cutoff = all_born ? INFINITY : e->p.born_cutoff;
+  a.born_c2 = all_born ? INFINITY : e->p.born_cutoff * e->p.born_cutoff;
+  const double rc = e->p.nb_cutoff;
+  a.kappa = all_nb ? 0.0 : 1.0 / (2.0 * rc * rc * rc);
+  a.crf = all_nb ? 0.0 : 3.0 / (2.0 * rc);
+  a.n_chunks = e->e_chunks; a.part = e->epart.p; a.pair_part = e->epair.p; a.pair_count = e->epair_count.p;
+
+  OG_CUDA(cudaMemsetAsync(e->clamp_count.p, 0, sizeof(int32_t) * n_sys, stream));
+  // the tile spheres of the cutoff culls and the surface term
+  if (areas || !all_nb || !all_born) ogk::launch_pack(e->atoms(), false, stream);
+  ogk::launch_born64(a, stream);
+  ogk::launch_born_finalize(e->atoms(), a.part, a.n_chunks, e->born_r64.p, false, e->clamp_count.p, stream);
+  ogk::launch_energy64(a, stream);
+  ogk::launch_bonded_energies(e->bonded_args(), stream);
+  if (areas) {
+    OG_CUDA(cudaMemsetAsync(e->sasa_area.p, 0, sizeof(double) * e->n_padded, stream));
+    OG_CUDA(cudaMemsetAsync(e->sasa_energy.p, 0, sizeof(double) * e->n_padded, stream));
+    ogk::launch_sasa_areas(e->sasa_args(false), stream);
+  }
+  ogk::EnergyTotals t{};
+  t.sasa = areas ? e->sasa_energy.p : nullptr;
+  t.bonded = e->bonded_e.p;
+  t.seg_begin = e->seg_begin.p;
+  t.seg_end = e->seg_end.p;
+  t.clamp_count = e->clamp_count.p;
+  t.out = e->seg_out.p;
+  ogk::launch_energy_totals(a, t, n_sys, stream);
+  return launch_check("energy kernels");
+}
+
+}  // namespace
+
 og_status og_compute_energies(og_engine* e, int32_t s, og_energies* out) {
   og_status st = check_ready(e);
   if (st != OG_OK) return st;
@@ -1988,96 +2001,32 @@ og_status og_compute_energies(og_engine* e, int32_t s, og_energies* out) {
   if (!out) return og_fail(OG_E_BADARG, "null output");
   if (s < -1 || s >= n_sys) return og_fail(OG_E_BADARG, "system index out of range");
   cudaStream_t stream = e->stream;
-  ogk::EnergyArgs a{};
-  a.x = e->x.p; a.y = e->y.p; a.z = e->z.p; a.q = e->q.p;
-  a.rmin = e->rmin.p; a.eps = e->eps.p; a.rmin14 = e->rmin14.p; a.eps14 = e->eps14.p;
-  a.rho_tilde = e->rho_tilde.p; a.srho = e->srho.p; a.born_r = e->born_r64.p;
-  a.atom_sys = e->atom_sys.p;
-  std::vector<int32_t> hb(n_sys), hc(n_sys);
-  for (int k = 0; k < n_sys; ++k) {
-    hb[k] = e->sys[k].atom_begin;
-    hc[k] = e->sys[k].topo.n;
-  }
-  DVec<int32_t> dbeg, dcnt;
-  OG_CUDA(dbeg.upload(hb, stream));
-  OG_CUDA(dcnt.upload(hc, stream));
-  a.sys_begin = dbeg.p;
-  a.sys_count = dcnt.p;
-  a.excl_row = e->excl_row.p; a.excl_col = e->excl_col.p; a.excl_kind = e->excl_kind.p;
-  a.n_atoms_padded = e->n_padded;
-  a.nb_c2 = no_cutoff(e->p.nb_cutoff) ? INFINITY : e->p.nb_cutoff * e->p.nb_cutoff;
-  a.born_c2 = no_cutoff(e->p.born_cutoff) ? INFINITY : e->p.born_cutoff * e->p.born_cutoff;
-  const double rc = e->p.nb_cutoff;
-  a.kappa = no_cutoff(rc) ? 0.0 : 1.0 / (2.0 * rc * rc * rc);
-  a.crf = no_cutoff(rc) ? 0.0 : 3.0 / (2.0 * rc);
-  a.integral = e->integral64.p;
-  a.e_lj = e->e_lj.p; a.e_coul = e->e_coul.p; a.e_gb = e->e_gb.p; a.e_self = e->e_self.p;
-  a.n_pairs = e->n_pairs.p;
-  a.n_chunks = e->e_chunks; a.part = e->epart.p; a.part_pairs = e->epart_pairs.p;
-
-  OG_CUDA(cudaMemsetAsync(e->clamp_count.p, 0, sizeof(int32_t) * n_sys, stream));
-  ogk::launch_born64(a, stream);
-  ogk::launch_born_finalize(e->atoms(), e->integral64.p, e->born_r64.p, false, e->clamp_count.p, stream);
-  ogk::launch_energy64(a, stream);
-  ogk::launch_bonded_energies(e->bonded_args(), stream);
-  if (e->p.include_sasa) {
-    OG_CUDA(cudaMemsetAsync(e->sasa_area.p, 0, sizeof(double) * e->n_padded, stream));
-    OG_CUDA(cudaMemsetAsync(e->sasa_energy.p, 0, sizeof(double) * e->n_padded, stream));
-    ogk::launch_pack(e->atoms(), false, stream);
-    ogk::launch_sasa_areas(e->sasa_args(false), stream);
-  }
-  if ((st = launch_check("energy kernels")) != OG_OK) return st;
-
-  // Deterministic per-system sums, all on the device, then one copy back:
-  // seg_out = [lj | coulomb | gb pair | gb self | sasa | bond | angle |
-  // dihedral | improper], n_sys each.
-  const double* per_atom[5] = {e->e_lj.p, e->e_coul.p, e->e_gb.p, e->e_self.p, e->sasa_energy.p};
-  const int n_terms = e->p.include_sasa ? 5 : 4;
-  for (int k = 0; k < n_terms; ++k)
-    ogk::launch_segment_sum(per_atom[k], e->seg_begin.p, e->seg_end.p, n_sys, e->seg_out.p + k * n_sys, stream);
-  ogk::launch_segment_sum(e->bonded_e.p, e->seg_begin.p + n_sys, e->seg_end.p + n_sys, 4 * n_sys,
-                          e->seg_out.p + 5 * n_sys, stream);
-  std::vector<double> all(9 * static_cast<size_t>(n_sys), 0.0);
-  OG_CUDA(cudaMemcpyAsync(all.data(), e->seg_out.p, sizeof(double) * (n_terms == 5 ? 9 : 4) * n_sys,
-                          cudaMemcpyDeviceToHost, stream));
-  if (n_terms < 5)
-    OG_CUDA(cudaMemcpyAsync(all.data() + 5 * n_sys, e->seg_out.p + 5 * n_sys, sizeof(double) * 4 * n_sys,
-                            cudaMemcpyDeviceToHost, stream));
-  std::vector<double> sums[5];
-  for (int k = 0; k < 5; ++k) sums[k].assign(all.begin() + k * n_sys, all.begin() + (k + 1) * n_sys);
-  std::vector<double> bonded(all.begin() + 5 * n_sys, all.end());
-  // Pair counts (int) summed on the host.
-  std::vector<int32_t> clamp(n_sys);
-  OG_CUDA(cudaMemcpyAsync(clamp.data(), e->clamp_count.p, sizeof(int32_t) * n_sys, cudaMemcpyDeviceToHost, stream));
-  std::vector<int32_t> pairs(e->n_padded);
-  OG_CUDA(cudaMemcpyAsync(pairs.data(), e->n_pairs.p, sizeof(int32_t) * e->n_padded, cudaMemcpyDeviceToHost,
-                          stream));
+  if ((st = enqueue_energies(e, e->p.include_sasa, stream)) != OG_OK) return st;
+  std::vector<double> all(ogk::kEnergyTerms * static_cast<size_t>(n_sys));
+  OG_CUDA(cudaMemcpyAsync(all.data(), e->seg_out.p, sizeof(double) * all.size(), cudaMemcpyDeviceToHost, stream));
   OG_CUDA(cudaStreamSynchronize(stream));
-  if ((st = launch_check("energy reductions")) != OG_OK) return st;
   if (e->p.include_sasa) {
     std::vector<ogk::SysState> hs;
     if ((st = read_status(e, &hs)) != OG_OK) return st;
   }
-
   for (int k = 0; k < n_sys; ++k) {
     if (s >= 0 && k != s) continue;
+    auto term = [&](ogk::EnergyTerm t) { return all[static_cast<size_t>(t) * n_sys + k]; };
     og_energies& o = out[s >= 0 ? 0 : k];
     o = og_energies{};
-    o.bond = bonded[0 * n_sys + k];
-    o.angle = bonded[1 * n_sys + k];
-    o.dihedral = bonded[2 * n_sys + k];
-    o.improper = bonded[3 * n_sys + k];
-    o.lj = 0.5 * sums[0][k] * ogk::kKcalToKj;
-    o.coulomb = 0.5 * sums[1][k] * ogk::kKcalToKj;
-    o.gb_pair = 0.5 * sums[2][k] * ogk::kKcalToKj;
-    o.gb_self = sums[3][k] * ogk::kKcalToKj;
+    o.bond = term(ogk::kTermBond);
+    o.angle = term(ogk::kTermAngle);
+    o.dihedral = term(ogk::kTermDihedral);
+    o.improper = term(ogk::kTermImproper);
+    o.lj = term(ogk::kTermLj);
+    o.coulomb = term(ogk::kTermCoulomb);
+    o.gb_pair = term(ogk::kTermGbPair);
+    o.gb_self = term(ogk::kTermGbSelf);
     o.gb = o.gb_self + o.gb_pair;
-    o.sasa = e->p.include_sasa ? sums[4][k] : 0.0;
+    o.sasa = term(ogk::kTermSasa);
     o.total = o.bond + o.angle + o.dihedral + o.improper + o.lj + o.coulomb + o.gb + o.sasa;
-    o.born_clamped = clamp[k];
-    long long np = 0;
-    for (int i = e->sys[k].atom_begin; i < e->sys[k].atom_begin + e->sys[k].topo.n; ++i) np += pairs[i];
-    o.nb_pairs = static_cast<int32_t>(np / 2);
+    o.born_clamped = static_cast<int32_t>(term(ogk::kTermClamped));
+    o.nb_pairs = static_cast<int32_t>(term(ogk::kTermPairs));
   }
   return OG_OK;
 }
@@ -2414,37 +2363,6 @@ og_status og_remd_swap(og_engine* e, int32_t parity, const double* uniforms, int
   return OG_OK;
 }
 
-namespace {
-
-// The FP64 energy kernels of og_compute_energies without its host reductions
-// (their per-atom and per-term outputs stay on the device).
-void enqueue_energy_kernels(og_engine* e, cudaStream_t stream) {
-  ogk::EnergyArgs a{};
-  a.x = e->x.p; a.y = e->y.p; a.z = e->z.p; a.q = e->q.p;
-  a.rmin = e->rmin.p; a.eps = e->eps.p; a.rmin14 = e->rmin14.p; a.eps14 = e->eps14.p;
-  a.rho_tilde = e->rho_tilde.p; a.srho = e->srho.p; a.born_r = e->born_r64.p;
-  a.atom_sys = e->atom_sys.p;
-  a.sys_begin = e->remd_begin.p;
-  a.sys_count = e->remd_count.p;
-  a.excl_row = e->excl_row.p; a.excl_col = e->excl_col.p; a.excl_kind = e->excl_kind.p;
-  a.n_atoms_padded = e->n_padded;
-  a.nb_c2 = no_cutoff(e->p.nb_cutoff) ? INFINITY : e->p.nb_cutoff * e->p.nb_cutoff;
-  a.born_c2 = no_cutoff(e->p.born_cutoff) ? INFINITY : e->p.born_cutoff * e->p.born_cutoff;
-  const double rc = e->p.nb_cutoff;
-  a.kappa = no_cutoff(rc) ? 0.0 : 1.0 / (2.0 * rc * rc * rc);
-  a.crf = no_cutoff(rc) ? 0.0 : 3.0 / (2.0 * rc);
-  a.integral = e->integral64.p;
-  a.e_lj = e->e_lj.p; a.e_coul = e->e_coul.p; a.e_gb = e->e_gb.p; a.e_self = e->e_self.p;
-  a.n_pairs = e->n_pairs.p;
-  a.n_chunks = e->e_chunks; a.part = e->epart.p; a.part_pairs = e->epart_pairs.p;
-  ogk::launch_born64(a, stream);
-  ogk::launch_born_finalize(e->atoms(), e->integral64.p, e->born_r64.p, false, e->clamp_count.p, stream);
-  ogk::launch_energy64(a, stream);
-  ogk::launch_bonded_energies(e->bonded_args(), stream);
-}
-
-}  // namespace
-
 og_status og_remd_run(og_engine* e, int32_t n_rounds, int32_t steps_per_swap, uint64_t seed, int64_t* attempts,
                       int64_t* accepts, int32_t* sys_of_slot) {
   og_status st = check_ready(e);
@@ -2457,20 +2375,14 @@ og_status og_remd_run(og_engine* e, int32_t n_rounds, int32_t steps_per_swap, ui
     if (sh.topo.n != e->sys[0].topo.n) return og_fail(OG_E_BADARG, "replica exchange between unequal systems");
   cudaStream_t stream = e->stream;
   if (!e->remd_ready) {
-    std::vector<int32_t> order(n), hb(n), hc(n);
+    std::vector<int32_t> order(n);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return e->sys[a].temperature < e->sys[b].temperature; });
     std::vector<double> temps(n);
-    for (int k = 0; k < n; ++k) {
-      temps[k] = e->sys[order[k]].temperature;
-      hb[k] = e->sys[k].atom_begin;
-      hc[k] = e->sys[k].topo.n;
-    }
+    for (int k = 0; k < n; ++k) temps[k] = e->sys[order[k]].temperature;
     OG_CUDA(e->remd_slot.upload(order, stream));
     OG_CUDA(e->remd_temps.upload(temps, stream));
-    OG_CUDA(e->remd_begin.upload(hb, stream));
-    OG_CUDA(e->remd_count.upload(hc, stream));
     OG_CUDA(e->remd_total.alloc(n));
     OG_CUDA(e->remd_vscale.alloc(n));
     OG_CUDA(e->remd_attempts.alloc(std::max(n - 1, 1)));
@@ -2488,15 +2400,12 @@ og_status og_remd_run(og_engine* e, int32_t n_rounds, int32_t steps_per_swap, ui
   r.vscale = e->remd_vscale.p;
   r.attempts = e->remd_attempts.p;
   r.accepts = e->remd_accepts.p;
-  r.e_lj = e->e_lj.p; r.e_coul = e->e_coul.p; r.e_gb = e->e_gb.p; r.e_self = e->e_self.p;
-  r.bonded_e = e->bonded_e.p;
-  r.seg_begin = e->seg_begin.p;
-  r.seg_end = e->seg_end.p;
+  r.terms = e->seg_out.p;
   r.n_slots = n;
   r.seed = seed;
   for (int round = 0; round < n_rounds; ++round) {
     if ((st = og_step(e, steps_per_swap)) != OG_OK && st != OG_E_NONFINITE) return st;
-    enqueue_energy_kernels(e, stream);
+    if ((st = enqueue_energies(e, false, stream)) != OG_OK) return st;
     ogk::launch_remd_round(e->atoms(), r, static_cast<int>(e->remd_round & 1u), e->remd_round, stream);
     e->remd_round += 1;
     if ((st = launch_check("replica exchange")) != OG_OK) return st;
@@ -2800,7 +2709,7 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
       pb.seg_end = e->seg_end_b.p;
     }
     ogk::launch_born_pass(pb, e->born_launch, e->stream);
-    ogk::launch_born_finalize(e->atoms(), nullptr, e->born_r.p, true, nullptr, e->stream);
+    ogk::launch_born_finalize(e->atoms(), nullptr, 0, e->born_r.p, true, nullptr, e->stream);
     OG_CUDA(cudaStreamSynchronize(e->stream));
     const int chunks[3] = {8, 16, 32};
     for (int pass = 0; pass < 2; ++pass) {

@@ -129,178 +129,271 @@ void launch_near_force64(const PairArgs& a, const int4* near, int n_near, cudaSt
 }
 
 // ----------------------------------------------------------------- FP64 path
+//
+// Energies: one warp owns a 32-atom i-tile and every n_chunks-th j-tile (its
+// j-tiles staged in the warp's shared memory, read back as broadcasts), so a
+// single chain spreads over n_tiles x n_chunks warps.  Bound by the FP64
+// pipe.  Three things cut its work per pair against a closed form per
+// ordered pair (0.60 ms for an energy of a 4 694-atom chain, all pairs):
+//   * the pair energies see each unordered pair once (tiles jt >= it) and
+//     take 1/r from one reciprocal square root;
+//   * distant pairs (a warp vote) need no exponential in the GB term, and in
+//     the descreening integral a short series in s/r instead of two
+//     divisions, a square root and a logarithm;
+//   * with cutoffs, tile pairs whose bounding spheres are apart are skipped.
+// Sums run in a fixed order: per lane over its pairs, warp butterflies,
+// then k_energy_totals.
 
 namespace {
 
-__device__ __forceinline__ double descreen64(double r, double rho_i, double s_rho_j) {
-  // energy/src/gb.rs:347-369, term for term.
+constexpr int kEnergyWarps = 4;
+
+__device__ __forceinline__ double descreen64(double r, double r2, double inv_r, double rho_i, double s_rho_j) {
+  // energy/src/gb.rs:347-369, with 1/r given.
   if (r + s_rho_j <= rho_i) return 0.0;
   const double l = (r - s_rho_j < rho_i) ? rho_i : r - s_rho_j;
   const double u = r + s_rho_j;
   if (u <= 0.0 || l <= 0.0) return 0.0;
   const double inv_l = 1.0 / l, inv_u = 1.0 / u;
+  const double d2 = inv_u * inv_u - inv_l * inv_l;
   const double term1 = 0.5 * (inv_l - inv_u);
-  const double term2 = (r / 4.0) * (inv_u * inv_u - inv_l * inv_l);
-  const double term3 = (1.0 / (2.0 * r)) * log(l / u);
-  const double term4 = (s_rho_j * s_rho_j - r * r) / (4.0 * r) * (inv_u * inv_u - inv_l * inv_l);
+  const double term2 = (r * 0.25) * d2;
+  const double term3 = (0.5 * inv_r) * log(l * inv_u);
+  const double term4 = (s_rho_j * s_rho_j - r2) * (0.25 * inv_r) * d2;
   return term1 + term2 + term3 + term4;
 }
 
-// j range `c` of `nc` over a system's atoms [b, b + n).
-__device__ __forceinline__ void chunk_range(int b, int n, int c, int nc, int* j0, int* j1) {
-  *j0 = b + static_cast<int>(static_cast<long long>(n) * c / nc);
-  *j1 = b + static_cast<int>(static_cast<long long>(n) * (c + 1) / nc);
+// The same function where the spheres do not overlap (l = r - s), as its
+// series in x = s/r (see k_born): h = -(x^3 / r) sum_k k (2k - 1) / (2k + 1)
+// x^(2 (k - 1)), kTerms terms, w = x^2.  Dropped terms stay below 2^-53 of
+// the first for x < 1/16 with 8 terms (256^-8 * 24 = 1.3e-18) and x < 1/4
+// with 15 (16^-15 * 45 = 3.9e-17).  The closed form loses digits to
+// cancellation at these distances; the series does not.
+template <int kTerms>
+__device__ __forceinline__ double descreen_series64(double w) {
+  double p = 0.0;
+#pragma unroll
+  for (int k = kTerms; k >= 1; --k) p = fma(p, w, static_cast<double>(k * (2 * k - 1)) / (2 * k + 1));
+  return p;
 }
 
-__global__ void k_born64(EnergyArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Tile spheres at least `cutoff` apart (FP64, the margin of k_cut_lists).
+__device__ __forceinline__ bool tiles_apart(double4 oi, double4 oj, double cutoff) {
+  const double dx = oj.x - oi.x, dy = oj.y - oi.y, dz = oj.z - oi.z;
+  const double lim = oi.w + oj.w + cutoff + 1e-3;
+  return dx * dx + dy * dy + dz * dz > lim * lim;
+}
+
+struct BornTile {
+  double4 p[kTile];  // x, y, z, s rho~
+};
+
+__global__ void __launch_bounds__(kEnergyWarps * 32) k_born64(EnergyArgs a) {
+  __shared__ BornTile tiles[kEnergyWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int it = blockIdx.x * kEnergyWarps + warp;
   const int c = blockIdx.y;
-  if (i >= a.n_atoms_padded) return;
-  const int sys = a.atom_sys[i];
-  if (sys < 0) return;
-  int j0, j1;
-  chunk_range(a.sys_begin[sys], a.sys_count[sys], c, a.n_chunks, &j0, &j1);
-  const double xi = a.x[i], yi = a.y[i], zi = a.z[i], rho = a.rho_tilde[i];
+  if (it >= a.n_tiles) return;
+  BornTile& t = tiles[warp];
+  const int sys = a.atom_sys[it * kTile];
+  const int2 st = a.sys_tiles[sys];
+  const int end = st.x * kTile + a.sys_state[sys].n_atoms;
+  const int i = it * kTile + lane;
+  const int il = i < end ? i : it * kTile;  // padding lanes repeat the tile's first atom (for the votes)
+  const double xi = a.x[il], yi = a.y[il], zi = a.z[il], rho = a.rho_tilde[il];
+  const bool cut = a.born_c2 != INFINITY;
+  const double4 oi = a.origin[it];
   double acc = 0.0;
-  for (int j = j0; j < j1; ++j) {
-    if (j == i) continue;
-    const double dx = a.x[j] - xi, dy = a.y[j] - yi, dz = a.z[j] - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 > a.born_c2 || r2 < 1e-18) continue;
-    acc += descreen64(sqrt(r2), rho, a.srho[j]);
-  }
-  if (a.n_chunks == 1) a.integral[i] = acc;
-  else a.part[static_cast<size_t>(c) * a.n_atoms_padded + i] = acc;
-}
-
-__global__ void k_born64_sum(EnergyArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n_atoms_padded || a.atom_sys[i] < 0) return;
-  double acc = 0.0;
-  for (int c = 0; c < a.n_chunks; ++c) acc += a.part[static_cast<size_t>(c) * a.n_atoms_padded + i];
-  a.integral[i] = acc;
-}
-
-// Per i atom, over every j != i of its system: LJ + RF Coulomb within the
-// nonbonded cutoff with exclusions / 1-4 parameters (nonbonded.rs:127-169)
-// and the GB pair energy over all pairs (gb.rs:160-173).  Each unordered pair
-// is seen from both ends, so the host halves the sums.
-__global__ void k_energy64(EnergyArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  if (i >= a.n_atoms_padded) return;
-  const int sys = a.atom_sys[i];
-  const double pref = -0.5 * (1.0 - 1.0 / kEpsWater) * kCoulomb;
-  if (sys < 0) {
-    if (a.n_chunks == 1) {
-      a.e_lj[i] = a.e_coul[i] = a.e_gb[i] = a.e_self[i] = 0.0;
-      a.n_pairs[i] = 0;
+  for (int jt = st.x + c; jt < st.x + st.y; jt += a.n_chunks) {
+    if (cut && tiles_apart(oi, a.origin[jt], a.born_cutoff)) continue;
+    const int j0 = jt * kTile, nj = min(kTile, end - j0);
+    __syncwarp();
+    if (lane < nj) t.p[lane] = make_double4(a.x[j0 + lane], a.y[j0 + lane], a.z[j0 + lane], a.srho[j0 + lane]);
+    __syncwarp();
+    const int self = il - j0;
+    for (int k = 0; k < nj; ++k) {
+      const double4 pj = t.p[k];
+      const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double inv_r = rsqrt(r2);
+      const double r = r2 * inv_r;
+      const double x = pj.w * inv_r;
+      const bool on = k != self && !(r2 > a.born_c2) && !(r2 < 1e-18);
+      const bool apart = r - pj.w >= rho;
+      const double w = x * x;
+      double h;
+      if (__all_sync(0xffffffffu, apart && x < 0.0625)) {
+        h = -(w * x * inv_r) * descreen_series64<8>(w);
+      } else if (__all_sync(0xffffffffu, apart && x < 0.25)) {
+        h = -(w * x * inv_r) * descreen_series64<15>(w);
+      } else {
+        h = on ? descreen64(r, r2, inv_r, rho, pj.w) : 0.0;
+      }
+      if (on) acc += h;
     }
-    return;
   }
-  int j0, j1;
-  chunk_range(a.sys_begin[sys], a.sys_count[sys], c, a.n_chunks, &j0, &j1);
-  const double xi = a.x[i], yi = a.y[i], zi = a.z[i], qi = a.q[i], Ri = a.born_r[i];
-  int ep = a.excl_row[i];
-  const int ee = a.excl_row[i + 1];
-  while (ep < ee && a.excl_col[ep] < j0) ++ep;
+  if (i < end) a.part[static_cast<size_t>(c) * a.n_tiles * kTile + i] = acc;
+}
+
+// The j-tile staged per warp.
+struct EnergyTile {
+  double4 p[kTile];  // x, y, z, q
+  double4 g[kTile];  // Rmin/2, sqrt(eps), R, 1/R
+};
+
+// LJ + RF Coulomb within the nonbonded cutoff with exclusions / 1-4
+// parameters (nonbonded.rs:127-169) and the GB pair energy over all pairs
+// (gb.rs:160-173), each unordered pair once.  LJ as sqrt(eps_i eps_j) (r6^2 -
+// 2 r6); every sum without its constant prefactor (k_energy_totals).
+__global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
+  __shared__ EnergyTile tiles[kEnergyWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int it = blockIdx.x * kEnergyWarps + warp;
+  const int c = blockIdx.y;
+  if (it >= a.n_tiles) return;
+  EnergyTile& t = tiles[warp];
+  const int sys = a.atom_sys[it * kTile];
+  const int2 st = a.sys_tiles[sys];
+  const int end = st.x * kTile + a.sys_state[sys].n_atoms;
+  const int i = it * kTile + lane;
+  const bool valid = i < end;
+  const int il = valid ? i : it * kTile;
+  const double xi = a.x[il], yi = a.y[il], zi = a.z[il], qi = a.q[il], Ri = a.born_r[il];
+  const double rmi = a.rmin[il], sepi = sqrt(a.eps[il]);
+  const double rm14i = a.rmin14[il], sep14i = sqrt(a.eps14[il]);
+  const double iRi4 = 0.25 / Ri;
+  const bool cut = a.nb_c2 != INFINITY;
+  const double4 oi = a.origin[it];
+  int mref = a.mask_begin[it];
+  const int mend = a.mask_begin[it + 1];
   double lj = 0.0, coul = 0.0, gb = 0.0;
   int pairs = 0;
-  for (int j = j0; j < j1; ++j) {
-    if (j == i) continue;
-    const double dx = a.x[j] - xi, dy = a.y[j] - yi, dz = a.z[j] - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    int kind = 0;
-    while (ep < ee && a.excl_col[ep] < j) ++ep;
-    if (ep < ee && a.excl_col[ep] == j) kind = a.excl_kind[ep];
-    const double qq = qi * a.q[j];
-    if (qq != 0.0) {
-      // Once r2 / (4 rp) >= 40, rp exp(-r2 / (4 rp)) < r2 2^-54 (e^-40 <
-      // 160 2^-54, and the gap only widens), below half an ulp of r2, so
-      // r2 + rp exp(...) rounds to r2: the exponential is skipped there
-      // with the same result bit for bit.
-      const double rp = Ri * a.born_r[j];
-      const double xg = r2 / (4.0 * rp);
-      const double fgb = xg >= 40.0 ? sqrt(r2) : sqrt(r2 + rp * exp(-xg));
-      gb += 2.0 * pref * qq / fgb;
+  for (int jt = it + c; jt < st.x + st.y; jt += a.n_chunks) {
+    while (mref < mend && a.mask_refs[mref].j_tile < jt) ++mref;
+    uint32_t ex = 0u, m14 = 0u;
+    if (mref < mend && a.mask_refs[mref].j_tile == jt) {
+      const int w = a.mask_refs[mref].offset * kTile + lane;
+      ex = a.mask_ex[w];
+      m14 = a.mask_14[w];
     }
-    if (r2 > a.nb_c2 || kind == 1) continue;
-    const double r = sqrt(r2);
-    double rmin, eps;
-    if (kind == 2) {
-      rmin = a.rmin14[i] + a.rmin14[j];
-      eps = sqrt(a.eps14[i] * a.eps14[j]);
-    } else {
-      rmin = a.rmin[i] + a.rmin[j];
-      eps = sqrt(a.eps[i] * a.eps[j]);
+    const bool any14 = __any_sync(0xffffffffu, m14 != 0u);
+    const bool nb_tile = !cut || !tiles_apart(oi, a.origin[jt], a.nb_cutoff);
+    const int j0 = jt * kTile, nj = min(kTile, end - j0);
+    __syncwarp();
+    if (lane < nj) {
+      const int j = j0 + lane;
+      t.p[lane] = make_double4(a.x[j], a.y[j], a.z[j], a.q[j]);
+      t.g[lane] = make_double4(a.rmin[j], sqrt(a.eps[j]), a.born_r[j], 1.0 / a.born_r[j]);
     }
-    const double x = rmin / r;
-    const double x2 = x * x;
-    const double r6 = x2 * x2 * x2;
-    lj += eps * (r6 * r6 - 2.0 * r6);
-    if (qq != 0.0) coul += kCoulomb * qq * (1.0 / r + a.kappa * r * r - a.crf);
-    ++pairs;
+    __syncwarp();
+    const int first = jt == it ? lane + 1 : 0;  // the diagonal tile's pairs once
+    for (int k = 0; k < nj; ++k) {
+      const double4 pj = t.p[k], gj = t.g[k];
+      const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const bool on = valid && k >= first;
+      const double inv_r = rsqrt(r2);
+      // Once r2 / (4 R_i R_j) >= 40, R_i R_j exp(-r2 / (4 R_i R_j)) < r2
+      // 2^-54 (e^-40 < 160 2^-54, and the gap only widens), below half an
+      // ulp of r2: f_GB = r there.
+      const double xg = r2 * (iRi4 * gj.w);
+      double inv_f = inv_r;
+      if (!__all_sync(0xffffffffu, xg >= 40.0)) inv_f = rsqrt(r2 + Ri * gj.z * exp(-xg));
+      if (on) gb += pj.w * inv_f;
+      if (!nb_tile) continue;
+      const bool nb = on && !(r2 > a.nb_c2) && !((ex >> k) & 1u);
+      if (!__any_sync(0xffffffffu, nb)) continue;
+      double rmin = rmi + gj.x, se = sepi * gj.y;
+      if (any14 && ((m14 >> k) & 1u)) {
+        rmin = rm14i + a.rmin14[j0 + k];
+        se = sep14i * sqrt(a.eps14[j0 + k]);
+      }
+      if (nb) {
+        const double x = rmin * inv_r;
+        const double x2 = x * x;
+        const double r6 = x2 * x2 * x2;
+        lj += se * (r6 * (r6 - 2.0));
+        const double rf = cut ? fma(a.kappa, r2, inv_r) - a.crf : inv_r;
+        if (pj.w != 0.0) coul += pj.w * rf;
+        ++pairs;
+      }
+    }
   }
-  if (a.n_chunks == 1) {
-    a.e_lj[i] = lj;
-    a.e_coul[i] = coul;
-    a.e_gb[i] = gb;
-    a.e_self[i] = (qi != 0.0) ? pref * (qi * qi) / Ri : 0.0;
-    a.n_pairs[i] = pairs;
-    return;
+  // a charge of zero contributes nothing, whatever its pairs
+  double v[3] = {valid ? lj : 0.0, valid && qi != 0.0 ? qi * coul : 0.0, valid && qi != 0.0 ? qi * gb : 0.0};
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
   }
-  const size_t np = a.n_atoms_padded, nc = a.n_chunks;
-  a.part[(0 * nc + c) * np + i] = lj;
-  a.part[(1 * nc + c) * np + i] = coul;
-  a.part[(2 * nc + c) * np + i] = gb;
-  a.part_pairs[c * np + i] = pairs;
+  if (lane == 0) {
+    const size_t m = static_cast<size_t>(a.n_tiles) * a.n_chunks, at = static_cast<size_t>(it) * a.n_chunks + c;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) a.pair_part[k * m + at] = v[k];
+    a.pair_count[at] = pairs;
+  }
 }
 
-__global__ void k_energy64_sum(EnergyArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n_atoms_padded) return;
-  if (a.atom_sys[i] < 0) {
-    a.e_lj[i] = a.e_coul[i] = a.e_gb[i] = a.e_self[i] = 0.0;
-    a.n_pairs[i] = 0;
-    return;
+// One block per (system, term): the sums of og_energies in kJ/mol, pair and
+// clamp counts as doubles, out[term * n_sys + system].
+constexpr int kTotalThreads = 256;
+
+__global__ void __launch_bounds__(kTotalThreads) k_energy_totals(EnergyArgs a, EnergyTotals t) {
+  const int sys = blockIdx.x, term = blockIdx.y;
+  const int2 st = a.sys_tiles[sys];
+  const double pref = -(1.0 - 1.0 / kEpsWater) * kCoulomb;
+  double acc = 0.0;
+  if (term <= kTermGbPair || term == kTermPairs) {
+    const size_t m = static_cast<size_t>(a.n_tiles) * a.n_chunks;
+    const size_t k0 = static_cast<size_t>(st.x) * a.n_chunks, k1 = k0 + static_cast<size_t>(st.y) * a.n_chunks;
+    for (size_t k = k0 + threadIdx.x; k < k1; k += kTotalThreads)
+      acc += term == kTermPairs ? static_cast<double>(a.pair_count[k]) : a.pair_part[term * m + k];
+    acc *= term == kTermLj ? kKcalToKj : term == kTermCoulomb ? kCoulomb * kKcalToKj : term == kTermGbPair ? pref * kKcalToKj : 1.0;
+  } else if (term == kTermGbSelf) {
+    const int i0 = st.x * kTile, i1 = i0 + a.sys_state[sys].n_atoms;
+    for (int i = i0 + threadIdx.x; i < i1; i += kTotalThreads) {
+      const double qi = a.q[i];
+      acc += qi != 0.0 ? (qi * qi) / a.born_r[i] : 0.0;
+    }
+    acc *= 0.5 * pref * kKcalToKj;
+  } else if (term == kTermClamped) {
+    acc = threadIdx.x == 0 ? static_cast<double>(t.clamp_count[sys]) : 0.0;
+  } else if (term == kTermSasa) {
+    if (t.sasa) {
+      const int i0 = st.x * kTile, i1 = i0 + a.sys_state[sys].n_atoms;
+      for (int i = i0 + threadIdx.x; i < i1; i += kTotalThreads) acc += t.sasa[i];
+    }
+  } else {
+    const int seg = (term - kTermBond + 1) * gridDim.x + sys;
+    for (int k = t.seg_begin[seg] + threadIdx.x; k < t.seg_end[seg]; k += kTotalThreads) acc += t.bonded[k];
   }
-  const size_t np = a.n_atoms_padded, nc = a.n_chunks;
-  double lj = 0.0, coul = 0.0, gb = 0.0;
-  int pairs = 0;
-  for (size_t c = 0; c < nc; ++c) {
-    lj += a.part[(0 * nc + c) * np + i];
-    coul += a.part[(1 * nc + c) * np + i];
-    gb += a.part[(2 * nc + c) * np + i];
-    pairs += a.part_pairs[c * np + i];
+  __shared__ double sh[kTotalThreads];
+  sh[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = kTotalThreads / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+    __syncthreads();
   }
-  const double pref = -0.5 * (1.0 - 1.0 / kEpsWater) * kCoulomb;
-  const double qi = a.q[i];
-  a.e_lj[i] = lj;
-  a.e_coul[i] = coul;
-  a.e_gb[i] = gb;
-  a.e_self[i] = (qi != 0.0) ? pref * (qi * qi) / a.born_r[i] : 0.0;
-  a.n_pairs[i] = pairs;
+  if (threadIdx.x == 0) t.out[term * gridDim.x + sys] = sh[0];
 }
 
 }  // namespace
 
 void launch_born64(const EnergyArgs& a, cudaStream_t s) {
-  const int bs = 128, nb = (a.n_atoms_padded + bs - 1) / bs;
-  k_born64<<<dim3(nb, a.n_chunks), bs, 0, s>>>(a);
-  if (a.n_chunks > 1) k_born64_sum<<<nb, bs, 0, s>>>(a);
+  k_born64<<<dim3((a.n_tiles + kEnergyWarps - 1) / kEnergyWarps, a.n_chunks), kEnergyWarps * 32, 0, s>>>(a);
 }
 
 void launch_energy64(const EnergyArgs& a, cudaStream_t s) {
-  const int bs = 128, nb = (a.n_atoms_padded + bs - 1) / bs;
-  k_energy64<<<dim3(nb, a.n_chunks), bs, 0, s>>>(a);
-  if (a.n_chunks > 1) k_energy64_sum<<<nb, bs, 0, s>>>(a);
+  k_energy64<<<dim3((a.n_tiles + kEnergyWarps - 1) / kEnergyWarps, a.n_chunks), kEnergyWarps * 32, 0, s>>>(a);
 }
 
-int energy_chunks(int n_atoms_padded, int max_system_atoms, int n_sm) {
-  const int blocks = (n_atoms_padded + 127) / 128;
-  int nc = (8 * n_sm + blocks - 1) / std::max(blocks, 1);
-  nc = std::min(nc, std::max(1, max_system_atoms / 64));
-  return std::max(1, std::min(nc, 32));
+void launch_energy_totals(const EnergyArgs& a, const EnergyTotals& t, int n_sys, cudaStream_t s) {
+  k_energy_totals<<<dim3(n_sys, kEnergyTerms), kTotalThreads, 0, s>>>(a, t);
+}
+
+int energy_chunks(int n_tiles, int max_system_tiles, int n_sm) {
+  const int nc = (24 * n_sm + n_tiles - 1) / std::max(n_tiles, 1);
+  return std::max(1, std::min(std::min(nc, max_system_tiles), 64));
 }
 
 }  // namespace ogk

@@ -5,6 +5,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "step_kernels.cuh"
+
 namespace ogk {
 
 // One unit of pair work: `n_i_tiles` (<= warps per CTA) consecutive i-tiles of
@@ -111,40 +113,53 @@ void launch_force_pass(const PairArgs& a, const PairLaunch& c, cudaStream_t s);
 // each pair once, both atoms' forces.
 void launch_near_force64(const PairArgs& a, const int4* near, int n_near, cudaStream_t s);
 
-// FP64 energy evaluation, one thread per i atom over every j of its system.
+// FP64 energy evaluation: one warp per i-tile and j range (pair_fp64.cu).
 struct EnergyArgs {
   const double* x; const double* y; const double* z;
   const double* q;
   const double* rmin; const double* eps; const double* rmin14; const double* eps14;
   const double* rho_tilde; const double* srho;  // srho = scale * rho_tilde
-  const double* born_r;                          // FP64 Born radii (output of born64)
+  const double* born_r;                          // FP64 Born radii
+  const double4* origin;                         // per tile, at the current positions
   const int32_t* atom_sys;
-  const int32_t* sys_begin;  // per system: first padded atom
-  const int32_t* sys_count;  // real atoms
-  const int32_t* excl_row;   // CSR over padded atoms: exclusion partners (both directions)
-  const int32_t* excl_col;
-  const int8_t* excl_kind;
-  int32_t n_atoms_padded;
-  double nb_c2;    // INFINITY = all pairs
-  double born_c2;
+  const int2* sys_tiles;      // per system: first tile, tiles
+  const SysState* sys_state;  // per system: real atoms
+  const int32_t* mask_begin;  // exclusion masks (PairArgs)
+  const TileMaskRef* mask_refs;
+  const uint32_t* mask_ex;
+  const uint32_t* mask_14;
+  int32_t n_tiles;
+  double nb_cutoff, nb_c2;      // A and A^2; INFINITY = all pairs
+  double born_cutoff, born_c2;
   double kappa, crf;  // reaction field constants (0 without cutoff)
-  // outputs, per padded atom
-  double* integral;   // born64
-  double* e_lj; double* e_coul; double* e_gb; double* e_self; int32_t* n_pairs;
-  // Each i atom's partners are split into n_chunks j ranges, one thread
-  // each (so that a single chain fills the GPU); with more than one, the
-  // range sums go to part ([3][n_chunks][n_atoms_padded] doubles: Born
-  // integral or LJ, Coulomb, GB) and part_pairs, and are added in range
-  // order by a second kernel.
+  // Each i-tile's j-tiles are dealt to n_chunks warps.  part: their Born
+  // integrals, [n_chunks][padded atoms]; pair_part: their LJ, Coulomb and GB
+  // sums, [3][n_tiles][n_chunks], and pair_count their LJ pairs.
   int32_t n_chunks;
   double* part;
-  int32_t* part_pairs;
+  double* pair_part;
+  int32_t* pair_count;
+};
+
+// The terms of launch_energy_totals, in its output order.
+enum EnergyTerm {
+  kTermLj = 0, kTermCoulomb, kTermGbPair, kTermGbSelf, kTermSasa, kTermBond, kTermAngle, kTermDihedral, kTermImproper,
+  kTermPairs, kTermClamped, kEnergyTerms
+};
+struct EnergyTotals {
+  const double* sasa;         // per padded atom, NULL without the surface term
+  const double* bonded;       // per bonded term
+  const int32_t* seg_begin;   // the engine's [atoms | bonds | angles | dihedrals | impropers] segments
+  const int32_t* seg_end;
+  const int32_t* clamp_count; // per system
+  double* out;                // [kEnergyTerms][n_sys], kJ/mol and counts
 };
 
 void launch_born64(const EnergyArgs& a, cudaStream_t s);
 void launch_energy64(const EnergyArgs& a, cudaStream_t s);
-// j ranges per i atom for the FP64 energy path: enough threads for eight
-// 128-thread blocks per SM, at least 64 partners per range, at most 32.
-int energy_chunks(int n_atoms_padded, int max_system_atoms, int n_sm);
+void launch_energy_totals(const EnergyArgs& a, const EnergyTotals& t, int n_sys, cudaStream_t s);
+// Warps per i-tile of the FP64 energy path: enough for 24 warps per SM, at
+// most one per j-tile of the largest system and 64.
+int energy_chunks(int n_tiles, int max_system_tiles, int n_sm);
 
 }  // namespace ogk

@@ -2,6 +2,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "pair_kernels.cuh"
 #include "step_kernels.cuh"
 
 namespace ogk {
@@ -79,7 +80,9 @@ __global__ void k_pack(AtomArrays a, bool zero_acc) {
 }
 
 // ------------------------------------------------------------ Born radii
-__global__ void k_born_finalize(AtomArrays a, const double* integral64, double* out_r, bool write_gb,
+// part64: the FP64 path's integrals, n_part range sums per atom added in
+// range order; NULL = the force path's fixed-point sums.
+__global__ void k_born_finalize(AtomArrays a, const double* part64, int32_t n_part, double* out_r, bool write_gb,
                                 int32_t* clamp_count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n_padded) return;
@@ -89,8 +92,12 @@ __global__ void k_born_finalize(AtomArrays a, const double* integral64, double* 
     out_r[i] = 1.0;
     return;
   }
-  const double integral = integral64 ? integral64[i]
-                                     : static_cast<double>(static_cast<long long>(a.born_sum[i])) * kBornUnscale;
+  double integral = 0.0;
+  if (part64) {
+    for (int c = 0; c < n_part; ++c) integral += part64[static_cast<size_t>(c) * a.n_padded + i];
+  } else {
+    integral = static_cast<double>(static_cast<long long>(a.born_sum[i])) * kBornUnscale;
+  }
   const double rt = a.rho_tilde[i];
   const double rho = a.rho[i];
   const double psi = integral * rt;
@@ -411,14 +418,6 @@ __device__ double block_sum_fixed_order(double v) {
   return sh[0];
 }
 
-__global__ void k_segment_sum(const double* v, const int32_t* begin, const int32_t* end, double* out) {
-  const int s = blockIdx.x;
-  double acc = 0.0;
-  for (int k = begin[s] + threadIdx.x; k < end[s]; k += kRedThreads) acc += v[k];
-  const double tot = block_sum_fixed_order(acc);
-  if (threadIdx.x == 0) out[s] = tot;
-}
-
 __global__ void k_kinetic(AtomArrays a, const int32_t* begin, const int32_t* end, double* out) {
   const int s = blockIdx.x;
   double acc = 0.0;
@@ -429,43 +428,26 @@ __global__ void k_kinetic(AtomArrays a, const int32_t* begin, const int32_t* end
 }
 
 // ------------------------------------------------------ replica exchange
-// Per system the potential energy og_compute_energies reports (bonded +
-// LJ/RF + GB, kJ/mol), from the per-atom and per-term FP64 energies: each
-// term summed exactly as k_segment_sum does, then combined in the same
-// order as the host, so the total is bit-identical to og_compute_energies'.
-__global__ void k_remd_totals(const double* e_lj, const double* e_coul, const double* e_gb, const double* e_self,
-                              const double* bonded_e, const int32_t* begin, const int32_t* end, int n_sys,
-                              double* total) {
-  const int s = blockIdx.x;
-  double part[8];
-  const double* per_atom[4] = {e_lj, e_coul, e_gb, e_self};
-  for (int t = 0; t < 8; ++t) {
-    const int seg = t < 4 ? s : (t - 3) * n_sys + s;
-    const double* v = t < 4 ? per_atom[t] : bonded_e;
-    double acc = 0.0;
-    for (int k = begin[seg] + threadIdx.x; k < end[seg]; k += kRedThreads) acc += v[k];
-    part[t] = block_sum_fixed_order(acc);
-    __syncthreads();  // the next sum reuses the shared buffer
-  }
-  if (threadIdx.x == 0) {
-    const double lj = 0.5 * part[0] * kKcalToKj, coul = 0.5 * part[1] * kKcalToKj;
-    const double gb_pair = 0.5 * part[2] * kKcalToKj, gb_self = part[3] * kKcalToKj;
-    const double gb = gb_self + gb_pair;
-    total[s] = part[4] + part[5] + part[6] + part[7] + lj + coul + gb;
-  }
-}
-
 // One swap round: neighbouring temperature slots (pi, pi + 1), pi = parity,
 // parity + 2, ... (remd.rs:425-474).  Slot pi holds system sys_of_slot[pi]
 // at temperature temps[pi]; an accepted exchange swaps the two systems'
 // slots (their temperatures) and marks their velocities for rescaling by
 // sqrt(T_new / T_old).  The uniform of pair pi in round r is Philox keyed by
-// (seed, r, pi).  One thread: the pairs are few and the decisions ordered.
-__global__ void k_remd_swap(SysState* sys, int32_t* sys_of_slot, const double* temps, const double* total,
-                            int n_slots, int parity, uint64_t seed, uint32_t round, long long* attempts,
-                            long long* accepts, double* vscale) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  for (int k = 0; k < n_slots; ++k) vscale[k] = 1.0;
+// (seed, r, pi).  One block: its threads form the systems' totals from the
+// energy terms in the order og_compute_energies adds them (the same value
+// bit for bit), then one thread decides (the pairs are few and ordered).
+__global__ void k_remd_swap(SysState* sys, int32_t* sys_of_slot, const double* temps, const double* terms,
+                            double* total, int n_slots, int parity, uint64_t seed, uint32_t round,
+                            long long* attempts, long long* accepts, double* vscale) {
+  for (int k = threadIdx.x; k < n_slots; k += blockDim.x) {
+    vscale[k] = 1.0;
+    auto term = [&](int t) { return terms[t * n_slots + k]; };
+    const double gb = term(kTermGbSelf) + term(kTermGbPair);
+    total[k] = term(kTermBond) + term(kTermAngle) + term(kTermDihedral) + term(kTermImproper) + term(kTermLj) +
+               term(kTermCoulomb) + gb;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   for (int pi = parity; pi + 1 < n_slots; pi += 2) {
     const int a = sys_of_slot[pi], b = sys_of_slot[pi + 1];
     if ((sys[a].status | sys[b].status) & kStatusDiverged) continue;
@@ -510,9 +492,9 @@ void launch_pack(const AtomArrays& a, bool zero_acc, cudaStream_t s) {
   k_pack<<<blocks_for(a.n_padded, 256), 256, 0, s>>>(a, zero_acc);
 }
 
-void launch_born_finalize(const AtomArrays& a, const double* integral64, double* out_r, bool write_gb,
+void launch_born_finalize(const AtomArrays& a, const double* part64, int32_t n_part, double* out_r, bool write_gb,
                           int32_t* clamp_count, cudaStream_t s) {
-  k_born_finalize<<<blocks_for(a.n_padded, 256), 256, 0, s>>>(a, integral64, out_r, write_gb, clamp_count);
+  k_born_finalize<<<blocks_for(a.n_padded, 256), 256, 0, s>>>(a, part64, n_part, out_r, write_gb, clamp_count);
 }
 
 __global__ void k_swap_systems(AtomArrays a, int32_t ba, int32_t bb, int32_t n, double scale_a, double scale_b) {
@@ -565,11 +547,6 @@ void launch_shake(const ShakeArgs& a, cudaStream_t s) {
   if (a.n_clusters > 0) k_shake<<<blocks_for(a.n_clusters, 128), 128, 0, s>>>(a);
 }
 
-void launch_segment_sum(const double* v, const int32_t* begin, const int32_t* end, int32_t n_seg, double* out,
-                        cudaStream_t s) {
-  if (n_seg > 0) k_segment_sum<<<n_seg, kRedThreads, 0, s>>>(v, begin, end, out);
-}
-
 void launch_kinetic(const AtomArrays& a, const int32_t* begin, const int32_t* end, int32_t n_sys, double* out,
                     cudaStream_t s) {
   if (n_sys > 0) k_kinetic<<<n_sys, kRedThreads, 0, s>>>(a, begin, end, out);
@@ -577,10 +554,8 @@ void launch_kinetic(const AtomArrays& a, const int32_t* begin, const int32_t* en
 
 void launch_remd_round(const AtomArrays& a, const RemdArgs& r, int parity, uint32_t round, cudaStream_t s) {
   if (r.n_slots < 2) return;
-  k_remd_totals<<<r.n_slots, kRedThreads, 0, s>>>(r.e_lj, r.e_coul, r.e_gb, r.e_self, r.bonded_e, r.seg_begin,
-                                                  r.seg_end, r.n_slots, r.total);
-  k_remd_swap<<<1, 32, 0, s>>>(r.sys, r.sys_of_slot, r.temps, r.total, r.n_slots, parity, r.seed, round, r.attempts,
-                               r.accepts, r.vscale);
+  k_remd_swap<<<1, 128, 0, s>>>(r.sys, r.sys_of_slot, r.temps, r.terms, r.total, r.n_slots, parity, r.seed, round,
+                                r.attempts, r.accepts, r.vscale);
   k_remd_rescale<<<blocks_for(a.n_padded, 256), 256, 0, s>>>(a, r.vscale);
 }
 

@@ -47,12 +47,13 @@ struct AtomArrays {
 void launch_pack(const AtomArrays& a, bool zero_acc, cudaStream_t s);
 
 // OBC-II map of the descreening integral to effective radii
-// (energy/src/gb.rs:326-341), FP64.  The integral comes from integral_fp64
-// when given, else from the fixed-point born_sum of the force path.  Radii go
+// (energy/src/gb.rs:326-341), FP64.  The integral is the sum of part64's
+// n_part ranges per padded atom ([n_part][n_padded]) when given, else the
+// fixed-point born_sum of the force path.  Radii go
 // to out_r and, when write_gb, to the gb float4s the force pass reads.
 // clamp_count (per system, optional) counts non-finite / non-positive
 // inverse radii.
-void launch_born_finalize(const AtomArrays& a, const double* integral_fp64, double* out_r, bool write_gb,
+void launch_born_finalize(const AtomArrays& a, const double* part64, int32_t n_part, double* out_r, bool write_gb,
                           int32_t* clamp_count, cudaStream_t s);
 
 // ------------------------------------------------------------------ bonded
@@ -104,11 +105,6 @@ struct ShakeArgs {
 };
 void launch_shake(const ShakeArgs& a, cudaStream_t s);
 
-// Per-system deterministic sums of a per-atom (or per-term) array:
-// out[s] = sum over [begin[s], end[s]) in a fixed order.
-void launch_segment_sum(const double* v, const int32_t* begin, const int32_t* end, int32_t n_seg, double* out,
-                        cudaStream_t s);
-
 // Replica exchange (remd.rs:442-465): swap positions, forces and Born radii
 // of two systems of equal size; velocities swap and are rescaled
 // (system a receives b's velocities times scale_a and vice versa).
@@ -139,9 +135,7 @@ struct RemdArgs {
   double* vscale;         // n_slots scratch: velocity factor per system
   long long* attempts;    // n_slots - 1 counters per slot pair
   long long* accepts;
-  const double* e_lj; const double* e_coul; const double* e_gb; const double* e_self; const double* bonded_e;
-  const int32_t* seg_begin;  // the engine's [atoms | bonds | angles | dihedrals | impropers] segments
-  const int32_t* seg_end;
+  const double* terms;    // launch_energy_totals' output
   int32_t n_slots;
   uint64_t seed;
 };
