@@ -396,15 +396,17 @@ og_status og_compute_sasa(og_engine* e, int32_t sys, int32_t method, int32_t n_d
  * the CPU.  Every variant computes the same sums; shapes differ in the
  * fixed-point rounding of partial sums only (well inside the force
  * tolerance), and for a fixed configuration runs are bit-reproducible.
- *   shape       0: 8 i-tiles (256 atoms) per CTA at the default occupancy
- *               target (Born 4 CTAs/SM, force 2); 1: 4 i-tiles (128 atoms)
- *               per CTA at twice the CTAs per SM; 2: 8 i-tiles at 3 CTAs/SM;
- *               force pass only: 3: two i-tiles per warp, 16 per CTA at 2
- *               CTAs/SM; 4: two i-tiles per warp, 8 per CTA at 4 CTAs/SM;
- *               5, 6: as 4 at 5 or 6 CTAs/SM
+ *   shape       0: one i-tile (32 atoms) per CTA, its four warps splitting
+ *               each j-tile; 1: 4 i-tiles per CTA, one per warp; Born pass 2:
+ *               8 i-tiles per CTA, one per warp; force pass 2 to 6: four
+ *               i-tiles per warp, 16 (2, 3), 8 (4, 5) or 4 (6) per CTA at
+ *               3, 4, 6, 7 or 14 CTAs/SM
  *   persistent  0: one CTA per work item; 1: resident CTAs taking items from
  *               an atomic work queue
- *   chunk       j-tiles per work item (default 16)
+ *   chunk       j-tiles per work item at most (default 16; halved while the
+ *               list has fewer than eight items per SM)
+ * An engine that is neither tuned nor set by hand takes its shapes from its
+ * tile count and cutoffs.
  * og_engine_autotune times every combination (3 Born / 7 force shapes x 2 x
  * chunks 8, 16, 32) of each pass on the engine's systems at their current positions and
  * keeps the fastest; the choice is cached in the JSON file cache_path (NULL
@@ -416,7 +418,7 @@ typedef struct og_autotune_result {
   int32_t born_shape, born_persistent, born_chunk;
   int32_t force_shape, force_persistent, force_chunk;
   double born_ms, force_ms;                 /* the chosen variants' times (ms per launch) */
-  double born_ms_default, force_ms_default; /* shape 0, one CTA per item, chunk 16; -1 from cache */
+  double born_ms_default, force_ms_default; /* the untuned engine's shape, one CTA per item, chunk 16; -1 from cache */
   int32_t from_cache;
 } og_autotune_result;
 og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_result* out);

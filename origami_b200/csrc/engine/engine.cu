@@ -18,6 +18,7 @@
 #include <numeric>
 #include <set>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../../include/origami_gpu.h"
@@ -210,7 +211,7 @@ struct og_engine {
   int64_t n_real = 0;
   DVec<double> stage_a, stage_b;
   DVec<int64_t> stage_f;
-  DVec<float> pq, lj, gb;  // tile-SoA, 4 columns per 32-atom tile
+  DVec<float> pq, lj, gb, bs;  // tile-SoA, 4 columns per 32-atom tile
   DVec<double4> origin;
   DVec<ogk::SysState> sys_state;
   // pair work
@@ -245,6 +246,7 @@ struct og_engine {
   // and the persistent launches' queue heads (Born, force)
   ogk::PairLaunch born_launch, force_launch;
   int chunk_b = 16, chunk_f = 16;
+  bool launch_set = false;  // by og_engine_set_pair_launch or og_engine_autotune; else default_launch
   DVec<int32_t> pair_queue;
   // device-side replica exchange (og_remd_run): temperature slots, counters
   bool remd_ready = false;
@@ -297,6 +299,7 @@ struct og_engine {
   bool tunnel_on = false;
   ogk::TunnelParams tunnel{};
   double sasa_rmax = 0.0;
+  double s_max = 0.0, rho_max = 0.0;  // largest s*rho~ and rho~ (series limits of the Born pass)
   // graph
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -367,7 +370,7 @@ struct og_engine {
 
   ogk::PairArgs pair_args() {
     ogk::PairArgs a{};
-    a.pq = pq.p; a.lj = lj.p; a.gb = gb.p; a.origin = origin.p; a.atom_valid = atom_valid.p;
+    a.pq = pq.p; a.lj = lj.p; a.gb = gb.p; a.bs = bs.p; a.origin = origin.p; a.atom_valid = atom_valid.p;
     a.work = work.p; a.n_work = n_work; a.jlist = jlist.p;
     a.mask_begin = mask_begin.p; a.mask_refs = mask_refs.p; a.mask_ex = mask_ex.p; a.mask_14 = mask_14.p;
     a.fx = fx.p; a.fy = fy.p; a.fz = fz.p; a.born_sum = born_sum.p;
@@ -375,11 +378,17 @@ struct og_engine {
     a.nb_c2 = c2(p.nb_cutoff);
     a.gb_c2 = c2(p.gb_force_cutoff);
     a.born_c2 = c2(p.born_cutoff);
+    auto c1 = [](double c) { return no_cutoff(c) ? INFINITY : static_cast<float>(c); };
+    a.pair_cutoff = std::max(c1(p.nb_cutoff), c1(p.gb_force_cutoff));
+    a.born_cutoff = c1(p.born_cutoff);
+    a.s_max = static_cast<float>(s_max);
+    a.rho_max = static_cast<float>(rho_max);
     a.inv_rc3 = no_cutoff(p.nb_cutoff) ? 0.0f
                                        : static_cast<float>(1.0 / (p.nb_cutoff * p.nb_cutoff * p.nb_cutoff));
     a.coul_kj = static_cast<float>(ogk::kCoulomb * ogk::kKcalToKj);
     a.lj_kj12 = static_cast<float>(12.0 * ogk::kKcalToKj);
     a.gb_pref_kj = static_cast<float>((1.0 - 1.0 / ogk::kEpsWater) * ogk::kCoulomb * ogk::kKcalToKj);
+    a.far_kj = static_cast<float>(-ogk::kCoulomb * ogk::kKcalToKj / ogk::kEpsWater);
     a.error_flag = error_flag.p;
     a.queue = pair_queue.p;
     a.atom_sys = atom_sys.p;
@@ -797,14 +806,25 @@ og_status set_xyz(og_engine* e, int s, DVec<double>& a, DVec<double>& b, DVec<do
   return OG_OK;
 }
 
+// Work items of a pass over i-blocks of W tiles in chunks of `chunk` j-tiles.
+int64_t count_items(const og_engine* e, int first_offset, int W, int chunk) {
+  int64_t n = 0;
+  for (const auto& s : e->sys)
+    for (int t0 = 0; t0 < s.n_tiles; t0 += W) n += std::max(0, (s.n_tiles - t0 - first_offset + chunk - 1) / chunk);
+  return n;
+}
+
 // Pair work (Newton-3 layout): i-blocks of W consecutive tiles (W from the
 // pass's launch shape) against the tiles from the block's first tile on
 // (Born pass: the block's own diagonal included) or after it (far-field
 // force pass), cut into chunks of at most `chunk` j-tiles and ordered
-// longest first; plus the i-blocks of cutoff mode's culled lists.
+// longest first; plus the i-blocks of cutoff mode's culled lists.  A list
+// too short to fill the GPU (eight items per SM) is cut finer: with few
+// tiles the longest item is the pass's time.
 og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec<ogk::PairWork>* work,
                           int* n_work, DVec<int32_t>* jlist, DVec<ogk::CutBlock>* cut, int* n_cut,
                           DVec<int32_t>* jlist_cut, DVec<int32_t>* seg_end, cudaStream_t st) {
+  while (chunk > 1 && count_items(e, first_offset, W, chunk) < 8ll * e->n_sm) chunk /= 2;
   std::vector<int32_t> hj;
   std::vector<ogk::PairWork> hw;
   std::vector<ogk::CutBlock> hc;
@@ -831,11 +851,37 @@ og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec
   return OG_OK;
 }
 
+// The launch variants of an engine nobody tuned, by its tile pairs (times in us
+// on B200; shapes in pair_kernels.cuh).  With cutoffs most tile pairs are
+// skipped and shape 0 wins throughout (32 x 4 668 atoms: Born 290 against 307
+// for shape 1, force 226 against 240).  Without, Born: shape 0 while the
+// tiles are few or the systems small (4.6k atoms in one system of 147 tiles:
+// 35 against 30; 64 systems of 20 tiles: 44 against 48), else shape 1.  Force:
+// shape 0 below 800 tile pairs (20 residues: 10.6 against 12.8; 80 residues:
+// 14.5 against 13.2), shape 4 from 40 000 on (8 x 4 694 atoms: 148 against
+// 155; one system of 10.9k tile pairs: 36 against 32), shape 1 between.
+void default_launch(og_engine* e) {
+  int64_t pairs = 0;
+  int max_tiles = 0;
+  for (const auto& s : e->sys) {
+    pairs += static_cast<int64_t>(s.n_tiles) * (s.n_tiles + 1) / 2;
+    max_tiles = std::max(max_tiles, s.n_tiles);
+  }
+  e->born_launch = ogk::PairLaunch{};
+  e->force_launch = ogk::PairLaunch{};
+  e->chunk_b = e->chunk_f = 16;
+  const bool small = pairs < 4000 || (pairs < 16000 && max_tiles < 32);
+  if (no_cutoff(e->p.born_cutoff)) e->born_launch.shape = small ? 0 : 1;
+  if (no_cutoff(e->p.nb_cutoff) || no_cutoff(e->p.gb_force_cutoff))
+    e->force_launch.shape = pairs < 800 ? 0 : pairs < 40000 ? 1 : 4;
+}
+
 og_status build_pair_lists(og_engine* e, cudaStream_t st) {
-  og_status s = build_pass_list(e, 0, ogk::pair_shape_tiles(e->born_launch.shape), e->chunk_b, &e->work, &e->n_work,
+  if (!e->launch_set) default_launch(e);
+  og_status s = build_pass_list(e, 0, ogk::pair_shape_tiles(true, e->born_launch.shape), e->chunk_b, &e->work, &e->n_work,
                                 &e->jlist, &e->cut_b, &e->n_cut_b, &e->jlist_cut_b, &e->seg_end_b, st);
   if (s != OG_OK) return s;
-  return build_pass_list(e, 1, ogk::pair_shape_tiles(e->force_launch.shape), e->chunk_f, &e->work_f, &e->n_work_f,
+  return build_pass_list(e, 1, ogk::pair_shape_tiles(false, e->force_launch.shape), e->chunk_f, &e->work_f, &e->n_work_f,
                          &e->jlist_f, &e->cut_f, &e->n_cut_f, &e->jlist_cut_f, &e->seg_end_f, st);
 }
 
@@ -879,7 +925,7 @@ og_status fill_atoms(og_engine* e, int a0, int a1, cudaStream_t st) {
   std::vector<double> hm(m, 1.0), him(m, 1.0), hq(m, 0.0), hrm(m, 0.0), hep(m, 0.0), hrm14(m, 0.0),
       hep14(m, 0.0), hrho(m, 1.0), hrt(m, 1.0), hsr(m, 0.0), hr(m, 0.0), hg(m, 0.0);
   std::vector<int32_t> hsys(m, -1), hloc(m, 0), hvalid(m, 0), hcls(m, 0);
-  std::vector<float> hlj(4 * m, 0.0f), hgb(4 * m);
+  std::vector<float> hlj(4 * m, 0.0f), hgb(4 * m), hbs(4 * m, 0.0f);
   for (size_t r = 0; r < m; ++r) {
     const int i = a0 + static_cast<int>(r);
     const int si = system_of(e, i);
@@ -910,6 +956,10 @@ og_status fill_atoms(og_engine* e, int a0, int a1, cudaStream_t st) {
     hlj[ogk::soa_index(ri, 1)] = static_cast<float>(std::sqrt(hep[r]));
     hlj[ogk::soa_index(ri, 2)] = static_cast<float>(hrm14[r]);
     hlj[ogk::soa_index(ri, 3)] = static_cast<float>(std::sqrt(hep14[r]));
+    const double s3 = hsr[r] * hsr[r] * hsr[r], s5 = s3 * hsr[r] * hsr[r], s7 = s5 * hsr[r] * hsr[r];
+    hbs[ogk::soa_index(ri, 0)] = static_cast<float>(s3 / 3.0);
+    hbs[ogk::soa_index(ri, 1)] = static_cast<float>(6.0 / 5.0 * s5);
+    hbs[ogk::soa_index(ri, 2)] = static_cast<float>(15.0 / 7.0 * s7);
     // The Born pass reads rho~ and s*rho~ before the first radii exist, so
     // the gb columns start out fully defined (R = rho~ until then).
     const bool real = si >= 0;
@@ -926,9 +976,15 @@ og_status fill_atoms(og_engine* e, int a0, int a1, cudaStream_t st) {
   OG_CUDA(put(e->atom_valid, a0, hvalid, st));
   OG_CUDA(put(e->lj, 4 * static_cast<size_t>(a0), hlj, st));
   OG_CUDA(put(e->gb, 4 * static_cast<size_t>(a0), hgb, st));
+  OG_CUDA(put(e->bs, 4 * static_cast<size_t>(a0), hbs, st));
   OG_CUDA(put(e->sasa_r, a0, hr, st)); OG_CUDA(put(e->sasa_gamma, a0, hg, st));
   OG_CUDA(put(e->lgb_class, a0, hcls, st));
   for (double v : hr) e->sasa_rmax = std::max(e->sasa_rmax, v);
+  for (size_t r = 0; r < m; ++r)
+    if (hvalid[r]) {
+      e->s_max = std::max(e->s_max, hsr[r]);
+      e->rho_max = std::max(e->rho_max, hrt[r]);
+    }
   return OG_OK;
 }
 
@@ -1260,6 +1316,7 @@ og_status finalize_impl(og_engine* e) {
   for (auto* v : {&e->atom_sys, &e->local_idx, &e->atom_valid, &e->lgb_class}) OG_CUDA(v->alloc(np));
   OG_CUDA(e->lj.alloc(4 * static_cast<size_t>(np)));
   OG_CUDA(e->gb.alloc(4 * static_cast<size_t>(np)));
+  OG_CUDA(e->bs.alloc(4 * static_cast<size_t>(np)));
   {
     og_status fs = fill_atoms(e, 0, np, st);
     if (fs == OG_OK) fs = fill_positions(e, 0, np, st);
@@ -1599,7 +1656,7 @@ og_status append_impl(og_engine* e, int si, const TopoCopy& grown, const double*
     OG_CUDA(v->grow(np, st));
   for (auto* v : {&e->fx, &e->fy, &e->fz, &e->born_sum}) OG_CUDA(v->grow(np, st));
   for (auto* v : {&e->atom_sys, &e->local_idx, &e->atom_valid, &e->lgb_class}) OG_CUDA(v->grow(np, st));
-  for (auto* v : {&e->pq, &e->lj, &e->gb}) OG_CUDA(v->grow(4 * static_cast<size_t>(np), st));
+  for (auto* v : {&e->pq, &e->lj, &e->gb, &e->bs}) OG_CUDA(v->grow(4 * static_cast<size_t>(np), st));
   OG_CUDA(e->origin.grow(e->n_tiles, st));
   const int a_first = sh.atom_begin + n_old;
   og_status s = fill_atoms(e, a_first / kTile * kTile, np, st);
@@ -2601,7 +2658,7 @@ og_status time_pass(og_engine* e, bool born, const ogk::PairLaunch& lc, int chun
   DVec<int32_t> jl, jl_cut, seg;
   DVec<ogk::CutBlock> cut;
   int n_work = 0, n_cut = 0;
-  og_status s = build_pass_list(e, born ? 0 : 1, ogk::pair_shape_tiles(lc.shape), chunk, &work, &n_work, &jl, &cut,
+  og_status s = build_pass_list(e, born ? 0 : 1, ogk::pair_shape_tiles(born, lc.shape), chunk, &work, &n_work, &jl, &cut,
                                 &n_cut, &jl_cut, &seg, st);
   if (s != OG_OK) return s;
   ogk::PairArgs a = e->pair_args();
@@ -2652,6 +2709,7 @@ og_status apply_launch(og_engine* e, const TuneEntry& t) {
   e->force_launch.shape = t.f[0];
   e->force_launch.persistent = t.f[1] != 0;
   e->chunk_f = t.f[2];
+  e->launch_set = true;
   OG_CUDA(cudaStreamSynchronize(e->stream));
   og_status s = build_pair_lists(e, e->stream);
   if (s != OG_OK) return s;
@@ -2712,6 +2770,13 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
     ogk::launch_born_finalize(e->atoms(), nullptr, 0, e->born_r.p, true, nullptr, e->stream);
     OG_CUDA(cudaStreamSynchronize(e->stream));
     const int chunks[3] = {8, 16, 32};
+    struct { int b, f; } untuned;  // default_launch's shapes
+    {
+      const auto keep = std::make_tuple(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f);
+      default_launch(e);
+      untuned = {e->born_launch.shape, e->force_launch.shape};
+      std::tie(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f) = keep;
+    }
     for (int pass = 0; pass < 2; ++pass) {
       double bt = 1e30;
       int bc[3] = {0, 0, 16};
@@ -2724,7 +2789,7 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
             lc.persistent = pers != 0;
             s = time_pass(e, pass == 0, lc, chunk, 3, &ms);
             if (s != OG_OK) return s;
-            if (shape == 0 && pers == 0 && chunk == 16) (pass == 0 ? b_def : f_def) = ms;
+            if (shape == (pass == 0 ? untuned.b : untuned.f) && pers == 0 && chunk == 16) (pass == 0 ? b_def : f_def) = ms;
             if (ms < bt) {
               bt = ms;
               bc[0] = shape;

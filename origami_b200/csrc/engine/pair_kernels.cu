@@ -24,11 +24,22 @@
 // accumulators; the i side accumulates FP32 per tile and FP64 across tiles.
 // Every sum therefore has a fixed order and results are bit-reproducible.
 //
-// Launch variants (PairConfig): W, the CTAs per SM the register budget is
-// sized for, and either one CTA per work item (the hardware assigns CTAs to
-// SMs as they free up) or a persistent grid of resident CTAs that take items
-// from an atomic queue.  The engine's autotuner times them on the actual
-// systems; every variant computes the same sums in the same order.
+// Launch variants (PairLaunch): how many i-tiles a CTA owns and how (the
+// split kernels: one, four warps sharing it; k_born and k_force: one per warp;
+// k_force_quad: four per warp), the CTAs per SM the register budget is sized
+// for, and either one CTA per work item (the hardware assigns CTAs to SMs as
+// they free up) or a persistent grid of resident CTAs that take items from an
+// atomic queue.  The engine picks by tile counts (default_launch) or its
+// autotuner times them on the actual systems; every variant computes the same
+// pair terms.
+//
+// Tile pairs are classed by the gap between their bounding spheres: distant
+// ones take shorter forms of the same sums (fewer series terms, the far GB
+// form without its exponential), with every pair's condition implied by the
+// gap.  64 x 4 694 atoms, all pairs, B200: Born 1.265 -> 0.668 ms (k_born, 64
+// registers, FMA pipe 62 % busy), force 1.105 -> 0.843 ms (k_force_quad, 162
+// registers, 12 warps per SM, FMA pipe 56 %); one 300-atom system 58 -> 5 and
+// 32 -> 5 us (split).
 //
 // Positions are FP32 offsets from a per-tile FP64 origin; the origin
 // difference of a tile pair is formed in FP64 once per tile, so |dx| keeps
@@ -64,6 +75,12 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float fast_rcp(float x) { return __fdividef(1.0f, x); }
+// 1 / x as the one special-function instruction (1 ulp; no range handling).
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
 // Reduce-scatter over the warp of four per-lane values v0..v3 (contributions
 // to four consecutive j atoms): afterwards every lane of the 8-lane group
@@ -197,6 +214,140 @@ __device__ __forceinline__ float2 born_pair(float dx, float dy, float dz, float 
   return on ? h : make_float2(0.0f, 0.0f);
 }
 
+// Lower bound (A) on the distance of any atom pair of two tiles, from their
+// bounding spheres; the margin covers the FP32 rounding.
+__device__ __forceinline__ float tile_gap(double4 oi, double4 oj) {
+  const float dx = static_cast<float>(oj.x - oi.x), dy = static_cast<float>(oj.y - oi.y),
+              dz = static_cast<float>(oj.z - oi.z);
+  const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+  return d * (1.0f - 1e-6f) - static_cast<float>(oi.w + oj.w) - 1e-3f;
+}
+
+// --------------------------------------------------- Born, distant tiles
+// A tile pair whose spheres leave a gap g takes its series length from the
+// largest possible x = s / r, s_max / g, instead of a vote per pair: 8 terms
+// for x < 1/4, 5 below 0.1135, 3 below 0.029 -- each drops less than 6e-9 of
+// the sum, as 8 terms at 1/4 do -- and needs no closed form, no root (only
+// u = 1 / r^2 enters: h_ij = -s_j^3 u^2 P(s_j^2 u)) and no overlap test.
+constexpr float kSeries5MaxX = 0.1135f, kSeries3MaxX = 0.0290f;
+
+// The gaps from which the series holds with 8, 5 and 3 terms.
+struct BornGaps {
+  float g8, g5, g3;
+};
+__device__ __forceinline__ BornGaps born_gaps(const PairArgs& a) {
+  return {fmaxf(a.s_max / kSeriesMaxX, a.s_max + a.rho_max), a.s_max / kSeries5MaxX, a.s_max / kSeries3MaxX};
+}
+
+template <int kTerms>
+__device__ __forceinline__ float2 descreen_poly2(float2 w) {
+  float2 p = bc(static_cast<float>(kTerms * (2 * kTerms - 1)) / (2 * kTerms + 1));
+#pragma unroll
+  for (int k = kTerms - 1; k >= 1; --k) p = fma2(p, w, bc(static_cast<float>(k * (2 * k - 1)) / (2 * k + 1)));
+  return p;
+}
+
+// Two pairs in the halves: adds -h_ij to *hi and returns -h_ji; (s2, s3) =
+// (s^2, s^3) of the two sides.
+template <int kTerms, bool kCut>
+__device__ __forceinline__ float2 born_far2(float2 dx, float2 dy, float2 dz, float2 si2, float2 si3, float2 sj2,
+                                            float2 sj3, float c2, float2* hi) {
+  const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+  float2 u = make_float2(rcp_approx(r2.x), rcp_approx(r2.y));
+  if (kCut) {
+    u.x = r2.x <= c2 ? u.x : 0.0f;
+    u.y = r2.y <= c2 ? u.y : 0.0f;
+  }
+  const float2 u2 = mul2(u, u);
+  *hi = fma2(mul2(u2, descreen_poly2<kTerms>(mul2(sj2, u))), sj3, *hi);
+  return mul2(mul2(u2, descreen_poly2<kTerms>(mul2(si2, u))), si3);
+}
+
+// The same with three terms, in powers of u with the series' coefficients per
+// atom (c.x = s^3 / 3, c.y = 6/5 s^5, c.z = 15/7 s^7, PairArgs::bs): six
+// packed operations after u^2 where the form above takes ten.  All but the
+// nearest tile pairs of an extended chain come here.
+struct Series3 {
+  float2 c0, c1, c2;
+};
+__device__ __forceinline__ float2 born_far3(float2 dx, float2 dy, float2 dz, const Series3& i, const Series3& j,
+                                            float2* hi) {
+  const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+  const float2 u = make_float2(rcp_approx(r2.x), rcp_approx(r2.y));
+  const float2 u2 = mul2(u, u);
+  *hi = fma2(u2, fma2(u, fma2(u, j.c2, j.c1), j.c0), *hi);
+  return mul2(u2, fma2(u, fma2(u, i.c2, i.c1), i.c0));
+}
+
+// One i atom per lane against j atoms k0, k0 + 4, .. of [k_begin, k_end) with
+// three terms; the columns at sp (x, y, z) and sb (the coefficients).
+template <class J>
+__device__ __forceinline__ float born_far_one3(const float* sp, const float* sb, int k_begin, int k_end, float xi,
+                                               float yi, float zi, float3 c, J j) {
+  const float2 nx = bc(-xi), ny = bc(-yi), nz = bc(-zi);
+  const Series3 i{bc(c.x), bc(c.y), bc(c.z)};
+  float2 hi = bc(0.0f);
+#pragma unroll 2
+  for (int k0 = k_begin; k0 < k_end; k0 += 4) {
+    const float4 X = *reinterpret_cast<const float4*>(&sp[k0]);
+    const float4 Y = *reinterpret_cast<const float4*>(&sp[32 + k0]);
+    const float4 Z = *reinterpret_cast<const float4*>(&sp[64 + k0]);
+    const float4 A = *reinterpret_cast<const float4*>(&sb[k0]);
+    const float4 B = *reinterpret_cast<const float4*>(&sb[32 + k0]);
+    const float4 C = *reinterpret_cast<const float4*>(&sb[64 + k0]);
+    const float2 a = born_far3(add2(make_float2(X.x, X.y), nx), add2(make_float2(Y.x, Y.y), ny),
+                               add2(make_float2(Z.x, Z.y), nz), i,
+                               Series3{make_float2(A.x, A.y), make_float2(B.x, B.y), make_float2(C.x, C.y)}, &hi);
+    const float2 b = born_far3(add2(make_float2(X.z, X.w), nx), add2(make_float2(Y.z, Y.w), ny),
+                               add2(make_float2(Z.z, Z.w), nz), i,
+                               Series3{make_float2(A.z, A.w), make_float2(B.z, B.w), make_float2(C.z, C.w)}, &hi);
+    j(k0, a.x, a.y, b.x, b.y);
+  }
+  return -(hi.x + hi.y);
+}
+
+// One i atom per lane against j atoms k0, k0 + 4, .. of [k_begin, k_end), two j
+// atoms per packed operation; the columns at sp (x, y, z) and sg (rho~, s~
+// from +64).  Returns the i side; j(k, v) receives the lane's four values for
+// the j atoms from k on, negated.
+template <int kTerms, bool kCut, class J>
+__device__ __forceinline__ float born_far_one(const float* sp, const float* sg, int k_begin, int k_end, float xi,
+                                              float yi, float zi, float s_i, float c2, J j) {
+  const float2 nx = bc(-xi), ny = bc(-yi), nz = bc(-zi), si2 = bc(s_i * s_i), si3 = bc(s_i * s_i * s_i);
+  float2 hi = bc(0.0f);
+#pragma unroll 2
+  for (int k0 = k_begin; k0 < k_end; k0 += 4) {
+    const float4 X = *reinterpret_cast<const float4*>(&sp[k0]);
+    const float4 Y = *reinterpret_cast<const float4*>(&sp[32 + k0]);
+    const float4 Z = *reinterpret_cast<const float4*>(&sp[64 + k0]);
+    const float4 S = *reinterpret_cast<const float4*>(&sg[96 + k0]);
+    const float2 sa = make_float2(S.x, S.y), sb = make_float2(S.z, S.w);
+    const float2 sa2 = mul2(sa, sa), sb2 = mul2(sb, sb);
+    const float2 a = born_far2<kTerms, kCut>(add2(make_float2(X.x, X.y), nx), add2(make_float2(Y.x, Y.y), ny),
+                                             add2(make_float2(Z.x, Z.y), nz), si2, si3, sa2, mul2(sa2, sa), c2, &hi);
+    const float2 b = born_far2<kTerms, kCut>(add2(make_float2(X.z, X.w), nx), add2(make_float2(Y.z, Y.w), ny),
+                                             add2(make_float2(Z.z, Z.w), nz), si2, si3, sb2, mul2(sb2, sb), c2, &hi);
+    j(k0, a.x, a.y, b.x, b.y);
+  }
+  return -(hi.x + hi.y);
+}
+// The series length by the gap; false for a gap the series does not hold for.
+template <class J>
+__device__ __forceinline__ bool born_far_tile(const BornGaps& gaps, float gap, const float* sp, const float* sg,
+                                              const float* sb, int k_begin, int k_end, float xi, float yi, float zi,
+                                              float s_i, float3 ci, float c2, float* hi, J j) {
+  if (gap < gaps.g8) return false;
+  if (c2 != INFINITY) {
+    *hi = gap >= gaps.g5 ? born_far_one<5, true>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j)
+                         : born_far_one<8, true>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j);
+  } else {
+    *hi = gap >= gaps.g3   ? born_far_one3(sp, sb, k_begin, k_end, xi, yi, zi, ci, j)
+          : gap >= gaps.g5 ? born_far_one<5, false>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j)
+                           : born_far_one<8, false>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j);
+  }
+  return true;
+}
+
 // The next work item of a CTA: its own (one CTA per item) or the queue's.
 template <bool kPersistent>
 __device__ __forceinline__ int next_item(const PairArgs& a, int* s_item, int prev) {
@@ -209,7 +360,7 @@ __device__ __forceinline__ int next_item(const PairArgs& a, int* s_item, int pre
 
 template <int W, int kMinBlocks, bool kPersistent>
 __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
-  __shared__ __align__(128) float s_buf[2][2][kStageFloats];          // columns of pq, gb
+  __shared__ __align__(128) float s_buf[2][3][kStageFloats];          // columns of pq, gb, bs
   __shared__ float s_part[W][1][kStageTiles * kTile];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_item;
@@ -221,6 +372,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
     fence_mbar_init();
   }
   __syncthreads();
+  const BornGaps gaps = born_gaps(a);
   uint32_t g = 0;  // stages this CTA has consumed
   for (int item = next_item<kPersistent>(a, &s_item, -1); item < a.n_work;
        item = next_item<kPersistent>(a, &s_item, item)) {
@@ -228,10 +380,10 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
   if (w.j_begin >= w.j_end) continue;  // chunk culled by the cutoff (block-uniform)
   const Stager st{a.jlist, w.j_begin, w.j_end, (w.j_end - w.j_begin + kStageTiles - 1) / kStageTiles, s_bar, g};
-  const float* src[2] = {a.pq, a.gb};
+  const float* src[3] = {a.pq, a.gb, a.bs};
   if (threadIdx.x == 0) {
-    if (st.n_stages > 0) st.issue<2>(0, s_buf, src);
-    if (st.n_stages > 1) st.issue<2>(1, s_buf, src);
+    if (st.n_stages > 0) st.issue<3>(0, s_buf, src);
+    if (st.n_stages > 1) st.issue<3>(1, s_buf, src);
   }
 
   const bool active = warp < w.n_i_tiles;
@@ -239,6 +391,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   const int i = it * kTile + lane;
   const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
   const float rho_i = a.gb[soa_index(i, 2)], s_i = a.gb[soa_index(i, 3)];
+  const float3 ci = make_float3(a.bs[soa_index(i, 0)], a.bs[soa_index(i, 1)], a.bs[soa_index(i, 2)]);
   const double4 oi = a.origin[it];
   const float c2 = a.born_c2;
   double acc = 0.0;
@@ -255,18 +408,25 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
     for (int t = 0; t < cnt; ++t) {
       const int jt = a.jlist[t0 + t];
       float* part = &s_part[warp][0][t * kTile];
-      if (!active || jt < it) {
+      const double4 oj = a.origin[jt];
+      if (!active || jt < it || (c2 != INFINITY && tile_gap(oi, oj) > a.born_cutoff)) {
         part[lane] = 0.0f;
         continue;
       }
-      const double4 oj = a.origin[jt];
       const float xi = px - static_cast<float>(oj.x - oi.x);
       const float yi = py - static_cast<float>(oj.y - oi.y);
       const float zi = pz - static_cast<float>(oj.z - oi.z);
       const float* sp = &s_buf[b][0][t * 128];
       const float* sg = &s_buf[b][1][t * 128];
       float hi = 0.0f;
-      if (jt == it) {
+      const bool series = born_far_tile(gaps, tile_gap(oi, oj), sp, sg, &s_buf[b][2][t * 128], 0, kTile, xi, yi, zi, s_i,
+                                        ci, c2, &hi,
+                                        [&](int k0, float v0, float v1, float v2, float v3) {
+                                          const float tot = reduce_scatter4(v0, v1, v2, v3, lane);
+                                          if ((lane & 7) == 0) part[k0 + (lane >> 3)] = -tot;
+                                        });
+      if (series) {
+      } else if (jt == it) {
         // Diagonal tile: every ordered pair from the i side.
 #pragma unroll 4
         for (int k = 0; k < kTile; ++k) {
@@ -295,7 +455,7 @@ OG_UNROLL(OG_BORN_UNROLL)
       acc += static_cast<double>(hi);
     }
     __syncthreads();  // every warp is done with buffer b and has written its j partials
-    if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<2>(s + 2, s_buf, src);
+    if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
     unsigned long long* dst[1] = {a.born_sum};
     flush_j<W, 1>(a, a.jlist, t0, cnt, s_part, dst, kBornScale);
   }
@@ -304,6 +464,91 @@ OG_UNROLL(OG_BORN_UNROLL)
     if (!isfinite(acc)) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
     add_fixed(a.born_sum + i, acc, kBornScale);
   }
+  }
+}
+
+// One i-tile per CTA, its four warps taking eight atoms of each j-tile: the
+// shape for engines of few tiles, where whole-tile work items leave most of
+// the chip idle and a tile pair's latency (about 1 500 cycles per group of
+// four j atoms in the closed form) is the pass's time; and with cutoffs, where
+// its list is culled per i-tile.  (Warps taking whole tile pairs of their own,
+// without the shared sums, were 0 to 50 % slower than the better of this and
+// k_born at every size tried.)
+constexpr int kSplitWarps = 4, kSplitJ = kTile / kSplitWarps;
+
+// The four warps' i-side sums of one component, in warp order.
+__device__ __forceinline__ double split_sum(const double (*s_acc)[kTile], int lane) {
+  double v = 0.0;
+#pragma unroll
+  for (int w = 0; w < kSplitWarps; ++w) v += s_acc[w][lane];
+  return v;
+}
+
+template <bool kPersistent>
+__global__ void __launch_bounds__(kSplitWarps * 32) k_born_split(PairArgs a) {
+  __shared__ double s_acc[kSplitWarps][kTile];
+  __shared__ int s_item;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float c2 = a.born_c2;
+  const BornGaps gaps = born_gaps(a);
+  for (int item = next_item<kPersistent>(a, &s_item, -1); item < a.n_work;
+       item = next_item<kPersistent>(a, &s_item, item)) {
+    PairWork w = a.work[item];
+    if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
+    if (w.j_begin >= w.j_end) continue;  // block-uniform
+    const int it = w.i_tile0, i = it * kTile + lane;
+    const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
+    const float rho_i = a.gb[soa_index(i, 2)], s_i = a.gb[soa_index(i, 3)];
+    const float3 ci = make_float3(a.bs[soa_index(i, 0)], a.bs[soa_index(i, 1)], a.bs[soa_index(i, 2)]);
+    const double4 oi = a.origin[it];
+    double acc = 0.0;
+    for (int p = w.j_begin; p < w.j_end; ++p) {
+      const int jt = a.jlist[p];
+      const double4 oj = a.origin[jt];
+      const bool diag = jt == it;
+      const float xi = px - static_cast<float>(oj.x - oi.x);
+      const float yi = py - static_cast<float>(oj.y - oi.y);
+      const float zi = pz - static_cast<float>(oj.z - oi.z);
+      float hi = 0.0f;
+      const float* sp = a.pq + static_cast<size_t>(jt) * 128;
+      const float* sg = a.gb + static_cast<size_t>(jt) * 128;
+      const float* sb = a.bs + static_cast<size_t>(jt) * 128;
+      auto add_j = [&](int k0, float v0, float v1, float v2, float v3) {
+        const float tot = reduce_scatter4(v0, v1, v2, v3, lane);
+        const int j = jt * kTile + k0 + (lane >> 3);
+        if ((lane & 7) == 0 && tot != 0.0f && a.atom_valid[j]) {
+          if (!isfinite(tot)) atomicOr(a.sys_nonfinite + a.atom_sys[j], 1);
+          add_fixed(a.born_sum + j, static_cast<double>(tot), kBornScale);
+        }
+      };
+      const int k_begin = warp * kSplitJ, k_end = k_begin + kSplitJ;
+      auto sub_j = [&](int k0, float v0, float v1, float v2, float v3) { add_j(k0, -v0, -v1, -v2, -v3); };
+      if (!born_far_tile(gaps, tile_gap(oi, oj), sp, sg, sb, k_begin, k_end, xi, yi, zi, s_i, ci, c2, &hi, sub_j)) {
+#pragma unroll 1
+        for (int k0 = k_begin; k0 < k_end; k0 += 4) {
+          const float4 X = *reinterpret_cast<const float4*>(sp + k0);
+          const float4 Y = *reinterpret_cast<const float4*>(sp + 32 + k0);
+          const float4 Z = *reinterpret_cast<const float4*>(sp + 64 + k0);
+          const float4 RH = *reinterpret_cast<const float4*>(sg + 64 + k0);
+          const float4 SR = *reinterpret_cast<const float4*>(sg + 96 + k0);
+          const float2 h0 = born_pair(X.x - xi, Y.x - yi, Z.x - zi, rho_i, s_i, RH.x, SR.x, c2);
+          const float2 h1 = born_pair(X.y - xi, Y.y - yi, Z.y - zi, rho_i, s_i, RH.y, SR.y, c2);
+          const float2 h2 = born_pair(X.z - xi, Y.z - yi, Z.z - zi, rho_i, s_i, RH.z, SR.z, c2);
+          const float2 h3 = born_pair(X.w - xi, Y.w - yi, Z.w - zi, rho_i, s_i, RH.w, SR.w, c2);
+          hi += (h0.x + h1.x) + (h2.x + h3.x);
+          if (!diag) add_j(k0, h0.y, h1.y, h2.y, h3.y);  // a diagonal tile's pairs are all seen from the i side
+        }
+      }
+      acc += static_cast<double>(hi);
+    }
+    s_acc[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && a.atom_valid[i]) {
+      const double v = split_sum(s_acc, lane);
+      if (!isfinite(v)) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
+      add_fixed(a.born_sum + i, v, kBornScale);
+    }
+    if (kPersistent) __syncthreads();  // s_acc is read before the next item writes it
   }
 }
 
@@ -318,13 +563,30 @@ struct IAtom2 {
   float2 R;            // Born radius
   float2 nexp;         // -log2(e) / (4 R_i)
   float2 nrc3;         // -1 / Rc^3
+  float2 cg;           // (gb_pref_kj - coul_kj) q_i
 };
+
+// One i atom in both halves (nx, ny, nz are set per j-tile).
+__device__ __forceinline__ IAtom2 i_atom(const PairArgs& a, int i) {
+  IAtom2 ia;
+  const float qi = a.pq[soa_index(i, 3)];
+  ia.rm = bc(a.lj[soa_index(i, 0)]);
+  ia.se = bc(a.lj_kj12 * a.lj[soa_index(i, 1)]);
+  ia.cq = bc(-a.coul_kj * qi);
+  ia.gq = bc(a.gb_pref_kj * qi);
+  ia.R = bc(a.gb[soa_index(i, 0)]);
+  ia.nexp = bc(-0.25f * kLog2e * a.gb[soa_index(i, 1)]);
+  ia.nrc3 = bc(-a.inv_rc3);
+  ia.cg = bc(a.far_kj * qi);
+  return ia;
+}
 
 // Separation d = x_j - x_i of two j atoms from the i atom, and r^2.
 struct Sep2 {
   float2 dx, dy, dz, r2;
 };
-__device__ __forceinline__ Sep2 sep2(float2 xj, float2 yj, float2 zj, const IAtom2& ia) {
+template <class I>
+__device__ __forceinline__ Sep2 sep2(float2 xj, float2 yj, float2 zj, const I& ia) {
   Sep2 s;
   s.dx = add2(xj, ia.nx);
   s.dy = add2(yj, ia.ny);
@@ -379,6 +641,81 @@ __device__ __forceinline__ float2 coeff2(const Sep2& s, float2 arg, float2 qj, f
   return c;
 }
 
+// Where a tile pair's spheres leave a gap g with g^2 > kFarGapSq R_i R_j for
+// the tiles' largest Born radii, every pair has the far GB form (kFarGb) and,
+// without cutoffs, Coulomb and GB share 1/r^3: one reciprocal square root and
+// thirteen packed operations per two pairs, no vote and no guard.
+// (arg < -30 in coeff2: r^2 log2(e) / (4 R_i R_j) > 30; a little above 120 ln 2)
+constexpr float kFarGapSq = 83.2f;
+__device__ __forceinline__ bool far_tiles(float gap, float ri_max, float rj_max) {
+  return gap > 0.0f && gap * gap > kFarGapSq * ri_max * rj_max;
+}
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// The coefficient of two such pairs; cg = (gb_pref - coul) q_i.
+template <class I>
+__device__ __forceinline__ float2 coeff_far2(float2 r2, float2 qj, float2 rmj, float2 sej, const I& ia) {
+  const float2 inv_r = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 inv_r2 = mul2(inv_r, inv_r);
+  const float2 rmin = add2(ia.rm, rmj);
+  const float2 ratio2 = mul2(mul2(rmin, rmin), inv_r2);
+  const float2 r6 = mul2(mul2(ratio2, ratio2), ratio2);
+  const float2 lj = mul2(mul2(ia.se, sej), mul2(r6, fma2(r6, bc(-1.0f), bc(1.0f))));
+  return mul2(inv_r2, fma2(mul2(ia.cg, qj), inv_r, lj));
+}
+
+// The pair forces c d of one i atom and four consecutive j atoms (a: the first
+// two, b: the others), the j columns at pq, lj, gb.
+struct Group4 {
+  float2 xa, ya, za, xb, yb, zb;
+};
+__device__ __forceinline__ Group4 force_far4(const float* pq, const float* lj, const IAtom2& ia) {
+  const float4 X = *reinterpret_cast<const float4*>(pq);
+  const float4 Y = *reinterpret_cast<const float4*>(pq + 32);
+  const float4 Z = *reinterpret_cast<const float4*>(pq + 64);
+  const float4 Q = *reinterpret_cast<const float4*>(pq + 96);
+  const float4 RM = *reinterpret_cast<const float4*>(lj);
+  const float4 SE = *reinterpret_cast<const float4*>(lj + 32);
+  const Sep2 sa = sep2(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), ia);
+  const Sep2 sb = sep2(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), ia);
+  const float2 ca = coeff_far2(sa.r2, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y), make_float2(SE.x, SE.y), ia);
+  const float2 cb = coeff_far2(sb.r2, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w), make_float2(SE.z, SE.w), ia);
+  return Group4{mul2(sa.dx, ca), mul2(sa.dy, ca), mul2(sa.dz, ca), mul2(sb.dx, cb), mul2(sb.dy, cb), mul2(sb.dz, cb)};
+}
+template <bool kAllPairs>
+__device__ __forceinline__ Group4 force_group4(const float* pq, const float* lj, const float* gb, const IAtom2& ia,
+                                               const PairArgs& a) {
+  const float4 X = *reinterpret_cast<const float4*>(pq);
+  const float4 Y = *reinterpret_cast<const float4*>(pq + 32);
+  const float4 Z = *reinterpret_cast<const float4*>(pq + 64);
+  const float4 Q = *reinterpret_cast<const float4*>(pq + 96);
+  const float4 RM = *reinterpret_cast<const float4*>(lj);
+  const float4 SE = *reinterpret_cast<const float4*>(lj + 32);
+  const float4 RB = *reinterpret_cast<const float4*>(gb);
+  const float4 IR = *reinterpret_cast<const float4*>(gb + 32);
+  const Sep2 sa = sep2(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), ia);
+  const Sep2 sb = sep2(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), ia);
+  const float2 arga = gb_arg2(sa, make_float2(IR.x, IR.y), ia), argb = gb_arg2(sb, make_float2(IR.z, IR.w), ia);
+  // the far GB form when every pair of the warp's group allows it
+  const bool far = __all_sync(0xffffffffu, fmaxf(fmaxf(arga.x, arga.y), fmaxf(argb.x, argb.y)) < -30.0f);
+  float2 ca, cb;
+  if (far) {
+    ca = coeff2<kAllPairs, true>(sa, arga, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y), make_float2(SE.x, SE.y),
+                                 make_float2(RB.x, RB.y), ia, a);
+    cb = coeff2<kAllPairs, true>(sb, argb, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w), make_float2(SE.z, SE.w),
+                                 make_float2(RB.z, RB.w), ia, a);
+  } else {
+    ca = coeff2<kAllPairs, false>(sa, arga, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y), make_float2(SE.x, SE.y),
+                                  make_float2(RB.x, RB.y), ia, a);
+    cb = coeff2<kAllPairs, false>(sb, argb, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w), make_float2(SE.z, SE.w),
+                                  make_float2(RB.z, RB.w), ia, a);
+  }
+  return Group4{mul2(sa.dx, ca), mul2(sa.dy, ca), mul2(sa.dz, ca), mul2(sb.dx, cb), mul2(sb.dy, cb), mul2(sb.dz, cb)};
+}
+
 template <bool kAllPairs, int W, int kMinBlocks, bool kPersistent>
 __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
   __shared__ __align__(128) float s_buf[2][3][kStageFloats];          // columns of pq, lj, gb
@@ -411,18 +748,8 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
   const int i = it * kTile + lane;
   const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
   const double4 oi = a.origin[it];
-  IAtom2 ia;
-  {
-    const float qi = a.pq[soa_index(i, 3)];
-    const float Ri = a.gb[soa_index(i, 0)], iRi = a.gb[soa_index(i, 1)];
-    ia.rm = bc(a.lj[soa_index(i, 0)]);
-    ia.se = bc(a.lj_kj12 * a.lj[soa_index(i, 1)]);
-    ia.cq = bc(-a.coul_kj * qi);
-    ia.gq = bc(a.gb_pref_kj * qi);
-    ia.R = bc(Ri);
-    ia.nexp = bc(-0.25f * kLog2e * iRi);
-    ia.nrc3 = bc(-a.inv_rc3);
-  }
+  IAtom2 ia = i_atom(a, i);
+  const float ri_max = kAllPairs ? warp_max(ia.R.x) : 0.0f;
   int mref = a.mask_begin[it];
   const int mend = a.mask_begin[it + 1];
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
@@ -444,13 +771,13 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
       float* jfx = &s_part[warp][0][t * kTile];
       float* jfy = &s_part[warp][1][t * kTile];
       float* jfz = &s_part[warp][2][t * kTile];
-      if (!(active && jt > it && !masked)) {
+      const double4 oj = a.origin[jt];
+      if (!(active && jt > it && !masked) || (!kAllPairs && tile_gap(oi, oj) > a.pair_cutoff)) {
         jfx[lane] = 0.0f;
         jfy[lane] = 0.0f;
         jfz[lane] = 0.0f;
         continue;
       }
-      const double4 oj = a.origin[jt];
       ia.nx = bc(-(px - static_cast<float>(oj.x - oi.x)));
       ia.ny = bc(-(py - static_cast<float>(oj.y - oi.y)));
       ia.nz = bc(-(pz - static_cast<float>(oj.z - oi.z)));
@@ -458,46 +785,26 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
       const float* sl = &s_buf[b][1][t * 128];
       const float* sg = &s_buf[b][2][t * 128];
       float2 fx = bc(0.0f), fy = bc(0.0f), fz = bc(0.0f);
-OG_UNROLL(OG_FORCE_UNROLL)
-      for (int k0 = 0; k0 < kTile; k0 += 4) {
-        const float4 X = *reinterpret_cast<const float4*>(&sp[k0]);
-        const float4 Y = *reinterpret_cast<const float4*>(&sp[32 + k0]);
-        const float4 Z = *reinterpret_cast<const float4*>(&sp[64 + k0]);
-        const float4 Q = *reinterpret_cast<const float4*>(&sp[96 + k0]);
-        const float4 RM = *reinterpret_cast<const float4*>(&sl[k0]);
-        const float4 SE = *reinterpret_cast<const float4*>(&sl[32 + k0]);
-        const float4 RB = *reinterpret_cast<const float4*>(&sg[k0]);
-        const float4 IR = *reinterpret_cast<const float4*>(&sg[32 + k0]);
-        const Sep2 sa = sep2(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), ia);
-        const Sep2 sb = sep2(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), ia);
-        const float2 arga = gb_arg2(sa, make_float2(IR.x, IR.y), ia), argb = gb_arg2(sb, make_float2(IR.z, IR.w), ia);
-        // the far GB form when every pair of the warp's group allows it
-        const bool far = __all_sync(0xffffffffu, fmaxf(fmaxf(arga.x, arga.y), fmaxf(argb.x, argb.y)) < -30.0f);
-        float2 ca, cb;
-        if (far) {
-          ca = coeff2<kAllPairs, true>(sa, arga, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y),
-                                       make_float2(SE.x, SE.y), make_float2(RB.x, RB.y), ia, a);
-          cb = coeff2<kAllPairs, true>(sb, argb, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w),
-                                       make_float2(SE.z, SE.w), make_float2(RB.z, RB.w), ia, a);
-        } else {
-          ca = coeff2<kAllPairs, false>(sa, arga, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y),
-                                        make_float2(SE.x, SE.y), make_float2(RB.x, RB.y), ia, a);
-          cb = coeff2<kAllPairs, false>(sb, argb, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w),
-                                        make_float2(SE.z, SE.w), make_float2(RB.z, RB.w), ia, a);
-        }
-        const float2 uxa = mul2(sa.dx, ca), uya = mul2(sa.dy, ca), uza = mul2(sa.dz, ca);
-        const float2 uxb = mul2(sb.dx, cb), uyb = mul2(sb.dy, cb), uzb = mul2(sb.dz, cb);
-        fx = add2(fx, add2(uxa, uxb));
-        fy = add2(fy, add2(uya, uyb));
-        fz = add2(fz, add2(uza, uzb));
-        const float tx = reduce_scatter4(uxa.x, uxa.y, uxb.x, uxb.y, lane);
-        const float ty = reduce_scatter4(uya.x, uya.y, uyb.x, uyb.y, lane);
-        const float tz = reduce_scatter4(uza.x, uza.y, uzb.x, uzb.y, lane);
+      auto add_group = [&](int k0, const Group4& u) {
+        fx = add2(fx, add2(u.xa, u.xb));
+        fy = add2(fy, add2(u.ya, u.yb));
+        fz = add2(fz, add2(u.za, u.zb));
+        const float tx = reduce_scatter4(u.xa.x, u.xa.y, u.xb.x, u.xb.y, lane);
+        const float ty = reduce_scatter4(u.ya.x, u.ya.y, u.yb.x, u.yb.y, lane);
+        const float tz = reduce_scatter4(u.za.x, u.za.y, u.zb.x, u.zb.y, lane);
         if ((lane & 7) == 0) {
           jfx[k0 + (lane >> 3)] = -tx;
           jfy[k0 + (lane >> 3)] = -ty;
           jfz[k0 + (lane >> 3)] = -tz;
         }
+      };
+      if (kAllPairs && far_tiles(tile_gap(oi, oj), ri_max, warp_max(sg[lane]))) {
+#pragma unroll 2
+        for (int k0 = 0; k0 < kTile; k0 += 4) add_group(k0, force_far4(sp + k0, sl + k0, ia));
+      } else {
+OG_UNROLL(OG_FORCE_UNROLL)
+        for (int k0 = 0; k0 < kTile; k0 += 4)
+          add_group(k0, force_group4<kAllPairs>(sp + k0, sl + k0, sg + k0, ia, a));
       }
       acc0 += static_cast<double>(fx.x + fx.y);
       acc1 += static_cast<double>(fy.x + fy.y);
@@ -518,30 +825,169 @@ OG_UNROLL(OG_FORCE_UNROLL)
   }
 }
 
-// ------------------------------------------------------ force, i pairs
-// The same pair terms with two i-tiles per warp: lane l holds atom l of the
-// block's tiles 2w and 2w + 1 in the two halves of every float2, so one
-// FP32x2 instruction evaluates a j atom against both, and the stage's j
-// columns are expanded in shared memory to (v, v) pairs to feed it.  A j
-// atom's contributions from the two i atoms are summed in the lane before
-// the warp reduce-scatter, which then serves eight pairs instead of four
-// (in k_force the reduce-scatter is about a third of all instructions).
-// Sums and their order per i atom and per j atom are as in k_force's
-// structure: FP32 per j-tile and 4-atom group, FP64 across tiles, warps
-// summed in a fixed order, fixed point at the end.
-// Four-warp blocks at up to four per SM stage six j-tiles at a time (four in
-// the other pair kernels): two block-wide barriers per stage, so a third
-// fewer per pair; eight-warp blocks keep four, within the 48 KB of static
-// shared memory, and so do five four-warp blocks per SM, within the SM's.
-template <int W, int kMinBlocks>
-constexpr int ip_stage_tiles() { return W <= 4 && kMinBlocks <= 4 ? 6 : kStageTiles; }
+// ------------------------------------------------------ force, four i-tiles
+// The same pair terms with four i-tiles per warp (one atom of each in every
+// lane, two per float2); the stage's j columns are expanded in shared memory
+// to (v, v) pairs to feed them.  For systems of many tiles: a distant j atom
+// costs one load of its columns and three reduce-scatters for 128 pairs, so
+// the packed pair arithmetic is the bound.  A j-tile that is not distant from
+// all four i-tiles goes through force_pair_tile, two i-tiles at a time.
+// Sums per i atom: FP32 per j-tile, FP64 across tiles; per j atom: the warp's
+// i atoms in FP32, warps in a fixed order, fixed point at the end.
+
+// The stage's j columns: x, y, z, q, Rmin/2, sqrt(eps), R, 1/R.
+constexpr int kForceCols = 8;
+
+struct ForceSum {
+  float2 x, y, z;
+};
+__device__ __forceinline__ float half_of(float2 v, int h) { return h ? v.y : v.x; }
+
+// What a lane keeps of its i atoms: the far form's data.  The general form's
+// are read again where a j-tile needs them (i_pair): 16 registers less in
+// the far loop.
+struct FarI2 {
+  float2 nx, ny, nz, rm, se, cg;
+};
+// The general form's data of atoms i and j in the halves.
+__device__ __forceinline__ IAtom2 i_pair(const PairArgs& a, int i, int j, const FarI2& f) {
+  IAtom2 ia;
+  ia.nx = f.nx;
+  ia.ny = f.ny;
+  ia.nz = f.nz;
+  ia.rm = f.rm;
+  ia.se = f.se;
+  ia.cg = f.cg;
+  const float2 qi = make_float2(a.pq[soa_index(i, 3)], a.pq[soa_index(j, 3)]);
+  ia.cq = mul2(bc(-a.coul_kj), qi);
+  ia.gq = mul2(bc(a.gb_pref_kj), qi);
+  ia.R = make_float2(a.gb[soa_index(i, 0)], a.gb[soa_index(j, 0)]);
+  ia.nexp = mul2(bc(-0.25f * kLog2e), make_float2(a.gb[soa_index(i, 1)], a.gb[soa_index(j, 1)]));
+  ia.nrc3 = bc(-a.inv_rc3);
+  return ia;
+}
+
+// Two i-tiles (the halves) against a j-tile, general form; va, vb: which of
+// them.  j totals are added to jfx, jfy, jfz (negated).
+template <bool kAllPairs>
+__device__ __forceinline__ void force_pair_tile(const float* dup, const IAtom2& ia, const PairArgs& a, bool va, bool vb,
+                                                float* jfx, float* jfy, float* jfz, int lane, ForceSum* f) {
+  const bool both = va && vb;
+#pragma unroll 1
+  for (int k0 = 0; k0 < kTile; k0 += 4) {
+    float tx[4], ty[4], tz[4];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float* d = dup + 2 * (k0 + 2 * p);  // two j atoms
+      const float4 X = *reinterpret_cast<const float4*>(d);
+      const float4 Y = *reinterpret_cast<const float4*>(d + 64);
+      const float4 Z = *reinterpret_cast<const float4*>(d + 128);
+      const float4 Q = *reinterpret_cast<const float4*>(d + 192);
+      const float4 RM = *reinterpret_cast<const float4*>(d + 256);
+      const float4 SE = *reinterpret_cast<const float4*>(d + 320);
+      const float4 RB = *reinterpret_cast<const float4*>(d + 384);
+      const float4 IR = *reinterpret_cast<const float4*>(d + 448);
+      const Sep2 s[2] = {sep2(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), ia),
+                         sep2(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), ia)};
+      const float2 q[2] = {make_float2(Q.x, Q.y), make_float2(Q.z, Q.w)};
+      const float2 rm[2] = {make_float2(RM.x, RM.y), make_float2(RM.z, RM.w)};
+      const float2 se[2] = {make_float2(SE.x, SE.y), make_float2(SE.z, SE.w)};
+      const float2 rb[2] = {make_float2(RB.x, RB.y), make_float2(RB.z, RB.w)};
+      const float2 arg[2] = {gb_arg2(s[0], make_float2(IR.x, IR.y), ia), gb_arg2(s[1], make_float2(IR.z, IR.w), ia)};
+      const bool far = __all_sync(0xffffffffu, fmaxf(fmaxf(arg[0].x, arg[0].y), fmaxf(arg[1].x, arg[1].y)) < -30.0f);
+      float2 c[2];
+      if (far) {
+        c[0] = coeff2<kAllPairs, true>(s[0], arg[0], q[0], rm[0], se[0], rb[0], ia, a);
+        c[1] = coeff2<kAllPairs, true>(s[1], arg[1], q[1], rm[1], se[1], rb[1], ia, a);
+      } else {
+        c[0] = coeff2<kAllPairs, false>(s[0], arg[0], q[0], rm[0], se[0], rb[0], ia, a);
+        c[1] = coeff2<kAllPairs, false>(s[1], arg[1], q[1], rm[1], se[1], rb[1], ia, a);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // one tile's pairs with this j-tile are near field or counted elsewhere
+        if (!both) c[h] = make_float2(va ? c[h].x : 0.0f, vb ? c[h].y : 0.0f);
+        const float2 ux = mul2(s[h].dx, c[h]), uy = mul2(s[h].dy, c[h]), uz = mul2(s[h].dz, c[h]);
+        f->x = add2(f->x, ux);
+        f->y = add2(f->y, uy);
+        f->z = add2(f->z, uz);
+        tx[2 * p + h] = ux.x + ux.y;
+        ty[2 * p + h] = uy.x + uy.y;
+        tz[2 * p + h] = uz.x + uz.y;
+      }
+    }
+    const float sx = reduce_scatter4(tx[0], tx[1], tx[2], tx[3], lane);
+    const float sy = reduce_scatter4(ty[0], ty[1], ty[2], ty[3], lane);
+    const float sz = reduce_scatter4(tz[0], tz[1], tz[2], tz[3], lane);
+    if ((lane & 7) == 0) {
+      jfx[k0 + (lane >> 3)] -= sx;
+      jfy[k0 + (lane >> 3)] -= sy;
+      jfz[k0 + (lane >> 3)] -= sz;
+    }
+  }
+}
+
+// Four i-tiles against a j-tile distant from all of them.
+__device__ __forceinline__ void force_far_four(const float* dup, const FarI2 (&ia)[2], float* jfx, float* jfy,
+                                               float* jfz, int lane, ForceSum (&f)[2]) {
+#pragma unroll 1
+  for (int k0 = 0; k0 < kTile; k0 += 4) {
+    float tx[4], ty[4], tz[4];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float* d = dup + 2 * (k0 + 2 * p);
+      const float4 X = *reinterpret_cast<const float4*>(d);
+      const float4 Y = *reinterpret_cast<const float4*>(d + 64);
+      const float4 Z = *reinterpret_cast<const float4*>(d + 128);
+      const float4 Q = *reinterpret_cast<const float4*>(d + 192);
+      const float4 RM = *reinterpret_cast<const float4*>(d + 256);
+      const float4 SE = *reinterpret_cast<const float4*>(d + 320);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float2 xj = h ? make_float2(X.z, X.w) : make_float2(X.x, X.y);
+        const float2 yj = h ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y);
+        const float2 zj = h ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y);
+        const float2 q = h ? make_float2(Q.z, Q.w) : make_float2(Q.x, Q.y);
+        const float2 rm = h ? make_float2(RM.z, RM.w) : make_float2(RM.x, RM.y);
+        const float2 se = h ? make_float2(SE.z, SE.w) : make_float2(SE.x, SE.y);
+        float2 ux, uy, uz;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const Sep2 s = sep2(xj, yj, zj, ia[t]);
+          const float2 c = coeff_far2(s.r2, q, rm, se, ia[t]);
+          f[t].x = fma2(s.dx, c, f[t].x);
+          f[t].y = fma2(s.dy, c, f[t].y);
+          f[t].z = fma2(s.dz, c, f[t].z);
+          ux = t ? fma2(s.dx, c, ux) : mul2(s.dx, c);
+          uy = t ? fma2(s.dy, c, uy) : mul2(s.dy, c);
+          uz = t ? fma2(s.dz, c, uz) : mul2(s.dz, c);
+        }
+        tx[2 * p + h] = ux.x + ux.y;
+        ty[2 * p + h] = uy.x + uy.y;
+        tz[2 * p + h] = uz.x + uz.y;
+      }
+    }
+    const float sx = reduce_scatter4(tx[0], tx[1], tx[2], tx[3], lane);
+    const float sy = reduce_scatter4(ty[0], ty[1], ty[2], ty[3], lane);
+    const float sz = reduce_scatter4(tz[0], tz[1], tz[2], tz[3], lane);
+    if ((lane & 7) == 0) {
+      jfx[k0 + (lane >> 3)] = -sx;
+      jfy[k0 + (lane >> 3)] = -sy;
+      jfz[k0 + (lane >> 3)] = -sz;
+    }
+  }
+}
 
 template <bool kAllPairs, int W, int kMinBlocks, bool kPersistent>
-__global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_ip(PairArgs a) {
-  constexpr int kST = ip_stage_tiles<W, kMinBlocks>();
-  __shared__ __align__(128) float s_buf[2][3][kST * 128];   // raw columns of pq, lj, gb (TMA)
-  __shared__ __align__(16) float s_dup[3][2 * kST * 128];    // the stage's columns, each value twice
-  __shared__ float s_part[W][3][kST * kTile];
+__global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_quad(PairArgs a) {
+  __shared__ __align__(128) float s_buf[2][3][kStageFloats];                  // raw columns of pq, lj, gb (TMA)
+  __shared__ __align__(16) float s_dup[kStageTiles][kForceCols * 2 * kTile];  // the stage's columns, each value twice
+  __shared__ float s_rmax[kStageTiles];
+  __shared__ int s_jt[2][kStageTiles];        // the stage's j-tiles and their spheres, loaded a stage ahead
+  __shared__ double4 s_oj[2][kStageTiles];
+  __shared__ double4 s_oi[W * 4];             // the block's i-tile spheres
+  __shared__ float s_part[W][3][kStageTiles * kTile];
+  __shared__ double s_acc[W][12][kTile];  // the lanes' sums over j-tiles, per i-tile and component
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_item;
 
@@ -558,38 +1004,60 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_ip(PairArgs a) {
   PairWork w = a.work[item];
   if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
   if (w.j_begin >= w.j_end) continue;  // chunk culled by the cutoff (block-uniform)
-  const StagerT<kST> st{a.jlist, w.j_begin, w.j_end, (w.j_end - w.j_begin + kST - 1) / kST, s_bar, g};
+  const Stager st{a.jlist, w.j_begin, w.j_end, (w.j_end - w.j_begin + kStageTiles - 1) / kStageTiles, s_bar, g};
   const float* src[3] = {a.pq, a.lj, a.gb};
   if (threadIdx.x == 0) {
     if (st.n_stages > 0) st.issue<3>(0, s_buf, src);
     if (st.n_stages > 1) st.issue<3>(1, s_buf, src);
   }
 
-  // tiles 2w (half x) and 2w + 1 (half y); a missing second tile repeats the
-  // first, with its pairs masked out
-  const bool act_a = 2 * warp < w.n_i_tiles, act_b = 2 * warp + 1 < w.n_i_tiles;
-  const int it_a = w.i_tile0 + (act_a ? 2 * warp : 0);
-  const int it_b = act_b ? it_a + 1 : it_a;
-  const int i_a = it_a * kTile + lane, i_b = it_b * kTile + lane;
-  const float2 px = make_float2(a.pq[soa_index(i_a, 0)], a.pq[soa_index(i_b, 0)]);
-  const float2 py = make_float2(a.pq[soa_index(i_a, 1)], a.pq[soa_index(i_b, 1)]);
-  const float2 pz = make_float2(a.pq[soa_index(i_a, 2)], a.pq[soa_index(i_b, 2)]);
-  IAtom2 ia;
-  {
-    const float2 qi = make_float2(a.pq[soa_index(i_a, 3)], a.pq[soa_index(i_b, 3)]);
-    const float2 Ri = make_float2(a.gb[soa_index(i_a, 0)], a.gb[soa_index(i_b, 0)]);
-    const float2 iRi = make_float2(a.gb[soa_index(i_a, 1)], a.gb[soa_index(i_b, 1)]);
-    ia.rm = make_float2(a.lj[soa_index(i_a, 0)], a.lj[soa_index(i_b, 0)]);
-    ia.se = mul2(bc(a.lj_kj12), make_float2(a.lj[soa_index(i_a, 1)], a.lj[soa_index(i_b, 1)]));
-    ia.cq = mul2(bc(-a.coul_kj), qi);
-    ia.gq = mul2(bc(a.gb_pref_kj), qi);
-    ia.R = Ri;
-    ia.nexp = mul2(bc(-0.25f * kLog2e), iRi);
-    ia.nrc3 = bc(-a.inv_rc3);
+  // tiles 4w .. 4w + 3 of the block; a missing one repeats the warp's first
+  // (or the block's), with its pairs masked out
+  const int n_own = max(0, min(4, w.n_i_tiles - 4 * warp));
+  const int it0 = w.i_tile0 + (n_own > 0 ? 4 * warp : 0);
+  FarI2 ia[2];
+  float2 px[2], py[2], pz[2];
+  float ri_max = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int ta = it0 + (2 * q < n_own ? 2 * q : 0), tb = it0 + (2 * q + 1 < n_own ? 2 * q + 1 : 0);
+    const int i = ta * kTile + lane, j = tb * kTile + lane;
+    px[q] = make_float2(a.pq[soa_index(i, 0)], a.pq[soa_index(j, 0)]);
+    py[q] = make_float2(a.pq[soa_index(i, 1)], a.pq[soa_index(j, 1)]);
+    pz[q] = make_float2(a.pq[soa_index(i, 2)], a.pq[soa_index(j, 2)]);
+    ia[q].rm = make_float2(a.lj[soa_index(i, 0)], a.lj[soa_index(j, 0)]);
+    ia[q].se = mul2(bc(a.lj_kj12), make_float2(a.lj[soa_index(i, 1)], a.lj[soa_index(j, 1)]));
+    ia[q].cg = mul2(bc(a.far_kj), make_float2(a.pq[soa_index(i, 3)], a.pq[soa_index(j, 3)]));
+    ri_max = fmaxf(ri_max, fmaxf(a.gb[soa_index(i, 0)], a.gb[soa_index(j, 0)]));
   }
-  int mref_a = a.mask_begin[it_a], mref_b = a.mask_begin[it_b];
-  const int mend_a = a.mask_begin[it_a + 1], mend_b = a.mask_begin[it_b + 1];
-  double acc_ax = 0.0, acc_ay = 0.0, acc_az = 0.0, acc_bx = 0.0, acc_by = 0.0, acc_bz = 0.0;
+  if (kAllPairs) ri_max = warp_max(ri_max);
+  // the next near-field j-tile of each own tile (refs are in j order)
+  int mref[4], mnext[4];
+  auto load_next = [&](int q, int from) {
+    const int end = a.mask_begin[it0 + q + 1];
+    mref[q] = from;
+    mnext[q] = from < end ? a.mask_refs[from].j_tile : 0x7fffffff;
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    mref[q] = 0;
+    mnext[q] = 0x7fffffff;
+    if (q < n_own) load_next(q, a.mask_begin[it0 + q]);
+  }
+  auto stage_info = [&](int st_index) {
+    const int t = static_cast<int>(threadIdx.x);
+    if (t < kStageTiles && w.j_begin + st_index * kStageTiles + t < w.j_end) {
+      const int jt = a.jlist[w.j_begin + st_index * kStageTiles + t], b = (g + st_index) & 1;
+      s_jt[b][t] = jt;
+      s_oj[b][t] = a.origin[jt];
+    }
+  };
+  __syncthreads();  // the previous item's info has been read
+  if (static_cast<int>(threadIdx.x) < w.n_i_tiles) s_oi[threadIdx.x] = a.origin[w.i_tile0 + threadIdx.x];
+  stage_info(0);
+  double(*acc)[kTile] = s_acc[warp];
+#pragma unroll
+  for (int q = 0; q < 12; ++q) acc[q][lane] = 0.0;
 
   for (int s = 0; s < st.n_stages; ++s) {
     const uint32_t gs = g + s;
@@ -599,120 +1067,167 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_ip(PairArgs a) {
       if (threadIdx.x == 0) atomicOr(a.error_flag, kStatusTimeout);
       return;
     }
-    const int t0 = w.j_begin + s * kST;
-    const int cnt = min(kST, w.j_end - t0);
-    // expand the stage's columns: value q of an array to entries 2q, 2q + 1
+    const int t0 = w.j_begin + s * kStageTiles;
+    const int cnt = min(kStageTiles, w.j_end - t0);
+    for (int q = threadIdx.x; q < cnt * kTile; q += W * 32) {  // one tile per warp and trip
+      const int t = q / kTile, l = q % kTile;
+      const float* p = &s_buf[b][0][t * 128 + l];
+      const float* pl = &s_buf[b][1][t * 128 + l];
+      const float* pg = &s_buf[b][2][t * 128 + l];
+      const float v[kForceCols] = {p[0], p[32], p[64], p[96], pl[0], pl[32], pg[0], pg[32]};
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      for (int q = threadIdx.x; q < cnt * 128; q += W * 32) {
-        const float v = s_buf[b][c][q];
-        *reinterpret_cast<float2*>(&s_dup[c][2 * q]) = make_float2(v, v);
+      for (int c = 0; c < kForceCols; ++c)
+        *reinterpret_cast<float2*>(&s_dup[t][64 * c + 2 * l]) = make_float2(v[c], v[c]);
+      if (kAllPairs) {
+        const float rmax = warp_max(v[6]);
+        if (l == 0) s_rmax[t] = rmax;
       }
+    }
     __syncthreads();  // s_dup is complete and raw buffer b is free
     if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
+    if (s + 1 < st.n_stages) stage_info(s + 1);
     for (int t = 0; t < cnt; ++t) {
-      const int jt = a.jlist[t0 + t];
-      while (mref_a < mend_a && a.mask_refs[mref_a].j_tile < jt) ++mref_a;
-      while (mref_b < mend_b && a.mask_refs[mref_b].j_tile < jt) ++mref_b;
-      const bool va = act_a && jt > it_a && !(mref_a < mend_a && a.mask_refs[mref_a].j_tile == jt);
-      const bool vb = act_b && jt > it_b && !(mref_b < mend_b && a.mask_refs[mref_b].j_tile == jt);
+      const int jt = s_jt[b][t];
+      const double4 oj = s_oj[b][t];
+      unsigned on = 0;  // own tiles that meet this j-tile here
+      float gap = INFINITY;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        while (mnext[q] < jt) load_next(q, mref[q] + 1);
+        const double4 oi = s_oi[it0 - w.i_tile0 + (q < n_own ? q : 0)];
+        const float gq = tile_gap(oi, oj);
+        if (q < n_own && jt > it0 + q && mnext[q] != jt && (kAllPairs || gq <= a.pair_cutoff)) {
+          on |= 1u << q;
+          gap = fminf(gap, gq);
+        }
+        const float ox = static_cast<float>(oj.x - oi.x), oy = static_cast<float>(oj.y - oi.y),
+                    oz = static_cast<float>(oj.z - oi.z);
+        if (q & 1) {
+          ia[q / 2].nx.y = ox - px[q / 2].y;
+          ia[q / 2].ny.y = oy - py[q / 2].y;
+          ia[q / 2].nz.y = oz - pz[q / 2].y;
+        } else {
+          ia[q / 2].nx.x = ox - px[q / 2].x;
+          ia[q / 2].ny.x = oy - py[q / 2].x;
+          ia[q / 2].nz.x = oz - pz[q / 2].x;
+        }
+      }
       float* jfx = &s_part[warp][0][t * kTile];
       float* jfy = &s_part[warp][1][t * kTile];
       float* jfz = &s_part[warp][2][t * kTile];
-      if (!(va || vb)) {
+      ForceSum f[2] = {{bc(0.0f), bc(0.0f), bc(0.0f)}, {bc(0.0f), bc(0.0f), bc(0.0f)}};
+      if (kAllPairs && on == 0xFu && far_tiles(gap, ri_max, s_rmax[t])) {
+        force_far_four(s_dup[t], ia, jfx, jfy, jfz, lane, f);
+      } else {
         jfx[lane] = 0.0f;
         jfy[lane] = 0.0f;
         jfz[lane] = 0.0f;
-        continue;
+        if (on == 0u) continue;
+        __syncwarp();
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q) {
+          const bool va = (on >> (2 * q)) & 1u, vb = (on >> (2 * q)) & 2u;
+          if (!(va || vb)) continue;
+          const int ta = it0 + (2 * q < n_own ? 2 * q : 0), tb = it0 + (2 * q + 1 < n_own ? 2 * q + 1 : 0);
+          const IAtom2 gi = i_pair(a, ta * kTile + lane, tb * kTile + lane, q ? ia[1] : ia[0]);
+          ForceSum fq{bc(0.0f), bc(0.0f), bc(0.0f)};
+          force_pair_tile<kAllPairs>(s_dup[t], gi, a, va, vb, jfx, jfy, jfz, lane, &fq);
+          if (q) f[1] = fq;
+          else f[0] = fq;
+        }
       }
-      const bool both = va && vb;
-      const double4 oj = a.origin[jt], oa = a.origin[it_a], ob = a.origin[it_b];
-      ia.nx = make_float2(-(px.x - static_cast<float>(oj.x - oa.x)), -(px.y - static_cast<float>(oj.x - ob.x)));
-      ia.ny = make_float2(-(py.x - static_cast<float>(oj.y - oa.y)), -(py.y - static_cast<float>(oj.y - ob.y)));
-      ia.nz = make_float2(-(pz.x - static_cast<float>(oj.z - oa.z)), -(pz.y - static_cast<float>(oj.z - ob.z)));
-      const float* dp = &s_dup[0][t * 256];
-      const float* dl = &s_dup[1][t * 256];
-      const float* dg = &s_dup[2][t * 256];
-      float2 fx = bc(0.0f), fy = bc(0.0f), fz = bc(0.0f);
-      for (int k0 = 0; k0 < kTile; k0 += 4) {
-        float tjx[4], tjy[4], tjz[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k2 = 2 * (k0 + 2 * h);  // two j atoms: entries k2 .. k2 + 3
-          const float4 X = *reinterpret_cast<const float4*>(&dp[k2]);
-          const float4 Y = *reinterpret_cast<const float4*>(&dp[64 + k2]);
-          const float4 Z = *reinterpret_cast<const float4*>(&dp[128 + k2]);
-          const float4 Q = *reinterpret_cast<const float4*>(&dp[192 + k2]);
-          const float4 RM = *reinterpret_cast<const float4*>(&dl[k2]);
-          const float4 SE = *reinterpret_cast<const float4*>(&dl[64 + k2]);
-          const float4 RB = *reinterpret_cast<const float4*>(&dg[k2]);
-          const float4 IR = *reinterpret_cast<const float4*>(&dg[64 + k2]);
-          const Sep2 s0 = sep2(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), ia);
-          const Sep2 s1 = sep2(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), ia);
-          const float2 arg0 = gb_arg2(s0, make_float2(IR.x, IR.y), ia);
-          const float2 arg1 = gb_arg2(s1, make_float2(IR.z, IR.w), ia);
-          const bool far = __all_sync(0xffffffffu, fmaxf(fmaxf(arg0.x, arg0.y), fmaxf(arg1.x, arg1.y)) < -30.0f);
-          float2 c0, c1;
-          if (far) {
-            c0 = coeff2<kAllPairs, true>(s0, arg0, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y),
-                                         make_float2(SE.x, SE.y), make_float2(RB.x, RB.y), ia, a);
-            c1 = coeff2<kAllPairs, true>(s1, arg1, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w),
-                                         make_float2(SE.z, SE.w), make_float2(RB.z, RB.w), ia, a);
-          } else {
-            c0 = coeff2<kAllPairs, false>(s0, arg0, make_float2(Q.x, Q.y), make_float2(RM.x, RM.y),
-                                          make_float2(SE.x, SE.y), make_float2(RB.x, RB.y), ia, a);
-            c1 = coeff2<kAllPairs, false>(s1, arg1, make_float2(Q.z, Q.w), make_float2(RM.z, RM.w),
-                                          make_float2(SE.z, SE.w), make_float2(RB.z, RB.w), ia, a);
-          }
-          if (!both) {  // one tile's pairs with this j-tile are near field or counted elsewhere
-            c0 = make_float2(va ? c0.x : 0.0f, vb ? c0.y : 0.0f);
-            c1 = make_float2(va ? c1.x : 0.0f, vb ? c1.y : 0.0f);
-          }
-          const float2 ux0 = mul2(s0.dx, c0), uy0 = mul2(s0.dy, c0), uz0 = mul2(s0.dz, c0);
-          const float2 ux1 = mul2(s1.dx, c1), uy1 = mul2(s1.dy, c1), uz1 = mul2(s1.dz, c1);
-          fx = add2(fx, add2(ux0, ux1));
-          fy = add2(fy, add2(uy0, uy1));
-          fz = add2(fz, add2(uz0, uz1));
-          tjx[2 * h] = ux0.x + ux0.y;
-          tjy[2 * h] = uy0.x + uy0.y;
-          tjz[2 * h] = uz0.x + uz0.y;
-          tjx[2 * h + 1] = ux1.x + ux1.y;
-          tjy[2 * h + 1] = uy1.x + uy1.y;
-          tjz[2 * h + 1] = uz1.x + uz1.y;
-        }
-        const float tx = reduce_scatter4(tjx[0], tjx[1], tjx[2], tjx[3], lane);
-        const float ty = reduce_scatter4(tjy[0], tjy[1], tjy[2], tjy[3], lane);
-        const float tz = reduce_scatter4(tjz[0], tjz[1], tjz[2], tjz[3], lane);
-        if ((lane & 7) == 0) {
-          jfx[k0 + (lane >> 3)] = -tx;
-          jfy[k0 + (lane >> 3)] = -ty;
-          jfz[k0 + (lane >> 3)] = -tz;
-        }
+      for (int q = 0; q < 4; ++q) {
+        acc[3 * q][lane] += static_cast<double>(half_of(f[q / 2].x, q & 1));
+        acc[3 * q + 1][lane] += static_cast<double>(half_of(f[q / 2].y, q & 1));
+        acc[3 * q + 2][lane] += static_cast<double>(half_of(f[q / 2].z, q & 1));
       }
-      acc_ax += static_cast<double>(fx.x);
-      acc_ay += static_cast<double>(fy.x);
-      acc_az += static_cast<double>(fz.x);
-      acc_bx += static_cast<double>(fx.y);
-      acc_by += static_cast<double>(fy.y);
-      acc_bz += static_cast<double>(fz.y);
     }
     __syncthreads();  // every warp is done with s_dup and has written its j partials
     unsigned long long* dst[3] = {a.fx, a.fy, a.fz};
-    flush_j<W, 3, kST>(a, a.jlist, t0, cnt, s_part, dst, kForceScale);
+    flush_j<W, 3>(a, a.jlist, t0, cnt, s_part, dst, kForceScale);
   }
   g += st.n_stages;
-  if (act_a && a.atom_valid[i_a]) {
-    if (!(isfinite(acc_ax) && isfinite(acc_ay) && isfinite(acc_az))) atomicOr(a.sys_nonfinite + a.atom_sys[i_a], 1);
-    add_fixed(a.fx + i_a, acc_ax, kForceScale);
-    add_fixed(a.fy + i_a, acc_ay, kForceScale);
-    add_fixed(a.fz + i_a, acc_az, kForceScale);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = (it0 + q) * kTile + lane;
+    if (q < n_own && a.atom_valid[i]) {
+      const double vx = acc[3 * q][lane], vy = acc[3 * q + 1][lane], vz = acc[3 * q + 2][lane];
+      if (!(isfinite(vx) && isfinite(vy) && isfinite(vz))) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
+      add_fixed(a.fx + i, vx, kForceScale);
+      add_fixed(a.fy + i, vy, kForceScale);
+      add_fixed(a.fz + i, vz, kForceScale);
+    }
   }
-  if (act_b && a.atom_valid[i_b]) {
-    if (!(isfinite(acc_bx) && isfinite(acc_by) && isfinite(acc_bz))) atomicOr(a.sys_nonfinite + a.atom_sys[i_b], 1);
-    add_fixed(a.fx + i_b, acc_bx, kForceScale);
-    add_fixed(a.fy + i_b, acc_by, kForceScale);
-    add_fixed(a.fz + i_b, acc_bz, kForceScale);
   }
+}
+
+// The force pass of k_born_split's shape.
+template <bool kAllPairs, bool kPersistent>
+__global__ void __launch_bounds__(kSplitWarps * 32) k_force_split(PairArgs a) {
+  __shared__ double s_acc[3][kSplitWarps][kTile];
+  __shared__ int s_item;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int item = next_item<kPersistent>(a, &s_item, -1); item < a.n_work;
+       item = next_item<kPersistent>(a, &s_item, item)) {
+    PairWork w = a.work[item];
+    if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
+    if (w.j_begin >= w.j_end) continue;  // block-uniform
+    const int it = w.i_tile0, i = it * kTile + lane;
+    const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
+    const double4 oi = a.origin[it];
+    IAtom2 ia = i_atom(a, i);
+    const float ri_max = kAllPairs ? warp_max(ia.R.x) : 0.0f;
+    int mref = a.mask_begin[it];
+    const int mend = a.mask_begin[it + 1];
+    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
+    for (int p = w.j_begin; p < w.j_end; ++p) {
+      const int jt = a.jlist[p];
+      while (mref < mend && a.mask_refs[mref].j_tile < jt) ++mref;
+      if (jt <= it || (mref < mend && a.mask_refs[mref].j_tile == jt)) continue;  // near field or counted elsewhere
+      const double4 oj = a.origin[jt];
+      const float gap = tile_gap(oi, oj);
+      if (!kAllPairs && gap > a.pair_cutoff) continue;
+      const size_t base = static_cast<size_t>(jt) * 128;
+      const bool far = kAllPairs && far_tiles(gap, ri_max, warp_max(a.gb[base + lane]));
+      ia.nx = bc(-(px - static_cast<float>(oj.x - oi.x)));
+      ia.ny = bc(-(py - static_cast<float>(oj.y - oi.y)));
+      ia.nz = bc(-(pz - static_cast<float>(oj.z - oi.z)));
+      float2 fx = bc(0.0f), fy = bc(0.0f), fz = bc(0.0f);
+#pragma unroll
+      for (int q = 0; q < kSplitJ; q += 4) {
+        const int k0 = warp * kSplitJ + q;
+        const Group4 u = far ? force_far4(a.pq + base + k0, a.lj + base + k0, ia)
+                             : force_group4<kAllPairs>(a.pq + base + k0, a.lj + base + k0, a.gb + base + k0, ia, a);
+        fx = add2(fx, add2(u.xa, u.xb));
+        fy = add2(fy, add2(u.ya, u.yb));
+        fz = add2(fz, add2(u.za, u.zb));
+        const float t[3] = {reduce_scatter4(u.xa.x, u.xa.y, u.xb.x, u.xb.y, lane),
+                            reduce_scatter4(u.ya.x, u.ya.y, u.yb.x, u.yb.y, lane),
+                            reduce_scatter4(u.za.x, u.za.y, u.zb.x, u.zb.y, lane)};
+        const int j = jt * kTile + k0 + (lane >> 3);
+        if ((lane & 7) == 0 && a.atom_valid[j]) {
+          if (!(isfinite(t[0]) && isfinite(t[1]) && isfinite(t[2]))) atomicOr(a.sys_nonfinite + a.atom_sys[j], 1);
+          add_fixed(a.fx + j, -static_cast<double>(t[0]), kForceScale);
+          add_fixed(a.fy + j, -static_cast<double>(t[1]), kForceScale);
+          add_fixed(a.fz + j, -static_cast<double>(t[2]), kForceScale);
+        }
+      }
+      acc0 += static_cast<double>(fx.x + fx.y);
+      acc1 += static_cast<double>(fy.x + fy.y);
+      acc2 += static_cast<double>(fz.x + fz.y);
+    }
+    s_acc[0][warp][lane] = acc0;
+    s_acc[1][warp][lane] = acc1;
+    s_acc[2][warp][lane] = acc2;
+    __syncthreads();
+    if (warp < 3 && a.atom_valid[i]) {
+      unsigned long long* dst = warp == 0 ? a.fx : warp == 1 ? a.fy : a.fz;
+      const double v = split_sum(s_acc[warp], lane);
+      if (!isfinite(v)) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
+      add_fixed(dst + i, v, kForceScale);
+    }
+    if (kPersistent) __syncthreads();  // s_acc is read before the next item writes it
   }
 }
 
@@ -775,73 +1290,52 @@ int persistent_grid(K kernel, int threads, int n_work) {
   return std::max(1, std::min(n_work, std::max(per_sm, 1) * std::max(n_sm, 1)));
 }
 
-template <int W, int MB, bool P>
-void born_variant(const PairArgs& a, cudaStream_t s) {
-  auto k = k_born<W, MB, P>;
+template <bool P, class K>
+void launch_items(K kernel, int threads, const PairArgs& a, cudaStream_t s) {
   if (P) {
     cudaMemsetAsync(a.queue, 0, sizeof(int32_t), s);
-    k<<<persistent_grid(k, W * 32, a.n_work), W * 32, 0, s>>>(a);
+    kernel<<<persistent_grid(kernel, threads, a.n_work), threads, 0, s>>>(a);
   } else {
-    k<<<a.n_work, W * 32, 0, s>>>(a);
-  }
-}
-
-template <bool AP, int W, int MB, bool P>
-void force_variant(const PairArgs& a, cudaStream_t s) {
-  auto k = k_force<AP, W, MB, P>;
-  if (P) {
-    cudaMemsetAsync(a.queue, 0, sizeof(int32_t), s);
-    k<<<persistent_grid(k, W * 32, a.n_work), W * 32, 0, s>>>(a);
-  } else {
-    k<<<a.n_work, W * 32, 0, s>>>(a);
-  }
-}
-
-template <bool AP, int W, int MB, bool P>
-void force_ip_variant(const PairArgs& a, cudaStream_t s) {
-  auto k = k_force_ip<AP, W, MB, P>;
-  if (P) {
-    cudaMemsetAsync(a.queue, 0, sizeof(int32_t), s);
-    k<<<persistent_grid(k, W * 32, a.n_work), W * 32, 0, s>>>(a);
-  } else {
-    k<<<a.n_work, W * 32, 0, s>>>(a);
+    kernel<<<a.n_work, threads, 0, s>>>(a);
   }
 }
 
 template <bool AP, bool P>
 void force_shape(const PairArgs& a, int shape, cudaStream_t s) {
   switch (shape) {
-    case 1: force_variant<AP, 4, 4, P>(a, s); break;
-    case 2: force_variant<AP, 8, 3, P>(a, s); break;
-    case 3: force_ip_variant<AP, 8, 2, P>(a, s); break;
-    case 4: force_ip_variant<AP, 4, 4, P>(a, s); break;
-    case 5: force_ip_variant<AP, 4, 5, P>(a, s); break;
-    case 6: force_ip_variant<AP, 4, 6, P>(a, s); break;
-    default: force_variant<AP, 8, 2, P>(a, s); break;
+    case 1: launch_items<P>(k_force<AP, 4, 4, P>, 4 * 32, a, s); break;
+    case 2: launch_items<P>(k_force_quad<AP, 4, 3, P>, 4 * 32, a, s); break;
+    case 3: launch_items<P>(k_force_quad<AP, 4, 4, P>, 4 * 32, a, s); break;
+    case 4: launch_items<P>(k_force_quad<AP, 2, 6, P>, 2 * 32, a, s); break;
+    case 5: launch_items<P>(k_force_quad<AP, 2, 7, P>, 2 * 32, a, s); break;
+    case 6: launch_items<P>(k_force_quad<AP, 1, 14, P>, 32, a, s); break;
+    default: launch_items<P>(k_force_split<AP, P>, kSplitWarps * 32, a, s); break;
+  }
+}
+
+template <bool P>
+void born_shape(const PairArgs& a, int shape, cudaStream_t s) {
+  switch (shape) {
+    case 1: launch_items<P>(k_born<4, 8, P>, 4 * 32, a, s); break;
+    case 2: launch_items<P>(k_born<8, 4, P>, 8 * 32, a, s); break;
+    default: launch_items<P>(k_born_split<P>, kSplitWarps * 32, a, s); break;
   }
 }
 
 }  // namespace
 
-int pair_shape_tiles(int shape) {
-  switch (shape) {
-    case 1: return 4;
-    case 3: return 16;
-    default: return 8;
-  }
+int pair_shape_tiles(bool born, int shape) {
+  if (shape == 0) return 1;
+  if (shape == 1) return 4;
+  if (born) return 8;
+  return shape <= 3 ? 16 : shape <= 5 ? 8 : 4;
 }
 
 void launch_born_pass(const PairArgs& a, const PairLaunch& c, cudaStream_t s) {
   if (a.n_work <= 0) return;
   if (c.persistent && !a.queue) return;
-  switch (c.shape * 2 + (c.persistent ? 1 : 0)) {
-    case 2: born_variant<4, 8, false>(a, s); break;
-    case 3: born_variant<4, 8, true>(a, s); break;
-    case 4: born_variant<8, 3, false>(a, s); break;
-    case 5: born_variant<8, 3, true>(a, s); break;
-    case 1: born_variant<8, 4, true>(a, s); break;
-    default: born_variant<8, 4, false>(a, s); break;
-  }
+  if (c.persistent) born_shape<true>(a, c.shape, s);
+  else born_shape<false>(a, c.shape, s);
 }
 
 void launch_force_pass(const PairArgs& a, const PairLaunch& c, cudaStream_t s) {

@@ -32,6 +32,7 @@ struct PairArgs {
   const float* pq;    // columns x_rel, y_rel, z_rel (A, from the tile origin), charge (e)
   const float* lj;    // columns rmin_half, sqrt(eps), rmin_half_14, sqrt(eps_14)   (kcal/mol)
   const float* gb;    // columns R_born, 1/R_born, rho_tilde, s*rho_tilde
+  const float* bs;    // with s = s*rho_tilde: columns s^3 / 3, 6/5 s^5, 15/7 s^7, 0
   const double4* origin;  // per tile
   const int32_t* atom_valid;  // 1 for real atoms
   // work
@@ -52,6 +53,9 @@ struct PairArgs {
   unsigned long long* born_sum;
   // cutoffs squared (INFINITY = none) and constants
   float nb_c2, gb_c2, born_c2;
+  float pair_cutoff, born_cutoff;  // A: the larger of the force pass's two, the Born pass's
+  float s_max, rho_max;            // largest s*rho_tilde and rho_tilde of any atom
+  float far_kj;                    // gb_pref_kj - coul_kj
   float inv_rc3;     // 1/Rc^3 of the reaction field (0 without cutoff)
   float coul_kj;     // 332.0637 * 4.184
   float lj_kj12;     // 12 * 4.184
@@ -88,20 +92,20 @@ struct CutBlock {
 void launch_cut_lists(const CutBlock* blocks, int32_t n_blocks, const int32_t* jlist_all, const double4* origin,
                       double cutoff, int32_t* jlist_out, int32_t* seg_end, cudaStream_t s);
 
-// How a pair pass is launched.  shape: 0 = 8 i-tiles per CTA (256 atoms)
-// at the default occupancy target (Born 4 CTAs/SM, force 2), 1 = 4 i-tiles
-// per CTA (128 atoms) at twice the CTAs, 2 = 8 i-tiles at 3 CTAs/SM; force
-// pass only: 3 = two i-tiles per warp (k_force_ip), 8 warps, 16 i-tiles per
-// CTA at 2 CTAs/SM, 4 = the same with 4 warps (8 i-tiles) at 4 CTAs/SM, 5 =
-// 4 warps at 5 CTAs/SM (96 registers), 6 = at 6 CTAs/SM (80 registers);
+// How a pair pass is launched.  shape:
+//   0 = one i-tile per CTA, the four warps splitting each j-tile (few tiles);
+//   1 = four i-tiles per CTA, one per warp;
+//   Born pass: 2 = eight i-tiles per CTA, one per warp;
+//   force pass: 2 to 6 = four i-tiles per warp (many tiles): 2, 3 sixteen per
+//       CTA at 3 and 4 CTAs per SM, 4, 5 eight at 6 and 7, 6 four at 14;
 // persistent: resident CTAs taking items from PairArgs::queue instead of
 // one CTA per item.  The work list must be built for
-// pair_shape_tiles(shape) i-tiles per item.
+// pair_shape_tiles i-tiles per item.
 struct PairLaunch {
   int shape = 0;
   bool persistent = false;
 };
-int pair_shape_tiles(int shape);
+int pair_shape_tiles(bool born, int shape);
 constexpr int kBornShapes = 3;   // shapes 0..2
 constexpr int kForceShapes = 7;  // shapes 0..6
 
