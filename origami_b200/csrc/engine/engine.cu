@@ -604,7 +604,7 @@ struct og_engine {
     }
     {
       Timer t(this, "near_force64");
-      ogk::launch_near_force64(pa, near.p, n_near, stream);
+      ogk::launch_near_force64(pa, near.p, n_near, n_sm, stream);
     }
     {
       Timer t(this, "bonded");

@@ -22,40 +22,59 @@ namespace ogk {
 // pair steps 1..16 cover every pair once (step 16 on the lower half-warp
 // only).  The pair coefficient is symmetric in i and j, so the j-side force
 // is exactly the negated i-side term.
+//
+// kSplit = 4 gives a tile pair to the four warps of a block, each taking
+// every fourth step, their sums added in warp order: a warp's 32 steps are a
+// chain of FP64 latency (about 20 us), which is the kernel's time when there
+// are too few tile pairs to fill the SMs.
 namespace {
 
 constexpr int kNearWarps = 4;
+// Tile pairs per SM up to which a block takes one.
+#ifndef OG_NEAR_SPLIT
+#define OG_NEAR_SPLIT 16
+#endif
+constexpr int kNearSplitPerSm = OG_NEAR_SPLIT;
 
 // The j-tile staged per warp: eps as its square root (the LJ mixing rule
 // sqrt(eps_i eps_j) as a product) and the Born radius with its inverse.
 struct NearTile {
   double x[kTile], y[kTile], z[kTile], q[kTile], r[kTile], ir[kTile];
   double rmin[kTile], seps[kTile], rmin14[kTile], seps14[kTile];
-  double fx[kTile], fy[kTile], fz[kTile];
   int32_t valid[kTile];
 };
+struct NearForce {
+  double x[kTile], y[kTile], z[kTile];
+};
 
+template <int kSplit>
 __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const int4* __restrict__ near, int n_near) {
-  __shared__ NearTile tiles[kNearWarps];
+  static_assert(kSplit == 1 || kSplit == kNearWarps, "a warp or a block per tile pair");
+  __shared__ NearTile tiles[kNearWarps / kSplit];
+  __shared__ NearForce jf[kNearWarps], sf[kSplit > 1 ? kNearWarps : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wid = blockIdx.x * kNearWarps + warp;
-  if (wid >= n_near) return;
-  NearTile& t = tiles[warp];
+  const int wid = kSplit > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kNearWarps + warp;
+  if (wid >= n_near) return;  // block-uniform when split
+  const int part = kSplit > 1 ? warp : 0;
+  NearTile& t = tiles[kSplit > 1 ? 0 : warp];
+  NearForce& f = jf[warp];
   const int4 w = near[wid];  // i_tile, j_tile (>= i_tile), mask block of (i_tile, j_tile)
   const int i = w.x * kTile + lane;
   const int jl = w.y * kTile + lane;  // this lane's j atom, staged for the warp
-  t.x[lane] = a.x64[jl];
-  t.y[lane] = a.y64[jl];
-  t.z[lane] = a.z64[jl];
-  t.q[lane] = a.q64[jl];
-  t.r[lane] = a.born_r64[jl];
-  t.ir[lane] = 1.0 / a.born_r64[jl];
-  t.rmin[lane] = a.rmin64[jl];
-  t.seps[lane] = sqrt(a.eps64[jl]);
-  t.rmin14[lane] = a.rmin14_64[jl];
-  t.seps14[lane] = sqrt(a.eps14_64[jl]);
-  t.valid[lane] = a.atom_valid[jl];
-  t.fx[lane] = t.fy[lane] = t.fz[lane] = 0.0;
+  if (part == 0) {
+    t.x[lane] = a.x64[jl];
+    t.y[lane] = a.y64[jl];
+    t.z[lane] = a.z64[jl];
+    t.q[lane] = a.q64[jl];
+    t.r[lane] = a.born_r64[jl];
+    t.ir[lane] = 1.0 / a.born_r64[jl];
+    t.rmin[lane] = a.rmin64[jl];
+    t.seps[lane] = sqrt(a.eps64[jl]);
+    t.rmin14[lane] = a.rmin14_64[jl];
+    t.seps14[lane] = sqrt(a.eps14_64[jl]);
+    t.valid[lane] = a.atom_valid[jl];
+  }
+  f.x[lane] = f.y[lane] = f.z[lane] = 0.0;
   const uint32_t ex = a.mask_ex[w.z * kTile + lane];
   const uint32_t m14 = a.mask_14[w.z * kTile + lane];
   const bool valid_i = a.atom_valid[i] != 0;
@@ -66,8 +85,9 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
   const double gb_pref = (1.0 - 1.0 / kEpsWater) * kCoulomb * kKcalToKj;
   const bool diag = w.x == w.y;
   double ax = 0.0, ay = 0.0, az = 0.0;
-  __syncwarp();
-  for (int k = diag ? 1 : 0; k < (diag ? 17 : kTile); ++k) {
+  if (kSplit > 1) __syncthreads();
+  else __syncwarp();
+  for (int k = (diag ? 1 : 0) + part; k < (diag ? 17 : kTile); k += kSplit) {
     const int p = (lane + k) & (kTile - 1);
     double coeff = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
     if (valid_i && t.valid[p] && !(diag && k == 16 && lane >= 16)) {
@@ -102,10 +122,35 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
     ax += dx * coeff;
     ay += dy * coeff;
     az += dz * coeff;
-    t.fx[p] -= dx * coeff;
-    t.fy[p] -= dy * coeff;
-    t.fz[p] -= dz * coeff;
+    f.x[p] -= dx * coeff;
+    f.y[p] -= dy * coeff;
+    f.z[p] -= dz * coeff;
     __syncwarp();
+  }
+  if (kSplit > 1) {
+    NearForce& fi = sf[warp];
+    fi.x[lane] = ax;
+    fi.y[lane] = ay;
+    fi.z[lane] = az;
+    __syncthreads();
+    if (warp >= 2) return;
+    // warp 0: the i side, warp 1: the j side, over the warps in order
+    const NearForce* side = warp == 0 ? sf : jf;
+    ax = ay = az = 0.0;
+#pragma unroll
+    for (int w = 0; w < kNearWarps; ++w) {
+      ax += side[w].x[lane];
+      ay += side[w].y[lane];
+      az += side[w].z[lane];
+    }
+    const int at = warp == 0 ? i : jl;
+    if (warp == 0 ? valid_i : t.valid[lane] != 0) {
+      if (!(isfinite(ax) && isfinite(ay) && isfinite(az))) atomicOr(a.sys_nonfinite + a.atom_sys[at], 1);
+      add_fixed(a.fx + at, ax, kForceScale);
+      add_fixed(a.fy + at, ay, kForceScale);
+      add_fixed(a.fz + at, az, kForceScale);
+    }
+    return;
   }
   if (valid_i) {
     if (!(isfinite(ax) && isfinite(ay) && isfinite(az))) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
@@ -114,7 +159,7 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
     add_fixed(a.fz + i, az, kForceScale);
   }
   if (t.valid[lane]) {
-    const double bx = t.fx[lane], by = t.fy[lane], bz = t.fz[lane];
+    const double bx = f.x[lane], by = f.y[lane], bz = f.z[lane];
     if (!(isfinite(bx) && isfinite(by) && isfinite(bz))) atomicOr(a.sys_nonfinite + a.atom_sys[jl], 1);
     add_fixed(a.fx + jl, bx, kForceScale);
     add_fixed(a.fy + jl, by, kForceScale);
@@ -124,8 +169,10 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
 
 }  // namespace
 
-void launch_near_force64(const PairArgs& a, const int4* near, int n_near, cudaStream_t s) {
-  if (n_near > 0) k_near64<<<(n_near + kNearWarps - 1) / kNearWarps, kNearWarps * 32, 0, s>>>(a, near, n_near);
+void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_sm, cudaStream_t s) {
+  if (n_near <= 0) return;
+  if (n_near <= kNearSplitPerSm * n_sm) k_near64<kNearWarps><<<n_near, kNearWarps * 32, 0, s>>>(a, near, n_near);
+  else k_near64<1><<<(n_near + kNearWarps - 1) / kNearWarps, kNearWarps * 32, 0, s>>>(a, near, n_near);
 }
 
 // ----------------------------------------------------------------- FP64 path

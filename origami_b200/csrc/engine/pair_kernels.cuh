@@ -115,7 +115,7 @@ void launch_force_pass(const PairArgs& a, const PairLaunch& c, cudaStream_t s);
 // Near field: near[k] = (i_tile, j_tile, mask block of (i_tile, j_tile), 0)
 // for every unordered tile pair (i_tile <= j_tile) that carries masks, FP64;
 // each pair once, both atoms' forces.
-void launch_near_force64(const PairArgs& a, const int4* near, int n_near, cudaStream_t s);
+void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_sm, cudaStream_t s);
 
 // FP64 energy evaluation: one warp per i-tile and j range (pair_fp64.cu).
 struct EnergyArgs {
