@@ -300,24 +300,36 @@ struct og_engine {
   ogk::TunnelParams tunnel{};
   double sasa_rmax = 0.0;
   double s_max = 0.0, rho_max = 0.0;  // largest s*rho~ and rho~ (series limits of the Born pass)
-  // graph
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t graph_exec = nullptr;
+  // captured launches: one MD step, and one force evaluation (from the
+  // second one on, while lgb_on() is what it was at the capture)
+  struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    void reset() {
+      if (exec) cudaGraphExecDestroy(exec);
+      if (graph) cudaGraphDestroy(graph);
+      exec = nullptr;
+      graph = nullptr;
+    }
+  };
+  StepGraph step_graph, force_graph;
+  bool capturing = false;  // enqueue_forces is being captured
+  bool force_graph_lgb = false;
+  int force_evals = 0;
   // profiling
   bool profile = false;
   std::map<std::string, std::pair<double, long long>> prof;
   std::vector<std::string> prof_names;
 
   ~og_engine() {
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
+    for (StepGraph* g : {&step_graph, &force_graph}) g->reset();
     if (own_stream && stream) cudaStreamDestroy(stream);
-    for (cudaStream_t* q : {&side, &hi})
+    for (cudaStream_t* q : {&side, &hi, &aux})
       if (*q) {
         cudaStreamSynchronize(*q);
         cudaStreamDestroy(*q);
       }
-    for (cudaEvent_t ev : {ev_fork, ev_join, ev_join_hi})
+    for (cudaEvent_t ev : {ev_fork, ev_join, ev_join_hi, ev_cut, ev_born, ev_join_aux})
       if (ev) cudaEventDestroy(ev);
   }
 
@@ -330,17 +342,21 @@ struct og_engine {
   // The pair kernels go to a high-priority internal stream and the surface
   // term to a low-priority one; in eager launches (judge, single force
   // evaluations) the block scheduler then places pair blocks first.
-  cudaStream_t side = nullptr, hi = nullptr;
+  // What needs no radii -- the force pass's cutoff lists, the bonded terms --
+  // runs on a third stream beside the Born pass, and the FP64 near field
+  // there beside the force pass: none of them fills the GPU by itself.
+  cudaStream_t side = nullptr, hi = nullptr, aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join_hi = nullptr;
+  cudaEvent_t ev_cut = nullptr, ev_born = nullptr, ev_join_aux = nullptr;
   cudaError_t ensure_side() {
-    if (side) return cudaSuccess;
+    if (ev_join_aux) return cudaSuccess;
     int least = 0, greatest = 0;
     cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, least);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&hi, cudaStreamNonBlocking, greatest);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev_join_hi, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, greatest);
+    for (cudaEvent_t* ev : {&ev_fork, &ev_join, &ev_join_hi, &ev_cut, &ev_born, &ev_join_aux})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     return e;
   }
 
@@ -556,17 +572,40 @@ struct og_engine {
   void enqueue_forces() {
     ogk::PairArgs pa = pair_args();
     ogk::AtomArrays at = atoms();
-    // the surface term on the side stream (profiling times kernels one by
-    // one, on the main stream)
-    const bool sasa_forked = p.include_sasa && !profile && ensure_side() == cudaSuccess;
+    // side streams: under capture, and with the surface term (profiling times
+    // kernels one by one, on the main stream; a first evaluation without the
+    // surface term would wait longer for the streams' creation than it gains)
+    const bool forked = !profile && (p.include_sasa || capturing) && ensure_side() == cudaSuccess;
+    const bool sasa_forked = p.include_sasa && forked;
     const cudaStream_t main_stream = stream;
-    if (sasa_forked) {
+    const bool cut_force = !no_cutoff(p.nb_cutoff) && !no_cutoff(p.gb_force_cutoff);
+    auto cut_lists = [&](cudaStream_t on) {
+      ogk::launch_cut_lists(cut_f.p, n_cut_f, jlist_f.p, origin.p, std::max(p.nb_cutoff, p.gb_force_cutoff),
+                            jlist_cut_f.p, seg_end_f.p, on);
+    };
+    auto bonded = [&](cudaStream_t on) {
+      Timer t(this, "bonded", on);
+      ogk::launch_bonded_forces(bonded_args(), on);
+    };
+    auto near_field = [&](cudaStream_t on) {
+      Timer t(this, "near_force64", on);
+      ogk::launch_near_force64(pa, near.p, n_near, n_sm, on);
+    };
+    if (forked) {
       cudaEventRecord(ev_fork, stream);
-      cudaStreamWaitEvent(side, ev_fork, 0);
-      cudaStreamWaitEvent(hi, ev_fork, 0);
-      ogk::launch_sasa_forces(sasa_args(false), side);
-      cudaEventRecord(ev_join, side);
-      stream = hi;  // the pair kernels below
+      cudaStreamWaitEvent(aux, ev_fork, 0);
+      if (sasa_forked) {
+        cudaStreamWaitEvent(side, ev_fork, 0);
+        cudaStreamWaitEvent(hi, ev_fork, 0);
+        ogk::launch_sasa_forces(sasa_args(false), side);
+        cudaEventRecord(ev_join, side);
+        stream = hi;  // the pair kernels below
+      }
+      if (cut_force) {
+        cut_lists(aux);
+        cudaEventRecord(ev_cut, aux);
+      }
+      bonded(aux);
     }
     if (lgb_on()) {
       enqueue_learned_radii();
@@ -587,6 +626,12 @@ struct og_engine {
         ogk::launch_born_finalize(at, nullptr, 0, born_r.p, true, nullptr, stream);
       }
     }
+    if (forked) {
+      cudaEventRecord(ev_born, stream);
+      cudaStreamWaitEvent(aux, ev_born, 0);
+      near_field(aux);
+      cudaEventRecord(ev_join_aux, aux);
+    }
     {
       Timer t(this, "force_pass");
       ogk::PairArgs pf = pa;
@@ -594,21 +639,17 @@ struct og_engine {
       pf.n_work = n_work_f;
       pf.jlist = jlist_f.p;
       pf.queue = pair_queue.p + 1;
-      if (!no_cutoff(p.nb_cutoff) && !no_cutoff(p.gb_force_cutoff)) {
-        ogk::launch_cut_lists(cut_f.p, n_cut_f, jlist_f.p, origin.p, std::max(p.nb_cutoff, p.gb_force_cutoff),
-                              jlist_cut_f.p, seg_end_f.p, stream);
+      if (cut_force) {
+        if (forked) cudaStreamWaitEvent(stream, ev_cut, 0);
+        else cut_lists(stream);
         pf.jlist = jlist_cut_f.p;
         pf.seg_end = seg_end_f.p;
       }
       ogk::launch_force_pass(pf, force_launch, stream);
     }
-    {
-      Timer t(this, "near_force64");
-      ogk::launch_near_force64(pa, near.p, n_near, n_sm, stream);
-    }
-    {
-      Timer t(this, "bonded");
-      ogk::launch_bonded_forces(bonded_args(), stream);
+    if (!forked) {
+      near_field(stream);
+      bonded(stream);
     }
     if (sasa_forked) {
       cudaEventRecord(ev_join_hi, hi);
@@ -619,6 +660,7 @@ struct og_engine {
       Timer t(this, "sasa");
       ogk::launch_sasa_forces(sasa_args(false), stream);
     }
+    if (forked) cudaStreamWaitEvent(stream, ev_join_aux, 0);
     if (tunnel_on) {
       Timer t(this, "tunnel");
       ogk::launch_tunnel(atoms(), tunnel, stream);
@@ -1462,22 +1504,71 @@ og_status finalize_impl(og_engine* e) {
   return OG_OK;
 }
 
+// Captures what enqueue() launches on e->stream into g.
+template <class F>
+og_status capture(og_engine* e, og_engine::StepGraph* g, F enqueue) {
+  cudaStream_t cap;
+  OG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  cudaStream_t saved = e->stream;
+  e->stream = cap;
+  cudaError_t err = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+  if (err == cudaSuccess) {
+    e->capturing = true;
+    enqueue();
+    e->capturing = false;
+    err = cudaStreamEndCapture(cap, &g->graph);
+  }
+  e->stream = saved;
+  cudaStreamDestroy(cap);
+  if (err != cudaSuccess) {
+    g->reset();
+    return cuda_fail(err, "graph capture");
+  }
+  // Kernel nodes run at the launch stream's priority: the surface term's
+  // blocks, launched first, are dispatched first and the pair kernels fill
+  // its tail.  (Honouring the captured node priorities, pair kernels first,
+  // measured slower: they displace surface warps, whose latency-bound work
+  // then stretches the step.)
+  err = cudaGraphInstantiate(&g->exec, g->graph, 0);
+  if (err != cudaSuccess) {
+    g->reset();
+    return cuda_fail(err, "graph instantiation");
+  }
+  return OG_OK;
+}
+
+// Forces at the current positions.  The first evaluation launches its
+// kernels one by one, later ones as one graph: an engine asked once does not
+// pay for a capture (about 0.2 ms), and one asked again (line searches,
+// external integrators) spends 6 us of host time per evaluation, not 30.
 og_status eval_forces(og_engine* e) {
   if (e->p.born_mode == 1 && !e->lgb_params_set)
     return og_fail(OG_E_STATE, "born_mode 1 needs the network's parameters (og_lgb_set_params)");
-  ogk::launch_pack(e->atoms(), true, e->stream);
-  e->enqueue_forces();
-  og_status st = launch_check("force evaluation");
+  auto enqueue = [e] {
+    ogk::launch_pack(e->atoms(), true, e->stream);
+    e->enqueue_forces();
+  };
+  og_status st;
+  if (e->profile || (e->force_graph.exec && e->force_graph_lgb != e->lgb_on()) ||
+      (!e->force_graph.exec && e->force_evals++ == 0)) {
+    enqueue();
+  } else {
+    if (!e->force_graph.exec) {
+      if ((st = capture(e, &e->force_graph, enqueue)) != OG_OK) return st;
+      e->force_graph_lgb = e->lgb_on();
+    }
+    OG_CUDA(cudaGraphLaunch(e->force_graph.exec, e->stream));
+  }
+  st = launch_check("force evaluation");
   if (st != OG_OK) return st;
   e->forces_valid = true;
   return OG_OK;
 }
 
 void reset_graph(og_engine* e) {
-  if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
-  if (e->graph) cudaGraphDestroy(e->graph);
-  e->graph_exec = nullptr;
-  e->graph = nullptr;
+  e->step_graph.reset();
+  e->force_graph.reset();
+  e->force_evals = 0;
 }
 
 og_status lgb_check(og_engine* e) {
@@ -1524,26 +1615,8 @@ og_status lgb_judge(og_engine* e, double* err_out) {
 }
 
 og_status build_graph(og_engine* e) {
-  if (e->graph_exec) return OG_OK;
-  cudaStream_t cap;
-  OG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-  cudaStream_t saved = e->stream;
-  e->stream = cap;
-  cudaError_t err = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-  if (err == cudaSuccess) {
-    e->enqueue_step();
-    err = cudaStreamEndCapture(cap, &e->graph);
-  }
-  e->stream = saved;
-  cudaStreamDestroy(cap);
-  if (err != cudaSuccess) return cuda_fail(err, "graph capture");
-  // Kernel nodes run at the launch stream's priority: the surface term's
-  // blocks, launched first, are dispatched first and the pair kernels fill
-  // its tail.  (Honouring the captured node priorities, pair kernels first,
-  // measured slower: they displace surface warps, whose latency-bound work
-  // then stretches the step.)
-  OG_CUDA(cudaGraphInstantiate(&e->graph_exec, e->graph, 0));
-  return OG_OK;
+  if (e->step_graph.exec) return OG_OK;
+  return capture(e, &e->step_graph, [e] { e->enqueue_step(); });
 }
 
 // ---- co-translational growth
@@ -2105,7 +2178,7 @@ og_status og_step(og_engine* e, int32_t n_steps) {
       if ((st = launch_check("step")) != OG_OK) return st;
     } else if (chunk > 0) {
       if ((st = build_graph(e)) != OG_OK) return st;
-      for (int k = 0; k < chunk; ++k) OG_CUDA(cudaGraphLaunch(e->graph_exec, e->stream));
+      for (int k = 0; k < chunk; ++k) OG_CUDA(cudaGraphLaunch(e->step_graph.exec, e->stream));
     }
     done += chunk;
     if (judging) {
