@@ -470,13 +470,13 @@ def run_b200(args):
     e2e_s = max_over_ranks((time.perf_counter() - t0) / e2e_steps, ws)
     e2e = aggregate_ns_per_day(ws, args.replicas, args.dt, e2e_s * 1e3)
 
-    # per step: BAOAB sub-steps and SHAKE (6), Born pass + finalize or
+    # per step: BAOAB sub-steps with SHAKE, pack, final kick (3), Born pass + finalize or
     # descriptors + fused network (2), force, near field, bonded (3), SASA
     # (boundary, its large-capacity queue, terms: 3), and in cutoff mode the
     # culled work lists (force; plus Born in the plain arm)
     sasa_k = 0 if args.no_sasa else 3
     cut_k = 0 if not args.cutoff else (2 if args.plain_only else 1)
-    launches = 6 + 2 + 3 + sasa_k + cut_k
+    launches = 3 + 2 + 3 + sasa_k + cut_k
     cfg = workload_config(args, atoms, "plain OBC-II pass" if args.plain_only
                           else "learned radii (network on tcgen05 GEMMs), plain-GB judge")
     cfg["system"] = system
@@ -586,7 +586,7 @@ def run_c3b(args):
                        "atoms_total": sum(atoms), "atoms_min": min(atoms), "atoms_max": max(atoms),
                        "l2": "inputs resident; timed as one region of K steps"},
             "pair_interactions_per_s": pairs / (per * 1e-3), "autotune": tune, "clocks": clk,
-            "gpu_launches": args.steps * 11}
+            "gpu_launches": args.steps * 8}
     eng.close()
     print(json.dumps(line))
 

@@ -265,6 +265,9 @@ struct og_engine {
   DVec<int2> cons_atoms;
   DVec<double> cons_d2;
   int n_clusters = 0;
+  // the fused step's slots; empty when some constraint is not a hydrogen on
+  // one heavy atom (build_slots)
+  DVec<ogk::MoveSlot> slots;
   // reductions
   DVec<int32_t> seg_begin, seg_end;  // [atoms per sys | bonds | angles | dihedrals | impropers], 5*n_sys
   DVec<double> seg_out;
@@ -667,13 +670,13 @@ struct og_engine {
     }
   }
 
-  void enqueue_step() {
-    ogk::StepArgs sa = step_args();
+  // The sub-steps before the forces for constraints of any shape.
+  void enqueue_move_general(const ogk::StepArgs& sa) {
     {
       Timer t(this, "step_pre");
       ogk::launch_step_pre(sa, stream);
     }
-    if (sa.use_shake) {
+    {
       Timer t(this, "shake");
       ogk::launch_shake(shake_args(), stream);
     }
@@ -681,13 +684,33 @@ struct og_engine {
       Timer t(this, "step_mid");
       ogk::launch_step_mid(sa, stream);
     }
-    if (sa.use_shake) {
+    {
       Timer t(this, "shake");
       ogk::launch_shake(shake_args(), stream);
     }
     {
       Timer t(this, "step_post");
       ogk::launch_step_post(sa, stream);
+    }
+  }
+
+  void enqueue_step() {
+    ogk::StepArgs sa = step_args();
+    if (!sa.use_shake) {
+      Timer t(this, "step_move");
+      ogk::launch_step_free(sa, stream);
+    } else if (slots.n > 0) {
+      Timer t(this, "step_move");
+      const ogk::ShakeArgs sh = shake_args();
+      ogk::MoveArgs m{};
+      m.slots = slots.p;
+      m.n_slots = static_cast<int32_t>(slots.n);
+      m.inv_mass = inv_mass.p;
+      m.tol_sq = sh.tol_sq;
+      m.max_iters = sh.max_iters;
+      ogk::launch_step_move(sa, m, stream);
+    } else {
+      enqueue_move_general(sa);
     }
     enqueue_forces();
     {
@@ -1275,6 +1298,52 @@ og_status append_clusters(og_engine* e, int si, const std::vector<int>& cons, co
   return OG_OK;
 }
 
+// Slots of the fused step (k_step_move): every atom once, a heavy atom
+// followed by its hydrogens in constraint order within one warp.  Left empty
+// -- the general launches then run -- when an atom is in two clusters or a
+// cluster has more than 31 constraints.
+og_status build_slots(og_engine* e, cudaStream_t st) {
+  e->slots.n = 0;
+  if (!e->p.constrain_h_bonds || e->n_clusters == 0) return OG_OK;
+  std::vector<ogk::MoveSlot> out;
+  for (const auto& s : e->sys) {
+    const TopoCopy& t = s.topo;
+    std::vector<std::vector<std::pair<int, double>>> h(t.n);  // per heavy atom: (hydrogen, squared length)
+    std::vector<int> owner(t.n, -1);
+    for (size_t k = 0; k < t.cons_d.size(); ++k) {
+      const int a = t.cons[2 * k], b = t.cons[2 * k + 1];
+      const int heavy = t.element[a] == 0 ? b : a, other = heavy == a ? b : a;
+      if (heavy == other || owner[other] >= 0) return OG_OK;
+      owner[other] = heavy;
+      h[heavy].push_back({other, t.cons_d[k] * t.cons_d[k]});
+    }
+    for (int a = 0; a < t.n; ++a) {
+      if (owner[a] >= 0) {
+        if (!h[a].empty()) return OG_OK;
+        continue;
+      }
+      const size_t n = h[a].size();
+      if (n > 31) return OG_OK;
+      const ogk::MoveSlot empty{-1, 0, 0, 0, 0, 0.0};
+      while (out.size() % 32 + n + 1 > 32) {
+        out.push_back(empty);
+        out.back().head = static_cast<uint8_t>((out.size() - 1) % 32);
+      }
+      const uint8_t head = static_cast<uint8_t>(out.size() % 32), nc = static_cast<uint8_t>(n);
+      out.push_back(ogk::MoveSlot{s.atom_begin + a, head, 0, nc, 0, 0.0});
+      for (size_t k = 0; k < n; ++k)
+        out.push_back(ogk::MoveSlot{s.atom_begin + h[a][k].first, head, static_cast<uint8_t>(k + 1), nc, 0, h[a][k].second});
+    }
+  }
+  while (out.size() % 32 != 0) {
+    out.push_back(ogk::MoveSlot{-1, static_cast<uint8_t>(out.size() % 32), 0, 0, 0, 0.0});
+  }
+  OG_CUDA(e->slots.grow(out.size(), st));
+  OG_CUDA(cudaMemcpyAsync(e->slots.p, out.data(), out.size() * sizeof(ogk::MoveSlot), cudaMemcpyHostToDevice, st));
+  OG_CUDA(cudaStreamSynchronize(st));  // `out` is read until here
+  return OG_OK;
+}
+
 og_status upload_sys_tiles(og_engine* e, cudaStream_t st) {
   std::vector<int2> hst;
   for (const auto& s : e->sys) hst.push_back(make_int2(s.tile_begin, s.n_tiles));
@@ -1488,6 +1557,10 @@ og_status finalize_impl(og_engine* e) {
       og_status cs = append_clusters(e, si, TermSel::all(e->sys[si].topo).cons, {}, st);
       if (cs != OG_OK) return cs;
     }
+  {
+    og_status ms = build_slots(e, st);
+    if (ms != OG_OK) return ms;
+  }
 
   OG_CUDA(e->clamp_count.alloc(n_sys));
   OG_CUDA(e->sys_nonfinite.alloc(n_sys));
@@ -1781,6 +1854,7 @@ og_status append_impl(og_engine* e, int si, const TopoCopy& grown, const double*
   if ((s = append_bonded(e, si, d, st)) != OG_OK) return s;
   if ((s = upload_segments(e, st)) != OG_OK) return s;
   if (e->p.constrain_h_bonds && (s = append_clusters(e, si, d.cons, old_heavy, st)) != OG_OK) return s;
+  if ((s = build_slots(e, st)) != OG_OK) return s;
 
   // the system's atom count and degrees of freedom (its step count, status
   // and temperature stay)

@@ -299,6 +299,28 @@ __device__ __forceinline__ void count_shake(const AtomArrays& a, int i, int sys)
   }
 }
 
+// O step (langevin.rs:260-271) of atom i with Philox noise keyed by (system,
+// step, atom).
+__device__ __forceinline__ void ornstein_uhlenbeck(const StepArgs& p, int i, int sys, double* vx, double* vy,
+                                                   double* vz) {
+  const AtomArrays& a = p.at;
+  const SysState& s = a.sys[sys];
+  const unsigned long long step = static_cast<unsigned long long>(s.steps) + 1ull;
+  const U4 r = philox4x32_10(U4{static_cast<uint32_t>(a.local_idx[i]), static_cast<uint32_t>(step),
+                                 static_cast<uint32_t>(step >> 32), static_cast<uint32_t>(sys)},
+                              p.seed_lo, p.seed_hi);
+  const double m1 = sqrt(-2.0 * log(u32_to_open01(r.x)));
+  const double m2 = sqrt(-2.0 * log(u32_to_open01(r.z)));
+  double s1, c1, s2, c2;
+  sincospi(2.0 * (static_cast<double>(r.y) * (1.0 / 4294967296.0)), &s1, &c1);
+  sincospi(2.0 * (static_cast<double>(r.w) * (1.0 / 4294967296.0)), &s2, &c2);
+  const double one_minus_a2 = 1.0 - p.alpha * p.alpha;
+  const double sigma = sqrt(one_minus_a2 * s.kbt * s.dof_corr * kAccel / a.mass[i]);
+  *vx = p.alpha * *vx + sigma * (m1 * c1);
+  *vy = p.alpha * *vy + sigma * (m1 * s1);
+  *vz = p.alpha * *vz + sigma * (m2 * c2);
+}
+
 __global__ void k_step_mid(StepArgs p) {
   const AtomArrays& a = p.at;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -313,22 +335,7 @@ __global__ void k_step_mid(StepArgs p) {
   } else {
     vx = a.vx[i]; vy = a.vy[i]; vz = a.vz[i];
   }
-  const SysState& s = a.sys[sys];
-  // O step (langevin.rs:260-271) with Philox noise keyed by (system, step, atom).
-  const unsigned long long step = static_cast<unsigned long long>(s.steps) + 1ull;
-  const U4 r = philox4x32_10(U4{static_cast<uint32_t>(a.local_idx[i]), static_cast<uint32_t>(step),
-                                 static_cast<uint32_t>(step >> 32), static_cast<uint32_t>(sys)},
-                              p.seed_lo, p.seed_hi);
-  const double m1 = sqrt(-2.0 * log(u32_to_open01(r.x)));
-  const double m2 = sqrt(-2.0 * log(u32_to_open01(r.z)));
-  double s1, c1, s2, c2;
-  sincospi(2.0 * (static_cast<double>(r.y) * (1.0 / 4294967296.0)), &s1, &c1);
-  sincospi(2.0 * (static_cast<double>(r.w) * (1.0 / 4294967296.0)), &s2, &c2);
-  const double one_minus_a2 = 1.0 - p.alpha * p.alpha;
-  const double sigma = sqrt(one_minus_a2 * s.kbt * s.dof_corr * kAccel / a.mass[i]);
-  vx = p.alpha * vx + sigma * (m1 * c1);
-  vy = p.alpha * vy + sigma * (m1 * s1);
-  vz = p.alpha * vz + sigma * (m2 * c2);
+  ornstein_uhlenbeck(p, i, sys, &vx, &vy, &vz);
   a.vx[i] = vx; a.vy[i] = vy; a.vz[i] = vz;
   const double x = a.x[i], y = a.y[i], z = a.z[i];
   if (p.use_shake) { a.rx[i] = x; a.ry[i] = y; a.rz[i] = z; }
@@ -347,6 +354,164 @@ __global__ void k_step_post(StepArgs p) {
     a.vy[i] = (a.y[i] - a.ry[i]) / p.half_dt;
     a.vz[i] = (a.z[i] - a.rz[i]) / p.half_dt;
     count_shake(a, i, sys);
+  }
+  pack_atom(a, i);
+  a.fx[i] = 0ull;
+  a.fy[i] = 0ull;
+  a.fz[i] = 0ull;
+  a.born_sum[i] = 0ull;
+}
+
+// ---- the same sub-steps in one kernel (B, A, O, A and the pack), for the
+// two common cases; k_step_pre, k_shake, k_step_mid and k_step_post remain for
+// constraints that are not hydrogens on one heavy atom each.  A step of a
+// small system is a chain of launches: five of them here are now one or two,
+// and the state is read and written once.
+
+// Without constraints: a thread per padded atom, a warp per tile.
+__global__ void k_step_free(StepArgs p) {
+  const AtomArrays& a = p.at;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n_padded) return;
+  int sys;
+  if (atom_live(a, i, &sys)) {
+    const double c = (kAccel / a.mass[i]) * p.half_dt;
+    double vx = a.vx[i] + fixed_to_f(a.fx[i]) * c;
+    double vy = a.vy[i] + fixed_to_f(a.fy[i]) * c;
+    double vz = a.vz[i] + fixed_to_f(a.fz[i]) * c;
+    const double x = a.x[i] + vx * p.half_dt, y = a.y[i] + vy * p.half_dt, z = a.z[i] + vz * p.half_dt;
+    ornstein_uhlenbeck(p, i, sys, &vx, &vy, &vz);
+    a.vx[i] = vx; a.vy[i] = vy; a.vz[i] = vz;
+    a.x[i] = x + vx * p.half_dt;
+    a.y[i] = y + vy * p.half_dt;
+    a.z[i] = z + vz * p.half_dt;
+  }
+  pack_atom(a, i);
+  a.fx[i] = 0ull;
+  a.fy[i] = 0ull;
+  a.fz[i] = 0ull;
+  a.born_sum[i] = 0ull;
+}
+
+// One lane's atom in the fused step with SHAKE.
+struct Mover {
+  double x, y, z;     // position
+  double rx, ry, rz;  // reference position of the constraints
+  double im;          // inverse mass
+};
+
+// SHAKE passes (shake.rs:86-125) over the warp's clusters at once: a cluster
+// is a heavy atom (lane head, k = 0) and its n hydrogens in the n lanes after
+// it (k = 1 .. n, in constraint order); constraint k is worked by its
+// hydrogen's lane, which hands the heavy atom's lane the displacement.  The
+// same Gauss-Seidel order and arithmetic as k_shake.  Returns whether the
+// lane's cluster converged.
+__device__ bool shake_lanes(Mover& m, int head, int k, int n, double d2, double tol_sq, int max_iters) {
+  const int lane = threadIdx.x & 31;
+  const int n_max = __reduce_max_sync(0xffffffffu, n);
+  const unsigned cluster = ((2u << n) - 1u) << head;
+  const double hrx = __shfl_sync(0xffffffffu, m.rx, head), hry = __shfl_sync(0xffffffffu, m.ry, head),
+               hrz = __shfl_sync(0xffffffffu, m.rz, head), him = __shfl_sync(0xffffffffu, m.im, head);
+  const double rox = hrx - m.rx, roy = hry - m.ry, roz = hrz - m.rz;
+  bool converged = n == 0;
+  for (int iter = 0; iter < max_iters; ++iter) {
+    if (__all_sync(0xffffffffu, converged)) break;
+    bool off = false;  // this lane's constraint is outside tolerance in this pass
+    for (int c = 1; c <= n_max; ++c) {
+      const double hx = __shfl_sync(0xffffffffu, m.x, head), hy = __shfl_sync(0xffffffffu, m.y, head),
+                   hz = __shfl_sync(0xffffffffu, m.z, head);
+      double dx = 0.0, dy = 0.0, dz = 0.0;
+      if (k == c && !converged) {
+        const double rnx = hx - m.x, rny = hy - m.y, rnz = hz - m.z;
+        const double err = (rnx * rnx + rny * rny + rnz * rnz) - d2;
+        off = fabs(err) >= tol_sq;
+        if (!(fabs(err) < tol_sq)) {
+          const double dotv = rnx * rox + rny * roy + rnz * roz;
+          const double denom = 2.0 * (him + m.im) * dotv;
+          if (!(fabs(denom) < 1e-18)) {
+            const double lambda = err / denom;
+            dx = rox * lambda;
+            dy = roy * lambda;
+            dz = roz * lambda;
+            m.x += dx * m.im;
+            m.y += dy * m.im;
+            m.z += dz * m.im;
+          }
+        }
+      }
+      const int from = (head + c) & 31;
+      dx = __shfl_sync(0xffffffffu, dx, from);
+      dy = __shfl_sync(0xffffffffu, dy, from);
+      dz = __shfl_sync(0xffffffffu, dz, from);
+      if (lane == head && c <= n) {
+        m.x -= dx * m.im;
+        m.y -= dy * m.im;
+        m.z -= dz * m.im;
+      }
+    }
+    if ((__ballot_sync(0xffffffffu, off) & cluster) == 0u) converged = true;
+  }
+  return converged;
+}
+
+__global__ void __launch_bounds__(128) k_step_move(StepArgs p, MoveArgs mv) {
+  const AtomArrays& a = p.at;
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= mv.n_slots) return;  // whole warps: n_slots is a multiple of 32
+  const MoveSlot slot = mv.slots[s];
+  const int i = slot.atom;
+  int sys = -1;
+  const bool live = i >= 0 && atom_live(a, i, &sys);
+  Mover m{};
+  double vx = 0.0, vy = 0.0, vz = 0.0;
+  const int n = live ? slot.n : 0;
+  if (live) {
+    const double c = (kAccel / a.mass[i]) * p.half_dt;
+    vx = a.vx[i] + fixed_to_f(a.fx[i]) * c;
+    vy = a.vy[i] + fixed_to_f(a.fy[i]) * c;
+    vz = a.vz[i] + fixed_to_f(a.fz[i]) * c;
+    m.im = mv.inv_mass[i];
+    m.rx = a.x[i]; m.ry = a.y[i]; m.rz = a.z[i];
+    m.x = m.rx + vx * p.half_dt;
+    m.y = m.ry + vy * p.half_dt;
+    m.z = m.rz + vz * p.half_dt;
+  }
+  int failed = 0;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+    if (!shake_lanes(m, slot.head, slot.k, n, slot.d2, mv.tol_sq, mv.max_iters)) failed |= 1 << half;
+    vx = (m.x - m.rx) / p.half_dt;
+    vy = (m.y - m.ry) / p.half_dt;
+    vz = (m.z - m.rz) / p.half_dt;
+    if (half == 0) {
+      if (live) ornstein_uhlenbeck(p, i, sys, &vx, &vy, &vz);
+      m.rx = m.x; m.ry = m.y; m.rz = m.z;
+      m.x += vx * p.half_dt;
+      m.y += vy * p.half_dt;
+      m.z += vz * p.half_dt;
+    }
+  }
+  if (live) {
+    a.vx[i] = vx; a.vy[i] = vy; a.vz[i] = vz;
+    a.x[i] = m.x; a.y[i] = m.y; a.z[i] = m.z;
+    if (failed && slot.k == 0) atomicOr(&a.sys[sys].shake_flag, failed);
+  }
+}
+
+// Pack and zero after k_step_move; counts its failed SHAKE calls (a bit per
+// half step).
+__global__ void k_step_pack(StepArgs p) {
+  const AtomArrays& a = p.at;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n_padded) return;
+  int sys;
+  if (atom_live(a, i, &sys) && a.local_idx[i] == 0) {
+    SysState& s = a.sys[sys];
+    if (s.shake_flag) {
+      s.shake_failures += __popc(s.shake_flag);
+      s.status |= kStatusShakeFail;
+      s.shake_flag = 0;
+    }
   }
   pack_atom(a, i);
   a.fx[i] = 0ull;
@@ -538,6 +703,13 @@ void launch_step_mid(const StepArgs& a, cudaStream_t s) {
 }
 void launch_step_post(const StepArgs& a, cudaStream_t s) {
   k_step_post<<<blocks_for(a.at.n_padded, 256), 256, 0, s>>>(a);
+}
+void launch_step_free(const StepArgs& a, cudaStream_t s) {
+  k_step_free<<<blocks_for(a.at.n_padded, 128), 128, 0, s>>>(a);
+}
+void launch_step_move(const StepArgs& a, const MoveArgs& m, cudaStream_t s) {
+  k_step_move<<<blocks_for(m.n_slots, 128), 128, 0, s>>>(a, m);
+  k_step_pack<<<blocks_for(a.at.n_padded, 256), 256, 0, s>>>(a);
 }
 void launch_step_end(const StepArgs& a, cudaStream_t s) {
   k_step_end<<<blocks_for(a.at.n_padded, 256), 256, 0, s>>>(a);

@@ -90,6 +90,27 @@ void launch_step_post(const StepArgs& a, cudaStream_t s);
 // B (second half), divergence check, step counter.
 void launch_step_end(const StepArgs& a, cudaStream_t s);
 
+// The sub-steps before the forces as one kernel (no constraints), or as one
+// and the pack (each constraint a hydrogen on one heavy atom): the same
+// results as the launches above, bit for bit.
+// Slots are warps of 32: a cluster's heavy atom, then its hydrogens, or single
+// atoms; a cluster stays within its warp.
+struct MoveSlot {
+  int32_t atom;        // padded atom, -1 = empty
+  uint8_t head, k, n;  // lane of the cluster's heavy atom, this atom's constraint (0: heavy or single), constraints
+  uint8_t pad;
+  double d2;           // squared length of constraint k
+};
+struct MoveArgs {
+  const MoveSlot* slots;
+  int32_t n_slots;  // a multiple of 32
+  const double* inv_mass;
+  double tol_sq;
+  int32_t max_iters;
+};
+void launch_step_free(const StepArgs& a, cudaStream_t s);
+void launch_step_move(const StepArgs& a, const MoveArgs& m, cudaStream_t s);
+
 struct ShakeArgs {
   double* x; double* y; double* z;
   const double* rx; const double* ry; const double* rz;
