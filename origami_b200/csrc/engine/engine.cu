@@ -120,6 +120,40 @@ struct DVec {
   }
 };
 
+// Staging of one engine's small host transfers, grown on demand and given back
+// with the engine: plain memory for the first use, page-locked (about 0.1 ms
+// to get) from the second on where it can be had.
+struct HostBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  bool pinned = false;
+  int uses = 0, uses_kept = 0;  // so far (2 = more), and when p was taken
+  HostBuf() = default;
+  HostBuf(const HostBuf&) = delete;
+  HostBuf& operator=(const HostBuf&) = delete;
+  ~HostBuf() { release(); }
+  void release() {
+    if (p && pinned) cudaFreeHost(p);
+    if (p && !pinned) std::free(p);
+    p = nullptr;
+    cap = 0;
+  }
+  bool reserve(size_t bytes) {
+    uses += uses < 2;
+    if (bytes <= cap && uses_kept == uses) return true;
+    release();
+    uses_kept = uses;
+    const size_t want = bytes + bytes / 2;
+    pinned = uses > 1 && cudaHostAlloc(&p, want, cudaHostAllocDefault) == cudaSuccess;
+    if (!pinned) {
+      if (uses > 1) cudaGetLastError();
+      p = std::malloc(want);
+    }
+    if (p) cap = want;
+    return p != nullptr;
+  }
+};
+
 struct TopoCopy {
   int n = 0;
   std::vector<double> charge, rmin, eps, rmin14, eps14, rho, scale, mass;
@@ -186,6 +220,7 @@ struct SysHost {
   std::vector<double> xyz;
   double temperature = 310.0;
   int atom_begin = 0, n_tiles = 0, tile_begin = 0;
+  int64_t real_begin = 0;  // real atoms of the systems before
 };
 
 double deg2rad(double d) { return d * M_PI / 180.0; }
@@ -211,6 +246,11 @@ struct og_engine {
   int64_t n_real = 0;
   DVec<double> stage_a, stage_b;
   DVec<int64_t> stage_f;
+  // one system's coordinates or forces on their way in (host_in; in_done:
+  // its last copy has been read) and out (host_out), by way of epart on the
+  // device, and the status words
+  HostBuf host_in, host_out, host_status;
+  cudaEvent_t in_done = nullptr;
   DVec<float> pq, lj, gb, bs;  // tile-SoA, 4 columns per 32-atom tile
   DVec<double4> origin;
   DVec<ogk::SysState> sys_state;
@@ -326,13 +366,14 @@ struct og_engine {
 
   ~og_engine() {
     for (StepGraph* g : {&step_graph, &force_graph}) g->reset();
+    if (in_done) cudaEventSynchronize(in_done);  // host_in is read until then
     if (own_stream && stream) cudaStreamDestroy(stream);
     for (cudaStream_t* q : {&side, &hi, &aux})
       if (*q) {
         cudaStreamSynchronize(*q);
         cudaStreamDestroy(*q);
       }
-    for (cudaEvent_t ev : {ev_fork, ev_join, ev_join_hi, ev_cut, ev_born, ev_join_aux})
+    for (cudaEvent_t ev : {in_done, ev_fork, ev_join, ev_join_hi, ev_cut, ev_born, ev_join_aux})
       if (ev) cudaEventDestroy(ev);
   }
 
@@ -741,13 +782,23 @@ og_status launch_check(const char* what) {
   return OG_OK;
 }
 
-og_status read_status(og_engine* e, std::vector<ogk::SysState>* out) {
+// The status words to host_status (queue_status), and what they say once the
+// stream has been waited for (status_words).
+og_status queue_status(og_engine* e) {
+  const size_t bytes = sizeof(ogk::SysState) * e->sys.size();
+  if (!e->host_status.reserve(bytes + sizeof(int32_t))) return og_fail(OG_E_NOMEM, "host staging");
+  char* h = static_cast<char*>(e->host_status.p);
+  OG_CUDA(cudaMemcpyAsync(h, e->sys_state.p, bytes, cudaMemcpyDeviceToHost, e->stream));
+  OG_CUDA(cudaMemcpyAsync(h + bytes, e->error_flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream));
+  return OG_OK;
+}
+
+og_status status_words(const og_engine* e, std::vector<ogk::SysState>* out) {
+  const char* h = static_cast<const char*>(e->host_status.p);
   out->resize(e->sys.size());
-  OG_CUDA(cudaMemcpyAsync(out->data(), e->sys_state.p, sizeof(ogk::SysState) * e->sys.size(),
-                          cudaMemcpyDeviceToHost, e->stream));
+  std::memcpy(out->data(), h, sizeof(ogk::SysState) * out->size());
   int32_t err_flag = 0;
-  OG_CUDA(cudaMemcpyAsync(&err_flag, e->error_flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, e->stream));
-  OG_CUDA(cudaStreamSynchronize(e->stream));
+  std::memcpy(&err_flag, h + sizeof(ogk::SysState) * out->size(), sizeof(int32_t));
   if (err_flag & ogk::kStatusTimeout) return og_fail(OG_E_TIMEOUT, "a pair-kernel pipeline wait timed out");
   for (const auto& s : *out)
     if (s.status & ogk::kStatusSasaOverflow)
@@ -755,6 +806,13 @@ og_status read_status(og_engine* e, std::vector<ogk::SysState>* out) {
                                        "caps, 254 transitions per circle, 128 arcs, or the term buffers); its "
                                        "surface term was not evaluated");
   return OG_OK;
+}
+
+og_status read_status(og_engine* e, std::vector<ogk::SysState>* out) {
+  og_status st = queue_status(e);
+  if (st != OG_OK) return st;
+  OG_CUDA(cudaStreamSynchronize(e->stream));
+  return status_words(e, out);
 }
 
 // Fibonacci test points of the Shrake-Rupley sampler (sasa.rs:182-197).
@@ -837,38 +895,32 @@ og_status copy_sys_range(og_engine* e, const DVec<T>& v, int s, T* host) {
   return OG_OK;
 }
 
-// Interleaved xyz <-> SoA device arrays of one system.
+// Interleaved xyz of one system <-> the SoA device arrays: one copy through
+// page-locked memory and one kernel each way.  (Three pageable copies per
+// call took 30 to 70 us and waited for each.)
 og_status get_xyz(og_engine* e, int s, const DVec<double>& a, const DVec<double>& b, const DVec<double>& c,
                   double* out) {
-  const int n = e->sys[s].topo.n;
-  std::vector<double> hx(n), hy(n), hz(n);
-  og_status st;
-  if ((st = copy_sys_range(e, a, s, hx.data())) != OG_OK) return st;
-  if ((st = copy_sys_range(e, b, s, hy.data())) != OG_OK) return st;
-  if ((st = copy_sys_range(e, c, s, hz.data())) != OG_OK) return st;
+  const SysHost& sh = e->sys[s];
+  const size_t bytes = 3 * sizeof(double) * static_cast<size_t>(sh.topo.n);
+  if (!e->host_out.reserve(bytes)) return og_fail(OG_E_NOMEM, "host staging");
+  ogk::launch_gather_xyz(a.p, b.p, c.p, e->real_map.p + sh.real_begin, sh.topo.n, e->epart.p, e->stream);
+  OG_CUDA(cudaMemcpyAsync(e->host_out.p, e->epart.p, bytes, cudaMemcpyDeviceToHost, e->stream));
   OG_CUDA(cudaStreamSynchronize(e->stream));
-  for (int i = 0; i < n; ++i) {
-    out[3 * i] = hx[i];
-    out[3 * i + 1] = hy[i];
-    out[3 * i + 2] = hz[i];
-  }
-  return OG_OK;
+  std::memcpy(out, e->host_out.p, bytes);
+  return launch_check("state gather");
 }
 
 og_status set_xyz(og_engine* e, int s, DVec<double>& a, DVec<double>& b, DVec<double>& c, const double* in) {
   const SysHost& sh = e->sys[s];
-  const int n = sh.topo.n;
-  std::vector<double> hx(n), hy(n), hz(n);
-  for (int i = 0; i < n; ++i) {
-    hx[i] = in[3 * i];
-    hy[i] = in[3 * i + 1];
-    hz[i] = in[3 * i + 2];
-  }
-  OG_CUDA(cudaMemcpyAsync(a.p + sh.atom_begin, hx.data(), sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
-  OG_CUDA(cudaMemcpyAsync(b.p + sh.atom_begin, hy.data(), sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
-  OG_CUDA(cudaMemcpyAsync(c.p + sh.atom_begin, hz.data(), sizeof(double) * n, cudaMemcpyHostToDevice, e->stream));
-  OG_CUDA(cudaStreamSynchronize(e->stream));
-  return OG_OK;
+  const size_t bytes = 3 * sizeof(double) * static_cast<size_t>(sh.topo.n);
+  if (!e->in_done) OG_CUDA(cudaEventCreateWithFlags(&e->in_done, cudaEventDisableTiming));
+  OG_CUDA(cudaEventSynchronize(e->in_done));  // the last call's copy
+  if (!e->host_in.reserve(bytes)) return og_fail(OG_E_NOMEM, "host staging");
+  std::memcpy(e->host_in.p, in, bytes);
+  OG_CUDA(cudaMemcpyAsync(e->epart.p, e->host_in.p, bytes, cudaMemcpyHostToDevice, e->stream));
+  OG_CUDA(cudaEventRecord(e->in_done, e->stream));
+  ogk::launch_scatter_xyz(e->epart.p, e->real_map.p + sh.real_begin, sh.topo.n, a.p, b.p, c.p, e->stream);
+  return launch_check("state scatter");
 }
 
 // Work items of a pass over i-blocks of W tiles in chunks of `chunk` j-tiles.
@@ -1383,7 +1435,7 @@ og_status size_energy_scratch(og_engine* e, cudaStream_t st) {
   for (const auto& s : e->sys) max_t = std::max(max_t, s.n_tiles);
   e->e_chunks = ogk::energy_chunks(e->n_tiles, max_t, e->n_sm);
   const size_t m = static_cast<size_t>(e->e_chunks) * e->n_tiles;
-  OG_CUDA(e->epart.grow(m * kTile, st));
+  OG_CUDA(e->epart.grow(std::max<size_t>(m, 3 * static_cast<size_t>(max_t)) * kTile, st));  // also one system's xyz
   OG_CUDA(e->epair.grow(3 * m, st));
   OG_CUDA(e->epair_count.grow(m, st));
   return OG_OK;
@@ -1409,10 +1461,13 @@ og_status finalize_impl(og_engine* e) {
 
   // ---- layout
   int atom = 0;
+  int64_t real = 0;
   for (auto& s : e->sys) {
     s.atom_begin = atom;
     s.n_tiles = (s.topo.n + kTile - 1) / kTile;
     s.tile_begin = atom / kTile;
+    s.real_begin = real;
+    real += s.topo.n;
     atom += s.n_tiles * kTile;
   }
   e->n_padded = atom;
@@ -2102,26 +2157,22 @@ og_status og_compute_forces(og_engine* e, int32_t s, double* f_out) {
   if (f_out && (s < 0 || s >= static_cast<int32_t>(e->sys.size())))
     return og_fail(OG_E_BADARG, "system index out of range");
   if ((st = eval_forces(e)) != OG_OK) return st;
+  const size_t n3 = f_out ? 3 * static_cast<size_t>(e->sys[s].topo.n) : 0;
+  if (f_out) {
+    const SysHost& sh = e->sys[s];
+    if (!e->host_out.reserve(n3 * sizeof(double))) return og_fail(OG_E_NOMEM, "host staging");
+    ogk::launch_gather_force(e->fx.p, e->fy.p, e->fz.p, e->real_map.p + sh.real_begin, sh.topo.n, e->epart.p,
+                             e->stream);
+    OG_CUDA(cudaMemcpyAsync(e->host_out.p, e->epart.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+  }
+  if (e->p.include_sasa && (st = queue_status(e)) != OG_OK) return st;
+  OG_CUDA(cudaStreamSynchronize(e->stream));
   if (e->p.include_sasa) {
     std::vector<ogk::SysState> hs;
-    if ((st = read_status(e, &hs)) != OG_OK) return st;
+    if ((st = status_words(e, &hs)) != OG_OK) return st;
   }
-  if (f_out) {
-    const int n = e->sys[s].topo.n;
-    std::vector<unsigned long long> h[3];
-    const DVec<unsigned long long>* src[3] = {&e->fx, &e->fy, &e->fz};
-    for (int c = 0; c < 3; ++c) {
-      h[c].resize(n);
-      if ((st = copy_sys_range(e, *src[c], s, h[c].data())) != OG_OK) return st;
-    }
-    OG_CUDA(cudaStreamSynchronize(e->stream));
-    for (int i = 0; i < n; ++i)
-      for (int c = 0; c < 3; ++c)
-        f_out[3 * i + c] = static_cast<double>(static_cast<long long>(h[c][i])) * ogk::kForceUnscale;
-  } else {
-    OG_CUDA(cudaStreamSynchronize(e->stream));
-  }
-  return OG_OK;
+  if (f_out) std::memcpy(f_out, e->host_out.p, n3 * sizeof(double));
+  return launch_check("force evaluation");
 }
 
 og_status og_get_born_radii(og_engine* e, int32_t s, double* radii) {
@@ -2206,12 +2257,15 @@ og_status og_compute_energies(og_engine* e, int32_t s, og_energies* out) {
   if (s < -1 || s >= n_sys) return og_fail(OG_E_BADARG, "system index out of range");
   cudaStream_t stream = e->stream;
   if ((st = enqueue_energies(e, e->p.include_sasa, stream)) != OG_OK) return st;
-  std::vector<double> all(ogk::kEnergyTerms * static_cast<size_t>(n_sys));
-  OG_CUDA(cudaMemcpyAsync(all.data(), e->seg_out.p, sizeof(double) * all.size(), cudaMemcpyDeviceToHost, stream));
+  const size_t bytes = sizeof(double) * ogk::kEnergyTerms * static_cast<size_t>(n_sys);
+  if (!e->host_out.reserve(bytes)) return og_fail(OG_E_NOMEM, "host staging");
+  const double* all = static_cast<const double*>(e->host_out.p);
+  OG_CUDA(cudaMemcpyAsync(e->host_out.p, e->seg_out.p, bytes, cudaMemcpyDeviceToHost, stream));
+  if (e->p.include_sasa && (st = queue_status(e)) != OG_OK) return st;
   OG_CUDA(cudaStreamSynchronize(stream));
   if (e->p.include_sasa) {
     std::vector<ogk::SysState> hs;
-    if ((st = read_status(e, &hs)) != OG_OK) return st;
+    if ((st = status_words(e, &hs)) != OG_OK) return st;
   }
   for (int k = 0; k < n_sys; ++k) {
     if (s >= 0 && k != s) continue;

@@ -16,6 +16,8 @@ void launch_scatter_xyz(const double* in, const int32_t* map, int64_t n, double*
                         cudaStream_t s);
 void launch_gather_fixed(const unsigned long long* a, const unsigned long long* b, const unsigned long long* c,
                          const int32_t* map, int64_t n, int64_t* out, cudaStream_t s);
+void launch_gather_force(const unsigned long long* a, const unsigned long long* b, const unsigned long long* c,
+                         const int32_t* map, int64_t n, double* out, cudaStream_t s);
 void launch_scatter_fixed(const int64_t* in, const int32_t* map, int64_t n, unsigned long long* a,
                           unsigned long long* b, unsigned long long* c, cudaStream_t s);
 
