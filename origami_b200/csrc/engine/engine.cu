@@ -2222,11 +2222,11 @@ og_status enqueue_energies(og_engine* e, bool areas, cudaStream_t stream) {
   const double rc = e->p.nb_cutoff;
   a.kappa = all_nb ? 0.0 : 1.0 / (2.0 * rc * rc * rc);
   a.crf = all_nb ? 0.0 : 3.0 / (2.0 * rc);
+  a.s_max = e->s_max; a.rho_max = e->rho_max;
   a.n_chunks = e->e_chunks; a.part = e->epart.p; a.pair_part = e->epair.p; a.pair_count = e->epair_count.p;
 
   OG_CUDA(cudaMemsetAsync(e->clamp_count.p, 0, sizeof(int32_t) * n_sys, stream));
-  // the tile spheres of the cutoff culls and the surface term
-  if (areas || !all_nb || !all_born) ogk::launch_pack(e->atoms(), false, stream);
+  ogk::launch_pack(e->atoms(), false, stream);  // the tile spheres at the current positions
   ogk::launch_born64(a, stream);
   ogk::launch_born_finalize(e->atoms(), a.part, a.n_chunks, e->born_r64.p, false, e->clamp_count.p, stream);
   ogk::launch_energy64(a, stream);

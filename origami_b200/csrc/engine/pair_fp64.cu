@@ -180,20 +180,41 @@ void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_
 // Energies: one warp owns a 32-atom i-tile and every n_chunks-th j-tile (its
 // j-tiles staged in the warp's shared memory, read back as broadcasts), so a
 // single chain spreads over n_tiles x n_chunks warps.  Bound by the FP64
-// pipe.  Three things cut its work per pair against a closed form per
-// ordered pair (0.60 ms for an energy of a 4 694-atom chain, all pairs):
-//   * the pair energies see each unordered pair once (tiles jt >= it) and
-//     take 1/r from one reciprocal square root;
-//   * distant pairs (a warp vote) need no exponential in the GB term, and in
-//     the descreening integral a short series in s/r instead of two
-//     divisions, a square root and a logarithm;
-//   * with cutoffs, tile pairs whose bounding spheres are apart are skipped.
+// pipe, so what counts is FP64 operations per pair; a closed form per ordered
+// pair with its roots, divisions, logarithm and exponential took 0.60 ms for
+// an energy of a 4 694-atom chain, all pairs.
+//   * The pair energies see each unordered pair once (tiles jt >= it) and
+//     take 1/r from one reciprocal square root.
+//   * Tile pairs are classed by the gap between their bounding spheres: the
+//     distant ones need no exponential in the GB term (and then share q / r
+//     with Coulomb: 20 operations per pair), and in the descreening integral
+//     a short series in u = 1/r^2 instead of two divisions, a square root and
+//     a logarithm (22 operations with 8 terms).
+//   * With cutoffs, tile pairs whose spheres are apart are skipped.
 // Sums run in a fixed order: per lane over its pairs, warp butterflies,
 // then k_energy_totals.
 
 namespace {
 
 constexpr int kEnergyWarps = 4;
+
+// 1 / a and 1 / sqrt(a) to an ulp or so: the special-function unit's
+// approximation (relative error below 2^-21) and one third-order
+// Newton-Householder step, whose error is the cube of that.  Without the
+// library's handling of zero (NaN here, infinity there), which the callers
+// do not need.
+__device__ __forceinline__ double rcp64(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt64(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 
 __device__ __forceinline__ double descreen64(double r, double r2, double inv_r, double rho_i, double s_rho_j) {
   // energy/src/gb.rs:347-369, with 1/r given.
@@ -211,11 +232,12 @@ __device__ __forceinline__ double descreen64(double r, double r2, double inv_r, 
 }
 
 // The same function where the spheres do not overlap (l = r - s), as its
-// series in x = s/r (see k_born): h = -(x^3 / r) sum_k k (2k - 1) / (2k + 1)
-// x^(2 (k - 1)), kTerms terms, w = x^2.  Dropped terms stay below 2^-53 of
-// the first for x < 1/16 with 8 terms (256^-8 * 24 = 1.3e-18) and x < 1/4
-// with 15 (16^-15 * 45 = 3.9e-17).  The closed form loses digits to
-// cancellation at these distances; the series does not.
+// series (see k_born): h = -s^3 u^2 sum_k k (2k - 1) / (2k + 1) w^(k - 1),
+// w = s^2 u, u = 1 / r^2.  Dropped terms stay below 2^-53 of the first: 15
+// terms for s / r < 1/4 (16^-15 * 45 = 3.9e-17), 8 below 1/16 (256^-8 * 24 =
+// 1.3e-18), 6 below 1/32 (1024^-6 * 18), 5 below 1/64 (4096^-5 * 15).  The
+// closed form loses digits to cancellation at these distances; the series
+// does not.
 template <int kTerms>
 __device__ __forceinline__ double descreen_series64(double w) {
   double p = 0.0;
@@ -224,16 +246,40 @@ __device__ __forceinline__ double descreen_series64(double w) {
   return p;
 }
 
-// Tile spheres at least `cutoff` apart (FP64, the margin of k_cut_lists).
-__device__ __forceinline__ bool tiles_apart(double4 oi, double4 oj, double cutoff) {
+// Lower bound on the distance of any atom pair of two tiles (spheres of the
+// current positions, the margin of k_cut_lists).
+__device__ __forceinline__ double tile_gap64(double4 oi, double4 oj) {
   const double dx = oj.x - oi.x, dy = oj.y - oi.y, dz = oj.z - oi.z;
-  const double lim = oi.w + oj.w + cutoff + 1e-3;
-  return dx * dx + dy * dy + dz * dz > lim * lim;
+  return sqrt(dx * dx + dy * dy + dz * dz) - (oi.w + oj.w + 1e-3);
+}
+
+__device__ __forceinline__ double warp_max64(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
 }
 
 struct BornTile {
   double4 p[kTile];  // x, y, z, s rho~
+  double2 s[kTile];  // s^2, s^3
 };
+
+// The negated sum over a distant j-tile.
+template <int kTerms, bool kCut>
+__device__ __forceinline__ double born_far64(const BornTile& t, int nj, double xi, double yi, double zi, double c2) {
+  double acc = 0.0;
+#pragma unroll 2
+  for (int k = 0; k < nj; ++k) {
+    const double4 pj = t.p[k];
+    const double2 sj = t.s[k];
+    const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double u = rcp64(r2);
+    const double h = (u * u * sj.y) * descreen_series64<kTerms>(sj.x * u);
+    if (!kCut || !(r2 > c2)) acc += h;
+  }
+  return acc;
+}
 
 __global__ void __launch_bounds__(kEnergyWarps * 32) k_born64(EnergyArgs a) {
   __shared__ BornTile tiles[kEnergyWarps];
@@ -250,29 +296,42 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_born64(EnergyArgs a) {
   const double xi = a.x[il], yi = a.y[il], zi = a.z[il], rho = a.rho_tilde[il];
   const bool cut = a.born_c2 != INFINITY;
   const double4 oi = a.origin[it];
+  const double gap15 = fmax(4.0 * a.s_max, a.s_max + a.rho_max);
   double acc = 0.0;
   for (int jt = st.x + c; jt < st.x + st.y; jt += a.n_chunks) {
-    if (cut && tiles_apart(oi, a.origin[jt], a.born_cutoff)) continue;
+    const double gap = tile_gap64(oi, a.origin[jt]);
+    if (cut && gap > a.born_cutoff) continue;
     const int j0 = jt * kTile, nj = min(kTile, end - j0);
     __syncwarp();
-    if (lane < nj) t.p[lane] = make_double4(a.x[j0 + lane], a.y[j0 + lane], a.z[j0 + lane], a.srho[j0 + lane]);
+    if (lane < nj) {
+      const double s = a.srho[j0 + lane];
+      t.p[lane] = make_double4(a.x[j0 + lane], a.y[j0 + lane], a.z[j0 + lane], s);
+      t.s[lane] = make_double2(s * s, s * s * s);
+    }
     __syncwarp();
+    if (gap >= gap15) {
+      const double q = gap / a.s_max;  // at least r / s for every pair
+      if (cut) acc -= q >= 16.0 ? born_far64<8, true>(t, nj, xi, yi, zi, a.born_c2)
+                                : born_far64<15, true>(t, nj, xi, yi, zi, a.born_c2);
+      else if (q >= 64.0) acc -= born_far64<5, false>(t, nj, xi, yi, zi, 0.0);
+      else if (q >= 32.0) acc -= born_far64<6, false>(t, nj, xi, yi, zi, 0.0);
+      else if (q >= 16.0) acc -= born_far64<8, false>(t, nj, xi, yi, zi, 0.0);
+      else acc -= born_far64<15, false>(t, nj, xi, yi, zi, 0.0);
+      continue;
+    }
     const int self = il - j0;
     for (int k = 0; k < nj; ++k) {
       const double4 pj = t.p[k];
       const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
       const double r2 = dx * dx + dy * dy + dz * dz;
-      const double inv_r = rsqrt(r2);
+      const double inv_r = rsqrt64(r2);
       const double r = r2 * inv_r;
-      const double x = pj.w * inv_r;
       const bool on = k != self && !(r2 > a.born_c2) && !(r2 < 1e-18);
-      const bool apart = r - pj.w >= rho;
-      const double w = x * x;
       double h;
-      if (__all_sync(0xffffffffu, apart && x < 0.0625)) {
-        h = -(w * x * inv_r) * descreen_series64<8>(w);
-      } else if (__all_sync(0xffffffffu, apart && x < 0.25)) {
-        h = -(w * x * inv_r) * descreen_series64<15>(w);
+      if (__all_sync(0xffffffffu, r - pj.w >= rho && r > 4.0 * pj.w)) {
+        const double2 sj = t.s[k];
+        const double u = inv_r * inv_r;
+        h = -(u * u * sj.y) * descreen_series64<15>(sj.x * u);
       } else {
         h = on ? descreen64(r, r2, inv_r, rho, pj.w) : 0.0;
       }
@@ -292,6 +351,10 @@ struct EnergyTile {
 // parameters (nonbonded.rs:127-169) and the GB pair energy over all pairs
 // (gb.rs:160-173), each unordered pair once.  LJ as sqrt(eps_i eps_j) (r6^2 -
 // 2 r6); every sum without its constant prefactor (k_energy_totals).
+//
+// Once r2 / (4 R_i R_j) >= 40, R_i R_j exp(-r2 / (4 R_i R_j)) < r2 2^-54 (e^-40
+// < 160 2^-54, and the gap only widens), below half an ulp of r2: f_GB = r
+// there, for a whole tile pair when its gap and largest radii say so.
 __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
   __shared__ EnergyTile tiles[kEnergyWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -309,57 +372,83 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
   const double rmi = a.rmin[il], sepi = sqrt(a.eps[il]);
   const double rm14i = a.rmin14[il], sep14i = sqrt(a.eps14[il]);
   const double iRi4 = 0.25 / Ri;
+  const double ri_max = warp_max64(Ri);
   const bool cut = a.nb_c2 != INFINITY;
   const double4 oi = a.origin[it];
   int mref = a.mask_begin[it];
   const int mend = a.mask_begin[it + 1];
-  double lj = 0.0, coul = 0.0, gb = 0.0;
+  // sums without the i atom's factor: LJ (the 1-4 pairs' with it), Coulomb,
+  // GB, and q_j / r of the pairs that count for both
+  double lj = 0.0, lj14 = 0.0, coul = 0.0, gb = 0.0, both = 0.0;
   int pairs = 0;
   for (int jt = it + c; jt < st.x + st.y; jt += a.n_chunks) {
     while (mref < mend && a.mask_refs[mref].j_tile < jt) ++mref;
     uint32_t ex = 0u, m14 = 0u;
-    if (mref < mend && a.mask_refs[mref].j_tile == jt) {
+    const bool masked = mref < mend && a.mask_refs[mref].j_tile == jt;
+    if (masked) {
       const int w = a.mask_refs[mref].offset * kTile + lane;
       ex = a.mask_ex[w];
       m14 = a.mask_14[w];
     }
-    const bool any14 = __any_sync(0xffffffffu, m14 != 0u);
-    const bool nb_tile = !cut || !tiles_apart(oi, a.origin[jt], a.nb_cutoff);
+    const double gap = tile_gap64(oi, a.origin[jt]);
+    const bool nb_tile = !cut || !(gap > a.nb_cutoff);
     const int j0 = jt * kTile, nj = min(kTile, end - j0);
+    double rj = 0.0;
     __syncwarp();
     if (lane < nj) {
       const int j = j0 + lane;
+      rj = a.born_r[j];
       t.p[lane] = make_double4(a.x[j], a.y[j], a.z[j], a.q[j]);
-      t.g[lane] = make_double4(a.rmin[j], sqrt(a.eps[j]), a.born_r[j], 1.0 / a.born_r[j]);
+      t.g[lane] = make_double4(a.rmin[j], sqrt(a.eps[j]), rj, 1.0 / rj);
     }
     __syncwarp();
+    const bool far = gap > 0.0 && gap * gap >= 160.0 * ri_max * warp_max64(rj);
+    if (far && !masked && !(cut && nb_tile)) {
+      if (nb_tile) {
+#pragma unroll 2
+        for (int k = 0; k < nj; ++k) {
+          const double4 pj = t.p[k], gj = t.g[k];
+          const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+          const double inv_r = rsqrt64(dx * dx + dy * dy + dz * dz);
+          const double x = (rmi + gj.x) * inv_r;
+          const double x2 = x * x;
+          const double r6 = x2 * x2 * x2;
+          lj = fma(gj.y, r6 * (r6 - 2.0), lj);
+          both = fma(pj.w, inv_r, both);
+        }
+        pairs += nj;
+      } else {
+#pragma unroll 2
+        for (int k = 0; k < nj; ++k) {
+          const double4 pj = t.p[k];
+          const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
+          gb = fma(pj.w, rsqrt64(dx * dx + dy * dy + dz * dz), gb);
+        }
+      }
+      continue;
+    }
     const int first = jt == it ? lane + 1 : 0;  // the diagonal tile's pairs once
     for (int k = 0; k < nj; ++k) {
       const double4 pj = t.p[k], gj = t.g[k];
       const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
       const double r2 = dx * dx + dy * dy + dz * dz;
       const bool on = valid && k >= first;
-      const double inv_r = rsqrt(r2);
-      // Once r2 / (4 R_i R_j) >= 40, R_i R_j exp(-r2 / (4 R_i R_j)) < r2
-      // 2^-54 (e^-40 < 160 2^-54, and the gap only widens), below half an
-      // ulp of r2: f_GB = r there.
+      const double inv_r = rsqrt64(r2);
       const double xg = r2 * (iRi4 * gj.w);
       double inv_f = inv_r;
-      if (!__all_sync(0xffffffffu, xg >= 40.0)) inv_f = rsqrt(r2 + Ri * gj.z * exp(-xg));
+      if (!__all_sync(0xffffffffu, xg >= 40.0)) inv_f = rsqrt64(r2 + Ri * gj.z * exp(-xg));
       if (on) gb += pj.w * inv_f;
       if (!nb_tile) continue;
       const bool nb = on && !(r2 > a.nb_c2) && !((ex >> k) & 1u);
       if (!__any_sync(0xffffffffu, nb)) continue;
-      double rmin = rmi + gj.x, se = sepi * gj.y;
-      if (any14 && ((m14 >> k) & 1u)) {
-        rmin = rm14i + a.rmin14[j0 + k];
-        se = sep14i * sqrt(a.eps14[j0 + k]);
-      }
       if (nb) {
-        const double x = rmin * inv_r;
+        const bool is14 = (m14 >> k) & 1u;
+        const double x = (is14 ? rm14i + a.rmin14[j0 + k] : rmi + gj.x) * inv_r;
         const double x2 = x * x;
         const double r6 = x2 * x2 * x2;
-        lj += se * (r6 * (r6 - 2.0));
+        const double e = r6 * (r6 - 2.0);
+        if (is14) lj14 += sep14i * sqrt(a.eps14[j0 + k]) * e;
+        else lj += gj.y * e;
         const double rf = cut ? fma(a.kappa, r2, inv_r) - a.crf : inv_r;
         if (pj.w != 0.0) coul += pj.w * rf;
         ++pairs;
@@ -367,7 +456,9 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
     }
   }
   // a charge of zero contributes nothing, whatever its pairs
-  double v[3] = {valid ? lj : 0.0, valid && qi != 0.0 ? qi * coul : 0.0, valid && qi != 0.0 ? qi * gb : 0.0};
+  const bool charged = valid && qi != 0.0;
+  double v[3] = {valid ? fma(sepi, lj, lj14) : 0.0, charged ? qi * (coul + both) : 0.0, charged ? qi * (gb + both) : 0.0};
+  if (!valid) pairs = 0;
   for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
@@ -383,7 +474,7 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
 
 // One block per (system, term): the sums of og_energies in kJ/mol, pair and
 // clamp counts as doubles, out[term * n_sys + system].
-constexpr int kTotalThreads = 256;
+constexpr int kTotalThreads = 1024;  // one system has a block per term: 21 us with 256, the longest sum's loads in turn
 
 __global__ void __launch_bounds__(kTotalThreads) k_energy_totals(EnergyArgs a, EnergyTotals t) {
   const int sys = blockIdx.x, term = blockIdx.y;

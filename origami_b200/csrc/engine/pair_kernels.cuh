@@ -136,6 +136,7 @@ struct EnergyArgs {
   double nb_cutoff, nb_c2;      // A and A^2; INFINITY = all pairs
   double born_cutoff, born_c2;
   double kappa, crf;  // reaction field constants (0 without cutoff)
+  double s_max, rho_max;  // largest srho and rho_tilde of any atom
   // Each i-tile's j-tiles are dealt to n_chunks warps.  part: their Born
   // integrals, [n_chunks][padded atoms]; pair_part: their LJ, Coulomb and GB
   // sums, [3][n_tiles][n_chunks], and pair_count their LJ pairs.
