@@ -21,7 +21,8 @@
 //    circles lie strictly inside the larger cap, where they only split
 //    buried segments.  The exposed arcs and vertices are unchanged.
 //  * A circle that the other caps bury all around is dropped before its
-//    transitions are built (cover_pair): it has no exposed segment.
+//    transitions are built: it has no exposed segment.  Of the others only
+//    the crossings that can bound an exposed segment are built.
 //  * Transitions on a circle are ordered by a pseudo-angle (monotone in the
 //    reference's atan2 angle, one division instead of an atan2), and the
 //    exposure test point of the segment from a to b -- a rotated by half the
@@ -30,6 +31,9 @@
 //    exposed arcs' central angles.
 //  * The gradient of A_i is taken term by term in reverse mode (sasa_geom.h)
 //    instead of one forward directional derivative per (atom, axis).
+//  * Clear cases of the three searches above (caps, contained caps, buried
+//    bins) are decided in FP32 with margins above its errors; what bounds an
+//    area or enters a gradient is FP64 throughout.
 #include <algorithm>
 #include <cstddef>
 #include <cmath>
@@ -50,7 +54,7 @@ using ogsasa::norm2;
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 4;
-constexpr int kSasaBatch = 32;        // circles per arrangement batch
+constexpr int kSasaBatch = 16;        // circles per arrangement batch (an atom has 4 to 6 to process)
 constexpr uint8_t kNoOther = 0xFF;    // pseudo entry of a transition-free circle
 constexpr int32_t kContained = 1 << 16;  // circle inside a cap it does not cross
 constexpr int32_t kCountMask = kContained - 1;
@@ -59,6 +63,9 @@ constexpr int32_t kCountMask = kContained - 1;
 constexpr int kMaskCircles = 56;
 constexpr uint64_t kMaskContained = 1ull << 63;
 constexpr double kPi = 3.14159265358979323846;
+// angular bins of a circle in which its burial is recorded (below)
+constexpr int kCoverBins = 32;
+using CoverMask = uint32_t;
 
 // Optional per-phase cycle counters of the boundary kernels (measurement
 // builds only: -DOG_SASA_PHASE_CLOCKS=1).  Lane 0 of each warp accumulates
@@ -125,7 +132,6 @@ __device__ __forceinline__ bool contains_strict(Cap c, D3 p) { return dot(p, c.a
 // pass (each ordered pair) classify every pair bit for bit alike.
 struct PairClass {
   double sigma, denom;
-  double nn;  // c_sq denom
   int count;  // transitions: 0, 1 (tangent) or 2
 };
 
@@ -133,14 +139,12 @@ __device__ __forceinline__ PairClass classify(Cap c1, Cap c2) {
   PairClass r;
   r.sigma = __fma_rn(c1.axis.x, c2.axis.x, __fma_rn(c1.axis.y, c2.axis.y, __dmul_rn(c1.axis.z, c2.axis.z)));
   r.denom = __fma_rn(-r.sigma, r.sigma, 1.0);
-  r.nn = 0.0;
   r.count = 0;
   if (fabs(r.denom) < 1e-12) return r;
   // every step is symmetric in the two caps, so (1, 2) and (2, 1) agree too
   const double t = __fma_rn(2.0 * r.sigma, __dmul_rn(c1.c, c2.c), r.denom);
   const double nn = __dsub_rn(t, __dadd_rn(__dmul_rn(c1.c, c1.c), __dmul_rn(c2.c, c2.c)));
   const double eps = 1e-9 * r.denom;
-  r.nn = nn;
   r.count = nn > eps ? 2 : (nn >= -eps ? 1 : 0);
   return r;
 }
@@ -257,6 +261,9 @@ struct WarpSmemT {
   uint8_t live[kCaps];
   // live circles that may have an exposed segment (indices into live)
   uint8_t circ[kCaps];
+  // buried bins of the circles in circ (the first kCoverKept of them)
+  static constexpr int kCoverKept = 24;
+  CoverMask circ_cover[kCoverKept];
   // per live circle either its transitions (low 16 bits) and kContained,
   // or -- up to kMaskCircles live circles, no tangent pair -- the mask of
   // the live circles it crosses (bit lm) and kMaskContained
@@ -264,30 +271,47 @@ struct WarpSmemT {
     int32_t tcnt[kCaps];
     uint64_t xmask[kCaps / 2];
   };
-  // transitions of the batch of circles being processed: unit radial
-  // direction, sort key (quantised angle over the slot, SlotKey), the other
-  // cap, the batch circle, the sorted order and each entry's rank in it
-  double tx[kTrans], ty[kTrans], tz[kTrans];
-  uint32_t tkey[kTrans];
-  uint8_t tother[kTrans];
-  uint8_t tseg[kTrans];
-  uint8_t torder[kTrans];
-  uint8_t trank[kTrans];
-  // a leaving crossing's entering partner (the other slot of its pair), or
-  // kNoOther when the pair is not one clean enter/leave crossing
-  uint8_t tpart[kTrans];
-  // per batch circle: first entry, entries kept after de-duplication,
-  // transition-free circles before it, sin(alpha) and 1 / sin(alpha)
-  uint16_t sbeg[kSasaBatch + 1];
-  uint8_t skept[kSasaBatch], zpre[kSasaBatch];
-  double bsk[kSasaBatch], binv[kSasaBatch];
-  // crossing toggle of each transition, the toggles up to it in angular
-  // order, and per batch circle the mode (0: burial
-  // depth by toggles, 1: explicit midpoint tests) and the depth before its
-  // first transition
-  int8_t ttog[kTrans], tdep[kTrans];
-  int32_t bmode[kSasaBatch];
-  int32_t bbase[kSasaBatch];
+  union {
+    // until the circles to process are known: FP32 copies of the caps (axis,
+    // cos alpha; after the nested-cap cull of the live ones), buried bins,
+    // neighbours waiting for their cap to be built
+    struct {
+      float4 fcap[kCaps];
+      union {
+        int32_t queue[96];
+        struct {
+          CoverMask cover[kCaps];    // buried bins of the circles in circ
+          uint64_t keep[kCaps / 2];  // and the crossings kept of them
+        };
+      };
+    };
+    struct {
+      // transitions of the batch of circles being processed: unit radial
+      // direction, sort key (quantised angle over the slot, SlotKey), the other
+      // cap, the batch circle, the sorted order and each entry's rank in it
+      double tx[kTrans], ty[kTrans], tz[kTrans];
+      uint32_t tkey[kTrans];
+      uint8_t tother[kTrans];
+      uint8_t tseg[kTrans];
+      uint8_t torder[kTrans];
+      uint8_t trank[kTrans];
+      // a leaving crossing's entering partner (the other slot of its pair), or
+      // kNoOther when the pair is not one clean enter/leave crossing
+      uint8_t tpart[kTrans];
+      // per batch circle: first entry, entries kept after de-duplication,
+      // transition-free circles before it, sin(alpha) and 1 / sin(alpha)
+      uint16_t sbeg[kSasaBatch + 1];
+      uint8_t skept[kSasaBatch], zpre[kSasaBatch];
+      double bsk[kSasaBatch], binv[kSasaBatch];
+      // crossing toggle of each transition, the toggles up to it in angular
+      // order, and per batch circle the mode (0: burial
+      // depth by toggles, 1: explicit midpoint tests) and the depth before its
+      // first transition
+      int8_t ttog[kTrans], tdep[kTrans];
+      int32_t bmode[kSasaBatch];
+      int32_t bbase[kSasaBatch];
+    };
+  };
   // exposed arcs
   double a_theta[kArcs], a_sx[kArcs], a_sy[kArcs], a_sz[kArcs];
   uint8_t a_cap[kArcs], a_full[kArcs], a_vis[kArcs];
@@ -337,74 +361,100 @@ __device__ __forceinline__ int32_t circle_tally(const W& w, int li, bool masks) 
 
 // ------------------------------------------------------- buried circles
 // On the circle of cap k, a cap m that it crosses buries one interval.  The
-// circle's angle range is divided into 64 bins of the pseudo-angle; each
-// crossing pair sets, on both circles, the bins that lie wholly inside its
-// interval, and a circle whose 64 bins are all set is buried all around: it
-// has no exposed segment, so none of its transitions is built, sorted or
-// tested.  Protein atoms have 20 to 50 live circles and a handful of exposed
-// arcs, so most circles go this way (about 15 in 20 on the relaxed 300-residue
-// chain, which took 546 transitions per atom before).
+// circle's angle range is divided into kCoverBins bins of the pseudo-angle;
+// every crossing cap sets the bins that lie wholly inside its interval, and a
+// circle whose bins are all set is buried all around: it has no exposed
+// segment, so none of its transitions is built, sorted or tested.  Protein
+// atoms have 20 to 50 live circles and a handful of exposed arcs, so most
+// circles go this way.
 //
 // With sigma = a_k.a_m, the interval is centred on the direction of a_m
-// projected on the circle's plane, (wx, wy) in the circle's frame (fu, fv) of
-// slot_frame, and its half width has cosine : sine = (c_m - c_k sigma) :
-// sqrt(nn) (nn as in classify; the squares sum to (1 - c_k^2) denom), so the
-// end points follow without a division or an arc function.  All of it is
-// FP32, from FP64 differences rounded once: each end's pseudo-angle is within
-// 4e-6 of the exact one, and bins are taken kCoverMargin / 16 = 2.4e-4 inside
-// the interval.  A point there is inside cap m by more than
-// (1 - c_k^2)^(1/2) denom^(1/2) 2e-8, above the 1e-12 of the exposure tests
-// for the pairs used here.
-constexpr float kCoverMargin = 1.0f / 256.0f;  // of a bin
+// projected on the circle's plane, (wx, wy) in an orthonormal frame, and its
+// half width has cosine : sine = (c_m - c_k sigma) : sqrt(nn) (nn as in
+// classify; the squares sum to R^2 = (1 - c_k^2) (1 - sigma^2)), so the end
+// points follow without an arc function.  All in FP32 from rounded caps: nn is
+// good to 7e-7, so for nn > 1e-3 and R > 0.1 (the pairs used) an end's angle
+// is good to 1.5e-4, and bins are taken kCoverMargin, 9.8e-4 rad or more,
+// inside the interval.  A point there is inside cap m by more than R (8e-4)^2
+// / 2 = 3e-8, far above the 1e-12 of the exposure tests.
+constexpr float kCoverMargin = 9.8e-4f * (kCoverBins / 4);  // in bins
 
+// Single special-function instructions (1 ulp class, within the error above).
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The pseudo-angle of (x, y) in bins, [0, kCoverBins].
 __device__ __forceinline__ float cover_bin(float x, float y) {
-  const float d = fabsf(x) + fabsf(y);
-  const float r = __fdividef(x, d);
-  return 16.0f * ((y >= 0.0f ? 1.0f - r : r - 1.0f) + 2.0f);
+  constexpr float q = kCoverBins / 4;
+  const float r = x * rcp_approx(fabsf(x) + fabsf(y));
+  return y >= 0.0f ? fmaf(-q, r, 3.0f * q) : fmaf(q, r, q);
 }
 
-// Bins [0, b) of 64.
-__device__ __forceinline__ uint64_t bins_below(int b) { return b >= 64 ? ~0ull : (b <= 0 ? 0ull : (1ull << b) - 1ull); }
-
-// The bins of circle k that cap m buries; root = sqrt(nn).
-__device__ __forceinline__ uint64_t covered_bins(Cap ck, Cap cm, double sigma, float root) {
-  const D3 a = ck.axis, b = cm.axis;
-  const double ax = fabs(a.x), ay = fabs(a.y), az = fabs(a.z);
-  // b.fu and b.fv of slot_frame(a): e - a (a.e) and a x e for helper axis e
-  double u, v;
-  if (ax < ay && ax < az) {
-    u = b.x - a.x * sigma;
-    v = b.y * a.z - b.z * a.y;
-  } else if (ay < az) {
-    u = b.y - a.y * sigma;
-    v = b.z * a.x - b.x * a.z;
-  } else {
-    u = b.z - a.z * sigma;
-    v = b.x * a.y - b.y * a.x;
-  }
-  const float wx = __double2float_rn(u), wy = __double2float_rn(v);
-  const float h = __double2float_rn(cm.c - ck.c * sigma);
-  if (!(h * h + root * root > 1e-6f)) return 0ull;
-  const float ts = cover_bin(h * wx + root * wy, h * wy - root * wx);
-  const float te = cover_bin(h * wx - root * wy, h * wy + root * wx);
-  const int bs = __float2int_ru(ts + kCoverMargin), be = __float2int_rd(te - kCoverMargin);
-  if (te > ts + kCoverMargin) return be > bs ? bins_below(be) & ~bins_below(bs) : 0ull;
-  if (ts > te + kCoverMargin) return ~bins_below(bs) | bins_below(be);
-  return 0ull;  // the ends coincide to rounding
+// Bins [0, b).
+__device__ __forceinline__ CoverMask bins_below(int b) {
+  return b >= kCoverBins ? ~CoverMask{0} : (CoverMask{1} << max(b, 0)) - CoverMask{1};
 }
 
-__device__ __forceinline__ void cover_or(uint64_t* cover, int li, uint64_t m) {
-  unsigned* p = reinterpret_cast<unsigned*>(cover + li);
-  const unsigned lo = static_cast<unsigned>(m), hi = static_cast<unsigned>(m >> 32);
-  if (lo) atomicOr(p, lo);
-  if (hi) atomicOr(p + 1, hi);
+// A circle as the cover pass sees it: cap a (axis, cos alpha) and the frame
+// (f, g) of its plane (Duff et al., Building an Orthonormal Basis, Revisited,
+// 2017).
+struct CoverCircle {
+  float4 a;
+  float fx, fy, fz, gx, gy, gz;
+};
+__device__ __forceinline__ CoverCircle cover_circle(float4 a) {
+  CoverCircle c;
+  c.a = a;
+  const float sgn = copysignf(1.0f, a.z);
+  const float q = __fdividef(-1.0f, sgn + a.z);
+  const float b = a.x * a.y * q;
+  c.fx = 1.0f + sgn * a.x * a.x * q;
+  c.fy = sgn * b;
+  c.fz = -sgn * a.x;
+  c.gx = b;
+  c.gy = sgn + a.y * a.y * q;
+  c.gz = -a.y;
+  return c;
 }
 
-// Sets bit b of circle li's crossing mask by a 32-bit atomic on the word
-// holding it (little-endian halves), which shared memory does natively.
+// The ends of the interval of circle c that cap b buries, in bins; false for
+// pairs outside the limits above and ends that coincide to rounding.
+__device__ __forceinline__ bool buried_interval(const CoverCircle& c, float4 b, float sigma, float nn, float* ts,
+                                                float* te) {
+  const float h = b.w - c.a.w * sigma;
+  const float root = sqrt_approx(nn);
+  const float wx = b.x * c.fx + b.y * c.fy + b.z * c.fz, wy = b.x * c.gx + b.y * c.gy + b.z * c.gz;
+  *ts = cover_bin(h * wx + root * wy, h * wy - root * wx);
+  *te = cover_bin(h * wx - root * wy, h * wy + root * wx);
+  return nn > 1e-3f && h * h + nn > 1e-2f && fabsf(*ts - *te) > kCoverMargin;
+}
+// The bins wholly inside the interval from ts counter-clockwise to te.
+__device__ __forceinline__ CoverMask covered_bins(float ts, float te) {
+  const CoverMask from = ~bins_below(__float2int_ru(ts + kCoverMargin)),
+                  to = bins_below(__float2int_rd(te - kCoverMargin));
+  return te > ts ? from & to : from | to;
+}
+// Whether an interval end lies in, or within twice the margin of, a bin that
+// `cover` leaves open.
+__device__ __forceinline__ bool end_open(float t, CoverMask cover) {
+  const int b0 = __float2int_rd(t - 2.0f * kCoverMargin) & (kCoverBins - 1),
+            b1 = __float2int_rd(t + 2.0f * kCoverMargin) & (kCoverBins - 1);
+  return !((cover >> b0) & 1u) || !((cover >> b1) & 1u);
+}
+
+// Sets bit b of keep[j] by a 32-bit atomic on the word holding it
+// (little-endian halves), which shared memory does natively.
 template <class W>
-__device__ __forceinline__ void mask_or(W& w, int li, int b) {
-  atomicOr(reinterpret_cast<unsigned*>(&w.xmask[li]) + (b >> 5), 1u << (b & 31));
+__device__ __forceinline__ void keep_or(W& w, int j, int b) {
+  atomicOr(reinterpret_cast<unsigned*>(&w.keep[j]) + (b >> 5), 1u << (b & 31));
 }
 
 enum Outcome { kExposed = 0, kBuried = 1, kBounded = 2, kInvalid = 3 };
@@ -501,8 +551,53 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   const int2 st = a.sys_tiles[sys];
 
   // ---- caps (build_caps), neighbours in ascending atom order
-  int n_caps = 0;
+  int n_caps = 0, queued = 0;
   bool enclosed = false;
+  auto near_atom = [&](int j) {
+    const double dx = a.x[j] - pi.x, dy = a.y[j] - pi.y, dz = a.z[j] - pi.z, rs = ri + a.radius[j];
+    return j != i && a.atom_sys[j] >= 0 && dx * dx + dy * dy + dz * dz <= rs * rs * (1.0 + 1e-12);
+  };
+  // caps of the first n queued neighbours
+  auto make_caps = [&](int n) {
+    bool is_cap = false;
+    int j = 0;
+    double ax = 0.0, ay = 0.0, az = 0.0, ca = 0.0;
+    if (lane < n) {
+      j = w.queue[lane];
+      const double dx = a.x[j] - pi.x, dy = a.y[j] - pi.y, dz = a.z[j] - pi.z;
+      const double rj = a.radius[j];
+      // d and 1/d from one reciprocal square root (d = 0 exactly for
+      // coincident centres); the quotients by d as products
+      const double d2 = dx * dx + dy * dy + dz * dz;
+      const double inv_d = rsqrt(d2);
+      const double d = d2 > 0.0 ? d2 * inv_d : 0.0;
+      if (d <= ri + rj) {
+        if (d + ri <= rj) {
+          enclosed = true;
+        } else if (!(d + rj <= ri || d >= ri + rj)) {
+          ca = (d2 + ri * ri - rj * rj) * (inv_d * half_inv_ri);
+          is_cap = ca >= -1.0 && ca <= 1.0;
+          ax = dx * inv_d;
+          ay = dy * inv_d;
+          az = dz * inv_d;
+        }
+      }
+    }
+    const unsigned caps = __ballot_sync(kFull, is_cap);
+    if (is_cap) {
+      const int slot = n_caps + __popc(caps & ((1u << lane) - 1u));
+      if (slot < W::kCaps) {
+        w.cx[slot] = ax;
+        w.cy[slot] = ay;
+        w.cz[slot] = az;
+        w.cc[slot] = ca;
+        w.owner[slot] = j;
+        w.fcap[slot] = make_float4(static_cast<float>(ax), static_cast<float>(ay), static_cast<float>(az),
+                                   static_cast<float>(ca));
+      }
+    }
+    n_caps += __popc(caps);
+  };
   for (int t0 = 0; t0 < st.y; t0 += 32) {
     const int t = t0 + lane;
     bool hit = false;
@@ -513,66 +608,38 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       hit = dx * dx + dy * dy + dz * dz <= lim * lim;
     }
     unsigned hits = __ballot_sync(kFull, hit);
-    // the atoms of two hit tiles per trip (independent loads in flight); the
-    // caps are written in ascending atom order, the first tile's first
-    struct Nb {
-      double x, y, z, r;
-      bool ok;
-    };
-    auto load = [&](int j) {
-      return Nb{a.x[j], a.y[j], a.z[j], a.radius[j], j != i && a.atom_sys[j] >= 0};
-    };
-    auto probe = [&](const Nb& n, double* ax, double* ay, double* az, double* ca) {
-      if (!n.ok) return false;
-      const double dx = n.x - pi.x, dy = n.y - pi.y, dz = n.z - pi.z;
-      const double rj = n.r;
-      // d and 1/d from one reciprocal square root (d = 0 exactly for
-      // coincident centres); the quotients by d as products
-      const double d2 = dx * dx + dy * dy + dz * dz;
-      const double inv_d = rsqrt(d2);
-      const double d = d2 > 0.0 ? d2 * inv_d : 0.0;
-      if (d > ri + rj) return false;
-      if (d + ri <= rj) {
-        enclosed = true;
-        return false;
-      }
-      if (d + rj <= ri || d >= ri + rj) return false;
-      *ca = (d2 + ri * ri - rj * rj) * (inv_d * half_inv_ri);
-      if (!(*ca >= -1.0 && *ca <= 1.0)) return false;
-      *ax = dx * inv_d;
-      *ay = dy * inv_d;
-      *az = dz * inv_d;
-      return true;
-    };
-    auto put_cap = [&](bool is_cap, int j, double ax, double ay, double az, double ca) {
-      const unsigned caps = __ballot_sync(kFull, is_cap);
-      if (is_cap) {
-        const int slot = n_caps + __popc(caps & ((1u << lane) - 1u));
-        if (slot < W::kCaps) {
-          w.cx[slot] = ax;
-          w.cy[slot] = ay;
-          w.cz[slot] = az;
-          w.cc[slot] = ca;
-          w.owner[slot] = j;
-        }
-      }
-      n_caps += __popc(caps);
-    };
+    // the atoms of two hit tiles per trip (independent loads in flight);
+    // those within R_i + R_j (with a margin) queue up in ascending order and
+    // are made into caps 32 at a time, so that the root and the quotients
+    // run with every lane busy (a hit tile has about four neighbours)
     while (hits) {
       const int b = __ffs(hits) - 1;
       hits &= hits - 1;
       const int b2 = hits ? __ffs(hits) - 1 : -1;
       if (b2 >= 0) hits &= hits - 1;
       const int j = (st.x + t0 + b) * 32 + lane;
-      const int j2 = (st.x + t0 + b2) * 32 + lane;
-      double ax = 0.0, ay = 0.0, az = 0.0, ca = 0.0, ax2 = 0.0, ay2 = 0.0, az2 = 0.0, ca2 = 0.0;
-      const Nb n1 = load(j), n2 = load(b2 >= 0 ? j2 : j);
-      const bool c1 = probe(n1, &ax, &ay, &az, &ca);
-      const bool c2 = b2 >= 0 && probe(n2, &ax2, &ay2, &az2, &ca2);
-      put_cap(c1, j, ax, ay, az, ca);
-      if (b2 >= 0) put_cap(c2, j2, ax2, ay2, az2, ca2);
+      const int j2 = b2 >= 0 ? (st.x + t0 + b2) * 32 + lane : j;
+      const bool c1 = near_atom(j), c2 = near_atom(j2) && b2 >= 0;
+      const unsigned m1 = __ballot_sync(kFull, c1), m2 = __ballot_sync(kFull, c2);
+      const unsigned below = (1u << lane) - 1u;
+      if (c1) w.queue[queued + __popc(m1 & below)] = j;
+      queued += __popc(m1);
+      if (c2) w.queue[queued + __popc(m2 & below)] = j2;
+      queued += __popc(m2);
+      __syncwarp();
+      while (queued >= 32) {
+        make_caps(32);
+        const int rest = queued - 32;
+        const int v0 = lane < rest ? w.queue[32 + lane] : 0, v1 = lane + 32 < rest ? w.queue[64 + lane] : 0;
+        __syncwarp();
+        if (lane < rest) w.queue[lane] = v0;
+        if (lane + 32 < rest) w.queue[32 + lane] = v1;
+        __syncwarp();
+        queued = rest;
+      }
     }
   }
+  make_caps(queued);
   ph.mark(0);
   ph.count(10, n_caps);
   if (__any_sync(kFull, enclosed)) return kBuried;
@@ -581,30 +648,29 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   __syncwarp();
 
   // ---- drop caps whose circle lies inside another cap: alpha_k < alpha_m
-  // and angle(axis_k, axis_m) < alpha_m - alpha_k, i.e. sigma - c_k c_m -
-  // margin > s_k s_m, compared squared (both sides positive)
+  // and angle(axis_k, axis_m) < alpha_m - alpha_k, i.e. sigma - c_k c_m >
+  // s_k s_m, compared squared (both sides positive).  In FP32 with a margin
+  // of 1e-4 on the left, for products s_k s_m above 0.01: the errors (4e-7
+  // on the left, 4e-7 / (2 s_k s_m) on the right) stay well below it, so
+  // only contained circles go; one that is kept within the margin changes
+  // nothing but the work.
   // Each lane tests two caps (k and k + 32) against the caps m in one pass,
   // so a cap m's data is read once for both; survivors keep ascending order.
   int n_live = 0;
   for (int k0 = 0; k0 < n_caps; k0 += 64) {
     const int ka = k0 + lane, kb = k0 + 32 + lane;
     bool la = ka < n_caps, lb = kb < n_caps;
-    const double ca = la ? w.cc[ka] : 0.0, cb = lb ? w.cc[kb] : 0.0;
-    const double sa2 = 1.0 - ca * ca, sb2 = 1.0 - cb * cb;
-    const D3 aa = la ? D3{w.cx[ka], w.cy[ka], w.cz[ka]} : D3{};
-    const D3 ab = lb ? D3{w.cx[kb], w.cy[kb], w.cz[kb]} : D3{};
-    for (int m = 0; m < n_caps && (la || lb); ++m) {
-      const double cm = w.cc[m];
-      const D3 am = {w.cx[m], w.cy[m], w.cz[m]};
-      const double sm2 = 1.0 - cm * cm;
-      if (la && m != ka && ca > cm) {
-        const double lhs = dot(aa, am) - cm * ca - 1e-6;
-        if (lhs > 0.0 && lhs * lhs > sa2 * sm2) la = false;
-      }
-      if (lb && m != kb && cb > cm) {
-        const double lhs = dot(ab, am) - cm * cb - 1e-6;
-        if (lhs > 0.0 && lhs * lhs > sb2 * sm2) lb = false;
-      }
+    const float4 fa = la ? w.fcap[ka] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+    const float4 fb = lb ? w.fcap[kb] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
+    const float sa2 = 1.0f - fa.w * fa.w, sb2 = 1.0f - fb.w * fb.w;
+#pragma unroll 2
+    for (int m = 0; m < n_caps; ++m) {
+      const float4 fm = w.fcap[m];
+      const float sm2 = 1.0f - fm.w * fm.w;
+      const float ha = fa.x * fm.x + fa.y * fm.y + fa.z * fm.z - fa.w * fm.w - 1e-4f, pa = sa2 * sm2;
+      const float hb = fb.x * fm.x + fb.y * fm.y + fb.z * fm.z - fb.w * fm.w - 1e-4f, pb = sb2 * sm2;
+      if (fa.w > fm.w && pa > 1e-4f && ha > 0.0f && ha * ha > pa) la = false;
+      if (fb.w > fm.w && pb > 1e-4f && hb > 0.0f && hb * hb > pb) lb = false;
     }
     const unsigned below = (1u << lane) - 1u;
     const unsigned lva = __ballot_sync(kFull, la);
@@ -619,8 +685,8 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   ph.count(11, n_live);
 
   // ---- boundary arcs (find_boundary), a batch of circles at a time: the
-  // transitions of every circle are counted first (each ordered pair once,
-  // by the same classification the writing pass uses), then consecutive
+  // transitions of every circle are counted first, as the writing pass's
+  // classification has them, then consecutive
   // circles whose transition lists fit the buffer are processed together --
   // their transitions written, sorted and tested across all lanes -- and the
   // exposed arcs appended in circle order and, within a circle, in angular
@@ -634,79 +700,112 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // p / n_live by a float reciprocal: exact here, since p + 0.5 keeps the
   // quotient at least 0.5 / n_live from an integer, far above the rounding
   const float inv_live = 1.0f / static_cast<float>(n_live);
-  bool masks = n_live <= kMaskCircles;
-  // buried bins per live circle, over the transition arrays (not in use yet)
-  static_assert(offsetof(W, ty) == offsetof(W, tx) + sizeof(w.tx) &&
-                    sizeof(w.tx) + sizeof(w.ty) >= W::kCaps * sizeof(uint64_t),
-                "cover scratch");
-  uint64_t* cover = reinterpret_cast<uint64_t*>(w.tx);
-  for (int li = lane; li < n_live; li += 32) cover[li] = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    if (masks) {
-      for (int li = lane; li < n_live; li += 32) w.xmask[li] = 0;
-    } else {
-      for (int li = lane; li < n_live; li += 32) w.tcnt[li] = 0;
-    }
+  for (int l0 = 0; l0 < n_live; l0 += 32) {  // live[k] >= k: a trip overwrites nothing a later one reads
+    const float4 f = l0 + lane < n_live ? w.fcap[w.live[l0 + lane]] : float4{};
     __syncwarp();
-    // the counts are symmetric (circle k crosses cap m where circle m
-    // crosses cap k), so each unordered pair is classified once: pair p of
-    // the n(n-1)/2 with li < lm, row-major.  Row l starts at
-    // S(l) = l (2n - 1 - l) / 2; the row of p is the floor of the smaller
-    // root of S(l) = p, corrected by one step for the rounding of sqrtf
-    // (the discriminant is an exact float: below 2^24).
-    const int n_pairs = n_live * (n_live - 1) / 2;
-    const float tn = static_cast<float>(2 * n_live - 1);
+    if (l0 + lane < n_live) w.fcap[l0 + lane] = f;
+    __syncwarp();
+  }
+  bool masks = n_live <= kMaskCircles;
+  int n_circ = 0;  // the circles left to process, in live order
+  for (int pass = 0; pass < 2; ++pass) {
+    // Lane = circle, all caps in turn (read as broadcasts): the lane keeps
+    // its circle's crossings and buried bins in registers.  (Each unordered
+    // pair once, with shared-memory atomics on both circles, took three times
+    // as long.)
+    n_circ = 0;
     bool tangent = false;
-    for (int p = lane; p < n_pairs; p += 32) {
-      int li = static_cast<int>((tn - sqrtf(tn * tn - 8.0f * static_cast<float>(p))) * 0.5f);
-      li = max(0, min(li, n_live - 2));
-      if ((li + 1) * (2 * n_live - 2 - li) / 2 <= p) {
-        ++li;
-      } else if (li * (2 * n_live - 1 - li) / 2 > p) {
-        --li;
+    for (int l0 = 0; l0 < n_live; l0 += 32) {
+      const int li = l0 + lane;
+      const bool own = li < n_live;
+      const CoverCircle c = cover_circle(w.fcap[own ? li : 0]);
+      CoverMask cover = 0;
+      uint64_t mask = 0;
+      int32_t tally = 0;
+      bool inside = false;  // in a cap without crossing its rim
+      for (int mb = 0; mb < n_live; mb += 32) {
+        const int mn = min(32, n_live - mb);
+        unsigned cross = 0, unclear = 0;
+#pragma unroll 2
+        for (int q = 0; q < mn; ++q) {
+          const float4 b = w.fcap[mb + q];
+          const unsigned bit = 1u << q;
+          const float sg = c.a.x * b.x + c.a.y * b.y + c.a.z * b.z;
+          const float nn = fmaf(2.0f * sg, c.a.w * b.w, fmaf(-sg, sg, 1.0f)) - (c.a.w * c.a.w + b.w * b.w);
+          // FP32 decides the clear cases (nn is good to 7e-7)
+          cross |= nn > 1e-5f ? bit : 0u;
+          unclear |= !(fabsf(nn) > 1e-5f) || (nn < 0.0f && !(c.a.w * sg - b.w < -1e-5f)) ? bit : 0u;
+          float ts, te;
+          const bool used = buried_interval(c, b, sg, nn, &ts, &te);
+          const CoverMask bins = covered_bins(ts, te);
+          cover |= used ? bins : CoverMask{0};
+        }
+        const unsigned self = li >= mb && li < mb + 32 ? 1u << (li - mb) : 0u;  // nn = 0 up to rounding
+        cross = own ? cross & ~self : 0u;
+        unclear = own ? unclear & ~self : 0u;
+        while (__any_sync(kFull, unclear != 0u)) {  // rarely: classify decides
+          if (unclear) {
+            const int q = __ffs(unclear) - 1;
+            unclear &= unclear - 1;
+            const Cap ck = cap_at(w, w.live[li]), cm = cap_at(w, w.live[mb + q]);
+            const PairClass pc = classify(ck, cm);
+            if (pc.count == 2) cross |= 1u << q;
+            inside |= !pc.count && ck.c * pc.sigma - cm.c > -1e-9;
+            tangent |= pc.count == 1;
+            tally += pc.count == 1;
+          }
+        }
+        tally += 2 * __popc(cross);
+        mask |= static_cast<uint64_t>(cross) << (mb & 32);
       }
-      const int lm = li + 1 + p - li * (2 * n_live - 1 - li) / 2;
-      const Cap ck = cap_at(w, w.live[li]), cm = cap_at(w, w.live[lm]);
-      const PairClass pc = classify(ck, cm);
-      if (pc.count == 2) {
-        const float root = sqrtf(__double2float_rn(pc.nn));
-        cover_or(cover, li, covered_bins(ck, cm, pc.sigma, root));
-        cover_or(cover, lm, covered_bins(cm, ck, pc.sigma, root));
-      }
-      // a circle inside the other cap without crossing its rim
-      const bool in_m = !pc.count && ck.c * pc.sigma - cm.c > -1e-9;
-      const bool in_k = !pc.count && cm.c * pc.sigma - ck.c > -1e-9;
       if (masks) {
-        tangent |= pc.count == 1;
-        if (pc.count == 2) {
-          mask_or(w, li, lm);
-          mask_or(w, lm, li);
-        }
-        if (in_m) mask_or(w, li, 63);
-        if (in_k) mask_or(w, lm, 63);
+        if (own) w.xmask[li] = mask | (inside ? kMaskContained : 0ull);
       } else {
-        if (pc.count) {
-          atomicAdd(&w.tcnt[li], pc.count);
-          atomicAdd(&w.tcnt[lm], pc.count);
-        }
-        if (in_m) atomicOr(&w.tcnt[li], kContained);
-        if (in_k) atomicOr(&w.tcnt[lm], kContained);
+        if (own) w.tcnt[li] = tally | (inside ? kContained : 0);
       }
+      const bool open = own && cover != ~CoverMask{0};
+      const unsigned m = __ballot_sync(kFull, open);
+      if (open) {
+        const int at = n_circ + __popc(m & ((1u << lane) - 1u));
+        w.circ[at] = static_cast<uint8_t>(li);
+        w.cover[at] = cover;
+        if (at < W::kCoverKept) w.circ_cover[at] = cover;
+      }
+      n_circ += __popc(m);
     }
     __syncwarp();
     if (!masks || !__any_sync(kFull, tangent)) break;
     masks = false;
   }
-  // the circles left to process, in live order
-  int n_circ = 0;
-  for (int l0 = 0; l0 < n_live; l0 += 32) {
-    const int li = l0 + lane;
-    const bool open = li < n_live && cover[li] != ~0ull;
-    const unsigned m = __ballot_sync(kFull, open);
-    if (open) w.circ[n_circ + __popc(m & ((1u << lane) - 1u))] = static_cast<uint8_t>(li);
-    n_circ += __popc(m);
+  // Of an open circle's crossings only those with an end in an open bin can
+  // bound an exposed segment: both ends of an exposed segment lie in open
+  // bins, and a cap with both ends inside buried bins either misses an open
+  // bin or would have buried it.  The others are dropped from the circle's
+  // mask (a fifth is left); depths counted over the rest are lower bounds, so
+  // a segment they find at depth 0 is tested explicitly below.
+  if (masks) {
+    for (int j = lane; j < n_circ; j += 32) w.keep[j] = 0ull;
+    __syncwarp();
+    const int n_pairs = n_circ * n_live;
+    for (int p = lane; p < n_pairs; p += 32) {
+      const int j = __float2int_rz((static_cast<float>(p) + 0.5f) * inv_live);
+      const int m = p - j * n_live, li = w.circ[j];
+      if (!((w.xmask[li] >> m) & 1ull)) continue;
+      const CoverCircle c = cover_circle(w.fcap[li]);
+      const float4 b = w.fcap[m];
+      const float sg = c.a.x * b.x + c.a.y * b.y + c.a.z * b.z;
+      const float nn = fmaf(2.0f * sg, c.a.w * b.w, fmaf(-sg, sg, 1.0f)) - (c.a.w * c.a.w + b.w * b.w);
+      float ts, te;
+      const bool used = buried_interval(c, b, sg, nn, &ts, &te);
+      if (!used || end_open(ts, w.cover[j]) || end_open(te, w.cover[j])) keep_or(w, j, m);
+    }
+    __syncwarp();
+    for (int j = lane; j < n_circ; j += 32) {
+      uint64_t& x = w.xmask[w.circ[j]];
+      x = w.keep[j] | (x & kMaskContained);
+    }
+    __syncwarp();
   }
-  __syncwarp();
   ph.mark(2);
   ph.count(14, n_circ);
 
@@ -714,17 +813,18 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   bool bad = false;
   for (int b0 = 0; b0 < n_circ && !bad;) {
     // the batch: consecutive circles of circ whose (padded) lists fit.  Lane j
-    // takes circle circ[b0 + j] (kSasaBatch == 32): an inclusive warp prefix of
+    // takes circle circ[b0 + j]: an inclusive warp prefix of
     // the list sizes gives every circle's first slot, and the lanes whose
     // prefix fits the buffer form the batch (a leading run, since the prefix
     // grows with j).  (Lane 0 alone walking the circles took twice as long.)
-    static_assert(kSasaBatch == 32, "one batch circle per lane");
+    static_assert(kSasaBatch <= 32, "one batch circle per lane");
     const int cj = b0 + lane;
-    const int lj = cj < n_circ ? w.circ[cj] : 0;
-    const int tally = cj < n_circ ? circle_tally(w, lj, masks) : 0;
+    const bool mine = lane < kSasaBatch && cj < n_circ;
+    const int lj = mine ? w.circ[cj] : 0;
+    const int tally = mine ? circle_tally(w, lj, masks) : 0;
     const int cnt_j = tally & kCountMask;
-    const int sz = cj < n_circ ? max(cnt_j, 1) : 0;
-    const int zero_j = (cj < n_circ && cnt_j == 0) ? 1 : 0;
+    const int sz = mine ? max(cnt_j, 1) : 0;
+    const int zero_j = (mine && cnt_j == 0) ? 1 : 0;
     int incl = sz, zincl = zero_j;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -734,7 +834,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         zincl += z;
       }
     }
-    const int nb = __popc(__ballot_sync(kFull, cj < n_circ && incl <= W::kTrans));
+    const int nb = __popc(__ballot_sync(kFull, mine && incl <= W::kTrans));
     if (nb == 0) {
       bad = true;  // one circle alone has more transitions than the buffer
       break;
@@ -1014,9 +1114,9 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     // crossing cap once, so the depth just after a transition is the toggles
     // up to it plus the depth before the first transition -- the number of
     // caps whose leaving crossing comes before their entering one in angular
-    // order, counted in the walk above.  A segment is exposed where the depth
-    // is 0.  The other circles test every segment's midpoint against every
-    // cap.
+    // order, counted in the walk above.  Only a segment at depth 0 can be
+    // exposed.  Its midpoint -- on the other circles every segment's -- is
+    // tested against every cap.
     __syncwarp();
     if (__any_sync(kFull, dup)) {
       if (lane == 0) compact_duplicates(w, nb);
@@ -1050,21 +1150,31 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
               const int m = w.live[lm];
               if (m != k && contains_strict(cap_at(w, m), probe)) exposed = false;
             }
-          } else if (w.bmode[j] == 0) {
-            sbn = w.torder[w.sbeg[j] + nxt];
-            if (w.bbase[j] + w.tdep[sa] == 0) {
-              // the reference's skip of a vanishing segment (ccw < 1e-9)
-              const D3 ua = tpoint(w, sa), ub = tpoint(w, sbn);
-              cos_ccw = dot(ua, ub);
-              sin_ccw = dot(D3{w.cx[k], w.cy[k], w.cz[k]}, cross(ua, ub));
-              exposed = !(cos_ccw > 0.0 && sin_ccw >= 0.0 && sin_ccw < 2e-9 && atan2(sin_ccw, cos_ccw) < 1e-9);
-            }
-          } else {
+          } else if (w.bmode[j] != 0 || w.bbase[j] + w.tdep[sa] == 0) {
             sbn = w.torder[w.sbeg[j] + nxt];
             const Cap ck = cap_at(w, k);
             D3 mid;
             if (segment_midpoint(tpoint(w, sa), tpoint(w, sbn), ck, w.bsk[j], kept == 1, &mid, &cos_ccw,
                                  &sin_ccw)) {
+              // In mask mode a segment at depth 0 is exposed or buried as a
+              // whole, and buried only by caps that bury the bins it lies
+              // in: its midpoint's bin decides unless it lies at a bin's edge
+              // between the two.
+              int known = -1;
+              if (masks && w.bmode[j] == 0 && b0 + j < W::kCoverKept) {
+                const CoverCircle cc = cover_circle(make_float4(static_cast<float>(ck.axis.x), static_cast<float>(ck.axis.y),
+                                                                static_cast<float>(ck.axis.z), 0.0f));
+                const float mx = static_cast<float>(mid.x), my = static_cast<float>(mid.y), mz = static_cast<float>(mid.z);
+                const float t = cover_bin(mx * cc.fx + my * cc.fy + mz * cc.fz, mx * cc.gx + my * cc.gy + mz * cc.gz);
+                const CoverMask cov = w.circ_cover[b0 + j];
+                const int q0 = __float2int_rd(t - 2.0f * kCoverMargin) & (kCoverBins - 1),
+                          q1 = __float2int_rd(t + 2.0f * kCoverMargin) & (kCoverBins - 1);
+                const int c0 = (cov >> q0) & 1u, c1 = (cov >> q1) & 1u;
+                if (w.bsk[j] > 0.1 && c0 == c1) known = c0;
+              }
+              if (known >= 0) {
+                exposed = known == 0;
+              } else {
               // a buried segment usually lies in one of the two caps whose
               // circles bound it; testing those first ends most searches early
               exposed = !contains_strict(cap_at(w, w.tother[sa]), mid) &&
@@ -1072,6 +1182,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
               for (int lm = 0; lm < n_live && exposed; ++lm) {
                 const int m = w.live[lm];
                 if (m != k && contains_strict(cap_at(w, m), mid)) exposed = false;
+              }
               }
             }
           }
@@ -1110,6 +1221,8 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
           w.v_z[v] = pa.z;
           w.v_in[v] = static_cast<uint8_t>(k);
           w.v_out[v] = w.tother[sa];
+          // in mask mode a pair's slots hold its + root, then its - root
+          w.v_sign[v] = masks ? (((sa - w.sbeg[j]) & 1) ? -1 : 1) : 0;
         }
       }
       n_arcs += __popc(ex);
@@ -1159,6 +1272,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
 template <class W>
 __device__ void link_boundary(W& w, int n_arcs, int n_verts, int lane) {
   for (int v = lane; v < n_verts; v += 32) {
+    if (w.v_sign[v] != 0) continue;  // known from the transition
     const Cap ci = cap_at(w, w.v_in[v]), co = cap_at(w, w.v_out[v]);
     w.v_sign[v] = static_cast<int8_t>(classify(ci, co).count == 1
                                           ? (w.v_in[v] < w.v_out[v] ? 1 : -1)
@@ -1269,13 +1383,22 @@ __device__ void boundary_task(const SasaArgs& a, W& w, int i, int lane, bool big
 // persistent grid of resident blocks): atoms differ several-fold in work,
 // and a warp whose atom was quick takes the next one instead of holding its
 // slot until the slowest warp of its block is done.
+//
+// Bound by latency: a warp's searches are chains of shared-memory reads,
+// votes and special functions over 20 to 90 caps, so what counts is work per
+// atom and warps in flight (24 per SM; registers and shared memory both end
+// there).  All kernels of the surface term together, before and after buried
+// circles and crossings were dropped in FP32 (of the cycles, a third goes to
+// the caps and contained caps, a quarter to the buried bins): 2057 -> 1297 us
+// for 64 chains of 300 residues, 819 -> 516 us for 16 compact folds of 306,
+// 184 -> 61 us for insulin (in the large-capacity kernel, see below).
 __device__ __forceinline__ int next_task(const SasaArgs& a, int lane) {
   int task = 0;
   if (lane == 0) task = atomicAdd(&a.counts[3], 1);
   return __shfl_sync(kFull, task, 0);
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 5) k_sasa_boundary(SasaArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, 6) k_sasa_boundary(SasaArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem& w = reinterpret_cast<WarpSmem*>(smem_raw)[warp];
@@ -1287,11 +1410,13 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_sasa_boundary(SasaArgs a) {
 // the queue length is known only on the device).
 // (One-warp blocks leave registers to spare; the cap keeps the compiler from
 // choosing a smaller allocation with spills.)
-__global__ void __maxnreg__(168) k_sasa_boundary_big(SasaArgs a) {
+// all: every task atom instead (launch_sasa_forces).
+__global__ void __maxnreg__(168) k_sasa_boundary_big(SasaArgs a, bool all) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSmemBig& w = *reinterpret_cast<WarpSmemBig*>(smem_raw);
-  const int n = min(a.counts[2], a.overflow_cap);
-  for (int q = blockIdx.x; q < n; q += gridDim.x) boundary_task(a, w, a.overflow[q], threadIdx.x, true);
+  const int32_t* atoms = all ? a.tasks : a.overflow;
+  const int n = all ? a.n_tasks : min(a.counts[2], a.overflow_cap);
+  for (int q = blockIdx.x; q < n; q += gridDim.x) boundary_task(a, w, atoms[q], threadIdx.x, true);
 }
 
 // Force path, stage 2: one term per thread, F_x += gamma_i R_i^2 dTerm/dr_x.
@@ -1477,7 +1602,7 @@ __device__ void areas_task(const SasaArgs& a, W& w, int i, int lane, bool big) {
   }
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 5) k_sasa_areas(SasaArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, 6) k_sasa_areas(SasaArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem& w = reinterpret_cast<WarpSmem*>(smem_raw)[warp];
@@ -1485,11 +1610,12 @@ __global__ void __launch_bounds__(kWarps * 32, 5) k_sasa_areas(SasaArgs a) {
     areas_task(a, w, a.tasks[task], lane, false);
 }
 
-__global__ void __launch_bounds__(32) k_sasa_areas_big(SasaArgs a) {
+__global__ void __launch_bounds__(32) k_sasa_areas_big(SasaArgs a, bool all) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSmemBig& w = *reinterpret_cast<WarpSmemBig*>(smem_raw);
-  const int n = min(a.counts[2], a.overflow_cap);
-  for (int q = blockIdx.x; q < n; q += gridDim.x) areas_task(a, w, a.overflow[q], threadIdx.x, true);
+  const int32_t* atoms = all ? a.tasks : a.overflow;
+  const int n = all ? a.n_tasks : min(a.counts[2], a.overflow_cap);
+  for (int q = blockIdx.x; q < n; q += gridDim.x) areas_task(a, w, atoms[q], threadIdx.x, true);
 }
 
 // Shrake-Rupley: one warp per atom, neighbours staged in shared memory,
@@ -1570,10 +1696,12 @@ __global__ void __launch_bounds__(kWarps * 32) k_shrake_rupley(SasaArgs a, const
 constexpr size_t kWarpSmemBytes = sizeof(WarpSmem) * kWarps;
 constexpr size_t kBigSmemBytes = sizeof(WarpSmemBig);
 constexpr int kBigGrid = 148 * 4;  // persistent one-warp blocks for the queue
-// five resident CTAs per SM (228 KB, 1 KB reserved per CTA): 20 warps; at
-// four (the capacities 128 caps, 128 transitions, 48 arcs) the kernel was
-// 1.6 % slower
-static_assert(5 * (kWarpSmemBytes + 1024) <= 228 * 1024, "boundary kernel no longer fits five CTAs per SM");
+// Up to this many atoms, all of them go to the large-capacity kernel at once,
+// one block each (all resident): the queue's second pass would take as long
+// as the first (insulin, 266 C and S atoms, 57 + 54 us).
+constexpr int kBigAllTasks = 148 * 8;
+// six resident CTAs per SM (228 KB, 1 KB reserved per CTA): 24 warps
+static_assert(6 * (kWarpSmemBytes + 1024) <= 228 * 1024, "boundary kernel no longer fits six CTAs per SM");
 
 }  // namespace
 
@@ -1610,16 +1738,24 @@ int resident_grid(K kernel, int n_tasks) {
 void launch_sasa_forces(const SasaArgs& a, cudaStream_t s) {
   if (a.n_tasks <= 0) return;
   cudaMemsetAsync(a.counts, 0, 4 * sizeof(int32_t), s);
-  k_sasa_boundary<<<resident_grid(k_sasa_boundary, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
-  k_sasa_boundary_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a);
+  if (a.n_tasks <= kBigAllTasks) {
+    k_sasa_boundary_big<<<a.n_tasks, 32, kBigSmemBytes, s>>>(a, true);
+  } else {
+    k_sasa_boundary<<<resident_grid(k_sasa_boundary, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
+    k_sasa_boundary_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a, false);
+  }
   k_sasa_terms<<<148 * 8, 128, 0, s>>>(a);
 }
 
 void launch_sasa_areas(const SasaArgs& a, cudaStream_t s) {
   if (a.n_tasks <= 0) return;
   cudaMemsetAsync(a.counts + 2, 0, 2 * sizeof(int32_t), s);
-  k_sasa_areas<<<resident_grid(k_sasa_areas, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
-  k_sasa_areas_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a);
+  if (a.n_tasks <= kBigAllTasks) {
+    k_sasa_areas_big<<<a.n_tasks, 32, kBigSmemBytes, s>>>(a, true);
+  } else {
+    k_sasa_areas<<<resident_grid(k_sasa_areas, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
+    k_sasa_areas_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a, false);
+  }
 }
 
 void launch_shrake_rupley(const SasaArgs& a, const double* dots, int n_dots, cudaStream_t s) {

@@ -14,15 +14,18 @@ namespace ogk {
 // Per-atom capacities of the on-chip boundary arrangement.  An atom that
 // exceeds one marks its system with kStatusSasaOverflow (the host reports
 // OG_E_UNSUPPORTED) instead of producing a wrong force.  Protein atoms reach
-// about 90 caps, 46 of them left after contained caps are dropped, 72
-// transitions on one circle and 19 exposed arcs.
+// about 90 caps, 46 of them left after contained caps are dropped, 4 to 6
+// circles that are not buried all around with 24 to 37 transitions between
+// them on average, and 19 exposed arcs.
 // Arrangement capacities per atom: the default kernels' (four warps per
-// block, five blocks per SM) and the large ones for the atoms that exceed
+// block, six blocks per SM) and the large ones for the atoms that exceed
 // them (caps cutting the atom's sphere, transitions of one batch of circles,
-// exposed arcs).
+// exposed arcs).  96 transitions and 34 arcs, five blocks per SM, took 1383
+// instead of 1297 us (64 chains of 300 residues) and 535 instead of 516 us
+// (16 compact folds of 306): more atoms fit, but fewer warps hide latency.
 constexpr int kSasaMaxCaps = 112;
-constexpr int kSasaMaxTrans = 96;
-constexpr int kSasaMaxArcs = 34;
+constexpr int kSasaMaxTrans = 64;
+constexpr int kSasaMaxArcs = 24;
 constexpr int kSasaBigCaps = 254;
 constexpr int kSasaBigTrans = 254;
 constexpr int kSasaBigArcs = 128;
