@@ -482,6 +482,7 @@ struct og_engine {
   ogk::SasaArgs sasa_args(bool all_atoms) {
     ogk::SasaArgs a{};
     a.x = x.p; a.y = y.p; a.z = z.p;
+    a.pq = pq.p;
     a.radius = sasa_r.p;
     a.gamma = sasa_gamma.p;
     a.tasks = all_atoms ? sasa_all.p : sasa_tasks.p;

@@ -31,8 +31,8 @@
 //    exposed arcs' central angles.
 //  * The gradient of A_i is taken term by term in reverse mode (sasa_geom.h)
 //    instead of one forward directional derivative per (atom, axis).
-//  * Clear cases of the three searches above (caps, contained caps, buried
-//    bins) are decided in FP32 with margins above its errors; what bounds an
+//  * Clear cases of the searches (neighbours, contained caps, buried bins)
+//    are decided in FP32 with margins above its errors; what bounds an
 //    area or enters a gradient is FP64 throughout.
 #include <algorithm>
 #include <cstddef>
@@ -253,6 +253,7 @@ __device__ int identify_root_sign(Cap c1, Cap c2, D3 ref) {
 template <int kCaps_, int kTrans_, int kArcs_>
 struct WarpSmemT {
   static constexpr int kCaps = kCaps_, kTrans = kTrans_, kArcs = kArcs_;
+  static constexpr bool kBig = kCaps_ > kSasaMaxCaps;  // alone takes atoms without crossing masks
   static_assert(kCaps <= 254 && kTrans <= 254, "byte-sized cap and transition indices");
   static_assert(kCaps / 2 >= kMaskCircles, "a crossing mask for every circle of mask mode");
   // caps (indices in neighbour order, i.e. ascending atom index)
@@ -278,7 +279,7 @@ struct WarpSmemT {
     struct {
       float4 fcap[kCaps];
       union {
-        int32_t queue[96];
+        int32_t queue[160];
         struct {
           CoverMask cover[kCaps];    // buried bins of the circles in circ
           uint64_t keep[kCaps / 2];  // and the crossings kept of them
@@ -400,7 +401,7 @@ __device__ __forceinline__ float cover_bin(float x, float y) {
 
 // Bins [0, b).
 __device__ __forceinline__ CoverMask bins_below(int b) {
-  return b >= kCoverBins ? ~CoverMask{0} : (CoverMask{1} << max(b, 0)) - CoverMask{1};
+  return ~__funnelshift_lc(0u, ~0u, static_cast<unsigned>(max(b, 0)));  // shifts of 32 clamp
 }
 
 // A circle as the cover pass sees it: cap a (axis, cos alpha) and the frame
@@ -469,7 +470,7 @@ __device__ __forceinline__ D3 circle_point(Cap ck, double sk, D3 u) { return ck.
 // (ccw < 1e-9); else the exposure test point *mid (ua rotated by half the ccw
 // angle, midpoint_on_circle) and the cosine / sine of the ccw angle.
 // single = the circle's only transition (the whole circle, ccw = 2 pi).
-__device__ __noinline__ bool segment_midpoint(D3 ua, D3 ub, Cap ck, double sk, bool single, D3* mid, double* cos_ccw,
+__device__ __forceinline__ bool segment_midpoint(D3 ua, D3 ub, Cap ck, double sk, bool single, D3* mid, double* cos_ccw,
                                  double* sin_ccw) {
   if (single) {
     *cos_ccw = 1.0;
@@ -481,17 +482,11 @@ __device__ __noinline__ bool segment_midpoint(D3 ua, D3 ub, Cap ck, double sk, b
   const double s = dot(ck.axis, cross(ua, ub));
   *cos_ccw = c;
   *sin_ccw = s;
-  if (c > 0.0 && s >= 0.0 && s < 2e-9 && atan2(s, c) < 1e-9) return false;
+  if (c > 0.0 && s >= 0.0 && s < 1e-9 * c) return false;  // the angle, s / c to rounding, is below 1e-9
   // cos / sin of half the ccw angle h in (0, pi], from c = cos 2h, s = sin 2h
-  double ch, sh;
-  if (c >= 0.0) {
-    const double r = sqrt((1.0 + c) * 0.5);
-    ch = s >= 0.0 ? r : -r;
-    sh = fabs(s) / (2.0 * r);
-  } else {
-    sh = sqrt((1.0 - c) * 0.5);
-    ch = s / (2.0 * sh);
-  }
+  const double r = sqrt((1.0 + fabs(c)) * 0.5), h = s / (2.0 * r);
+  const double ch = c >= 0.0 ? (s >= 0.0 ? r : -r) : h;
+  const double sh = c >= 0.0 ? fabs(h) : r;
   *mid = circle_point(ck, sk, ua * ch + cross(ck.axis, ua) * sh);
   return true;
 }
@@ -553,17 +548,13 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // ---- caps (build_caps), neighbours in ascending atom order
   int n_caps = 0, queued = 0;
   bool enclosed = false;
-  auto near_atom = [&](int j) {
-    const double dx = a.x[j] - pi.x, dy = a.y[j] - pi.y, dz = a.z[j] - pi.z, rs = ri + a.radius[j];
-    return j != i && a.atom_sys[j] >= 0 && dx * dx + dy * dy + dz * dz <= rs * rs * (1.0 + 1e-12);
-  };
-  // caps of the first n queued neighbours
-  auto make_caps = [&](int n) {
+  // caps of the n queued neighbours from `head` on
+  auto make_caps = [&](int head, int n) {
     bool is_cap = false;
     int j = 0;
     double ax = 0.0, ay = 0.0, az = 0.0, ca = 0.0;
     if (lane < n) {
-      j = w.queue[lane];
+      j = w.queue[head + lane];
       const double dx = a.x[j] - pi.x, dy = a.y[j] - pi.y, dz = a.z[j] - pi.z;
       const double rj = a.radius[j];
       // d and 1/d from one reciprocal square root (d = 0 exactly for
@@ -598,48 +589,71 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     }
     n_caps += __popc(caps);
   };
-  for (int t0 = 0; t0 < st.y; t0 += 32) {
-    const int t = t0 + lane;
-    bool hit = false;
-    if (t < st.y) {
-      const double4 o = a.origin[st.x + t];
-      const double dx = o.x - pi.x, dy = o.y - pi.y, dz = o.z - pi.z;
-      const double lim = o.w + ri + a.r_max + 1e-6;
-      hit = dx * dx + dy * dy + dz * dz <= lim * lim;
-    }
-    unsigned hits = __ballot_sync(kFull, hit);
-    // the atoms of two hit tiles per trip (independent loads in flight);
-    // those within R_i + R_j (with a margin) queue up in ascending order and
-    // are made into caps 32 at a time, so that the root and the quotients
-    // run with every lane busy (a hit tile has about four neighbours)
-    while (hits) {
-      const int b = __ffs(hits) - 1;
-      hits &= hits - 1;
-      const int b2 = hits ? __ffs(hits) - 1 : -1;
-      if (b2 >= 0) hits &= hits - 1;
-      const int j = (st.x + t0 + b) * 32 + lane;
-      const int j2 = b2 >= 0 ? (st.x + t0 + b2) * 32 + lane : j;
-      const bool c1 = near_atom(j), c2 = near_atom(j2) && b2 >= 0;
-      const unsigned m1 = __ballot_sync(kFull, c1), m2 = __ballot_sync(kFull, c2);
-      const unsigned below = (1u << lane) - 1u;
-      if (c1) w.queue[queued + __popc(m1 & below)] = j;
-      queued += __popc(m1);
-      if (c2) w.queue[queued + __popc(m2 & below)] = j2;
-      queued += __popc(m2);
-      __syncwarp();
-      while (queued >= 32) {
-        make_caps(32);
-        const int rest = queued - 32;
-        const int v0 = lane < rest ? w.queue[32 + lane] : 0, v1 = lane + 32 < rest ? w.queue[64 + lane] : 0;
-        __syncwarp();
-        if (lane < rest) w.queue[lane] = v0;
-        if (lane + 32 < rest) w.queue[32 + lane] = v1;
-        __syncwarp();
-        queued = rest;
+  // The atoms of up to kTilesPerTrip hit tiles per trip (independent loads in
+  // flight); those within R_i + R_j in FP32, with a margin above its error
+  // (coordinates relative to the tile's centre, rounded to 6e-8 of its radius
+  // and of its distance), queue up in ascending order and are made into caps
+  // 32 at a time, so that the root and the quotients run with every lane busy
+  // (a hit tile has about four neighbours).
+  constexpr int kTilesPerTrip = 2;
+  int t0 = 0;
+  unsigned hits = 0;
+  float4 rel{};  // this lane's tile: centre - p_i, R_i + margin
+#pragma unroll 1
+  while (true) {
+    // the next group of tiles with a hit
+    while (!hits && t0 < st.y) {
+      const int t = t0 + lane;
+      bool hit = false;
+      if (t < st.y) {
+        const double4 o = a.origin[st.x + t];
+        const double dx = o.x - pi.x, dy = o.y - pi.y, dz = o.z - pi.z;
+        const double lim = o.w + ri + a.r_max + 1e-6;
+        hit = dx * dx + dy * dy + dz * dz <= lim * lim;
+        rel = make_float4(static_cast<float>(dx), static_cast<float>(dy), static_cast<float>(dz),
+                          static_cast<float>(ri) + 1e-4f + 1e-6f * static_cast<float>(o.w));
       }
+      hits = __ballot_sync(kFull, hit);
+      t0 += 32;
     }
+    const bool last = !hits;
+    if (!last) {
+      const int tile0 = st.x + t0 - 32;
+      int tile[kTilesPerTrip];
+      bool near[kTilesPerTrip];
+#pragma unroll
+      for (int u = 0; u < kTilesPerTrip; ++u) {
+        const bool any = hits != 0u;
+        const int b = any ? __ffs(hits) - 1 : 0;
+        hits &= hits - 1;
+        tile[u] = tile0 + b;
+        const float* c = a.pq + soa_index(tile[u] * 32 + lane, 0);
+        const float dx = c[0] + __shfl_sync(kFull, rel.x, b), dy = c[32] + __shfl_sync(kFull, rel.y, b),
+                    dz = c[64] + __shfl_sync(kFull, rel.z, b);
+        const float rs = static_cast<float>(a.radius[tile[u] * 32 + lane]) + __shfl_sync(kFull, rel.w, b);
+        near[u] = any && tile[u] * 32 + lane != i && dx * dx + dy * dy + dz * dz <= rs * rs;
+      }
+#pragma unroll
+      for (int u = 0; u < kTilesPerTrip; ++u) {
+        const unsigned m = __ballot_sync(kFull, near[u]);
+        if (near[u]) w.queue[queued + __popc(m & ((1u << lane) - 1u))] = tile[u] * 32 + lane;
+        queued += __popc(m);
+      }
+      __syncwarp();
+    }
+    int head = 0;
+#pragma unroll 1
+    for (; queued - head >= 32 || (last && queued > head); head += 32) make_caps(head, min(queued - head, 32));
+    if (last) break;
+    if (head > 0) {
+      const int rest = queued - head;
+      const int v = lane < rest ? w.queue[head + lane] : 0;
+      __syncwarp();
+      if (lane < rest) w.queue[lane] = v;
+      queued = rest;
+    }
+    __syncwarp();
   }
-  make_caps(queued);
   ph.mark(0);
   ph.count(10, n_caps);
   if (__any_sync(kFull, enclosed)) return kBuried;
@@ -657,6 +671,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // Each lane tests two caps (k and k + 32) against the caps m in one pass,
   // so a cap m's data is read once for both; survivors keep ascending order.
   int n_live = 0;
+#pragma unroll 1
   for (int k0 = 0; k0 < n_caps; k0 += 64) {
     const int ka = k0 + lane, kb = k0 + 32 + lane;
     bool la = ka < n_caps, lb = kb < n_caps;
@@ -700,14 +715,17 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // p / n_live by a float reciprocal: exact here, since p + 0.5 keeps the
   // quotient at least 0.5 / n_live from an integer, far above the rounding
   const float inv_live = 1.0f / static_cast<float>(n_live);
+#pragma unroll 1
   for (int l0 = 0; l0 < n_live; l0 += 32) {  // live[k] >= k: a trip overwrites nothing a later one reads
     const float4 f = l0 + lane < n_live ? w.fcap[w.live[l0 + lane]] : float4{};
     __syncwarp();
     if (l0 + lane < n_live) w.fcap[l0 + lane] = f;
     __syncwarp();
   }
+  if (!W::kBig && n_live > kMaskCircles) return kInvalid;
   bool masks = n_live <= kMaskCircles;
   int n_circ = 0;  // the circles left to process, in live order
+#pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     // Lane = circle, all caps in turn (read as broadcasts): the lane keeps
     // its circle's crossings and buried bins in registers.  (Each unordered
@@ -715,6 +733,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     // as long.)
     n_circ = 0;
     bool tangent = false;
+#pragma unroll 1
     for (int l0 = 0; l0 < n_live; l0 += 32) {
       const int li = l0 + lane;
       const bool own = li < n_live;
@@ -723,10 +742,11 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       uint64_t mask = 0;
       int32_t tally = 0;
       bool inside = false;  // in a cap without crossing its rim
+#pragma unroll 1
       for (int mb = 0; mb < n_live; mb += 32) {
         const int mn = min(32, n_live - mb);
         unsigned cross = 0, unclear = 0;
-#pragma unroll 2
+#pragma unroll (W::kBig ? 2 : 1)
         for (int q = 0; q < mn; ++q) {
           const float4 b = w.fcap[mb + q];
           const unsigned bit = 1u << q;
@@ -775,6 +795,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     }
     __syncwarp();
     if (!masks || !__any_sync(kFull, tangent)) break;
+    if (!W::kBig) return kInvalid;
     masks = false;
   }
   // Of an open circle's crossings only those with an end in an open bin can
@@ -784,9 +805,11 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // mask (a fifth is left); depths counted over the rest are lower bounds, so
   // a segment they find at depth 0 is tested explicitly below.
   if (masks) {
+#pragma unroll 1
     for (int j = lane; j < n_circ; j += 32) w.keep[j] = 0ull;
     __syncwarp();
     const int n_pairs = n_circ * n_live;
+#pragma unroll 1
     for (int p = lane; p < n_pairs; p += 32) {
       const int j = __float2int_rz((static_cast<float>(p) + 0.5f) * inv_live);
       const int m = p - j * n_live, li = w.circ[j];
@@ -800,6 +823,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       if (!used || end_open(ts, w.cover[j]) || end_open(te, w.cover[j])) keep_or(w, j, m);
     }
     __syncwarp();
+#pragma unroll 1
     for (int j = lane; j < n_circ; j += 32) {
       uint64_t& x = w.xmask[w.circ[j]];
       x = w.keep[j] | (x & kMaskContained);
@@ -846,7 +870,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       const double c = w.cc[w.live[lj]];
       const double sk = sqrt(fmax(1.0 - c * c, 0.0));
       w.bsk[lane] = sk;
-      w.binv[lane] = sk > 0.0 ? 1.0 / sk : 0.0;
+      w.binv[lane] = sk > 0.0 ? rsqrt(fmax(1.0 - c * c, 0.0)) : 0.0;
       w.bmode[lane] = (tally & kContained) ? 1 : 0;
       w.bbase[lane] = 0;
     }
@@ -864,7 +888,6 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     int run = 0;
     bool mismatch = false, nonfinite = false;
     using Key = SlotKey<W::kTrans>;
-    // the transitions of batch circle j with cap m from slot base on
     // batch circle j's transitions on its crossing with cap m, the points
     // in the order of the pair (circle j, cap m), from slot base on
     // (the two slots of a pair unrolled side by side)
@@ -900,7 +923,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         w.tpart[sl] = (e == 0 && clean) ? static_cast<uint8_t>(base + 1) : kNoOther;
       }
     };
-    if (masks) {
+    if (!W::kBig || masks) {
       // the crossing pairs straight from the masks, 32 at a time: entry e
       // belongs to the batch circle whose inclusive prefix of crossing
       // partners first exceeds e, and is its r-th partner in ascending live
@@ -915,6 +938,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         if (lane >= d) incl += v;
       }
       const int n_ent = __shfl_sync(kFull, incl, 31);
+#pragma unroll 1
       for (int e0 = 0; e0 < n_ent; e0 += 32) {
         const int e = e0 + lane;
         int j = 0;
@@ -1000,6 +1024,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       bad = true;  // the two passes disagree: never expected, but never written past
       break;
     }
+#pragma unroll 1
     for (int j = lane; j < nb; j += 32) {
       if ((circle_tally(w, w.circ[b0 + j], masks) & kCountMask) != 0) continue;
       const int sl = w.sbeg[j];
@@ -1019,12 +1044,13 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     // toggles on the way; four of those per trip with their loads issued
     // together had measured 1.8x slower.)
     constexpr int kShift = Key::kShift;
+#pragma unroll 1
     for (int sl = lane; sl < n_tr; sl += 32) {
       const int j = w.tseg[sl];
       const int sb = w.sbeg[j], se = w.sbeg[j + 1];
       const uint32_t ks = w.tkey[sl];
       int rank = 0;
-#pragma unroll 4
+#pragma unroll 1
       for (int t = sb; t < se; ++t) rank += w.tkey[t] < ks ? 1 : 0;
       rank = min(rank, se - sb - 1);
       w.torder[sb + rank] = static_cast<uint8_t>(sl);
@@ -1044,10 +1070,12 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     // circle with such neighbours (rare: the quantum is 2^-21 of the angle's
     // range) is ordered again from the FP64 angles and the walk repeated.
     bool dup = false;
+#pragma unroll 1
     for (int walk = 0; walk < 2; ++walk) {
       unsigned tied = 0;
       int carry = 0;
       dup = false;
+#pragma unroll 1
       for (int r0 = 0; r0 < n_tr; r0 += 32) {
         const int r = r0 + lane;
         int sl = 0, v = 0;
@@ -1121,12 +1149,14 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     if (__any_sync(kFull, dup)) {
       if (lane == 0) compact_duplicates(w, nb);
     } else {
+#pragma unroll 1
       for (int j = lane; j < nb; j += 32) w.skept[j] = static_cast<uint8_t>(w.sbeg[j + 1] - w.sbeg[j]);
     }
     __syncwarp();
     ph.mark(6);
 
     // exposure of every segment (and of every transition-free circle)
+#pragma unroll 1
     for (int r0 = 0; r0 < n_tr; r0 += 32) {
       const int r = r0 + lane;
       bool exposed = false, full = false;
@@ -1146,6 +1176,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
             full = true;
             probe = sample_circle_point(cap_at(w, k));
             exposed = true;
+#pragma unroll 1
             for (int lm = 0; lm < n_live && exposed; ++lm) {
               const int m = w.live[lm];
               if (m != k && contains_strict(cap_at(w, m), probe)) exposed = false;
@@ -1175,14 +1206,15 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
               if (known >= 0) {
                 exposed = known == 0;
               } else {
-              // a buried segment usually lies in one of the two caps whose
-              // circles bound it; testing those first ends most searches early
-              exposed = !contains_strict(cap_at(w, w.tother[sa]), mid) &&
-                        !contains_strict(cap_at(w, w.tother[sbn]), mid);
-              for (int lm = 0; lm < n_live && exposed; ++lm) {
-                const int m = w.live[lm];
-                if (m != k && contains_strict(cap_at(w, m), mid)) exposed = false;
-              }
+                // a buried segment usually lies in one of the two caps whose
+                // circles bound it; testing those first ends most searches early
+                exposed = !contains_strict(cap_at(w, w.tother[sa]), mid) &&
+                          !contains_strict(cap_at(w, w.tother[sbn]), mid);
+#pragma unroll 1
+                for (int lm = 0; lm < n_live && exposed; ++lm) {
+                  const int m = w.live[lm];
+                  if (m != k && contains_strict(cap_at(w, m), mid)) exposed = false;
+                }
               }
             }
           }
@@ -1239,6 +1271,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // instead of one lane at a time there): the cosine and sine of the angle
   // from p_start - a c to p_end - a c about the axis, as segment_midpoint
   // takes them from the unit radial directions, up to a positive factor.
+#pragma unroll 1
   for (int e = lane; e < n_arcs; e += 32) {
     if (w.a_full[e]) continue;
     const Cap ck = cap_at(w, w.a_cap[e]);
@@ -1271,19 +1304,22 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
 // signs crossed).
 template <class W>
 __device__ void link_boundary(W& w, int n_arcs, int n_verts, int lane) {
+#pragma unroll 1
   for (int v = lane; v < n_verts; v += 32) {
-    if (w.v_sign[v] != 0) continue;  // known from the transition
+    if (!W::kBig || w.v_sign[v] != 0) continue;  // known from the transition
     const Cap ci = cap_at(w, w.v_in[v]), co = cap_at(w, w.v_out[v]);
     w.v_sign[v] = static_cast<int8_t>(classify(ci, co).count == 1
                                           ? (w.v_in[v] < w.v_out[v] ? 1 : -1)
                                           : identify_root_sign(ci, co, {w.v_x[v], w.v_y[v], w.v_z[v]}));
   }
+#pragma unroll 1
   for (int e = lane; e < n_arcs; e += 32) {
     int vs = -1, ve = -1;
     if (!w.a_full[e]) {
       const D3 s = {w.a_sx[e], w.a_sy[e], w.a_sz[e]};
       const int own = w.a_own[e];
       const D3 t = {w.v_x[own], w.v_y[own], w.v_z[own]};
+#pragma unroll 1
       for (int v = 0; v < n_verts && (vs < 0 || ve < 0); ++v) {
         const D3 p = {w.v_x[v], w.v_y[v], w.v_z[v]};
         if (vs < 0 && norm2(p - s) < 1e-10) vs = v;
@@ -1353,6 +1389,7 @@ __device__ void boundary_task(const SasaArgs& a, W& w, int i, int lane, bool big
     if (lane == 0) atomicOr(&a.sys[sys].status, kStatusSasaOverflow);
     return;
   }
+#pragma unroll 1
   for (int e = lane; e < n_arcs; e += 32) {
     SasaArcTerm t;
     const int kc = w.a_cap[e];
@@ -1387,11 +1424,18 @@ __device__ void boundary_task(const SasaArgs& a, W& w, int i, int lane, bool big
 // Bound by latency: a warp's searches are chains of shared-memory reads,
 // votes and special functions over 20 to 90 caps, so what counts is work per
 // atom and warps in flight (24 per SM; registers and shared memory both end
-// there).  All kernels of the surface term together, before and after buried
-// circles and crossings were dropped in FP32 (of the cycles, a third goes to
-// the caps and contained caps, a quarter to the buried bins): 2057 -> 1297 us
-// for 64 chains of 300 residues, 819 -> 516 us for 16 compact folds of 306,
-// 184 -> 61 us for insulin (in the large-capacity kernel, see below).
+// there) -- and code size: the warps of a scheduler are in different phases
+// of a long program, and with loops unrolled 31 % of the stalls were waits for
+// instructions (59 % of issue slots used).  Hence loops that run a few trips
+// an atom are not unrolled, nor is the hot one over the caps (80 us of 1180),
+// the roots of a midpoint are taken once for both of its cases, and what only
+// rare atoms need -- plain counts instead of crossing masks -- lives in the
+// large-capacity kernel alone.
+// All kernels of the surface term together, first after buried circles and
+// crossings were dropped in FP32, then with the smaller code and the FP32
+// neighbour search: 2057 -> 1297 -> 998 us for 64 chains of 300 residues,
+// 819 -> 516 -> 413 us for 16 compact folds of 306, 184 -> 61 -> 56 us for
+// insulin (in the large-capacity kernel, see below).
 __device__ __forceinline__ int next_task(const SasaArgs& a, int lane) {
   int task = 0;
   if (lane == 0) task = atomicAdd(&a.counts[3], 1);
@@ -1698,7 +1742,7 @@ constexpr size_t kBigSmemBytes = sizeof(WarpSmemBig);
 constexpr int kBigGrid = 148 * 4;  // persistent one-warp blocks for the queue
 // Up to this many atoms, all of them go to the large-capacity kernel at once,
 // one block each (all resident): the queue's second pass would take as long
-// as the first (insulin, 266 C and S atoms, 57 + 54 us).
+// as the first (insulin, 266 C and S atoms: 57 + 54 us, 61 in one).
 constexpr int kBigAllTasks = 148 * 8;
 // six resident CTAs per SM (228 KB, 1 KB reserved per CTA): 24 warps
 static_assert(6 * (kWarpSmemBytes + 1024) <= 228 * 1024, "boundary kernel no longer fits six CTAs per SM");

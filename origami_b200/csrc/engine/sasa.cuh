@@ -52,6 +52,7 @@ struct SasaArgs {
   const double* x;
   const double* y;
   const double* z;
+  const float* pq;            // tile-SoA FP32 coordinates relative to the tile's origin
   const double* radius;       // per padded atom: vdW + 1.4 A probe
   const double* gamma;        // per padded atom: surface tension, kJ/mol/A^2
   const int32_t* tasks;       // padded atom indices to evaluate

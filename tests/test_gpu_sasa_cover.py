@@ -79,3 +79,24 @@ def test_buried_circles_leave_forces_and_areas_as_the_oracle(origami, kind, p, q
     area = np.zeros(x.shape[0])
     o.orc_sasa_areas(x.shape[0], dp(x), dp(rad), dp(area))
     assert np.max(np.abs(got - area) / (4 * np.pi * rad ** 2)) < 1e-9
+
+
+@pytest.mark.parametrize("apart", [30.0, 2000.0])
+def test_neighbours_in_wide_tiles_match_oracle(origami, apart):
+    """Two clusters whose atoms alternate, so that every tile spans both and
+    its FP32 coordinates are coarse (1e-4 A at 2000 A): the neighbour search
+    has to find each atom's own cluster all the same."""
+    xa, ea = _cluster(23, 3.5, 7)
+    xb, eb = _cluster(23, 3.5, 8)
+    x = np.ascontiguousarray(np.stack([xa, xb + np.array([apart, 0.3 * apart, 0.0])], 1).reshape(-1, 3))
+    el = np.ascontiguousarray(np.stack([ea, eb], 1).reshape(-1))
+    o = oracle()
+    rad = np.array([o.orc_sasa_radius(int(e)) for e in el])
+    gam = np.array([o.orc_sasa_gamma(int(e), 1.0) for e in el])
+    ref = np.zeros_like(x)
+    o.orc_sasa_forces_tangent_one_root(x.shape[0], dp(x), dp(rad), dp(gam), dp(ref))
+    force, got = _gpu(origami, x, el)
+    assert np.max(np.abs(force - ref)) < 1e-6
+    area = np.zeros(x.shape[0])
+    o.orc_sasa_areas(x.shape[0], dp(x), dp(rad), dp(area))
+    assert np.max(np.abs(got - area) / (4 * np.pi * rad ** 2)) < 1e-9
