@@ -938,11 +938,25 @@ int64_t count_items(const og_engine* e, int first_offset, int W, int chunk) {
 // force pass), cut into chunks of at most `chunk` j-tiles and ordered
 // longest first; plus the i-blocks of cutoff mode's culled lists.  A list
 // too short to fill the GPU (eight items per SM) is cut finer: with few
-// tiles the longest item is the pass's time.
+// tiles the longest item is the pass's time.  All-pairs passes are cut on
+// until the items make a few waves of resident blocks, so that the last one
+// weighs little: 32 items per SM for Born (15 600 atoms: 148 us with chunks of
+// 16, 139 of 8, 129 of 4; 4 x 4 668 atoms: 103, 103, 89, and 83 of 2), 16 for
+// the force pass (179, 179, 166; 12 x 4 694 atoms: 221, 192, 185), whose items
+// cost more to start, so that chunks of 1 lose again (12 x 4 694: 214).  With
+// cutoffs the culled lists are shorter than they count here, and finer items
+// lost (15 600 atoms, Born: 38 us of 16, 43 of 8).
 og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec<ogk::PairWork>* work,
                           int* n_work, DVec<int32_t>* jlist, DVec<ogk::CutBlock>* cut, int* n_cut,
                           DVec<int32_t>* jlist_cut, DVec<int32_t>* seg_end, cudaStream_t st) {
-  while (chunk > 1 && count_items(e, first_offset, W, chunk) < 8ll * e->n_sm) chunk /= 2;
+  const bool born = first_offset == 0;
+  const bool all_pairs = born ? no_cutoff(e->p.born_cutoff) : no_cutoff(e->p.nb_cutoff) || no_cutoff(e->p.gb_force_cutoff);
+  const int64_t waves = all_pairs ? (born ? 32 : 16) : 8;
+  while (chunk > 1) {
+    const int64_t items = count_items(e, first_offset, W, chunk);
+    if (items >= waves * e->n_sm || (items >= 8ll * e->n_sm && !born && chunk <= 3)) break;
+    chunk /= 2;
+  }
   std::vector<int32_t> hj;
   std::vector<ogk::PairWork> hw;
   std::vector<ogk::CutBlock> hc;
@@ -972,24 +986,19 @@ og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec
 // The launch variants of an engine nobody tuned, by its tile pairs (times in us
 // on B200; shapes in pair_kernels.cuh).  With cutoffs most tile pairs are
 // skipped and shape 0 wins throughout (32 x 4 668 atoms: Born 290 against 307
-// for shape 1, force 226 against 240).  Without, Born: shape 0 while the
-// tiles are few or the systems small (4.6k atoms in one system of 147 tiles:
-// 35 against 30; 64 systems of 20 tiles: 44 against 48), else shape 1.  Force:
-// shape 0 below 800 tile pairs (20 residues: 10.6 against 12.8; 80 residues:
-// 14.5 against 13.2), shape 4 from 40 000 on (8 x 4 694 atoms: 148 against
-// 155; one system of 10.9k tile pairs: 36 against 32), shape 1 between.
+// for shape 1, force 226 against 240).  Without, Born: shape 0 below 4 000
+// tile pairs (1 770: 15.0 against 16.4; 64 systems of 20 tiles, 13 440: 44.7
+// against 43.3; one system of 147 tiles, 10 878: 35 against 27), else shape 1.
+// Force: shape 0 below 800 tile pairs (20 residues: 10.6 against 12.8; 80
+// residues: 14.5 against 13.2), shape 4 from 40 000 on (8 x 4 694 atoms: 148
+// against 155; one system of 10.9k tile pairs: 36 against 32), shape 1 between.
 void default_launch(og_engine* e) {
   int64_t pairs = 0;
-  int max_tiles = 0;
-  for (const auto& s : e->sys) {
-    pairs += static_cast<int64_t>(s.n_tiles) * (s.n_tiles + 1) / 2;
-    max_tiles = std::max(max_tiles, s.n_tiles);
-  }
+  for (const auto& s : e->sys) pairs += static_cast<int64_t>(s.n_tiles) * (s.n_tiles + 1) / 2;
   e->born_launch = ogk::PairLaunch{};
   e->force_launch = ogk::PairLaunch{};
   e->chunk_b = e->chunk_f = 16;
-  const bool small = pairs < 4000 || (pairs < 16000 && max_tiles < 32);
-  if (no_cutoff(e->p.born_cutoff)) e->born_launch.shape = small ? 0 : 1;
+  if (no_cutoff(e->p.born_cutoff)) e->born_launch.shape = pairs < 4000 ? 0 : 1;
   if (no_cutoff(e->p.nb_cutoff) || no_cutoff(e->p.gb_force_cutoff))
     e->force_launch.shape = pairs < 800 ? 0 : pairs < 40000 ? 1 : 4;
 }
