@@ -154,6 +154,36 @@ __device__ __forceinline__ void flush_j(const PairArgs& a, const int32_t* jlist,
   }
 }
 
+// Lower bound (A) on the distance of any atom pair of two tiles, from their
+// bounding spheres; the margin covers the FP32 rounding.
+__device__ __forceinline__ float tile_gap(double4 oi, double4 oj) {
+  const float dx = static_cast<float>(oj.x - oi.x), dy = static_cast<float>(oj.y - oi.y),
+              dz = static_cast<float>(oj.z - oi.z);
+  const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+  return d * (1.0f - 1e-6f) - static_cast<float>(oi.w + oj.w) - 1e-3f;
+}
+
+// A stage's j-tiles as the block's kI i-tiles see them: the offset of the
+// tiles' origins (x, y, z: j minus i) and the gap between their spheres (w),
+// one thread per (i-tile, j-tile) a stage ahead.  (Every warp for itself, for
+// each tile pair: 35 to 100 instructions of 900 and two dependent loads.)
+template <int kI>
+struct StageTilesT {
+  int jt[kStageTiles];
+  float4 off[kStageTiles][kI];
+};
+template <int kI>
+__device__ __forceinline__ void stage_tiles(const PairArgs& a, const PairWork& w, int stage, StageTilesT<kI>& s) {
+  const int t = threadIdx.x % kStageTiles, q = threadIdx.x / kStageTiles;
+  const int at = w.j_begin + stage * kStageTiles + t;
+  if (at >= w.j_end || q >= w.n_i_tiles) return;  // at most kI i-tiles
+  const int jt = a.jlist[at];
+  const double4 oj = a.origin[jt], oi = a.origin[w.i_tile0 + q];
+  s.off[t][q] = make_float4(static_cast<float>(oj.x - oi.x), static_cast<float>(oj.y - oi.y),
+                            static_cast<float>(oj.z - oi.z), tile_gap(oi, oj));
+  if (q == 0) s.jt[t] = jt;
+}
+
 // ---------------------------------------------------------------- Born
 // origami's pairwise_descreening (gb.rs:347-369) is
 //   h = 1/2 (1/L - 1/U) + (r/4)(1/U^2 - 1/L^2) + ln(L/U)/(2r)
@@ -212,15 +242,6 @@ __device__ __forceinline__ float2 born_pair(float dx, float dy, float dz, float 
   }
   const bool on = (r2 <= c2) && (r2 >= 1e-18f);
   return on ? h : make_float2(0.0f, 0.0f);
-}
-
-// Lower bound (A) on the distance of any atom pair of two tiles, from their
-// bounding spheres; the margin covers the FP32 rounding.
-__device__ __forceinline__ float tile_gap(double4 oi, double4 oj) {
-  const float dx = static_cast<float>(oj.x - oi.x), dy = static_cast<float>(oj.y - oi.y),
-              dz = static_cast<float>(oj.z - oi.z);
-  const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-  return d * (1.0f - 1e-6f) - static_cast<float>(oi.w + oj.w) - 1e-3f;
 }
 
 // --------------------------------------------------- Born, distant tiles
@@ -362,6 +383,7 @@ template <int W, int kMinBlocks, bool kPersistent>
 __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   __shared__ __align__(128) float s_buf[2][3][kStageFloats];          // columns of pq, gb, bs
   __shared__ float s_part[W][1][kStageTiles * kTile];
+  __shared__ StageTilesT<W> s_tiles[2];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_item;
 
@@ -392,9 +414,9 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
   const float rho_i = a.gb[soa_index(i, 2)], s_i = a.gb[soa_index(i, 3)];
   const float3 ci = make_float3(a.bs[soa_index(i, 0)], a.bs[soa_index(i, 1)], a.bs[soa_index(i, 2)]);
-  const double4 oi = a.origin[it];
   const float c2 = a.born_c2;
   double acc = 0.0;
+  stage_tiles(a, w, 0, s_tiles[g & 1]);
   for (int s = 0; s < st.n_stages; ++s) {
     const uint32_t gs = g + s;
     const int b = gs & 1;
@@ -405,21 +427,22 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
     }
     const int t0 = w.j_begin + s * kStageTiles;
     const int cnt = min(kStageTiles, w.j_end - t0);
+    stage_tiles(a, w, s + 1, s_tiles[b ^ 1]);
     for (int t = 0; t < cnt; ++t) {
-      const int jt = a.jlist[t0 + t];
+      const int jt = s_tiles[b].jt[t];
       float* part = &s_part[warp][0][t * kTile];
-      const double4 oj = a.origin[jt];
-      if (!active || jt < it || (c2 != INFINITY && tile_gap(oi, oj) > a.born_cutoff)) {
+      const float4 off = s_tiles[b].off[t][warp];
+      if (!active || jt < it || (c2 != INFINITY && off.w > a.born_cutoff)) {
         part[lane] = 0.0f;
         continue;
       }
-      const float xi = px - static_cast<float>(oj.x - oi.x);
-      const float yi = py - static_cast<float>(oj.y - oi.y);
-      const float zi = pz - static_cast<float>(oj.z - oi.z);
+      const float xi = px - off.x;
+      const float yi = py - off.y;
+      const float zi = pz - off.z;
       const float* sp = &s_buf[b][0][t * 128];
       const float* sg = &s_buf[b][1][t * 128];
       float hi = 0.0f;
-      const bool series = born_far_tile(gaps, tile_gap(oi, oj), sp, sg, &s_buf[b][2][t * 128], 0, kTile, xi, yi, zi, s_i,
+      const bool series = born_far_tile(gaps, off.w, sp, sg, &s_buf[b][2][t * 128], 0, kTile, xi, yi, zi, s_i,
                                         ci, c2, &hi,
                                         [&](int k0, float v0, float v1, float v2, float v3) {
                                           const float tot = reduce_scatter4(v0, v1, v2, v3, lane);
@@ -720,6 +743,7 @@ template <bool kAllPairs, int W, int kMinBlocks, bool kPersistent>
 __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
   __shared__ __align__(128) float s_buf[2][3][kStageFloats];          // columns of pq, lj, gb
   __shared__ float s_part[W][3][kStageTiles * kTile];
+  __shared__ StageTilesT<W> s_tiles[2];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_item;
 
@@ -747,12 +771,12 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
   const int it = w.i_tile0 + (active ? warp : 0);
   const int i = it * kTile + lane;
   const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
-  const double4 oi = a.origin[it];
   IAtom2 ia = i_atom(a, i);
   const float ri_max = kAllPairs ? warp_max(ia.R.x) : 0.0f;
   int mref = a.mask_begin[it];
   const int mend = a.mask_begin[it + 1];
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
+  stage_tiles(a, w, 0, s_tiles[g & 1]);
 
   for (int s = 0; s < st.n_stages; ++s) {
     const uint32_t gs = g + s;
@@ -764,23 +788,24 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
     }
     const int t0 = w.j_begin + s * kStageTiles;
     const int cnt = min(kStageTiles, w.j_end - t0);
+    stage_tiles(a, w, s + 1, s_tiles[b ^ 1]);
     for (int t = 0; t < cnt; ++t) {
-      const int jt = a.jlist[t0 + t];
+      const int jt = s_tiles[b].jt[t];
       while (mref < mend && a.mask_refs[mref].j_tile < jt) ++mref;
       const bool masked = mref < mend && a.mask_refs[mref].j_tile == jt;
       float* jfx = &s_part[warp][0][t * kTile];
       float* jfy = &s_part[warp][1][t * kTile];
       float* jfz = &s_part[warp][2][t * kTile];
-      const double4 oj = a.origin[jt];
-      if (!(active && jt > it && !masked) || (!kAllPairs && tile_gap(oi, oj) > a.pair_cutoff)) {
+      const float4 off = s_tiles[b].off[t][warp];
+      if (!(active && jt > it && !masked) || (!kAllPairs && off.w > a.pair_cutoff)) {
         jfx[lane] = 0.0f;
         jfy[lane] = 0.0f;
         jfz[lane] = 0.0f;
         continue;
       }
-      ia.nx = bc(-(px - static_cast<float>(oj.x - oi.x)));
-      ia.ny = bc(-(py - static_cast<float>(oj.y - oi.y)));
-      ia.nz = bc(-(pz - static_cast<float>(oj.z - oi.z)));
+      ia.nx = bc(-(px - off.x));
+      ia.ny = bc(-(py - off.y));
+      ia.nz = bc(-(pz - off.z));
       const float* sp = &s_buf[b][0][t * 128];
       const float* sl = &s_buf[b][1][t * 128];
       const float* sg = &s_buf[b][2][t * 128];
@@ -798,7 +823,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
           jfz[k0 + (lane >> 3)] = -tz;
         }
       };
-      if (kAllPairs && far_tiles(tile_gap(oi, oj), ri_max, warp_max(sg[lane]))) {
+      if (kAllPairs && far_tiles(off.w, ri_max, warp_max(sg[lane]))) {
 #pragma unroll 2
         for (int k0 = 0; k0 < kTile; k0 += 4) add_group(k0, force_far4(sp + k0, sl + k0, ia));
       } else {
@@ -983,9 +1008,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_quad(PairArgs a) {
   __shared__ __align__(128) float s_buf[2][3][kStageFloats];                  // raw columns of pq, lj, gb (TMA)
   __shared__ __align__(16) float s_dup[kStageTiles][kForceCols * 2 * kTile];  // the stage's columns, each value twice
   __shared__ float s_rmax[kStageTiles];
-  __shared__ int s_jt[2][kStageTiles];        // the stage's j-tiles and their spheres, loaded a stage ahead
-  __shared__ double4 s_oj[2][kStageTiles];
-  __shared__ double4 s_oi[W * 4];             // the block's i-tile spheres
+  __shared__ StageTilesT<W * 4> s_tiles[2];
   __shared__ float s_part[W][3][kStageTiles * kTile];
   __shared__ double s_acc[W][12][kTile];  // the lanes' sums over j-tiles, per i-tile and component
   __shared__ __align__(8) uint64_t s_bar[2];
@@ -1044,17 +1067,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_quad(PairArgs a) {
     mnext[q] = 0x7fffffff;
     if (q < n_own) load_next(q, a.mask_begin[it0 + q]);
   }
-  auto stage_info = [&](int st_index) {
-    const int t = static_cast<int>(threadIdx.x);
-    if (t < kStageTiles && w.j_begin + st_index * kStageTiles + t < w.j_end) {
-      const int jt = a.jlist[w.j_begin + st_index * kStageTiles + t], b = (g + st_index) & 1;
-      s_jt[b][t] = jt;
-      s_oj[b][t] = a.origin[jt];
-    }
-  };
-  __syncthreads();  // the previous item's info has been read
-  if (static_cast<int>(threadIdx.x) < w.n_i_tiles) s_oi[threadIdx.x] = a.origin[w.i_tile0 + threadIdx.x];
-  stage_info(0);
+  stage_tiles(a, w, 0, s_tiles[g & 1]);
   double(*acc)[kTile] = s_acc[warp];
 #pragma unroll
   for (int q = 0; q < 12; ++q) acc[q][lane] = 0.0;
@@ -1085,31 +1098,27 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_quad(PairArgs a) {
     }
     __syncthreads();  // s_dup is complete and raw buffer b is free
     if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
-    if (s + 1 < st.n_stages) stage_info(s + 1);
+    stage_tiles(a, w, s + 1, s_tiles[b ^ 1]);
     for (int t = 0; t < cnt; ++t) {
-      const int jt = s_jt[b][t];
-      const double4 oj = s_oj[b][t];
+      const int jt = s_tiles[b].jt[t];
       unsigned on = 0;  // own tiles that meet this j-tile here
       float gap = INFINITY;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         while (mnext[q] < jt) load_next(q, mref[q] + 1);
-        const double4 oi = s_oi[it0 - w.i_tile0 + (q < n_own ? q : 0)];
-        const float gq = tile_gap(oi, oj);
-        if (q < n_own && jt > it0 + q && mnext[q] != jt && (kAllPairs || gq <= a.pair_cutoff)) {
+        const float4 off = s_tiles[b].off[t][it0 - w.i_tile0 + (q < n_own ? q : 0)];
+        if (q < n_own && jt > it0 + q && mnext[q] != jt && (kAllPairs || off.w <= a.pair_cutoff)) {
           on |= 1u << q;
-          gap = fminf(gap, gq);
+          gap = fminf(gap, off.w);
         }
-        const float ox = static_cast<float>(oj.x - oi.x), oy = static_cast<float>(oj.y - oi.y),
-                    oz = static_cast<float>(oj.z - oi.z);
         if (q & 1) {
-          ia[q / 2].nx.y = ox - px[q / 2].y;
-          ia[q / 2].ny.y = oy - py[q / 2].y;
-          ia[q / 2].nz.y = oz - pz[q / 2].y;
+          ia[q / 2].nx.y = off.x - px[q / 2].y;
+          ia[q / 2].ny.y = off.y - py[q / 2].y;
+          ia[q / 2].nz.y = off.z - pz[q / 2].y;
         } else {
-          ia[q / 2].nx.x = ox - px[q / 2].x;
-          ia[q / 2].ny.x = oy - py[q / 2].x;
-          ia[q / 2].nz.x = oz - pz[q / 2].x;
+          ia[q / 2].nx.x = off.x - px[q / 2].x;
+          ia[q / 2].ny.x = off.y - py[q / 2].x;
+          ia[q / 2].nz.x = off.z - pz[q / 2].x;
         }
       }
       float* jfx = &s_part[warp][0][t * kTile];
