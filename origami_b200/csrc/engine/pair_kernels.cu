@@ -130,11 +130,11 @@ using Stager = StagerT<>;
 // Adds the stage's j partials (s_part[w][c][q], summed over warps in a fixed
 // order) to the fixed-point accumulators.
 template <int W, int kComps, int kST = kStageTiles>
-__device__ __forceinline__ void flush_j(const PairArgs& a, const int32_t* jlist, int t0, int cnt,
+__device__ __forceinline__ void flush_j(const PairArgs& a, const int* jt, int cnt,
                                         float (*s_part)[kComps][kST * kTile], unsigned long long* const* dst,
                                         double scale) {
   for (int q = threadIdx.x; q < cnt * kTile; q += blockDim.x) {
-    const int j = jlist[t0 + q / kTile] * kTile + (q % kTile);
+    const int j = jt[q / kTile] * kTile + (q % kTile);
     if (!a.atom_valid[j]) continue;
     float v[kComps];
     bool any = false, finite = true;
@@ -480,7 +480,7 @@ OG_UNROLL(OG_BORN_UNROLL)
     __syncthreads();  // every warp is done with buffer b and has written its j partials
     if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
     unsigned long long* dst[1] = {a.born_sum};
-    flush_j<W, 1>(a, a.jlist, t0, cnt, s_part, dst, kBornScale);
+    flush_j<W, 1>(a, s_tiles[b].jt, cnt, s_part, dst, kBornScale);
   }
   g += st.n_stages;
   if (active && a.atom_valid[i]) {
@@ -773,8 +773,10 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
   const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
   IAtom2 ia = i_atom(a, i);
   const float ri_max = kAllPairs ? warp_max(ia.R.x) : 0.0f;
+  // the next near-field j-tile (refs are in j order)
   int mref = a.mask_begin[it];
   const int mend = a.mask_begin[it + 1];
+  int mnext = mref < mend ? a.mask_refs[mref].j_tile : 0x7fffffff;
   double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
   stage_tiles(a, w, 0, s_tiles[g & 1]);
 
@@ -791,8 +793,8 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force(PairArgs a) {
     stage_tiles(a, w, s + 1, s_tiles[b ^ 1]);
     for (int t = 0; t < cnt; ++t) {
       const int jt = s_tiles[b].jt[t];
-      while (mref < mend && a.mask_refs[mref].j_tile < jt) ++mref;
-      const bool masked = mref < mend && a.mask_refs[mref].j_tile == jt;
+      while (mnext < jt) mnext = ++mref < mend ? a.mask_refs[mref].j_tile : 0x7fffffff;
+      const bool masked = mnext == jt;
       float* jfx = &s_part[warp][0][t * kTile];
       float* jfy = &s_part[warp][1][t * kTile];
       float* jfz = &s_part[warp][2][t * kTile];
@@ -838,7 +840,7 @@ OG_UNROLL(OG_FORCE_UNROLL)
     __syncthreads();  // every warp is done with buffer b and has written its j partials
     if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
     unsigned long long* dst[3] = {a.fx, a.fy, a.fz};
-    flush_j<W, 3>(a, a.jlist, t0, cnt, s_part, dst, kForceScale);
+    flush_j<W, 3>(a, s_tiles[b].jt, cnt, s_part, dst, kForceScale);
   }
   g += st.n_stages;
   if (active && a.atom_valid[i]) {
@@ -1154,7 +1156,7 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_force_quad(PairArgs a) {
     }
     __syncthreads();  // every warp is done with s_dup and has written its j partials
     unsigned long long* dst[3] = {a.fx, a.fy, a.fz};
-    flush_j<W, 3>(a, a.jlist, t0, cnt, s_part, dst, kForceScale);
+    flush_j<W, 3>(a, s_tiles[b].jt, cnt, s_part, dst, kForceScale);
   }
   g += st.n_stages;
 #pragma unroll
