@@ -382,8 +382,8 @@ __device__ __forceinline__ int next_item(const PairArgs& a, int* s_item, int pre
 template <int W, int kMinBlocks, bool kPersistent>
 __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   __shared__ __align__(128) float s_buf[2][3][kStageFloats];          // columns of pq, gb, bs
-  __shared__ float s_part[W][1][kStageTiles * kTile];
-  __shared__ StageTilesT<W> s_tiles[2];
+  __shared__ float s_part[2][W][1][kStageTiles * kTile];
+  __shared__ StageTilesT<W> s_tiles[3];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ int s_item;
 
@@ -416,7 +416,13 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
   const float3 ci = make_float3(a.bs[soa_index(i, 0)], a.bs[soa_index(i, 1)], a.bs[soa_index(i, 2)]);
   const float c2 = a.born_c2;
   double acc = 0.0;
-  stage_tiles(a, w, 0, s_tiles[g & 1]);
+  stage_tiles(a, w, 0, s_tiles[g % 3]);
+  // the j sums of stage s, once every warp has written its own
+  auto flush = [&](int s) {
+    unsigned long long* dst[1] = {a.born_sum};
+    const int cnt = min(kStageTiles, w.j_end - (w.j_begin + s * kStageTiles));
+    flush_j<W, 1>(a, s_tiles[(g + s) % 3].jt, cnt, s_part[(g + s) & 1], dst, kBornScale);
+  };
   for (int s = 0; s < st.n_stages; ++s) {
     const uint32_t gs = g + s;
     const int b = gs & 1;
@@ -425,13 +431,21 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
       if (threadIdx.x == 0) atomicOr(a.error_flag, kStatusTimeout);
       return;
     }
-    const int t0 = w.j_begin + s * kStageTiles;
-    const int cnt = min(kStageTiles, w.j_end - t0);
-    stage_tiles(a, w, s + 1, s_tiles[b ^ 1]);
+    // one barrier per stage: here every warp is done with the stage before, whose
+    // raw buffer is free and whose j sums are complete (a second barrier before
+    // the flush: 650 -> 640 us for 64 chains of 300 residues; k_force, with
+    // three components to buffer twice, lost 1 % by it)
+    if (s > 0) {
+      if (threadIdx.x == 0 && s + 1 < st.n_stages) st.issue<3>(s + 1, s_buf, src);
+      flush(s - 1);
+    }
+    const int cnt = min(kStageTiles, w.j_end - (w.j_begin + s * kStageTiles));
+    stage_tiles(a, w, s + 1, s_tiles[(gs + 1) % 3]);
+    const StageTilesT<W>& tiles = s_tiles[gs % 3];
     for (int t = 0; t < cnt; ++t) {
-      const int jt = s_tiles[b].jt[t];
-      float* part = &s_part[warp][0][t * kTile];
-      const float4 off = s_tiles[b].off[t][warp];
+      const int jt = tiles.jt[t];
+      float* part = &s_part[b][warp][0][t * kTile];
+      const float4 off = tiles.off[t][warp];
       if (!active || jt < it || (c2 != INFINITY && off.w > a.born_cutoff)) {
         part[lane] = 0.0f;
         continue;
@@ -477,11 +491,9 @@ OG_UNROLL(OG_BORN_UNROLL)
       }
       acc += static_cast<double>(hi);
     }
-    __syncthreads();  // every warp is done with buffer b and has written its j partials
-    if (threadIdx.x == 0 && s + 2 < st.n_stages) st.issue<3>(s + 2, s_buf, src);
-    unsigned long long* dst[1] = {a.born_sum};
-    flush_j<W, 1>(a, s_tiles[b].jt, cnt, s_part, dst, kBornScale);
   }
+  __syncthreads();
+  flush(st.n_stages - 1);
   g += st.n_stages;
   if (active && a.atom_valid[i]) {
     if (!isfinite(acc)) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
