@@ -23,59 +23,11 @@ namespace ogk {
 // only).  The pair coefficient is symmetric in i and j, so the j-side force
 // is exactly the negated i-side term.
 //
-// Bound by the FP64 pipe: 61 operations per pair and lane, of which the two
-// roots take 10 and the exponential 11 (rsqrt64, exp_neg64), with the pair
-// constants folded into the i atom's.  The library's rsqrt and exp, and the
-// constants applied per pair, took 73 us (now 66)
-// for 256 chains of 10 to 80 residues and 113 (now 101) for 64 chains of 300.
-//
 // kSplit = 4 gives a tile pair to the four warps of a block, each taking
 // every fourth step, their sums added in warp order: a warp's 32 steps are a
 // chain of FP64 latency (about 20 us), which is the kernel's time when there
 // are too few tile pairs to fill the SMs.
 namespace {
-
-// 1 / a and 1 / sqrt(a) to an ulp or so: the special-function unit's
-// approximation (relative error below 2^-21) and one third-order
-// Newton-Householder step, whose error is the cube of that.  Without the
-// library's handling of zero (NaN here, infinity there), which the callers
-// do not need.
-__device__ __forceinline__ double rcp64(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double rsqrt64(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
-// e^x for x <= 0 to an ulp or so: x = k ln2 / 32 + r, |r| <= ln2 / 64, as
-// 2^(k / 32) -- `table` holds the 32 fractional powers -- times the Taylor
-// polynomial of e^r, whose first dropped term is r^7 / 5040 < 4e-18 (table
-// method: P. T. P. Tang, Table-driven implementation of the exponential
-// function in IEEE floating-point arithmetic, 1989).  Below -700, e^-700.
-__device__ __forceinline__ double exp_neg64(double x, const double* table) {
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word holds the rounded integer
-  x = fmax(x, -700.0);
-  const double t = fma(x, 46.16624130844683, kMagic);  // 32 / ln2
-  const int k = __double2loint(t);
-  const double n = t - kMagic;
-  // ln2 / 32 in two parts, the first with its low 21 bits zero (n < 2^15)
-  double r = fma(n, -0.02166084938653512, x);
-  r = fma(n, -5.9631716539705866e-12, r);
-  double q = fma(r, 1.0 / 720.0, 1.0 / 120.0);
-  q = fma(q, r, 1.0 / 24.0);
-  q = fma(q, r, 1.0 / 6.0);
-  q = fma(q, r, 0.5);
-  const double p = fma(r * r, q, r);
-  const double f = table[k & 31];
-  const double v = fma(f, p, f);
-  return __hiloint2double(__double2hiint(v) + ((k >> 5) << 20), __double2loint(v));
-}
 
 constexpr int kNearWarps = 4;
 // Tile pairs per SM up to which a block takes one.
@@ -89,6 +41,7 @@ constexpr int kNearSplitPerSm = OG_NEAR_SPLIT;
 struct NearTile {
   double x[kTile], y[kTile], z[kTile], q[kTile], r[kTile], ir[kTile];
   double rmin[kTile], seps[kTile], rmin14[kTile], seps14[kTile];
+  int32_t valid[kTile];
 };
 struct NearForce {
   double x[kTile], y[kTile], z[kTile];
@@ -99,11 +52,8 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
   static_assert(kSplit == 1 || kSplit == kNearWarps, "a warp or a block per tile pair");
   __shared__ NearTile tiles[kNearWarps / kSplit];
   __shared__ NearForce jf[kNearWarps], sf[kSplit > 1 ? kNearWarps : 1];
-  __shared__ double pow2[kTile];  // 2^(k / 32)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wid = kSplit > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kNearWarps + warp;
-  if (threadIdx.x < kTile) pow2[lane] = exp2(lane * (1.0 / kTile));
-  if (kSplit == 1) __syncthreads();
   if (wid >= n_near) return;  // block-uniform when split
   const int part = kSplit > 1 ? warp : 0;
   NearTile& t = tiles[kSplit > 1 ? 0 : warp];
@@ -122,51 +72,51 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
     t.seps[lane] = sqrt(a.eps64[jl]);
     t.rmin14[lane] = a.rmin14_64[jl];
     t.seps14[lane] = sqrt(a.eps14_64[jl]);
+    t.valid[lane] = a.atom_valid[jl];
   }
   f.x[lane] = f.y[lane] = f.z[lane] = 0.0;
   const uint32_t ex = a.mask_ex[w.z * kTile + lane];
   const uint32_t m14 = a.mask_14[w.z * kTile + lane];
-  const bool valid_i = a.atom_valid[i] != 0, valid_j = a.atom_valid[jl] != 0;
-  const uint32_t j_set = __ballot_sync(0xffffffffu, valid_j);
-  const double xi = a.x64[i], yi = a.y64[i], zi = a.z64[i], Ri = a.born_r64[i];
-  const double rmi = a.rmin64[i], rm14i = a.rmin14_64[i];
-  // the pair constants are folded into the i atom's
-  const double se_kj = 12.0 * kKcalToKj * sqrt(a.eps64[i]), se14_kj = 12.0 * kKcalToKj * sqrt(a.eps14_64[i]);
-  const double coul_q = -kCoulomb * kKcalToKj * a.q64[i];
-  const double gb_q = (1.0 - 1.0 / kEpsWater) * kCoulomb * kKcalToKj * a.q64[i];
-  const double exp_r = -0.25 / Ri;
+  const bool valid_i = a.atom_valid[i] != 0;
+  const double xi = a.x64[i], yi = a.y64[i], zi = a.z64[i], qi = a.q64[i], Ri = a.born_r64[i];
+  const double rmi = a.rmin64[i], sepi = sqrt(a.eps64[i]), rm14i = a.rmin14_64[i], sep14i = sqrt(a.eps14_64[i]);
+  const double iRi = 1.0 / Ri;
+  const double coul_kj = kCoulomb * kKcalToKj;
+  const double gb_pref = (1.0 - 1.0 / kEpsWater) * kCoulomb * kKcalToKj;
   const bool diag = w.x == w.y;
   double ax = 0.0, ay = 0.0, az = 0.0;
   if (kSplit > 1) __syncthreads();
   else __syncwarp();
   for (int k = (diag ? 1 : 0) + part; k < (diag ? 17 : kTile); k += kSplit) {
     const int p = (lane + k) & (kTile - 1);
-    const double dx = t.x[p] - xi, dy = t.y[p] - yi, dz = t.z[p] - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const bool on = valid_i && ((j_set >> p) & 1u) && r2 >= 1e-18 && !(diag && k == 16 && lane >= 16);
-    double coeff = 0.0;
-    if (on) {
-      const double qj = t.q[p];
-      // 1/r from one reciprocal square root; the GB factor
-      // (1/f^2) ((2r - r e / 2) / (2f)) / r of the reference is
-      // (1 - e/4) / f^3, and f^-1 another reciprocal square root
-      if (r2 <= a.gb_c2_64) {
-        const double e = exp_neg64(r2 * (exp_r * t.ir[p]), pow2);
-        const double inv_f = rsqrt64(fma(Ri * t.r[p], e, r2));
-        coeff = (gb_q * qj) * fma(-0.25, e, 1.0) * (inv_f * inv_f * inv_f);
-      }
-      if (!((ex >> p) & 1u) && r2 <= a.nb_c2_64) {
-        const double inv_r = rsqrt64(r2);
+    double coeff = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
+    if (valid_i && t.valid[p] && !(diag && k == 16 && lane >= 16)) {
+      dx = t.x[p] - xi;
+      dy = t.y[p] - yi;
+      dz = t.z[p] - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double qq = qi * t.q[p];
+      if (r2 >= 1e-18) {
+        // 1/r from one reciprocal square root; the GB factor
+        // (1/f^2) ((2r - r e / 2) / (2f)) / r of the reference is
+        // (1 - e/4) / f^3, and f^-1 another reciprocal square root
+        const double inv_r = rsqrt(r2);
         const double inv_r2 = inv_r * inv_r;
-        double rmin = rmi + t.rmin[p], eps = se_kj * t.seps[p];
-        if ((m14 >> p) & 1u) {
-          rmin = rm14i + t.rmin14[p];
-          eps = se14_kj * t.seps14[p];
+        if (!((ex >> p) & 1u) && r2 <= a.nb_c2_64) {
+          const bool is14 = (m14 >> p) & 1u;
+          const double rmin = is14 ? rm14i + t.rmin14[p] : rmi + t.rmin[p];
+          const double eps = is14 ? sep14i * t.seps14[p] : sepi * t.seps[p];
+          const double ratio2 = rmin * rmin * inv_r2;
+          const double r6 = ratio2 * ratio2 * ratio2;
+          coeff += 12.0 * eps * inv_r2 * (r6 - r6 * r6) * kKcalToKj;
+          if (qq != 0.0) coeff += -coul_kj * qq * (inv_r2 * inv_r - a.inv_rc3_64);
         }
-        const double ratio2 = rmin * rmin * inv_r2;
-        const double r6 = ratio2 * ratio2 * ratio2;
-        coeff = fma(eps * inv_r2, fma(-r6, r6, r6), coeff);
-        coeff = fma(coul_q * qj, fma(inv_r2, inv_r, -a.inv_rc3_64), coeff);
+        if (qq != 0.0 && r2 <= a.gb_c2_64) {
+          const double rp = Ri * t.r[p];
+          const double e = exp(-0.25 * r2 * (iRi * t.ir[p]));
+          const double inv_f = rsqrt(r2 + rp * e);
+          coeff += gb_pref * qq * (1.0 - 0.25 * e) * (inv_f * inv_f * inv_f);
+        }
       }
     }
     ax += dx * coeff;
@@ -194,7 +144,7 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
       az += side[w].z[lane];
     }
     const int at = warp == 0 ? i : jl;
-    if (warp == 0 ? valid_i : valid_j) {
+    if (warp == 0 ? valid_i : t.valid[lane] != 0) {
       if (!(isfinite(ax) && isfinite(ay) && isfinite(az))) atomicOr(a.sys_nonfinite + a.atom_sys[at], 1);
       add_fixed(a.fx + at, ax, kForceScale);
       add_fixed(a.fy + at, ay, kForceScale);
@@ -208,7 +158,7 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
     add_fixed(a.fy + i, ay, kForceScale);
     add_fixed(a.fz + i, az, kForceScale);
   }
-  if (valid_j) {
+  if (t.valid[lane]) {
     const double bx = f.x[lane], by = f.y[lane], bz = f.z[lane];
     if (!(isfinite(bx) && isfinite(by) && isfinite(bz))) atomicOr(a.sys_nonfinite + a.atom_sys[jl], 1);
     add_fixed(a.fx + jl, bx, kForceScale);
@@ -247,6 +197,24 @@ void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_
 namespace {
 
 constexpr int kEnergyWarps = 4;
+
+// 1 / a and 1 / sqrt(a) to an ulp or so: the special-function unit's
+// approximation (relative error below 2^-21) and one third-order
+// Newton-Householder step, whose error is the cube of that.  Without the
+// library's handling of zero (NaN here, infinity there), which the callers
+// do not need.
+__device__ __forceinline__ double rcp64(double a) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt64(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 
 __device__ __forceinline__ double descreen64(double r, double r2, double inv_r, double rho_i, double s_rho_j) {
   // energy/src/gb.rs:347-369, with 1/r given.
