@@ -40,10 +40,10 @@ sys.path.insert(0, ROOT)
 AA_ORDER = "ARNDCQEGHILKMFPSTWYV"  # AminoAcid::ALL (chem/src/amino_acid.rs:31)
 METRIC = "aggregate ns/day (64 replicas, 5k atoms, GB+SASA): learned-GB vs plain GB"
 # DRAM bytes (read + write) of one force-pass launch per replica of the
-# 4 694-atom chain: ncu at 4 replicas read 1.51 MB and wrote nothing; each
+# 4 694-atom chain: ncu at 4 replicas read 1.57 MB and wrote nothing; each
 # replica's packed arrays stay in L2 across its tile sweep, so the traffic
 # grows with replicas, not with pairs.
-FORCE_PASS_DRAM_BYTES_PER_REPLICA = 1.514496e6 / 4
+FORCE_PASS_DRAM_BYTES_PER_REPLICA = 1.570816e6 / 4
 FIXTURE = os.path.join(ROOT, "tests", "golden", "bench_chain_300.npz")
 TOPO_FIELDS = ("charge", "rmin_half", "epsilon", "rmin_half_14", "epsilon_14", "gb_rho", "gb_scale", "mass",
                "element", "bonds", "bond_k", "bond_r0", "angles", "angle_k", "angle_theta0", "dihedrals",
@@ -495,20 +495,17 @@ def run_b200(args):
                      "note": ("cutoff mode: the pairs evaluated are not counted, so no throughput is reported"
                               if args.cutoff else None),
                      "traffic": FORCE_PASS_DRAM_BYTES_PER_REPLICA * args.replicas,
-                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_force<1> at 4 "
-                                       "replicas (profiles/pair_kernels_4x4694_extended.md; the relaxed chain and the "
-                                       "two-i-tile k_force_ip give the same 1.51 MB, "
-                                       "profiles/force_ip_instruction_mix_4x4694.md), per replica x replicas",
+                     "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_force_quad at 4 "
+                                       "replicas (profiles/step_kernels_4x4694.md), per replica x replicas",
                      "peak_source": "measured FP32 FMA chain (og_measure_fp32_peak); the pair math is FP32 "
                                     "CUDA-core work, so neither the HBM copy nor the BF16 tensor peak bounds it",
                      "work": "55 flop per unordered pair (include/flops.h) x N(N-1)/2 x replicas"},
         "dominant_kernel": {
             "kernel": "k_sasa_boundary + k_sasa_terms (PowerSasa, FP64)",
             "ms_per_step": (prof["sasa"][0] / prof["sasa"][1]) if "sasa" in prof else None,
-            "bound": "dependency latency at 20 warps per SM (ncu on the relaxed chain: issue active 52 %, "
-                     "FP64 pipe 14 %, DRAM 0.03 %, 23 of 32 lanes active); data-dependent geometry, no flop "
-                     "or byte roofline",
-            "profile": "profiles/sasa_boundary_4x4694_relaxed.md",
+            "bound": "issue slots at 24 warps per SM and code size (ncu, 16 folds of 306 residues: issue active "
+                     "76 %, ALU 51 %, FP64 pipe 5 %); data-dependent geometry, no flop or byte roofline",
+            "profile": "profiles/step_kernels_4x4694.md",
             "launch_list": "profiles/launch_list_64x4694_plain_step.md"},
         "sasa_share_of_step": (prof["sasa"][0] / prof["sasa"][1] / plain_ms) if "sasa" in prof else None,
         "born_pass_tflops": born_tflops,

@@ -36,10 +36,11 @@
 // Tile pairs are classed by the gap between their bounding spheres: distant
 // ones take shorter forms of the same sums (fewer series terms, the far GB
 // form without its exponential), with every pair's condition implied by the
-// gap.  64 x 4 694 atoms, all pairs, B200: Born 1.265 -> 0.668 ms (k_born, 64
-// registers, FMA pipe 62 % busy), force 1.105 -> 0.843 ms (k_force_quad, 162
-// registers, 12 warps per SM, FMA pipe 56 %); one 300-atom system 58 -> 5 and
-// 32 -> 5 us (split).
+// gap.  64 x 4 694 atoms, all pairs, B200: Born 1.265 -> 0.668 ms by the
+// tiers and shapes (k_born, 64 registers, FMA pipe 62 % busy) -> 0.640 with the
+// tile offsets taken once per stage and one barrier per stage; force 1.105 ->
+// 0.843 (k_force_quad, 162 registers, 12 warps per SM, FMA pipe 56 %) -> 0.817;
+// one 300-atom system 58 -> 5 and 32 -> 5 us (split).
 //
 // Positions are FP32 offsets from a per-tile FP64 origin; the origin
 // difference of a tile pair is formed in FP64 once per tile, so |dx| keeps
@@ -166,7 +167,9 @@ __device__ __forceinline__ float tile_gap(double4 oi, double4 oj) {
 // A stage's j-tiles as the block's kI i-tiles see them: the offset of the
 // tiles' origins (x, y, z: j minus i) and the gap between their spheres (w),
 // one thread per (i-tile, j-tile) a stage ahead.  (Every warp for itself, for
-// each tile pair: 35 to 100 instructions of 900 and two dependent loads.)
+// each tile pair: 35 to 100 instructions of 900 and two dependent loads; 675
+// against 650 us of the Born pass and 846 against 819 of the force pass for 64
+// chains of 300 residues.)
 template <int kI>
 struct StageTilesT {
   int jt[kStageTiles];
