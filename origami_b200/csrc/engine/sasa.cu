@@ -458,6 +458,23 @@ __device__ __forceinline__ void keep_or(W& w, int j, int b) {
   atomicOr(reinterpret_cast<unsigned*>(&w.keep[j]) + (b >> 5), 1u << (b & 31));
 }
 
+// How many lanes (1, 2 or 4, as a power of two) share an item when `left` are
+// left, `full` of which occupy the warp -- in the large-capacity kernel, whose
+// warps run alone on their scheduler, so that the last, partly filled trip's
+// latency counts (insulin: 55.6 -> 53.5 us, a step 77 -> 72).  In the default kernel the shared
+// trips won 6 % for compact folds and lost 3 % for extended chains.
+template <class W>
+__device__ __forceinline__ int lane_split_log2(int left, int full) {
+  return !W::kBig || left > full ? 0 : left > full / 2 ? 1 : 2;
+}
+// A ballot of shared items: the bits of an item's lanes (32 >> lg apart)
+// combined, in all of them.
+__device__ __forceinline__ unsigned split_and(unsigned v, int lg) {
+  if (lg >= 2) v &= __funnelshift_l(v, v, 8);
+  if (lg >= 1) v &= __funnelshift_l(v, v, 16);
+  return v;
+}
+
 enum Outcome { kExposed = 0, kBuried = 1, kBounded = 2, kInvalid = 3 };
 
 // A point of circle k (cos alpha_k = ck.c, radius sk = sin alpha_k) from its
@@ -595,7 +612,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // and of its distance), queue up in ascending order and are made into caps
   // 32 at a time, so that the root and the quotients run with every lane busy
   // (a hit tile has about four neighbours).
-  constexpr int kTilesPerTrip = 2;
+  constexpr int kTilesPerTrip = W::kBig ? 4 : 2;
   int t0 = 0;
   unsigned hits = 0;
   float4 rel{};  // this lane's tile: centre - p_i, R_i + margin
@@ -668,18 +685,20 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
   // on the left, 4e-7 / (2 s_k s_m) on the right) stay well below it, so
   // only contained circles go; one that is kept within the margin changes
   // nothing but the work.
-  // Each lane tests two caps (k and k + 32) against the caps m in one pass,
-  // so a cap m's data is read once for both; survivors keep ascending order.
+  // Each lane tests two caps against the caps m in one pass, so a cap m's data
+  // is read once for both (lanes that share a cap take every second or fourth
+  // m); survivors keep ascending order.
   int n_live = 0;
 #pragma unroll 1
-  for (int k0 = 0; k0 < n_caps; k0 += 64) {
-    const int ka = k0 + lane, kb = k0 + 32 + lane;
+  for (int k0 = 0; k0 < n_caps;) {
+    const int lg = lane_split_log2<W>(n_caps - k0, 32), per = 32 >> lg;
+    const int ka = k0 + (lane & (per - 1)), kb = ka + per;
     bool la = ka < n_caps, lb = kb < n_caps;
     const float4 fa = la ? w.fcap[ka] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
     const float4 fb = lb ? w.fcap[kb] : make_float4(0.0f, 0.0f, 0.0f, -2.0f);
     const float sa2 = 1.0f - fa.w * fa.w, sb2 = 1.0f - fb.w * fb.w;
 #pragma unroll 2
-    for (int m = 0; m < n_caps; ++m) {
+    for (int m = lane >> (5 - lg); m < n_caps; m += 1 << lg) {
       const float4 fm = w.fcap[m];
       const float sm2 = 1.0f - fm.w * fm.w;
       const float ha = fa.x * fm.x + fa.y * fm.y + fa.z * fm.z - fa.w * fm.w - 1e-4f, pa = sa2 * sm2;
@@ -687,13 +706,14 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
       if (fa.w > fm.w && pa > 1e-4f && ha > 0.0f && ha * ha > pa) la = false;
       if (fb.w > fm.w && pb > 1e-4f && hb > 0.0f && hb * hb > pb) lb = false;
     }
-    const unsigned below = (1u << lane) - 1u;
-    const unsigned lva = __ballot_sync(kFull, la);
-    if (la) w.live[n_live + __popc(lva & below)] = static_cast<uint8_t>(ka);
+    const unsigned below = (1u << lane) - 1u, group = per == 32 ? kFull : (1u << per) - 1u;
+    const unsigned lva = split_and(__ballot_sync(kFull, la), lg) & group;
+    if ((lva >> lane) & 1u) w.live[n_live + __popc(lva & below)] = static_cast<uint8_t>(ka);
     n_live += __popc(lva);
-    const unsigned lvb = __ballot_sync(kFull, lb);
-    if (lb) w.live[n_live + __popc(lvb & below)] = static_cast<uint8_t>(kb);
+    const unsigned lvb = split_and(__ballot_sync(kFull, lb), lg) & group;
+    if ((lvb >> lane) & 1u) w.live[n_live + __popc(lvb & below)] = static_cast<uint8_t>(kb);
     n_live += __popc(lvb);
+    k0 += 2 * per;
   }
   __syncwarp();
   ph.mark(1);
@@ -734,20 +754,21 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
     n_circ = 0;
     bool tangent = false;
 #pragma unroll 1
-    for (int l0 = 0; l0 < n_live; l0 += 32) {
-      const int li = l0 + lane;
+    for (int l0 = 0; l0 < n_live;) {
+      const int lg = lane_split_log2<W>(n_live - l0, 16), per = 32 >> lg, part = lane >> (5 - lg);
+      const int li = l0 + (lane & (per - 1));
       const bool own = li < n_live;
       const CoverCircle c = cover_circle(w.fcap[own ? li : 0]);
       CoverMask cover = 0;
       uint64_t mask = 0;
-      int32_t tally = 0;
+      int pairs = 0, singles = 0;  // crossings; tangent pairs
       bool inside = false;  // in a cap without crossing its rim
 #pragma unroll 1
       for (int mb = 0; mb < n_live; mb += 32) {
         const int mn = min(32, n_live - mb);
         unsigned cross = 0, unclear = 0;
 #pragma unroll (W::kBig ? 2 : 1)
-        for (int q = 0; q < mn; ++q) {
+        for (int q = part; q < mn; q += 1 << lg) {
           const float4 b = w.fcap[mb + q];
           const unsigned bit = 1u << q;
           const float sg = c.a.x * b.x + c.a.y * b.y + c.a.z * b.z;
@@ -771,19 +792,25 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
             const PairClass pc = classify(ck, cm);
             if (pc.count == 2) cross |= 1u << q;
             inside |= !pc.count && ck.c * pc.sigma - cm.c > -1e-9;
-            tangent |= pc.count == 1;
-            tally += pc.count == 1;
+            singles += pc.count == 1;
           }
         }
-        tally += 2 * __popc(cross);
+        for (int d = per; d < 32; d <<= 1) cross |= __shfl_xor_sync(kFull, cross, d);
+        pairs += __popc(cross);
         mask |= static_cast<uint64_t>(cross) << (mb & 32);
       }
+      for (int d = per; d < 32; d <<= 1) {
+        cover |= __shfl_xor_sync(kFull, cover, d);
+        inside |= __shfl_xor_sync(kFull, static_cast<int>(inside), d) != 0;
+        singles += __shfl_xor_sync(kFull, singles, d);
+      }
+      tangent |= singles > 0;
       if (masks) {
         if (own) w.xmask[li] = mask | (inside ? kMaskContained : 0ull);
       } else {
-        if (own) w.tcnt[li] = tally | (inside ? kContained : 0);
+        if (own) w.tcnt[li] = (2 * pairs + singles) | (inside ? kContained : 0);
       }
-      const bool open = own && cover != ~CoverMask{0};
+      const bool open = own && lane < per && cover != ~CoverMask{0};
       const unsigned m = __ballot_sync(kFull, open);
       if (open) {
         const int at = n_circ + __popc(m & ((1u << lane) - 1u));
@@ -792,6 +819,7 @@ __device__ int build_boundary(const SasaArgs& a, W& w, int i, int lane, int* n_a
         if (at < W::kCoverKept) w.circ_cover[at] = cover;
       }
       n_circ += __popc(m);
+      l0 += per;
     }
     __syncwarp();
     if (!masks || !__any_sync(kFull, tangent)) break;
@@ -1434,7 +1462,7 @@ __device__ void boundary_task(const SasaArgs& a, W& w, int i, int lane, bool big
 // All kernels of the surface term together, first after buried circles and
 // crossings were dropped in FP32, then with the smaller code and the FP32
 // neighbour search: 2057 -> 1297 -> 998 us for 64 chains of 300 residues,
-// 819 -> 516 -> 413 us for 16 compact folds of 306, 184 -> 61 -> 56 us for
+// 819 -> 516 -> 413 us for 16 compact folds of 306, 184 -> 61 -> 54 us for
 // insulin (in the large-capacity kernel, see below).
 __device__ __forceinline__ int next_task(const SasaArgs& a, int lane) {
   int task = 0;
