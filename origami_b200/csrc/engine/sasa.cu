@@ -461,8 +461,9 @@ __device__ __forceinline__ void keep_or(W& w, int j, int b) {
 // How many lanes (1, 2 or 4, as a power of two) share an item when `left` are
 // left, `full` of which occupy the warp -- in the large-capacity kernel, whose
 // warps run alone on their scheduler, so that the last, partly filled trip's
-// latency counts (insulin: 55.6 -> 53.5 us, a step 77 -> 72).  In the default kernel the shared
-// trips won 6 % for compact folds and lost 3 % for extended chains.
+// latency counts (insulin: 55.6 -> 53.5 us, a step 77 -> 72).  In the default
+// kernel the shared trips won 6 % for compact folds and lost 3 % for extended
+// chains.
 template <class W>
 __device__ __forceinline__ int lane_split_log2(int left, int full) {
   return !W::kBig || left > full ? 0 : left > full / 2 ? 1 : 2;
