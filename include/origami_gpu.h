@@ -397,7 +397,11 @@ og_status og_compute_sasa(og_engine* e, int32_t sys, int32_t method, int32_t n_d
  * fixed-point rounding of partial sums only (well inside the force
  * tolerance), and for a fixed configuration runs are bit-reproducible.
  *   shape       0: one i-tile (32 atoms) per CTA, its four warps splitting
- *               each j-tile; 1: 4 i-tiles per CTA, one per warp; Born pass 2:
+ *               each j-tile, where every pair counts; with a cutoff the sums
+ *               of 8 i-tiles per CTA, one per warp, bit for bit, taken tile
+ *               pair by tile pair in engines of few tiles (so that an untuned
+ *               engine's results with cutoffs do not depend on what else is
+ *               in it); 1: 4 i-tiles per CTA, one per warp; Born pass 2:
  *               8 i-tiles per CTA, one per warp; force pass 2 to 6: four
  *               i-tiles per warp, 16 (2, 3), 8 (4, 5) or 4 (6) per CTA at
  *               3, 4, 6, 7 or 14 CTAs/SM
@@ -405,7 +409,8 @@ og_status og_compute_sasa(og_engine* e, int32_t sys, int32_t method, int32_t n_d
  *               an atomic work queue
  *   chunk       j-tiles per work item at most (default 16; halved while the
  *               list has fewer than eight items per SM, without cutoffs
- *               fewer than 32 in the Born pass and 16 in the force pass)
+ *               fewer than 32 in the Born pass and 16 in the force pass;
+ *               shape 0 with a cutoff takes it as it is)
  * An engine that is neither tuned nor set by hand takes its shapes from its
  * tile count and cutoffs.
  * og_engine_autotune times every combination (3 Born / 7 force shapes x 2 x

@@ -286,6 +286,12 @@ struct og_engine {
   // and the persistent launches' queue heads (Born, force)
   ogk::PairLaunch born_launch, force_launch;
   int chunk_b = 16, chunk_f = 16;
+  // tile pairs of every system (PairArgs::tile_pairs), with a cutoff and while
+  // there are at most kMaxTilePairs; both passes' sums share pair_part
+  DVec<int2> tile_pairs;
+  DVec<int32_t> pair_row;
+  DVec<float> pair_part;
+  DVec<uint8_t> pair_on;
   bool launch_set = false;  // by og_engine_set_pair_launch or og_engine_autotune; else default_launch
   DVec<int32_t> pair_queue;
   // device-side replica exchange (og_remd_run): temperature slots, counters
@@ -453,6 +459,15 @@ struct og_engine {
     a.queue = pair_queue.p;
     a.atom_sys = atom_sys.p;
     a.sys_nonfinite = sys_nonfinite.p;
+    if (tile_pairs.n > 0) {
+      a.tile_pairs = tile_pairs.p;
+      a.n_tile_pairs = static_cast<int32_t>(tile_pairs.n);
+      a.pair_row = pair_row.p;
+      a.pair_on = pair_on.p;
+      a.pair_i = pair_part.p;
+      a.pair_j = pair_part.p + 3 * kTile * tile_pairs.n;
+    }
+    a.n_sm = n_sm;
     a.x64 = x.p; a.y64 = y.p; a.z64 = z.p; a.q64 = q.p;
     a.rmin64 = rmin.p; a.eps64 = eps.p; a.rmin14_64 = rmin14.p; a.eps14_64 = eps14.p;
     a.born_r64 = born_r.p;
@@ -662,6 +677,9 @@ struct og_engine {
                                 stream);
           pb.jlist = jlist_cut_b.p;
           pb.seg_end = seg_end_b.p;
+          pb.blocks = cut_b.p;
+          pb.n_blocks = n_cut_b;
+          pb.chunk = chunk_b;
         }
         ogk::launch_born_pass(pb, born_launch, stream);
       }
@@ -697,6 +715,9 @@ struct og_engine {
         else cut_lists(stream);
         pf.jlist = jlist_cut_f.p;
         pf.seg_end = seg_end_f.p;
+        pf.blocks = cut_f.p;
+        pf.n_blocks = n_cut_f;
+        pf.chunk = chunk_f;
       }
       ogk::launch_force_pass(pf, force_launch, stream);
     }
@@ -940,31 +961,44 @@ int64_t count_items(const og_engine* e, int first_offset, int W, int chunk) {
   return n;
 }
 
-// Pair work (Newton-3 layout): i-blocks of W consecutive tiles (W from the
-// pass's launch shape) against the tiles from the block's first tile on
-// (Born pass: the block's own diagonal included) or after it (far-field
-// force pass), cut into chunks of at most `chunk` j-tiles and ordered
-// longest first; plus the i-blocks of cutoff mode's culled lists.  A list
-// too short to fill the GPU (eight items per SM) is cut finer: with few
-// tiles the longest item is the pass's time.  All-pairs passes are cut on
+// Whether a pass walks lists culled by its cutoff.
+bool culled_pass(const og_engine* e, bool born) {
+  return born ? !no_cutoff(e->p.born_cutoff) : !no_cutoff(e->p.nb_cutoff) && !no_cutoff(e->p.gb_force_cutoff);
+}
+
+// The chunk of a list too short to fill the GPU (eight items per SM), cut finer:
+// with few tiles the longest item is the pass's time.  All-pairs passes are cut on
 // until the items make a few waves of resident blocks, so that the last one
 // weighs little: 32 items per SM for Born (15 600 atoms: 148 us with chunks of
 // 16, 139 of 8, 129 of 4; 4 x 4 668 atoms: 103, 103, 89, and 83 of 2), 16 for
 // the force pass (179, 179, 166; 12 x 4 694 atoms: 221, 192, 185), whose items
 // cost more to start, so that chunks of 1 lose again (12 x 4 694: 214).  With
 // cutoffs the culled lists are shorter than they count here, and finer items
-// lost (15 600 atoms, Born: 38 us of 16, 43 of 8).
-og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec<ogk::PairWork>* work,
-                          int* n_work, DVec<int32_t>* jlist, DVec<ogk::CutBlock>* cut, int* n_cut,
-                          DVec<int32_t>* jlist_cut, DVec<int32_t>* seg_end, cudaStream_t st) {
-  const bool born = first_offset == 0;
+// lost (15 600 atoms, Born: 38 us of 16, 43 of 8); shape 0's are never cut: its
+// results are those of the chunk it is given, whatever else is in the engine.
+int refine_chunk(const og_engine* e, bool born, int shape, int chunk) {
+  const bool culled = culled_pass(e, born);
+  if (culled && shape == 0) return chunk;
+  const int W = ogk::pair_shape_tiles(born, shape, culled);
   const bool all_pairs = born ? no_cutoff(e->p.born_cutoff) : no_cutoff(e->p.nb_cutoff) || no_cutoff(e->p.gb_force_cutoff);
   const int64_t waves = all_pairs ? (born ? 32 : 16) : 8;
   while (chunk > 1) {
-    const int64_t items = count_items(e, first_offset, W, chunk);
+    const int64_t items = count_items(e, born ? 0 : 1, W, chunk);
     if (items >= waves * e->n_sm || (items >= 8ll * e->n_sm && !born && chunk <= 3)) break;
     chunk /= 2;
   }
+  return chunk;
+}
+
+// Pair work (Newton-3 layout): i-blocks of W consecutive tiles (W from the
+// pass's launch shape) against the tiles from the block's first tile on
+// (Born pass: the block's own diagonal included) or after it (far-field
+// force pass), cut into chunks of at most `chunk` j-tiles and ordered
+// longest first; plus the i-blocks of cutoff mode's culled lists.
+og_status build_pass_list(og_engine* e, bool born, int shape, int chunk, DVec<ogk::PairWork>* work, int* n_work,
+                          DVec<int32_t>* jlist, DVec<ogk::CutBlock>* cut, int* n_cut, DVec<int32_t>* jlist_cut,
+                          DVec<int32_t>* seg_end, cudaStream_t st) {
+  const int first_offset = born ? 0 : 1, W = ogk::pair_shape_tiles(born, shape, culled_pass(e, born));
   std::vector<int32_t> hj;
   std::vector<ogk::PairWork> hw;
   std::vector<ogk::CutBlock> hc;
@@ -973,7 +1007,7 @@ og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec
       const int jb = static_cast<int>(hj.size());
       for (int t = t0 + first_offset; t < s.n_tiles; ++t) hj.push_back(s.tile_begin + t);
       const int je = static_cast<int>(hj.size());
-      hc.push_back(ogk::CutBlock{s.tile_begin + t0, std::min(W, s.n_tiles - t0), jb, je});
+      hc.push_back(ogk::CutBlock{s.tile_begin + t0, std::min(W, s.n_tiles - t0), jb, je, s.tile_begin});
       for (int j0 = jb; j0 < je; j0 += chunk)
         hw.push_back(ogk::PairWork{s.tile_begin + t0, std::min(W, s.n_tiles - t0), j0, std::min(je, j0 + chunk)});
     }
@@ -992,9 +1026,9 @@ og_status build_pass_list(og_engine* e, int first_offset, int W, int chunk, DVec
 }
 
 // The launch variants of an engine nobody tuned, by its tile pairs (times in us
-// on B200; shapes in pair_kernels.cuh).  With cutoffs most tile pairs are
-// skipped and shape 0 wins throughout (32 x 4 668 atoms: Born 290 against 307
-// for shape 1, force 226 against 240).  Without, Born: shape 0 below 4 000
+// on B200; shapes in pair_kernels.cuh).  With cutoffs shape 0, whose sums have
+// one order whatever else is in the engine (pair_kernels.cu, k_born_pair).
+// Without, Born: shape 0 below 4 000
 // tile pairs (1 770: 15.0 against 16.4; 64 systems of 20 tiles, 13 440: 44.7
 // against 43.3; one system of 147 tiles, 10 878: 35 against 27), else shape 1.
 // Force: shape 0 below 800 tile pairs (20 residues: 10.6 against 12.8; 80
@@ -1011,13 +1045,36 @@ void default_launch(og_engine* e) {
     e->force_launch.shape = pairs < 800 ? 0 : pairs < 40000 ? 1 : 4;
 }
 
+// The tile pairs of every system, i <= j, in rows of i (PairArgs::tile_pairs).
+og_status build_tile_pairs(og_engine* e, cudaStream_t st) {
+  int64_t n = 0;
+  for (const auto& s : e->sys) n += static_cast<int64_t>(s.n_tiles) * (s.n_tiles + 1) / 2;
+  e->tile_pairs.n = 0;
+  if (n > ogk::kMaxTilePairs || !(culled_pass(e, true) || culled_pass(e, false))) return OG_OK;
+  std::vector<int2> pairs;
+  std::vector<int32_t> row;
+  for (const auto& s : e->sys)
+    for (int i = s.tile_begin; i < s.tile_begin + s.n_tiles; ++i) {
+      row.push_back(static_cast<int32_t>(pairs.size()));
+      for (int j = i; j < s.tile_begin + s.n_tiles; ++j) pairs.push_back(make_int2(i, j));
+    }
+  OG_CUDA(e->tile_pairs.upload(pairs, st));
+  OG_CUDA(e->pair_row.upload(row, st));
+  OG_CUDA(e->pair_part.alloc(6 * kTile * pairs.size()));
+  OG_CUDA(e->pair_on.alloc(pairs.size()));
+  return OG_OK;
+}
+
 og_status build_pair_lists(og_engine* e, cudaStream_t st) {
   if (!e->launch_set) default_launch(e);
-  og_status s = build_pass_list(e, 0, ogk::pair_shape_tiles(true, e->born_launch.shape), e->chunk_b, &e->work, &e->n_work,
-                                &e->jlist, &e->cut_b, &e->n_cut_b, &e->jlist_cut_b, &e->seg_end_b, st);
+  const int cb = refine_chunk(e, true, e->born_launch.shape, e->chunk_b);
+  const int cf = refine_chunk(e, false, e->force_launch.shape, e->chunk_f);
+  og_status s = build_pass_list(e, true, e->born_launch.shape, cb, &e->work, &e->n_work, &e->jlist, &e->cut_b,
+                                &e->n_cut_b, &e->jlist_cut_b, &e->seg_end_b, st);
   if (s != OG_OK) return s;
-  return build_pass_list(e, 1, ogk::pair_shape_tiles(false, e->force_launch.shape), e->chunk_f, &e->work_f, &e->n_work_f,
-                         &e->jlist_f, &e->cut_f, &e->n_cut_f, &e->jlist_cut_f, &e->seg_end_f, st);
+  s = build_pass_list(e, false, e->force_launch.shape, cf, &e->work_f, &e->n_work_f, &e->jlist_f, &e->cut_f,
+                      &e->n_cut_f, &e->jlist_cut_f, &e->seg_end_f, st);
+  return s != OG_OK ? s : build_tile_pairs(e, st);
 }
 
 template <class T>
@@ -2877,7 +2934,7 @@ og_status time_pass(og_engine* e, bool born, const ogk::PairLaunch& lc, int chun
   DVec<int32_t> jl, jl_cut, seg;
   DVec<ogk::CutBlock> cut;
   int n_work = 0, n_cut = 0;
-  og_status s = build_pass_list(e, born ? 0 : 1, ogk::pair_shape_tiles(born, lc.shape), chunk, &work, &n_work, &jl, &cut,
+  og_status s = build_pass_list(e, born, lc.shape, refine_chunk(e, born, lc.shape, chunk), &work, &n_work, &jl, &cut,
                                 &n_cut, &jl_cut, &seg, st);
   if (s != OG_OK) return s;
   ogk::PairArgs a = e->pair_args();
@@ -2886,10 +2943,13 @@ og_status time_pass(og_engine* e, bool born, const ogk::PairLaunch& lc, int chun
   a.jlist = jl.p;
   a.queue = e->pair_queue.p + (born ? 0 : 1);
   const double cutoff = born ? e->p.born_cutoff : std::max(e->p.nb_cutoff, e->p.gb_force_cutoff);
-  const bool culled = born ? !no_cutoff(e->p.born_cutoff) : (!no_cutoff(e->p.nb_cutoff) && !no_cutoff(e->p.gb_force_cutoff));
+  const bool culled = culled_pass(e, born);
   if (culled) {
     a.jlist = jl_cut.p;
     a.seg_end = seg.p;
+    a.blocks = cut.p;
+    a.n_blocks = n_cut;
+    a.chunk = chunk;
   }
   cudaEvent_t t0, t1;
   OG_CUDA(cudaEventCreate(&t0));
@@ -2984,6 +3044,9 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
                             e->seg_end_b.p, e->stream);
       pb.jlist = e->jlist_cut_b.p;
       pb.seg_end = e->seg_end_b.p;
+      pb.blocks = e->cut_b.p;
+      pb.n_blocks = e->n_cut_b;
+      pb.chunk = e->chunk_b;
     }
     ogk::launch_born_pass(pb, e->born_launch, e->stream);
     ogk::launch_born_finalize(e->atoms(), nullptr, 0, e->born_r.p, true, nullptr, e->stream);

@@ -23,10 +23,16 @@ namespace ogk {
 // only).  The pair coefficient is symmetric in i and j, so the j-side force
 // is exactly the negated i-side term.
 //
-// kSplit = 4 gives a tile pair to the four warps of a block, each taking
-// every fourth step, their sums added in warp order: a warp's 32 steps are a
-// chain of FP64 latency (about 20 us), which is the kernel's time when there
-// are too few tile pairs to fill the SMs.
+// kBlock and kBlockInOrder give a tile pair to the four warps of a block, each
+// taking every fourth step: a warp's 32 steps are a chain of FP64 latency (about
+// 20 us), which is the kernel's time when there are too few tile pairs to fill
+// the SMs.  kBlock adds the warps' sums in warp order.  kBlockInOrder, for
+// engines with cutoffs, whose results do not depend on what else is in the
+// engine (pair_kernels.cu, k_born_pair), keeps the steps' coefficients in shared
+// memory, and two warps add the i and the j side step by step: the sums of
+// kWarp, bit for bit (20 residues 12.7 us, by events around the launch, against
+// 12.5 of kBlock and 22.3 of kWarp).
+enum NearShape { kWarp, kBlock, kBlockInOrder };
 namespace {
 
 constexpr int kNearWarps = 4;
@@ -47,17 +53,19 @@ struct NearForce {
   double x[kTile], y[kTile], z[kTile];
 };
 
-template <int kSplit>
+template <NearShape kShape>
 __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const int4* __restrict__ near, int n_near) {
-  static_assert(kSplit == 1 || kSplit == kNearWarps, "a warp or a block per tile pair");
-  __shared__ NearTile tiles[kNearWarps / kSplit];
-  __shared__ NearForce jf[kNearWarps], sf[kSplit > 1 ? kNearWarps : 1];
+  constexpr bool kSplit = kShape != kWarp, kInOrder = kShape == kBlockInOrder;
+  __shared__ NearTile tiles[kSplit ? 1 : kNearWarps];
+  __shared__ NearForce jf[kInOrder ? 1 : kNearWarps];      // j sums; in order: the i atoms' positions
+  __shared__ NearForce sf[kShape == kBlock ? kNearWarps : 1];
+  __shared__ double s_coeff[kInOrder ? kTile : 1][kTile];  // in order: [step][lane]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wid = kSplit > 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kNearWarps + warp;
+  const int wid = kSplit ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kNearWarps + warp;
   if (wid >= n_near) return;  // block-uniform when split
-  const int part = kSplit > 1 ? warp : 0;
-  NearTile& t = tiles[kSplit > 1 ? 0 : warp];
-  NearForce& f = jf[warp];
+  const int part = kSplit ? warp : 0;
+  NearTile& t = tiles[kSplit ? 0 : warp];
+  NearForce& f = jf[kInOrder ? 0 : warp];
   const int4 w = near[wid];  // i_tile, j_tile (>= i_tile), mask block of (i_tile, j_tile)
   const int i = w.x * kTile + lane;
   const int jl = w.y * kTile + lane;  // this lane's j atom, staged for the warp
@@ -74,7 +82,7 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
     t.seps14[lane] = sqrt(a.eps14_64[jl]);
     t.valid[lane] = a.atom_valid[jl];
   }
-  f.x[lane] = f.y[lane] = f.z[lane] = 0.0;
+  if (!kInOrder) f.x[lane] = f.y[lane] = f.z[lane] = 0.0;
   const uint32_t ex = a.mask_ex[w.z * kTile + lane];
   const uint32_t m14 = a.mask_14[w.z * kTile + lane];
   const bool valid_i = a.atom_valid[i] != 0;
@@ -85,9 +93,14 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
   const double gb_pref = (1.0 - 1.0 / kEpsWater) * kCoulomb * kKcalToKj;
   const bool diag = w.x == w.y;
   double ax = 0.0, ay = 0.0, az = 0.0;
-  if (kSplit > 1) __syncthreads();
+  if (kInOrder && part == 0) {
+    f.x[lane] = xi;
+    f.y[lane] = yi;
+    f.z[lane] = zi;
+  }
+  if (kSplit) __syncthreads();
   else __syncwarp();
-  for (int k = (diag ? 1 : 0) + part; k < (diag ? 17 : kTile); k += kSplit) {
+  for (int k = (diag ? 1 : 0) + part; k < (diag ? 17 : kTile); k += kSplit ? kNearWarps : 1) {
     const int p = (lane + k) & (kTile - 1);
     double coeff = 0.0, dx = 0.0, dy = 0.0, dz = 0.0;
     if (valid_i && t.valid[p] && !(diag && k == 16 && lane >= 16)) {
@@ -119,29 +132,58 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
         }
       }
     }
-    ax += dx * coeff;
-    ay += dy * coeff;
-    az += dz * coeff;
-    f.x[p] -= dx * coeff;
-    f.y[p] -= dy * coeff;
-    f.z[p] -= dz * coeff;
-    __syncwarp();
+    if (kInOrder) {
+      s_coeff[k][lane] = coeff;
+    } else {
+      ax += dx * coeff;
+      ay += dy * coeff;
+      az += dz * coeff;
+      f.x[p] -= dx * coeff;
+      f.y[p] -= dy * coeff;
+      f.z[p] -= dz * coeff;
+      __syncwarp();
+    }
   }
-  if (kSplit > 1) {
-    NearForce& fi = sf[warp];
-    fi.x[lane] = ax;
-    fi.y[lane] = ay;
-    fi.z[lane] = az;
+  if (kSplit) {
+    if (kShape == kBlock) {
+      sf[warp].x[lane] = ax;
+      sf[warp].y[lane] = ay;
+      sf[warp].z[lane] = az;
+    }
     __syncthreads();
     if (warp >= 2) return;
-    // warp 0: the i side, warp 1: the j side, over the warps in order
-    const NearForce* side = warp == 0 ? sf : jf;
-    ax = ay = az = 0.0;
+    // warp 0: the i side, warp 1: the j side
+    if (kShape == kBlock) {
+      const NearForce* side = warp == 0 ? sf : jf;
+      ax = ay = az = 0.0;
 #pragma unroll
-    for (int w = 0; w < kNearWarps; ++w) {
-      ax += side[w].x[lane];
-      ay += side[w].y[lane];
-      az += side[w].z[lane];
+      for (int w = 0; w < kNearWarps; ++w) {
+        ax += side[w].x[lane];
+        ay += side[w].y[lane];
+        az += side[w].z[lane];
+      }
+    } else if (warp == 0) {
+      // atom `lane` with partner (lane + k) mod 32 at step k; a pair that is not
+      // counted has the coefficient 0
+#pragma unroll 8
+      for (int k = diag ? 1 : 0; k < (diag ? 17 : kTile); ++k) {
+        const int p = (lane + k) & (kTile - 1);
+        const double c = s_coeff[k][lane];
+        ax += (t.x[p] - xi) * c;
+        ay += (t.y[p] - yi) * c;
+        az += (t.z[p] - zi) * c;
+      }
+    } else {
+      // atom `lane` with the i atom (lane - k) mod 32
+      const double xj = t.x[lane], yj = t.y[lane], zj = t.z[lane];
+#pragma unroll 8
+      for (int k = diag ? 1 : 0; k < (diag ? 17 : kTile); ++k) {
+        const int l = (lane - k) & (kTile - 1);
+        const double c = s_coeff[k][l];
+        ax -= (xj - f.x[l]) * c;
+        ay -= (yj - f.y[l]) * c;
+        az -= (zj - f.z[l]) * c;
+      }
     }
     const int at = warp == 0 ? i : jl;
     if (warp == 0 ? valid_i : t.valid[lane] != 0) {
@@ -171,8 +213,13 @@ __global__ void __launch_bounds__(kNearWarps * 32) k_near64(PairArgs a, const in
 
 void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_sm, cudaStream_t s) {
   if (n_near <= 0) return;
-  if (n_near <= kNearSplitPerSm * n_sm) k_near64<kNearWarps><<<n_near, kNearWarps * 32, 0, s>>>(a, near, n_near);
-  else k_near64<1><<<(n_near + kNearWarps - 1) / kNearWarps, kNearWarps * 32, 0, s>>>(a, near, n_near);
+  const int block = kNearWarps * 32;
+  if (n_near > kNearSplitPerSm * n_sm)
+    k_near64<kWarp><<<(n_near + kNearWarps - 1) / kNearWarps, block, 0, s>>>(a, near, n_near);
+  else if (a.nb_c2_64 != INFINITY || a.gb_c2_64 != INFINITY)
+    k_near64<kBlockInOrder><<<n_near, block, 0, s>>>(a, near, n_near);
+  else
+    k_near64<kBlock><<<n_near, block, 0, s>>>(a, near, n_near);
 }
 
 // ----------------------------------------------------------------- FP64 path

@@ -31,7 +31,8 @@
 // they free up) or a persistent grid of resident CTAs that take items from an
 // atomic queue.  The engine picks by tile counts (default_launch) or its
 // autotuner times them on the actual systems; every variant computes the same
-// pair terms.
+// pair terms.  With cutoffs shape 0 keeps one order of every sum, by two sets
+// of kernels (k_born_pair).
 //
 // Tile pairs are classed by the gap between their bounding spheres: distant
 // ones take shorter forms of the same sums (fewer series terms, the far GB
@@ -255,6 +256,9 @@ __device__ __forceinline__ float2 born_pair(float dx, float dy, float dz, float 
 // u = 1 / r^2 enters: h_ij = -s_j^3 u^2 P(s_j^2 u)) and no overlap test.
 constexpr float kSeries5MaxX = 0.1135f, kSeries3MaxX = 0.0290f;
 
+// Not with a cutoff: there every pair takes the form that its own distance gives
+// it, whichever kernel meets it (see k_born_pair).
+
 // The gaps from which the series holds with 8, 5 and 3 terms.
 struct BornGaps {
   float g8, g5, g3;
@@ -273,15 +277,11 @@ __device__ __forceinline__ float2 descreen_poly2(float2 w) {
 
 // Two pairs in the halves: adds -h_ij to *hi and returns -h_ji; (s2, s3) =
 // (s^2, s^3) of the two sides.
-template <int kTerms, bool kCut>
+template <int kTerms>
 __device__ __forceinline__ float2 born_far2(float2 dx, float2 dy, float2 dz, float2 si2, float2 si3, float2 sj2,
-                                            float2 sj3, float c2, float2* hi) {
+                                            float2 sj3, float2* hi) {
   const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-  float2 u = make_float2(rcp_approx(r2.x), rcp_approx(r2.y));
-  if (kCut) {
-    u.x = r2.x <= c2 ? u.x : 0.0f;
-    u.y = r2.y <= c2 ? u.y : 0.0f;
-  }
+  const float2 u = make_float2(rcp_approx(r2.x), rcp_approx(r2.y));
   const float2 u2 = mul2(u, u);
   *hi = fma2(mul2(u2, descreen_poly2<kTerms>(mul2(sj2, u))), sj3, *hi);
   return mul2(mul2(u2, descreen_poly2<kTerms>(mul2(si2, u))), si3);
@@ -334,9 +334,9 @@ __device__ __forceinline__ float born_far_one3(const float* sp, const float* sb,
 // atoms per packed operation; the columns at sp (x, y, z) and sg (rho~, s~
 // from +64).  Returns the i side; j(k, v) receives the lane's four values for
 // the j atoms from k on, negated.
-template <int kTerms, bool kCut, class J>
+template <int kTerms, class J>
 __device__ __forceinline__ float born_far_one(const float* sp, const float* sg, int k_begin, int k_end, float xi,
-                                              float yi, float zi, float s_i, float c2, J j) {
+                                              float yi, float zi, float s_i, J j) {
   const float2 nx = bc(-xi), ny = bc(-yi), nz = bc(-zi), si2 = bc(s_i * s_i), si3 = bc(s_i * s_i * s_i);
   float2 hi = bc(0.0f);
 #pragma unroll 2
@@ -347,10 +347,10 @@ __device__ __forceinline__ float born_far_one(const float* sp, const float* sg, 
     const float4 S = *reinterpret_cast<const float4*>(&sg[96 + k0]);
     const float2 sa = make_float2(S.x, S.y), sb = make_float2(S.z, S.w);
     const float2 sa2 = mul2(sa, sa), sb2 = mul2(sb, sb);
-    const float2 a = born_far2<kTerms, kCut>(add2(make_float2(X.x, X.y), nx), add2(make_float2(Y.x, Y.y), ny),
-                                             add2(make_float2(Z.x, Z.y), nz), si2, si3, sa2, mul2(sa2, sa), c2, &hi);
-    const float2 b = born_far2<kTerms, kCut>(add2(make_float2(X.z, X.w), nx), add2(make_float2(Y.z, Y.w), ny),
-                                             add2(make_float2(Z.z, Z.w), nz), si2, si3, sb2, mul2(sb2, sb), c2, &hi);
+    const float2 a = born_far2<kTerms>(add2(make_float2(X.x, X.y), nx), add2(make_float2(Y.x, Y.y), ny),
+                                       add2(make_float2(Z.x, Z.y), nz), si2, si3, sa2, mul2(sa2, sa), &hi);
+    const float2 b = born_far2<kTerms>(add2(make_float2(X.z, X.w), nx), add2(make_float2(Y.z, Y.w), ny),
+                                       add2(make_float2(Z.z, Z.w), nz), si2, si3, sb2, mul2(sb2, sb), &hi);
     j(k0, a.x, a.y, b.x, b.y);
   }
   return -(hi.x + hi.y);
@@ -359,16 +359,11 @@ __device__ __forceinline__ float born_far_one(const float* sp, const float* sg, 
 template <class J>
 __device__ __forceinline__ bool born_far_tile(const BornGaps& gaps, float gap, const float* sp, const float* sg,
                                               const float* sb, int k_begin, int k_end, float xi, float yi, float zi,
-                                              float s_i, float3 ci, float c2, float* hi, J j) {
-  if (gap < gaps.g8) return false;
-  if (c2 != INFINITY) {
-    *hi = gap >= gaps.g5 ? born_far_one<5, true>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j)
-                         : born_far_one<8, true>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j);
-  } else {
-    *hi = gap >= gaps.g3   ? born_far_one3(sp, sb, k_begin, k_end, xi, yi, zi, ci, j)
-          : gap >= gaps.g5 ? born_far_one<5, false>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j)
-                           : born_far_one<8, false>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, c2, j);
-  }
+                                              float s_i, float3 ci, float* hi, J j) {
+  if (!(gap >= gaps.g8)) return false;
+  *hi = gap >= gaps.g3   ? born_far_one3(sp, sb, k_begin, k_end, xi, yi, zi, ci, j)
+        : gap >= gaps.g5 ? born_far_one<5>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, j)
+                         : born_far_one<8>(sp, sg, k_begin, k_end, xi, yi, zi, s_i, j);
   return true;
 }
 
@@ -459,9 +454,9 @@ __global__ void __launch_bounds__(W * 32, kMinBlocks) k_born(PairArgs a) {
       const float* sp = &s_buf[b][0][t * 128];
       const float* sg = &s_buf[b][1][t * 128];
       float hi = 0.0f;
-      const bool series = born_far_tile(gaps, off.w, sp, sg, &s_buf[b][2][t * 128], 0, kTile, xi, yi, zi, s_i,
-                                        ci, c2, &hi,
-                                        [&](int k0, float v0, float v1, float v2, float v3) {
+      const bool series = c2 == INFINITY &&
+                          born_far_tile(gaps, off.w, sp, sg, &s_buf[b][2][t * 128], 0, kTile, xi, yi, zi, s_i, ci,
+                                        &hi, [&](int k0, float v0, float v1, float v2, float v3) {
                                           const float tot = reduce_scatter4(v0, v1, v2, v3, lane);
                                           if ((lane & 7) == 0) part[k0 + (lane >> 3)] = -tot;
                                         });
@@ -508,8 +503,7 @@ OG_UNROLL(OG_BORN_UNROLL)
 // One i-tile per CTA, its four warps taking eight atoms of each j-tile: the
 // shape for engines of few tiles, where whole-tile work items leave most of
 // the chip idle and a tile pair's latency (about 1 500 cycles per group of
-// four j atoms in the closed form) is the pass's time; and with cutoffs, where
-// its list is culled per i-tile.  (Warps taking whole tile pairs of their own,
+// four j atoms in the closed form) is the pass's time.  (Warps taking whole tile pairs of their own,
 // without the shared sums, were 0 to 50 % slower than the better of this and
 // k_born at every size tried.)
 constexpr int kSplitWarps = 4, kSplitJ = kTile / kSplitWarps;
@@ -527,13 +521,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_born_split(PairArgs a) {
   __shared__ double s_acc[kSplitWarps][kTile];
   __shared__ int s_item;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float c2 = a.born_c2;
   const BornGaps gaps = born_gaps(a);
   for (int item = next_item<kPersistent>(a, &s_item, -1); item < a.n_work;
        item = next_item<kPersistent>(a, &s_item, item)) {
-    PairWork w = a.work[item];
-    if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
-    if (w.j_begin >= w.j_end) continue;  // block-uniform
+    const PairWork w = a.work[item];
     const int it = w.i_tile0, i = it * kTile + lane;
     const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
     const float rho_i = a.gb[soa_index(i, 2)], s_i = a.gb[soa_index(i, 3)];
@@ -561,7 +552,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_born_split(PairArgs a) {
       };
       const int k_begin = warp * kSplitJ, k_end = k_begin + kSplitJ;
       auto sub_j = [&](int k0, float v0, float v1, float v2, float v3) { add_j(k0, -v0, -v1, -v2, -v3); };
-      if (!born_far_tile(gaps, tile_gap(oi, oj), sp, sg, sb, k_begin, k_end, xi, yi, zi, s_i, ci, c2, &hi, sub_j)) {
+      if (!born_far_tile(gaps, tile_gap(oi, oj), sp, sg, sb, k_begin, k_end, xi, yi, zi, s_i, ci, &hi, sub_j)) {
 #pragma unroll 1
         for (int k0 = k_begin; k0 < k_end; k0 += 4) {
           const float4 X = *reinterpret_cast<const float4*>(sp + k0);
@@ -569,10 +560,10 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_born_split(PairArgs a) {
           const float4 Z = *reinterpret_cast<const float4*>(sp + 64 + k0);
           const float4 RH = *reinterpret_cast<const float4*>(sg + 64 + k0);
           const float4 SR = *reinterpret_cast<const float4*>(sg + 96 + k0);
-          const float2 h0 = born_pair(X.x - xi, Y.x - yi, Z.x - zi, rho_i, s_i, RH.x, SR.x, c2);
-          const float2 h1 = born_pair(X.y - xi, Y.y - yi, Z.y - zi, rho_i, s_i, RH.y, SR.y, c2);
-          const float2 h2 = born_pair(X.z - xi, Y.z - yi, Z.z - zi, rho_i, s_i, RH.z, SR.z, c2);
-          const float2 h3 = born_pair(X.w - xi, Y.w - yi, Z.w - zi, rho_i, s_i, RH.w, SR.w, c2);
+          const float2 h0 = born_pair(X.x - xi, Y.x - yi, Z.x - zi, rho_i, s_i, RH.x, SR.x, INFINITY);
+          const float2 h1 = born_pair(X.y - xi, Y.y - yi, Z.y - zi, rho_i, s_i, RH.y, SR.y, INFINITY);
+          const float2 h2 = born_pair(X.z - xi, Y.z - yi, Z.z - zi, rho_i, s_i, RH.z, SR.z, INFINITY);
+          const float2 h3 = born_pair(X.w - xi, Y.w - yi, Z.w - zi, rho_i, s_i, RH.w, SR.w, INFINITY);
           hi += (h0.x + h1.x) + (h2.x + h3.x);
           if (!diag) add_j(k0, h0.y, h1.y, h2.y, h3.y);  // a diagonal tile's pairs are all seen from the i side
         }
@@ -587,6 +578,178 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_born_split(PairArgs a) {
       add_fixed(a.born_sum + i, v, kBornScale);
     }
     if (kPersistent) __syncthreads();  // s_acc is read before the next item writes it
+  }
+}
+
+// ------------------------------------------- tile pairs, summed in k_born's order
+// The eight-tile kernels' sums for engines of few tiles with culled lists: a
+// CTA per tile pair (its four warps taking eight j atoms each) keeps the pair's
+// sums, and k_collect adds them in the order in which k_born<8> / k_force<8>
+// do -- an i atom's eight groups of a tile in FP32, a chunk's tiles in FP64, a
+// j atom's sums over a block's eight tiles in FP32 -- so that the results are
+// those kernels' bit for bit, whatever else is in the engine.  (A sum in
+// another order is as good by itself, but a trajectory at its limit of
+// stability shows the last bit: of 400 starts of unrelaxed insulin at 2 fs, 26
+// had parted by more than 2e-5 of the velocities after 50 steps.)
+// Bound by latency while the tile pairs fit the chip at once: insulin (25 tiles)
+// 21 us for each pass with its list and k_collect, against 98 and 63 for
+// k_born<8> and k_force<8>, and 15 and 14 for sums in no set order, added
+// straight to the accumulators.  The line is kMaxTilePairs: 16 folds of 4.7k
+// atoms (174k tile pairs) 235 and 179 us against 266 and 191; 32 extended
+// chains of 4.7k (348k) 195 and 133 against 113 and 77, since a culled tile pair
+// costs a lane here and nothing there.
+
+__device__ __forceinline__ size_t pair_at(size_t slot, int comps, int c, int lane) {
+  return (slot * comps + c) * kTile + lane;
+}
+
+// A CTA's tile pairs are blockIdx.x, + gridDim.x, ..: up to kPairsPerCta, so that
+// the culled ones (nearly all, in a long chain) cost a lane each and the others
+// spread over the CTAs.  Thread q tests pair q; returns the ones to evaluate.
+constexpr int kPairsPerCta = 32;
+template <class Skip>
+__device__ __forceinline__ unsigned live_pairs(const PairArgs& a, unsigned* s_live, Skip skip) {
+  if (threadIdx.x < kPairsPerCta) {
+    const size_t slot = blockIdx.x + static_cast<size_t>(threadIdx.x) * gridDim.x;
+    bool on = slot < static_cast<size_t>(a.n_tile_pairs);
+    if (on) {
+      const int2 ij = a.tile_pairs[slot];
+      on = !skip(ij.x, ij.y);
+      a.pair_on[slot] = on ? 1 : 0;
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, on);
+    if (threadIdx.x == 0) *s_live = live;
+  }
+  __syncthreads();
+  return *s_live;
+}
+
+__global__ void __launch_bounds__(kSplitWarps * 32) k_born_pair(PairArgs a) {
+  __shared__ float s_h[kTile][kTile];  // the i side's terms, in the order they are added
+  __shared__ unsigned s_live;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float c2 = a.born_c2;
+  unsigned live = live_pairs(a, &s_live, [&](int it, int jt) { return tile_gap(a.origin[it], a.origin[jt]) > a.born_cutoff; });
+  for (; live; live &= live - 1) {
+    const size_t slot = blockIdx.x + static_cast<size_t>(__ffs(live) - 1) * gridDim.x;
+    const int2 ij = a.tile_pairs[slot];
+    const int it = ij.x, jt = ij.y, i = it * kTile + lane;
+    const double4 oi = a.origin[it], oj = a.origin[jt];
+    const bool diag = jt == it;
+    const float rho_i = a.gb[soa_index(i, 2)], s_i = a.gb[soa_index(i, 3)];
+    const float xi = a.pq[soa_index(i, 0)] - static_cast<float>(oj.x - oi.x);
+    const float yi = a.pq[soa_index(i, 1)] - static_cast<float>(oj.y - oi.y);
+    const float zi = a.pq[soa_index(i, 2)] - static_cast<float>(oj.z - oi.z);
+    const float* sp = a.pq + static_cast<size_t>(jt) * 128;
+    const float* sg = a.gb + static_cast<size_t>(jt) * 128;
+    const int k_begin = warp * kSplitJ;
+    if (diag) {  // every ordered pair from the i side
+#pragma unroll 4
+      for (int k = k_begin; k < k_begin + kSplitJ; ++k)
+        s_h[k][lane] = born_pair(sp[k] - xi, sp[32 + k] - yi, sp[64 + k] - zi, rho_i, s_i, sg[64 + k], sg[96 + k], c2).x;
+    } else {
+#pragma unroll 1
+      for (int k0 = k_begin; k0 < k_begin + kSplitJ; k0 += 4) {
+        const float4 X = *reinterpret_cast<const float4*>(sp + k0);
+        const float4 Y = *reinterpret_cast<const float4*>(sp + 32 + k0);
+        const float4 Z = *reinterpret_cast<const float4*>(sp + 64 + k0);
+        const float4 RH = *reinterpret_cast<const float4*>(sg + 64 + k0);
+        const float4 SR = *reinterpret_cast<const float4*>(sg + 96 + k0);
+        const float2 h0 = born_pair(X.x - xi, Y.x - yi, Z.x - zi, rho_i, s_i, RH.x, SR.x, c2);
+        const float2 h1 = born_pair(X.y - xi, Y.y - yi, Z.y - zi, rho_i, s_i, RH.y, SR.y, c2);
+        const float2 h2 = born_pair(X.z - xi, Y.z - yi, Z.z - zi, rho_i, s_i, RH.z, SR.z, c2);
+        const float2 h3 = born_pair(X.w - xi, Y.w - yi, Z.w - zi, rho_i, s_i, RH.w, SR.w, c2);
+        s_h[k0 / 4][lane] = (h0.x + h1.x) + (h2.x + h3.x);
+        const float tot = reduce_scatter4(h0.y, h1.y, h2.y, h3.y, lane);
+        if ((lane & 7) == 0) a.pair_j[pair_at(slot, 1, 0, k0 + (lane >> 3))] = tot;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      float hi = 0.0f;
+      const int n = diag ? kTile : kTile / 4;
+#pragma unroll 8
+      for (int k = 0; k < n; ++k) hi += s_h[k][lane];
+      a.pair_i[pair_at(slot, 1, 0, lane)] = hi;
+      if (diag) a.pair_j[pair_at(slot, 1, 0, lane)] = 0.0f;
+    }
+    __syncthreads();  // s_h is read before the next pair writes it
+  }
+}
+
+// One CTA per (i-block, tile t of it): the tile's i sums chunk by chunk of the
+// block's list, and its j sums block by block, the warps taking them in turn.
+constexpr int kBlockTiles = 8, kCollectWarps = 8;
+
+template <int kComps>
+__global__ void __launch_bounds__(kCollectWarps * 32) k_collect(PairArgs a, unsigned long long* d0,
+                                                                unsigned long long* d1, unsigned long long* d2,
+                                                                double scale) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const CutBlock cb = a.blocks[blockIdx.x / kBlockTiles];
+  const int t = blockIdx.x % kBlockTiles;
+  if (t >= cb.n_i_tiles) return;
+  const int it = cb.i_tile0 + t, i = it * kTile + lane;
+  unsigned long long* const dst[3] = {d0, d1, d2};
+  const int je = a.seg_end[cb.i_tile0];
+  const int n_chunks = (je - cb.jb + a.chunk - 1) / a.chunk;
+  const int n_parts = n_chunks + (it - cb.sys_tile0) / kBlockTiles + 1;
+  const bool valid = a.atom_valid[i] != 0;
+  for (int part = warp; part < n_parts; part += kCollectWarps) {
+    double v[kComps];
+#pragma unroll
+    for (int c = 0; c < kComps; ++c) v[c] = 0.0;
+    bool any = true, finite = true;
+    if (part < n_chunks) {
+      const int row = a.pair_row[it];
+      const int p0 = cb.jb + part * a.chunk, p1 = min(je, p0 + a.chunk);
+      for (int q0 = p0; q0 < p1; q0 += 32) {  // lane q looks up tile q of the chunk
+        const int jt = q0 + lane < p1 ? a.jlist[q0 + lane] : -1;
+        const int at = row + jt - it;
+        unsigned live = __ballot_sync(0xffffffffu, jt >= it && a.pair_on[at] != 0);
+        while (live) {  // eight tiles' loads in flight
+          float x[8][kComps];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const bool on = live != 0u;
+            const int slot = __shfl_sync(0xffffffffu, at, on ? __ffs(live) - 1 : 0);
+#pragma unroll
+            for (int c = 0; c < kComps; ++c) x[u][c] = on ? a.pair_i[pair_at(slot, kComps, c, lane)] : 0.0f;
+            live &= live - 1;
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int c = 0; c < kComps; ++c) v[c] += static_cast<double>(x[u][c]);
+        }
+      }
+    } else {
+      const int t0 = cb.sys_tile0 + (part - n_chunks) * kBlockTiles;
+      const int ti = t0 + (lane & (kBlockTiles - 1));  // lane w looks up tile w of the block
+      const int at = ti < it ? a.pair_row[ti] + it - ti : 0;
+      const unsigned live = __ballot_sync(0xffffffffu, ti < it && a.pair_on[at] != 0);
+      float sum[kComps];
+#pragma unroll
+      for (int c = 0; c < kComps; ++c) sum[c] = 0.0f;
+#pragma unroll
+      for (int w = 0; w < kBlockTiles; ++w) {
+        const int slot = __shfl_sync(0xffffffffu, at, w);
+#pragma unroll
+        for (int c = 0; c < kComps; ++c) sum[c] += (live >> w) & 1u ? a.pair_j[pair_at(slot, kComps, c, lane)] : 0.0f;
+      }
+      any = false;
+#pragma unroll
+      for (int c = 0; c < kComps; ++c) {
+        any = any || sum[c] != 0.0f;
+        v[c] = static_cast<double>(sum[c]);
+      }
+    }
+    if (!any || !valid) continue;
+#pragma unroll
+    for (int c = 0; c < kComps; ++c) finite = finite && isfinite(v[c]);
+    if (!finite) atomicOr(a.sys_nonfinite + a.atom_sys[i], 1);
+#pragma unroll
+    for (int c = 0; c < kComps; ++c) add_fixed(dst[c] + i, v[c], scale);
   }
 }
 
@@ -1196,9 +1359,7 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_force_split(PairArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int item = next_item<kPersistent>(a, &s_item, -1); item < a.n_work;
        item = next_item<kPersistent>(a, &s_item, item)) {
-    PairWork w = a.work[item];
-    if (a.seg_end) w.j_end = min(w.j_end, a.seg_end[w.i_tile0]);
-    if (w.j_begin >= w.j_end) continue;  // block-uniform
+    const PairWork w = a.work[item];
     const int it = w.i_tile0, i = it * kTile + lane;
     const float px = a.pq[soa_index(i, 0)], py = a.pq[soa_index(i, 1)], pz = a.pq[soa_index(i, 2)];
     const double4 oi = a.origin[it];
@@ -1254,6 +1415,55 @@ __global__ void __launch_bounds__(kSplitWarps * 32) k_force_split(PairArgs a) {
       add_fixed(dst + i, v, kForceScale);
     }
     if (kPersistent) __syncthreads();  // s_acc is read before the next item writes it
+  }
+}
+
+// The force pass of k_born_pair's shape, over culled lists.
+__global__ void __launch_bounds__(kSplitWarps * 32) k_force_pair(PairArgs a) {
+  __shared__ float2 s_f[kTile / 4][3][kTile];  // the i side's sums of four j atoms, in the order they are added
+  __shared__ unsigned s_live;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned live = live_pairs(a, &s_live, [&](int it, int jt) {
+    bool off = jt == it || tile_gap(a.origin[it], a.origin[jt]) > a.pair_cutoff;
+#pragma unroll 4
+    for (int m = a.mask_begin[it]; m < a.mask_begin[it + 1]; ++m) off |= a.mask_refs[m].j_tile == jt;  // near field
+    return off;
+  });
+  for (; live; live &= live - 1) {
+    const size_t slot = blockIdx.x + static_cast<size_t>(__ffs(live) - 1) * gridDim.x;
+    const int2 ij = a.tile_pairs[slot];
+    const int it = ij.x, jt = ij.y, i = it * kTile + lane;
+    const double4 oi = a.origin[it], oj = a.origin[jt];
+    IAtom2 ia = i_atom(a, i);
+    ia.nx = bc(-(a.pq[soa_index(i, 0)] - static_cast<float>(oj.x - oi.x)));
+    ia.ny = bc(-(a.pq[soa_index(i, 1)] - static_cast<float>(oj.y - oi.y)));
+    ia.nz = bc(-(a.pq[soa_index(i, 2)] - static_cast<float>(oj.z - oi.z)));
+    const size_t base = static_cast<size_t>(jt) * 128;
+#pragma unroll
+    for (int q = 0; q < kSplitJ; q += 4) {
+      const int k0 = warp * kSplitJ + q;
+      const Group4 u = force_group4<false>(a.pq + base + k0, a.lj + base + k0, a.gb + base + k0, ia, a);
+      s_f[k0 / 4][0][lane] = add2(u.xa, u.xb);
+      s_f[k0 / 4][1][lane] = add2(u.ya, u.yb);
+      s_f[k0 / 4][2][lane] = add2(u.za, u.zb);
+      const float tx = reduce_scatter4(u.xa.x, u.xa.y, u.xb.x, u.xb.y, lane);
+      const float ty = reduce_scatter4(u.ya.x, u.ya.y, u.yb.x, u.yb.y, lane);
+      const float tz = reduce_scatter4(u.za.x, u.za.y, u.zb.x, u.zb.y, lane);
+      if ((lane & 7) == 0) {
+        const int j = k0 + (lane >> 3);
+        a.pair_j[pair_at(slot, 3, 0, j)] = -tx;
+        a.pair_j[pair_at(slot, 3, 1, j)] = -ty;
+        a.pair_j[pair_at(slot, 3, 2, j)] = -tz;
+      }
+    }
+    __syncthreads();
+    if (warp < 3) {
+      float2 f = bc(0.0f);
+#pragma unroll
+      for (int k = 0; k < kTile / 4; ++k) f = add2(f, s_f[k][warp][lane]);
+      a.pair_i[pair_at(slot, 3, warp, lane)] = f.x + f.y;
+    }
+    __syncthreads();  // s_f is read before the next pair writes it
   }
 }
 
@@ -1326,6 +1536,13 @@ void launch_items(K kernel, int threads, const PairArgs& a, cudaStream_t s) {
   }
 }
 
+// CTAs of k_born_pair and k_force_pair: one per tile pair while they fit the
+// chip at once (sixteen per SM), more pairs per CTA then.
+int pair_grid(const PairArgs& a) {
+  const int most = 16 * std::max(a.n_sm, 1);
+  return std::max((a.n_tile_pairs + kPairsPerCta - 1) / kPairsPerCta, std::min(a.n_tile_pairs, most));
+}
+
 template <bool AP, bool P>
 void force_shape(const PairArgs& a, int shape, cudaStream_t s) {
   switch (shape) {
@@ -1335,7 +1552,16 @@ void force_shape(const PairArgs& a, int shape, cudaStream_t s) {
     case 4: launch_items<P>(k_force_quad<AP, 2, 6, P>, 2 * 32, a, s); break;
     case 5: launch_items<P>(k_force_quad<AP, 2, 7, P>, 2 * 32, a, s); break;
     case 6: launch_items<P>(k_force_quad<AP, 1, 14, P>, 32, a, s); break;
-    default: launch_items<P>(k_force_split<AP, P>, kSplitWarps * 32, a, s); break;
+    default:
+      if (AP || !a.seg_end) {
+        launch_items<P>(k_force_split<AP, P>, kSplitWarps * 32, a, s);
+      } else if (a.tile_pairs) {
+        k_force_pair<<<pair_grid(a), kSplitWarps * 32, 0, s>>>(a);
+        k_collect<3><<<a.n_blocks * kBlockTiles, kCollectWarps * 32, 0, s>>>(a, a.fx, a.fy, a.fz, kForceScale);
+      } else {
+        launch_items<P>(k_force<false, kBlockTiles, 2, P>, kBlockTiles * 32, a, s);
+      }
+      break;
   }
 }
 
@@ -1344,14 +1570,23 @@ void born_shape(const PairArgs& a, int shape, cudaStream_t s) {
   switch (shape) {
     case 1: launch_items<P>(k_born<4, 8, P>, 4 * 32, a, s); break;
     case 2: launch_items<P>(k_born<8, 4, P>, 8 * 32, a, s); break;
-    default: launch_items<P>(k_born_split<P>, kSplitWarps * 32, a, s); break;
+    default:
+      if (!a.seg_end) {
+        launch_items<P>(k_born_split<P>, kSplitWarps * 32, a, s);
+      } else if (a.tile_pairs) {
+        k_born_pair<<<pair_grid(a), kSplitWarps * 32, 0, s>>>(a);
+        k_collect<1><<<a.n_blocks * kBlockTiles, kCollectWarps * 32, 0, s>>>(a, a.born_sum, nullptr, nullptr, kBornScale);
+      } else {
+        launch_items<P>(k_born<kBlockTiles, 4, P>, kBlockTiles * 32, a, s);
+      }
+      break;
   }
 }
 
 }  // namespace
 
-int pair_shape_tiles(bool born, int shape) {
-  if (shape == 0) return 1;
+int pair_shape_tiles(bool born, int shape, bool culled) {
+  if (shape == 0) return culled ? kBlockTiles : 1;
   if (shape == 1) return 4;
   if (born) return 8;
   return shape <= 3 ? 16 : shape <= 5 ? 8 : 4;

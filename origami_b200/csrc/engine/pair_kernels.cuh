@@ -18,6 +18,12 @@ struct PairWork {
   int32_t j_end;
 };
 
+// One i-block of a pair work list: W i-tiles from i_tile0 against the j-tiles
+// jlist[jb, je); the system's first tile.
+struct CutBlock {
+  int32_t i_tile0, n_i_tiles, jb, je, sys_tile0;
+};
+
 // Exclusion masks of one ordered (i-tile, j-tile) pair: for i-lane l, bit k
 // of ex[l] marks pair (i0+l, j0+k) as excluded (1-2, 1-3 or self), bit k of
 // m14[l] as a 1-4 pair.  Entries of one i-tile are sorted by j-tile.
@@ -46,6 +52,19 @@ struct PairArgs {
   const TileMaskRef* mask_refs;
   const uint32_t* mask_ex;
   const uint32_t* mask_14;
+  // shape 0 over culled lists, while there are few tile pairs: one CTA per
+  // tile pair (i, j >= i), its sums kept as [slot][component][atom] of the
+  // i-tile and of the j-tile; the pair of tiles (i, j) is at pair_row[i] + j - i.
+  // NULL = the eight-tile kernels
+  const int2* tile_pairs;
+  int32_t n_tile_pairs;
+  const int32_t* pair_row;
+  uint8_t* pair_on;  // whether the slot's pair was evaluated; its sums are zero otherwise
+  float* pair_i;
+  float* pair_j;
+  int32_t n_sm;
+  const CutBlock* blocks;  // the pass's i-blocks, and its chunk
+  int32_t n_blocks, chunk;
   // outputs (fixed point)
   unsigned long long* fx;
   unsigned long long* fy;
@@ -77,11 +96,6 @@ struct PairArgs {
   double nb_c2_64, gb_c2_64, inv_rc3_64;
 };
 
-// One i-block of a pair work list: W i-tiles from i_tile0 against the j-tiles
-// jlist[jb, je).
-struct CutBlock {
-  int32_t i_tile0, n_i_tiles, jb, je;
-};
 // Cutoff-mode j lists, rebuilt from the tile origins every force evaluation:
 // for each i-block, the j-tiles of jlist_all[jb, je) whose bounding sphere
 // comes within `cutoff` of any of the block's tile spheres, kept in order and
@@ -93,7 +107,10 @@ void launch_cut_lists(const CutBlock* blocks, int32_t n_blocks, const int32_t* j
                       double cutoff, int32_t* jlist_out, int32_t* seg_end, cudaStream_t s);
 
 // How a pair pass is launched.  shape:
-//   0 = one i-tile per CTA, the four warps splitting each j-tile (few tiles);
+//   0 = all pairs: one i-tile per CTA, the four warps splitting each j-tile (few
+//       tiles); culled lists (a cutoff): the sums of eight i-tiles per CTA, one
+//       per warp, taken by a CTA per tile pair while there are few
+//       (kMaxTilePairs), with the same results bit for bit;
 //   1 = four i-tiles per CTA, one per warp;
 //   Born pass: 2 = eight i-tiles per CTA, one per warp;
 //   force pass: 2 to 6 = four i-tiles per warp (many tiles): 2, 3 sixteen per
@@ -105,7 +122,8 @@ struct PairLaunch {
   int shape = 0;
   bool persistent = false;
 };
-int pair_shape_tiles(bool born, int shape);
+int pair_shape_tiles(bool born, int shape, bool culled);
+constexpr int64_t kMaxTilePairs = 1 << 18;  // 200 MB of sums at most
 constexpr int kBornShapes = 3;   // shapes 0..2
 constexpr int kForceShapes = 7;  // shapes 0..6
 
