@@ -51,6 +51,10 @@ using ogsasa::cross;
 using ogsasa::dot;
 using ogsasa::norm;
 using ogsasa::norm2;
+using ogsasa::CoverMask;
+using ogsasa::covered_bins;
+using ogsasa::kCoverBins;
+using ogsasa::kCoverMargin;
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarps = 4;
@@ -63,9 +67,6 @@ constexpr int32_t kCountMask = kContained - 1;
 constexpr int kMaskCircles = 56;
 constexpr uint64_t kMaskContained = 1ull << 63;
 constexpr double kPi = 3.14159265358979323846;
-// angular bins of a circle in which its burial is recorded (below)
-constexpr int kCoverBins = 32;
-using CoverMask = uint32_t;
 
 // Optional per-phase cycle counters of the boundary kernels (measurement
 // builds only: -DOG_SASA_PHASE_CLOCKS=1).  Lane 0 of each warp accumulates
@@ -378,7 +379,6 @@ __device__ __forceinline__ int32_t circle_tally(const W& w, int li, bool masks) 
 // is good to 1.5e-4, and bins are taken kCoverMargin, 9.8e-4 rad or more,
 // inside the interval.  A point there is inside cap m by more than R (8e-4)^2
 // / 2 = 3e-8, far above the 1e-12 of the exposure tests.
-constexpr float kCoverMargin = 9.8e-4f * (kCoverBins / 4);  // in bins
 
 // Single special-function instructions (1 ulp class, within the error above).
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -397,11 +397,6 @@ __device__ __forceinline__ float cover_bin(float x, float y) {
   constexpr float q = kCoverBins / 4;
   const float r = x * rcp_approx(fabsf(x) + fabsf(y));
   return y >= 0.0f ? fmaf(-q, r, 3.0f * q) : fmaf(q, r, q);
-}
-
-// Bins [0, b).
-__device__ __forceinline__ CoverMask bins_below(int b) {
-  return ~__funnelshift_lc(0u, ~0u, static_cast<unsigned>(max(b, 0)));  // shifts of 32 clamp
 }
 
 // A circle as the cover pass sees it: cap a (axis, cos alpha) and the frame
@@ -441,12 +436,6 @@ __device__ __forceinline__ bool buried_interval(const CoverCircle& c, float4 b, 
   *ts = cover_bin(h * wx + root * wy, h * wy - root * wx);
   *te = cover_bin(h * wx - root * wy, h * wy + root * wx);
   return nn > limits * 1e-3f && h * h + nn > limits * 1e-2f && fabsf(*ts - *te) > limits * kCoverMargin;
-}
-// The bins wholly inside the interval from ts counter-clockwise to te.
-__device__ __forceinline__ CoverMask covered_bins(float ts, float te) {
-  const CoverMask from = ~bins_below(__float2int_ru(ts + kCoverMargin)),
-                  to = bins_below(__float2int_rd(te - kCoverMargin));
-  return te > ts ? from & to : from | to;
 }
 // Whether an interval end lies in, or within twice the margin of, a bin that
 // `cover` leaves open.

@@ -1,6 +1,7 @@
-// Test shim: exposes the product's reverse-mode PowerSasa term gradients
-// (origami_b200/csrc/engine/sasa_geom.h, compiled here as plain C++) so the
-// CPU tests can compare them with the oracle's directional derivatives.
+// Test shim: exposes the product's reverse-mode PowerSasa term gradients and
+// the buried bins of an interval (origami_b200/csrc/engine/sasa_geom.h, compiled
+// here as plain C++) so the CPU tests can compare them with the oracle's
+// directional derivatives and with the intervals themselves.
 #include "../origami_b200/csrc/engine/sasa_geom.h"
 
 using ogsasa::D3;
@@ -30,3 +31,9 @@ extern "C" void shim_vertex_gradient(const double* p, const double* r, int sign,
   put(g, 1, gk);
   put(g, 2, gl);
 }
+
+extern "C" void shim_covered_bins(int n, const float* ts, const float* te, unsigned* bins) {
+  for (int k = 0; k < n; ++k) bins[k] = ogsasa::covered_bins(ts[k], te[k]);
+}
+
+extern "C" float shim_cover_margin() { return ogsasa::kCoverMargin; }
