@@ -407,10 +407,11 @@ og_status og_compute_sasa(og_engine* e, int32_t sys, int32_t method, int32_t n_d
  *               3, 4, 6, 7 or 14 CTAs/SM
  *   persistent  0: one CTA per work item; 1: resident CTAs taking items from
  *               an atomic work queue
- *   chunk       j-tiles per work item at most (default 16; halved while the
- *               list has fewer than eight items per SM, without cutoffs
- *               fewer than 32 in the Born pass and 16 in the force pass;
- *               shape 0 with a cutoff takes it as it is)
+ *   chunk       j-tiles per work item.  og_engine_set_pair_launch takes it as it
+ *               is; untuned engines (16) and the autotuner halve it while the
+ *               list has fewer than eight items per SM, without cutoffs fewer
+ *               than 32 in the Born pass and 16 in the force pass (shape 0 with
+ *               a cutoff never)
  * An engine that is neither tuned nor set by hand takes its shapes from its
  * tile count and cutoffs.
  * og_engine_autotune times every combination (3 Born / 7 force shapes x 2 x

@@ -286,6 +286,7 @@ struct og_engine {
   // and the persistent launches' queue heads (Born, force)
   ogk::PairLaunch born_launch, force_launch;
   int chunk_b = 16, chunk_f = 16;
+  bool chunk_set_b = false, chunk_set_f = false;  // by og_engine_set_pair_launch: taken as it is, not refined
   // tile pairs of every system (PairArgs::tile_pairs), with a cutoff and while
   // there are at most kMaxTilePairs; both passes' sums share pair_part
   DVec<int2> tile_pairs;
@@ -1040,6 +1041,7 @@ void default_launch(og_engine* e) {
   e->born_launch = ogk::PairLaunch{};
   e->force_launch = ogk::PairLaunch{};
   e->chunk_b = e->chunk_f = 16;
+  e->chunk_set_b = e->chunk_set_f = false;
   if (no_cutoff(e->p.born_cutoff)) e->born_launch.shape = pairs < 4000 ? 0 : 1;
   if (no_cutoff(e->p.nb_cutoff) || no_cutoff(e->p.gb_force_cutoff))
     e->force_launch.shape = pairs < 800 ? 0 : pairs < 40000 ? 1 : 4;
@@ -1067,8 +1069,8 @@ og_status build_tile_pairs(og_engine* e, cudaStream_t st) {
 
 og_status build_pair_lists(og_engine* e, cudaStream_t st) {
   if (!e->launch_set) default_launch(e);
-  const int cb = refine_chunk(e, true, e->born_launch.shape, e->chunk_b);
-  const int cf = refine_chunk(e, false, e->force_launch.shape, e->chunk_f);
+  const int cb = e->chunk_set_b ? e->chunk_b : refine_chunk(e, true, e->born_launch.shape, e->chunk_b);
+  const int cf = e->chunk_set_f ? e->chunk_f : refine_chunk(e, false, e->force_launch.shape, e->chunk_f);
   og_status s = build_pass_list(e, true, e->born_launch.shape, cb, &e->work, &e->n_work, &e->jlist, &e->cut_b,
                                 &e->n_cut_b, &e->jlist_cut_b, &e->seg_end_b, st);
   if (s != OG_OK) return s;
@@ -3017,6 +3019,7 @@ og_status og_engine_set_pair_launch(og_engine* e, int32_t pass, int32_t shape, i
   dst[0] = shape;
   dst[1] = persistent;
   dst[2] = chunk;
+  (pass == 0 ? e->chunk_set_b : e->chunk_set_f) = true;
   return apply_launch(e, t);
 }
 
@@ -3054,10 +3057,11 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
     const int chunks[3] = {8, 16, 32};
     struct { int b, f; } untuned;  // default_launch's shapes
     {
-      const auto keep = std::make_tuple(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f);
+      const auto keep =
+          std::make_tuple(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f, e->chunk_set_b, e->chunk_set_f);
       default_launch(e);
       untuned = {e->born_launch.shape, e->force_launch.shape};
-      std::tie(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f) = keep;
+      std::tie(e->born_launch, e->force_launch, e->chunk_b, e->chunk_f, e->chunk_set_b, e->chunk_set_f) = keep;
     }
     for (int pass = 0; pass < 2; ++pass) {
       double bt = 1e30;
@@ -3087,6 +3091,7 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
     if (!write_tune_cache(cache_path, cache)) return og_fail(OG_E_IO, std::string("cannot write ") + cache_path);
   }
   OG_CUDA(cudaMemsetAsync(e->sys_nonfinite.p, 0, sizeof(int32_t) * e->sys.size(), e->stream));
+  e->chunk_set_b = e->chunk_set_f = false;
   s = apply_launch(e, best);
   if (s != OG_OK) return s;
   if (out) {
