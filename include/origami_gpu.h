@@ -418,7 +418,8 @@ og_status og_compute_sasa(og_engine* e, int32_t sys, int32_t method, int32_t n_d
  * chunks 8, 16, 32) of each pass on the engine's systems at their current positions and
  * keeps the fastest; the choice is cached in the JSON file cache_path (NULL
  * = no cache) under the workload's bucket (mode, total 32-atom tiles and
- * the largest system's tiles rounded up to powers of two), so a later
+ * the largest system's tiles rounded up to powers of two, and the version of
+ * the kernels the shape numbers stand for), so a later
  * engine in the same bucket is configured without timing.  The next step
  * re-evaluates the forces. */
 typedef struct og_autotune_result {

@@ -2880,12 +2880,16 @@ int pow2_bucket(int x) {
   return b;
 }
 
+// What the shape numbers and chunks stand for; raised when that changes, so that
+// entries timed for other kernels are not found.
+constexpr int kTuneVersion = 3;
+
 std::string tune_key(const og_engine* e) {
   int max_tiles = 0;
   for (const auto& s : e->sys) max_tiles = std::max(max_tiles, s.n_tiles);
   const bool all_pairs = no_cutoff(e->p.nb_cutoff) && no_cutoff(e->p.gb_force_cutoff) && no_cutoff(e->p.born_cutoff);
   return std::string(all_pairs ? "all_pairs" : "cutoff") + "|tiles<=" + std::to_string(pow2_bucket(e->n_tiles)) +
-         "|system_tiles<=" + std::to_string(pow2_bucket(max_tiles));
+         "|system_tiles<=" + std::to_string(pow2_bucket(max_tiles)) + "|kernels=" + std::to_string(kTuneVersion);
 }
 
 struct TuneEntry {
