@@ -350,8 +350,9 @@ struct og_engine {
   ogk::TunnelParams tunnel{};
   double sasa_rmax = 0.0;
   double s_max = 0.0, rho_max = 0.0;  // largest s*rho~ and rho~ (series limits of the Born pass)
-  // captured launches: one MD step, and one force evaluation (from the
-  // second one on, while lgb_on() is what it was at the capture)
+  // captured launches: one MD step, and one force evaluation with plain and
+  // one with learned radii (each from its second evaluation on; the judge
+  // evaluates both)
   struct StepGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -362,17 +363,16 @@ struct og_engine {
       graph = nullptr;
     }
   };
-  StepGraph step_graph, force_graph;
+  StepGraph step_graph, force_graph[2];  // [lgb_on()]
   bool capturing = false;  // enqueue_forces is being captured
-  bool force_graph_lgb = false;
-  int force_evals = 0;
+  int force_evals[2] = {0, 0};
   // profiling
   bool profile = false;
   std::map<std::string, std::pair<double, long long>> prof;
   std::vector<std::string> prof_names;
 
   ~og_engine() {
-    for (StepGraph* g : {&step_graph, &force_graph}) g->reset();
+    for (StepGraph* g : {&step_graph, &force_graph[0], &force_graph[1]}) g->reset();
     if (in_done) cudaEventSynchronize(in_done);  // host_in is read until then
     if (own_stream && stream) cudaStreamDestroy(stream);
     for (cudaStream_t* q : {&side, &hi, &aux})
@@ -1754,15 +1754,12 @@ og_status eval_forces(og_engine* e) {
     e->enqueue_forces();
   };
   og_status st;
-  if (e->profile || (e->force_graph.exec && e->force_graph_lgb != e->lgb_on()) ||
-      (!e->force_graph.exec && e->force_evals++ == 0)) {
+  og_engine::StepGraph& graph = e->force_graph[e->lgb_on()];
+  if (e->profile || (!graph.exec && e->force_evals[e->lgb_on()]++ == 0)) {
     enqueue();
   } else {
-    if (!e->force_graph.exec) {
-      if ((st = capture(e, &e->force_graph, enqueue)) != OG_OK) return st;
-      e->force_graph_lgb = e->lgb_on();
-    }
-    OG_CUDA(cudaGraphLaunch(e->force_graph.exec, e->stream));
+    if (!graph.exec && (st = capture(e, &graph, enqueue)) != OG_OK) return st;
+    OG_CUDA(cudaGraphLaunch(graph.exec, e->stream));
   }
   st = launch_check("force evaluation");
   if (st != OG_OK) return st;
@@ -1772,8 +1769,10 @@ og_status eval_forces(og_engine* e) {
 
 void reset_graph(og_engine* e) {
   e->step_graph.reset();
-  e->force_graph.reset();
-  e->force_evals = 0;
+  for (int learned = 0; learned < 2; ++learned) {
+    e->force_graph[learned].reset();
+    e->force_evals[learned] = 0;
+  }
 }
 
 og_status lgb_check(og_engine* e) {
