@@ -1762,11 +1762,18 @@ __global__ void __launch_bounds__(kWarps * 32) k_shrake_rupley(SasaArgs a, const
 
 constexpr size_t kWarpSmemBytes = sizeof(WarpSmem) * kWarps;
 constexpr size_t kBigSmemBytes = sizeof(WarpSmemBig);
-constexpr int kBigGrid = 148 * 4;  // persistent one-warp blocks for the queue
-// Up to this many atoms, all of them go to the large-capacity kernel at once,
-// one block each (all resident): the queue's second pass would take as long
-// as the first (insulin, 266 C and S atoms: 57 + 54 us, 61 in one).
-constexpr int kBigAllTasks = 148 * 8;
+constexpr int kBigPerSm = 4;  // persistent one-warp blocks for the queue
+// Up to this many atoms per SM, all of them go to the large-capacity kernel at
+// once, one block each: the queue's second pass would take as long as the first.
+// Seven blocks are resident; the few beyond start as the quickest atoms end.
+// The whole term in us, one pass against two (148 SMs):
+//   atoms            98  263  294  526  636  849 1041 1052 1217 1315 1352 1578
+//   compact folds    44   54        59                  63        78        79
+//                    55   90        98                 102       107       108
+//   extended chains            42        45   46   47        55        57
+//                              47        50   51   52        55        55
+constexpr int kBigAllPerSm = 8;
+static_assert(7 * (kBigSmemBytes + 1024) <= 228 * 1024, "large-capacity kernel no longer fits seven blocks per SM");
 // six resident CTAs per SM (228 KB, 1 KB reserved per CTA): 24 warps
 static_assert(6 * (kWarpSmemBytes + 1024) <= 228 * 1024, "boundary kernel no longer fits six CTAs per SM");
 
@@ -1787,41 +1794,45 @@ cudaError_t sasa_prepare() {
   return e;
 }
 
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+  }();
+  return n;
+}
+
 // Resident blocks of a queue-driven kernel: the SM count times the blocks
 // that fit (no more than the atoms need).
 template <class K>
 int resident_grid(K kernel, int n_tasks) {
-  static int n_sm = 0;
-  if (n_sm == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  }
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kWarps * 32, kWarpSmemBytes);
-  return std::max(1, std::min((n_tasks + kWarps - 1) / kWarps, std::max(per_sm, 1) * std::max(n_sm, 1)));
+  return std::max(1, std::min((n_tasks + kWarps - 1) / kWarps, std::max(per_sm, 1) * sm_count()));
 }
 
 void launch_sasa_forces(const SasaArgs& a, cudaStream_t s) {
   if (a.n_tasks <= 0) return;
   cudaMemsetAsync(a.counts, 0, 4 * sizeof(int32_t), s);
-  if (a.n_tasks <= kBigAllTasks) {
+  if (a.n_tasks <= kBigAllPerSm * sm_count()) {
     k_sasa_boundary_big<<<a.n_tasks, 32, kBigSmemBytes, s>>>(a, true);
   } else {
     k_sasa_boundary<<<resident_grid(k_sasa_boundary, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
-    k_sasa_boundary_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a, false);
+    k_sasa_boundary_big<<<kBigPerSm * sm_count(), 32, kBigSmemBytes, s>>>(a, false);
   }
-  k_sasa_terms<<<148 * 8, 128, 0, s>>>(a);
+  k_sasa_terms<<<8 * sm_count(), 128, 0, s>>>(a);
 }
 
 void launch_sasa_areas(const SasaArgs& a, cudaStream_t s) {
   if (a.n_tasks <= 0) return;
   cudaMemsetAsync(a.counts + 2, 0, 2 * sizeof(int32_t), s);
-  if (a.n_tasks <= kBigAllTasks) {
+  if (a.n_tasks <= kBigAllPerSm * sm_count()) {
     k_sasa_areas_big<<<a.n_tasks, 32, kBigSmemBytes, s>>>(a, true);
   } else {
     k_sasa_areas<<<resident_grid(k_sasa_areas, a.n_tasks), kWarps * 32, kWarpSmemBytes, s>>>(a);
-    k_sasa_areas_big<<<kBigGrid, 32, kBigSmemBytes, s>>>(a, false);
+    k_sasa_areas_big<<<kBigPerSm * sm_count(), 32, kBigSmemBytes, s>>>(a, false);
   }
 }
 
