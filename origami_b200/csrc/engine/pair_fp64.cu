@@ -228,8 +228,10 @@ void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_
 // j-tiles staged in the warp's shared memory, read back as broadcasts), so a
 // single chain spreads over n_tiles x n_chunks warps.  Bound by the FP64
 // pipe, so what counts is FP64 operations per pair; a closed form per ordered
-// pair with its roots, divisions, logarithm and exponential took 0.60 ms for
-// an energy of a 4 694-atom chain, all pairs.
+// pair with its roots, divisions, logarithm and exponential took 620 us for the
+// call for a 4 694-atom chain, all pairs; this takes 153.  (A reciprocal and a
+// root of our own took 137, without CUDA's handling of zero: coincident atoms
+// need it.)
 //   * The pair energies see each unordered pair once (tiles jt >= it) and
 //     take 1/r from one reciprocal square root.
 //   * Tile pairs are classed by the gap between their bounding spheres: the
@@ -244,24 +246,6 @@ void launch_near_force64(const PairArgs& a, const int4* near, int n_near, int n_
 namespace {
 
 constexpr int kEnergyWarps = 4;
-
-// 1 / a and 1 / sqrt(a) to an ulp or so: the special-function unit's
-// approximation (relative error below 2^-21) and one third-order
-// Newton-Householder step, whose error is the cube of that.  Without the
-// library's handling of zero (NaN here, infinity there), which the callers
-// do not need.
-__device__ __forceinline__ double rcp64(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double rsqrt64(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  const double e = fma(-a * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
 
 __device__ __forceinline__ double descreen64(double r, double r2, double inv_r, double rho_i, double s_rho_j) {
   // energy/src/gb.rs:347-369, with 1/r given.
@@ -321,7 +305,7 @@ __device__ __forceinline__ double born_far64(const BornTile& t, int nj, double x
     const double2 sj = t.s[k];
     const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
     const double r2 = dx * dx + dy * dy + dz * dz;
-    const double u = rcp64(r2);
+    const double u = 1.0 / r2;
     const double h = (u * u * sj.y) * descreen_series64<kTerms>(sj.x * u);
     if (!kCut || !(r2 > c2)) acc += h;
   }
@@ -371,7 +355,7 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_born64(EnergyArgs a) {
       const double4 pj = t.p[k];
       const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
       const double r2 = dx * dx + dy * dy + dz * dz;
-      const double inv_r = rsqrt64(r2);
+      const double inv_r = rsqrt(r2);
       const double r = r2 * inv_r;
       const bool on = k != self && !(r2 > a.born_c2) && !(r2 < 1e-18);
       double h;
@@ -456,7 +440,7 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
         for (int k = 0; k < nj; ++k) {
           const double4 pj = t.p[k], gj = t.g[k];
           const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
-          const double inv_r = rsqrt64(dx * dx + dy * dy + dz * dz);
+          const double inv_r = rsqrt(dx * dx + dy * dy + dz * dz);
           const double x = (rmi + gj.x) * inv_r;
           const double x2 = x * x;
           const double r6 = x2 * x2 * x2;
@@ -469,7 +453,7 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
         for (int k = 0; k < nj; ++k) {
           const double4 pj = t.p[k];
           const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
-          gb = fma(pj.w, rsqrt64(dx * dx + dy * dy + dz * dz), gb);
+          gb = fma(pj.w, rsqrt(dx * dx + dy * dy + dz * dz), gb);
         }
       }
       continue;
@@ -480,10 +464,10 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
       const double dx = pj.x - xi, dy = pj.y - yi, dz = pj.z - zi;
       const double r2 = dx * dx + dy * dy + dz * dz;
       const bool on = valid && k >= first;
-      const double inv_r = rsqrt64(r2);
+      const double inv_r = rsqrt(r2);
       const double xg = r2 * (iRi4 * gj.w);
       double inv_f = inv_r;
-      if (!__all_sync(0xffffffffu, xg >= 40.0)) inv_f = rsqrt64(r2 + Ri * gj.z * exp(-xg));
+      if (!__all_sync(0xffffffffu, xg >= 40.0)) inv_f = rsqrt(r2 + Ri * gj.z * exp(-xg));
       if (on) gb += pj.w * inv_f;
       if (!nb_tile) continue;
       const bool nb = on && !(r2 > a.nb_c2) && !((ex >> k) & 1u);
@@ -493,7 +477,7 @@ __global__ void __launch_bounds__(kEnergyWarps * 32) k_energy64(EnergyArgs a) {
         const double x = (is14 ? rm14i + a.rmin14[j0 + k] : rmi + gj.x) * inv_r;
         const double x2 = x * x;
         const double r6 = x2 * x2 * x2;
-        const double e = r6 * (r6 - 2.0);
+        const double e = r6 * r6 - 2.0 * r6;  // NaN for coincident atoms, as the reference has it
         if (is14) lj14 += sep14i * sqrt(a.eps14[j0 + k]) * e;
         else lj += gj.y * e;
         const double rf = cut ? fma(a.kappa, r2, inv_r) - a.crf : inv_r;
