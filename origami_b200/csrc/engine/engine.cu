@@ -530,7 +530,6 @@ struct og_engine {
     s.alpha = std::exp(-p.friction_ps_inv * p.dt_fs * 1.0e-3);
     s.seed_lo = static_cast<uint32_t>(p.seed);
     s.seed_hi = static_cast<uint32_t>(p.seed >> 32);
-    s.use_shake = (p.constrain_h_bonds && n_clusters > 0) ? 1 : 0;
     return s;
   }
 
@@ -768,7 +767,7 @@ struct og_engine {
 
   void enqueue_step() {
     ogk::StepArgs sa = step_args();
-    if (!sa.use_shake) {
+    if (!p.constrain_h_bonds || n_clusters == 0) {
       Timer t(this, "step_move");
       ogk::launch_step_free(sa, stream);
     } else if (slots.n > 0) {

@@ -271,6 +271,9 @@ __global__ void k_bonded(BondedArgs a) {
 }
 
 // ------------------------------------------------------------------ BAOAB
+// k_step_pre, k_shake, k_step_mid, k_shake, k_step_post: the sub-steps before the
+// forces for constraints of any shape (the common cases have kernels of their own
+// below).
 __global__ void k_step_pre(StepArgs p) {
   const AtomArrays& a = p.at;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -282,7 +285,7 @@ __global__ void k_step_pre(StepArgs p) {
   double vz = a.vz[i] + fixed_to_f(a.fz[i]) * c;
   a.vx[i] = vx; a.vy[i] = vy; a.vz[i] = vz;
   const double x = a.x[i], y = a.y[i], z = a.z[i];
-  if (p.use_shake) { a.rx[i] = x; a.ry[i] = y; a.rz[i] = z; }
+  a.rx[i] = x; a.ry[i] = y; a.rz[i] = z;
   a.x[i] = x + vx * p.half_dt;
   a.y[i] = y + vy * p.half_dt;
   a.z[i] = z + vz * p.half_dt;
@@ -326,19 +329,12 @@ __global__ void k_step_mid(StepArgs p) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int sys;
   if (!atom_live(a, i, &sys)) return;
-  double vx, vy, vz;
-  if (p.use_shake) {
-    vx = (a.x[i] - a.rx[i]) / p.half_dt;
-    vy = (a.y[i] - a.ry[i]) / p.half_dt;
-    vz = (a.z[i] - a.rz[i]) / p.half_dt;
-    count_shake(a, i, sys);
-  } else {
-    vx = a.vx[i]; vy = a.vy[i]; vz = a.vz[i];
-  }
+  double vx = (a.x[i] - a.rx[i]) / p.half_dt, vy = (a.y[i] - a.ry[i]) / p.half_dt, vz = (a.z[i] - a.rz[i]) / p.half_dt;
+  count_shake(a, i, sys);
   ornstein_uhlenbeck(p, i, sys, &vx, &vy, &vz);
   a.vx[i] = vx; a.vy[i] = vy; a.vz[i] = vz;
   const double x = a.x[i], y = a.y[i], z = a.z[i];
-  if (p.use_shake) { a.rx[i] = x; a.ry[i] = y; a.rz[i] = z; }
+  a.rx[i] = x; a.ry[i] = y; a.rz[i] = z;
   a.x[i] = x + vx * p.half_dt;
   a.y[i] = y + vy * p.half_dt;
   a.z[i] = z + vz * p.half_dt;
@@ -349,7 +345,7 @@ __global__ void k_step_post(StepArgs p) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n_padded) return;
   int sys;
-  if (p.use_shake && atom_live(a, i, &sys)) {
+  if (atom_live(a, i, &sys)) {
     a.vx[i] = (a.x[i] - a.rx[i]) / p.half_dt;
     a.vy[i] = (a.y[i] - a.ry[i]) / p.half_dt;
     a.vz[i] = (a.z[i] - a.rz[i]) / p.half_dt;

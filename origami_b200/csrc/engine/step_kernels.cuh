@@ -79,20 +79,19 @@ struct StepArgs {
   double half_dt;
   double alpha;          // exp(-gamma dt)
   uint32_t seed_lo, seed_hi;
-  int32_t use_shake;
 };
-// B (first half) + A (first half); stores SHAKE reference positions.
+// Constraints of any shape: B (first half) + A (first half); stores SHAKE reference positions.
 void launch_step_pre(const StepArgs& a, cudaStream_t s);
-// [SHAKE velocity fix] + O + A (second half).
+// SHAKE velocity fix + O + A (second half).
 void launch_step_mid(const StepArgs& a, cudaStream_t s);
-// [SHAKE velocity fix] + pack + zero accumulators.
+// SHAKE velocity fix + pack + zero accumulators.
 void launch_step_post(const StepArgs& a, cudaStream_t s);
 // B (second half), divergence check, step counter.
 void launch_step_end(const StepArgs& a, cudaStream_t s);
 
 // The sub-steps before the forces as one kernel (no constraints), or as one
-// and the pack (each constraint a hydrogen on one heavy atom): the same
-// results as the launches above, bit for bit.
+// and the pack (each constraint a hydrogen on one heavy atom): the arithmetic of
+// the launches above in the same order.
 // Slots are warps of 32: a cluster's heavy atom, then its hydrogens, or single
 // atoms; a cluster stays within its warp.
 struct MoveSlot {
