@@ -3068,16 +3068,23 @@ og_status og_engine_autotune(og_engine* e, const char* cache_path, og_autotune_r
     for (int pass = 0; pass < 2; ++pass) {
       double bt = 1e30;
       int bc[3] = {0, 0, 16};
-      for (int shape = 0; shape < (pass == 0 ? ogk::kBornShapes : ogk::kForceShapes); ++shape)
+      const bool born = pass == 0, tile_pairs = culled_pass(e, born) && e->tile_pairs.n > 0;
+      std::map<std::tuple<int, int, int>, double> timed;  // by what is launched: equal variants once
+      for (int shape = 0; shape < (born ? ogk::kBornShapes : ogk::kForceShapes); ++shape)
         for (int pers = 0; pers <= 1; ++pers)
           for (int chunk : chunks) {
-            double ms = 0.0;
             ogk::PairLaunch lc;
             lc.shape = shape;
             lc.persistent = pers != 0;
-            s = time_pass(e, pass == 0, lc, chunk, 3, &ms);
-            if (s != OG_OK) return s;
-            if (shape == (pass == 0 ? untuned.b : untuned.f) && pers == 0 && chunk == 16) (pass == 0 ? b_def : f_def) = ms;
+            const auto what = std::make_tuple(shape, shape == 0 && tile_pairs ? 0 : pers, refine_chunk(e, born, shape, chunk));
+            if (!timed.count(what)) {
+              double t = 0.0;
+              s = time_pass(e, born, lc, chunk, 3, &t);
+              if (s != OG_OK) return s;
+              timed[what] = t;
+            }
+            const double ms = timed[what];
+            if (shape == (born ? untuned.b : untuned.f) && pers == 0 && chunk == 16) (born ? b_def : f_def) = ms;
             if (ms < bt) {
               bt = ms;
               bc[0] = shape;
