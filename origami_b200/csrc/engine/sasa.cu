@@ -1458,7 +1458,8 @@ __device__ void boundary_task(const SasaArgs& a, W& w, int i, int lane, bool big
 // crossings were dropped in FP32, then with the smaller code and the FP32
 // neighbour search: 2057 -> 1297 -> 998 us for 64 chains of 300 residues,
 // 819 -> 516 -> 413 us for 16 compact folds of 306, 184 -> 61 -> 54 us for
-// insulin (in the large-capacity kernel, see below).
+// insulin (in the large-capacity kernel, see below); 1017, 420 and 53 with the
+// bins' margin at the seam (covered_bins).
 __device__ __forceinline__ int next_task(const SasaArgs& a, int lane) {
   int task = 0;
   if (lane == 0) task = atomicAdd(&a.counts[3], 1);
