@@ -1047,23 +1047,32 @@ void default_launch(og_engine* e) {
 }
 
 // The tile pairs of every system, i <= j, in rows of i (PairArgs::tile_pairs).
+// Buffers keep half as much again, so that a growing engine makes new ones rarely.
 og_status build_tile_pairs(og_engine* e, cudaStream_t st) {
   int64_t n = 0;
   for (const auto& s : e->sys) n += static_cast<int64_t>(s.n_tiles) * (s.n_tiles + 1) / 2;
   e->tile_pairs.n = 0;
   if (n > ogk::kMaxTilePairs || !(culled_pass(e, true) || culled_pass(e, false))) return OG_OK;
-  std::vector<int2> pairs;
+  auto reserve = [](auto& v, size_t count) {
+    const cudaError_t err = count <= v.cap ? cudaSuccess : v.alloc(v.cap ? count + count / 2 : count);
+    v.n = count;
+    return err;
+  };
   std::vector<int32_t> row;
+  int32_t at = 0;
   for (const auto& s : e->sys)
-    for (int i = s.tile_begin; i < s.tile_begin + s.n_tiles; ++i) {
-      row.push_back(static_cast<int32_t>(pairs.size()));
-      for (int j = i; j < s.tile_begin + s.n_tiles; ++j) pairs.push_back(make_int2(i, j));
+    for (int k = s.n_tiles; k > 0; --k) {
+      row.push_back(at);
+      at += k;
     }
-  OG_CUDA(e->tile_pairs.upload(pairs, st));
-  OG_CUDA(e->pair_row.upload(row, st));
-  OG_CUDA(e->pair_part.alloc(6 * kTile * pairs.size()));
-  OG_CUDA(e->pair_on.alloc(pairs.size()));
-  return OG_OK;
+  row.push_back(at);
+  OG_CUDA(reserve(e->pair_row, row.size()));
+  OG_CUDA(cudaMemcpyAsync(e->pair_row.p, row.data(), row.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  OG_CUDA(reserve(e->pair_part, 6 * kTile * static_cast<size_t>(n)));
+  OG_CUDA(reserve(e->pair_on, static_cast<size_t>(n)));
+  OG_CUDA(reserve(e->tile_pairs, static_cast<size_t>(n)));
+  ogk::launch_tile_pairs(e->pair_row.p, e->n_tiles, e->tile_pairs.p, st);
+  return launch_check("tile pairs");
 }
 
 og_status build_pair_lists(og_engine* e, cudaStream_t st) {

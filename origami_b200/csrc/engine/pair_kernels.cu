@@ -1585,6 +1585,17 @@ void born_shape(const PairArgs& a, int shape, cudaStream_t s) {
 
 }  // namespace
 
+namespace {
+__global__ void k_tile_pairs(const int32_t* row, int2* pairs) {
+  const int i = blockIdx.x, first = row[i], n = row[i + 1] - first;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) pairs[first + k] = make_int2(i, i + k);
+}
+}  // namespace
+
+void launch_tile_pairs(const int32_t* pair_row, int n_tiles, int2* tile_pairs, cudaStream_t s) {
+  if (n_tiles > 0) k_tile_pairs<<<n_tiles, 128, 0, s>>>(pair_row, tile_pairs);
+}
+
 int pair_shape_tiles(bool born, int shape, bool culled) {
   if (shape == 0) return culled ? kBlockTiles : 1;
   if (shape == 1) return 4;

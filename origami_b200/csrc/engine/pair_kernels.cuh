@@ -123,6 +123,9 @@ struct PairLaunch {
   bool persistent = false;
 };
 int pair_shape_tiles(bool born, int shape, bool culled);
+// PairArgs::tile_pairs from the rows' first slots (n_tiles + 1 of them): row i
+// holds (i, i), (i, i + 1), ..
+void launch_tile_pairs(const int32_t* pair_row, int n_tiles, int2* tile_pairs, cudaStream_t s);
 constexpr int64_t kMaxTilePairs = 1 << 18;  // 200 MB of sums at most
 constexpr int kBornShapes = 3;   // shapes 0..2
 constexpr int kForceShapes = 7;  // shapes 0..6
