@@ -455,7 +455,9 @@ __device__ __forceinline__ void keep_or(W& w, int j, int b) {
 // How many lanes (1, 2 or 4, as a power of two) share an item when `left` are
 // left, `full` of which occupy the warp -- in the large-capacity kernel, whose
 // warps run alone on their scheduler, so that the last, partly filled trip's
-// latency counts (insulin: 55.6 -> 53.5 us, a step 77 -> 72).  In the default
+// latency counts (the term for compact folds of 98, 263, 526, 789 and 1 052
+// surface atoms: 49.0, 58.1, 62.7, 68.0 and 67.6 us without, 44.6, 54.1, 59.0,
+// 62.4 and 62.6 with; extended chains the same either way).  In the default
 // kernel the shared trips won 6 % for compact folds and lost 3 % for extended
 // chains.
 template <class W>
